@@ -14,8 +14,8 @@ Kinds of case, and what each stands for:
   twists       a twist average: a batch that differs by twist, solved and downloaded
   scan         an r_s scan at one size: a batch that differs by r_s, solved and downloaded
   stream       a mixed cohort of the serving loop: incremental solve, results as they stop
-  pipeline     a new twist batch made, solved, downloaded and released, as each step of a
-               twist-averaging program with fresh twists does
+  pipeline     a new twist batch made, solved (CCD or dRPA), downloaded and released, as each
+               step of a twist-averaging program with fresh twists does
 
 A drawn case is one of these kinds with its sizes spread over the same ranges.
 """
@@ -44,18 +44,17 @@ def listed():
         # the reference's dRPA benchmark size
         dict(name="drpa_n14", kind="drpa", electrons=14, basis=8.15, rs=1.0),
         # the reference's own twist average: 100 twists of a small system, its own iteration
-        dict(name="ccd_n14_twists100", kind="twists", method="ccd", electrons=14, basis=8.0, rs=1.0, count=100,
+        dict(name="ccd_n14_twists100", kind="twists", electrons=14, basis=8.0, rs=1.0, count=100,
              scheme="replay", precision=0),
         # one mid-size system solved by a host program
         dict(name="ccd_n54", kind="ccd", electrons=54, basis=17.963, rs=5.0),
         # the batched twist average, FP64 and mixed precision
-        dict(name="ccd_n54_twists100", kind="twists", method="ccd", electrons=54, basis=17.963, rs=1.0, count=100,
+        dict(name="ccd_n54_twists100", kind="twists", electrons=54, basis=17.963, rs=1.0, count=100,
              scheme="diis", precision=0),
-        dict(name="ccd_n54_twists100_mixed", kind="twists", method="ccd", electrons=54, basis=17.963, rs=1.0,
+        dict(name="ccd_n54_twists100_mixed", kind="twists", electrons=54, basis=17.963, rs=1.0,
              count=100, scheme="diis", precision=1),
-        # the twist average of the other method
-        dict(name="drpa_n54_twists30", kind="twists", method="drpa", electrons=54, basis=17.963, rs=1.0, count=30,
-             scheme="replay", precision=0),
+        # the twist average of the other method, a fresh batch per step
+        dict(name="drpa_n54_twists30", kind="pipeline", method="drpa", electrons=54, basis=17.963, rs=1.0, count=30),
         # the largest system, over r_s
         dict(name="ccd_n114_scan4", kind="scan", electrons=114, basis=18.333, count=4),
         # one residual for a host's own loop, ragged sizes
@@ -65,7 +64,7 @@ def listed():
         # a serving cohort of mixed sizes
         dict(name="stream_12", kind="stream", count=12, pick=3),
         # a fresh batch per step
-        dict(name="pipeline_n54_twists25", kind="pipeline", electrons=54, basis=12.0, rs=1.0, count=25),
+        dict(name="ccd_n54_pipeline25", kind="pipeline", method="ccd", electrons=54, basis=12.0, rs=1.0, count=25),
     ]
 
 
@@ -89,8 +88,7 @@ def draw(rng):
         n = rng.choice([14, 24, 38, 54, 66])
         most = {14: 100, 24: 100, 38: 100, 54: 60, 66: 30}[n]
         precision = rng.choice([0, 0, 0, 1])
-        method = "drpa" if precision == 0 and rng.random() < 0.3 else "ccd"
-        return dict(kind=kind, method=method, electrons=n, basis=round(rng.uniform(4.0, 17.0), 2), rs=rs(2.0),
+        return dict(kind=kind, electrons=n, basis=round(rng.uniform(4.0, 17.0), 2), rs=rs(2.0),
                     count=log_int(3, most), scheme="diis" if precision else rng.choice(["diis", "replay"]),
                     precision=precision)
     if kind == "scan":
@@ -98,8 +96,8 @@ def draw(rng):
                     count=rng.randint(2, 4))
     if kind == "stream":
         return dict(kind=kind, count=rng.randint(2, 12), pick=rng.randint(1, 999))
-    return dict(kind=kind, electrons=2 * rng.randint(7, 33), basis=round(rng.uniform(4.0, 12.0), 2), rs=rs(2.0),
-                count=log_int(3, 25))
+    return dict(kind=kind, method=rng.choice(["ccd", "drpa"]), electrons=2 * rng.randint(7, 33),
+                basis=round(rng.uniform(4.0, 16.0), 2), rs=rs(2.0), count=log_int(3, 25))
 
 
 # ------------------------------------------------------------------------------ inputs
@@ -157,6 +155,8 @@ def _screening(nocc, length):
 
 
 def _options(case):
+    if case.get("method") == "drpa":
+        return dict(REPLAY)
     if case["kind"] in ("scan", "pipeline"):
         return dict(DIIS, tol=1e-9)
     if case["kind"] == "stream":
@@ -279,10 +279,10 @@ def work(case):
         sizes = [(case["electrons"], case["basis"])] * case.get("count", 1)
     # iterations a solve of each scheme takes at these sizes
     iterations = {"mp2": 0, "residual": 1, "flags": 1, "drpa": 22, "ccd": 14, "two_channel": 33, "scan": 13,
-                  "stream": 12, "pipeline": 12}.get(kind)
+                  "stream": 12, "pipeline": 22 if case.get("method") == "drpa" else 12}.get(kind)
     drpa = kind == "drpa" or case.get("method") == "drpa"
     if iterations is None:
-        iterations = 12 if case["scheme"] == "diis" else 25 if drpa else 33
+        iterations = 12 if case["scheme"] == "diis" else 33
     nbytes = flops = 0
     for electrons, basis in sizes:
         O, V, amps, ladder, rings = _shape(electrons, basis)
