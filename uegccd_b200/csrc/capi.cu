@@ -889,7 +889,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->alloc(d.g, amp0))) return rc;
     if ((rc = b->alloc(d.jvv, jvv0))) return rc;
     if ((rc = b->alloc(d.joo, joo0))) return rc;
-    d.ph_total = ph0;
     if ((rc = b->alloc(d.hh, hhoff))) return rc;
     const size_t npart = std::max(chunks.size(), hchunks.size());   // per full or half chunk
     if ((rc = b->alloc(d.part_e, npart))) return rc;
@@ -1070,6 +1069,44 @@ int mixed_alloc(UegccdBatch &b)
         CU(cudaGetLastError());
         d.w16_valid = true;
     }
+    return 0;
+}
+
+// Lookups and sums of the dRPA terms, on the first dRPA solve.
+int drpa_alloc(UegccdBatch &b)
+{
+    DevBatch &d = b.d;
+    if (d.drs2) return 0;
+    const int n = d.nsolves;
+    std::vector<int2> list;
+    std::vector<DrpaSolveDev> ds(n);
+    int64_t rij = 0, cp = 0, ph = 0;
+    for (int s = 0; s < n; s++) {
+        const SolvePlan &P = b.plans[s];
+        ds[s] = DrpaSolveDev{rij, cp};
+        rij += (int64_t)P.O * P.O;
+        cp += (int64_t)P.blocks.size() * P.V;
+        ph += (int64_t)P.O * P.V;
+        for (int i = 0; i < P.O; i++) list.push_back(make_int2(s, i));
+    }
+    const UegccdBatch::Mark m = b.mark();
+    DevBatch x = d;
+    int rc = 0;
+    if ((rc = b.upload(x.drlist, list)) || (rc = b.upload(x.drsolves, ds)) || (rc = b.alloc(x.drows, (size_t)rij)) ||
+        (rc = b.alloc(x.colpos, (size_t)cp)) || (rc = b.alloc(x.drdone, n)) || (rc = b.alloc(x.dru, (size_t)ph)) ||
+        (rc = b.alloc(x.drs2, (size_t)ph))) {
+        cudaStreamSynchronize(b.stream);   // the uploads above read host vectors of this call
+        b.rollback(m);
+        return rc;
+    }
+    x.ndrlist = (int)list.size();
+    CU(cudaMemsetAsync(x.drows, 0xff, (size_t)rij * sizeof(int4), b.stream));
+    CU(cudaMemsetAsync(x.colpos, 0xff, (size_t)cp * sizeof(int16_t), b.stream));
+    CU(cudaMemsetAsync(x.drdone, 0, n * sizeof(int), b.stream));
+    launch_drpa_tables(x, b.stream);
+    CU(cudaGetLastError());
+    CU(cudaStreamSynchronize(b.stream));
+    d = x;
     return 0;
 }
 
@@ -1259,7 +1296,7 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
     CU(cudaMemsetAsync(b.ctl.Bm, 0, (size_t)n * kDiisMax * kDiisMax * sizeof(double), b.stream));
     if ((rc = set_active_all(b, 1))) return rc;
     if (opt->precision == UEGCCD_MIXED && (rc = mixed_alloc(b))) return rc;
-    if (drpa && !d.J1 && (rc = b.alloc(d.J1, (size_t)d.ph_total))) return rc;
+    if (drpa && (rc = drpa_alloc(b))) return rc;
     if (d.tc_err) CU(cudaMemsetAsync(d.tc_err, 0, sizeof(int), b.stream));
     if (!b.rings_tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch_rings(b))) return rc;
     b.launches = 0;
@@ -1401,7 +1438,7 @@ int session_start(UegccdBatch &b, const UegccdOptions *opt, int drpa)
     CU(cudaMemcpyAsync(b.ctl.state, st0.data(), n * sizeof(IterState), cudaMemcpyHostToDevice, b.stream));
     CU(cudaMemsetAsync(b.ctl.Bm, 0, (size_t)n * kDiisMax * kDiisMax * sizeof(double), b.stream));
     if ((rc = set_active_all(b, 1))) return rc;
-    if (drpa && !d.J1 && (rc = b.alloc(d.J1, (size_t)d.ph_total))) return rc;
+    if (drpa && (rc = drpa_alloc(b))) return rc;
     if (!b.rings_tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch_rings(b))) return rc;
     launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
     launch_reduce(d, b.stream);
@@ -1967,7 +2004,6 @@ int uegccd_batch_solve(UegccdBatch *b, const UegccdOptions *opt, int32_t drpa, d
     if (drpa) {
         // the reference starts dRPA from T2aaaa of the MP2 step (Main.f90:85-91)
         launch_to_aaaa(b->d, b->stream);
-        std::swap(b->d.t, b->d.t_new);
     }
     int st = two ? run_two_channel_solves(*b, opt, results) : run_solves(*b, opt, drpa, results);
     if (st < 0) return st;
@@ -2000,7 +2036,6 @@ int uegccd_batch_start(UegccdBatch *b, const UegccdOptions *opt, int32_t drpa, d
         for (int s = 0; s < b->d.nsolves; s++) e2[s] = b->red[3 * s];
     if (drpa) {
         launch_to_aaaa(b->d, b->stream);   // the dRPA start is T2aaaa of the MP2 step (Main.f90:85-91)
-        std::swap(b->d.t, b->d.t_new);
         b->launches++;
     }
     return session_start(*b, opt, drpa);
@@ -2085,7 +2120,7 @@ int uegccd_footprint(const UegccdSystem *sys, int32_t ndiis, int32_t mixed, int6
     b += A * (8 * 3 + 16 + sizeof(AmpInfo) + 4 + 4); // t, t_new, g; Coulomb factors; amps; partner, mirror
     b += sum_ov * (8 + 4) + (V + O + 1) * (4 + 8);   // mosaic partials and target lists
     b += O * O * V * 4;                              // pos
-    b += O * V * O * 8;                              // dRPA ring intermediate (allocated for dRPA only)
+    b += O * V * 8 * 2 + O * O * 16 + nblk * V * 2;  // dRPA sums and lookups (allocated for dRPA only)
     b += O * V * 2 * 2;                              // ph rows
     int64_t xy = 0;                                  // particle-hole operands and results of the rings
     for (size_t gi = 0; gi < P.groups.size(); gi++) {

@@ -48,8 +48,15 @@ struct DevBatch {
     double *t = nullptr, *t_new = nullptr, *g = nullptr;
     double2 *vcoef = nullptr;         // per amplitude {v(i-a), v(a-j)} (k_vcoef, once per batch)
     double *jvv = nullptr, *joo = nullptr;
-    double *J1 = nullptr;             // dRPA ring intermediate (on the first dRPA solve)
-    int64_t ph_total = 0;             // O*V*O entries summed over the solves
+    // dRPA (on the first dRPA solve): k_drpa_sums' CTA list {solve, i}, row and column lookups,
+    // and its U, S2 per (i, x) at phr0 + i*V + x - O; per solve the count of finished CTAs
+    int2 *drlist = nullptr;
+    int ndrlist = 0;
+    DrpaSolveDev *drsolves = nullptr;
+    int4 *drows = nullptr;
+    int16_t *colpos = nullptr;
+    double *dru = nullptr, *drs2 = nullptr;
+    int *drdone = nullptr;
     int64_t *hh0 = nullptr;          // per block: offset of H_K in hh
     double *hh = nullptr;
     double *part_e = nullptr, *part_dt = nullptr, *part_r = nullptr;
@@ -131,7 +138,7 @@ int tune_rings(DevBatch &d, cudaStream_t st);
 constexpr int kDiisMax = 16;   // DIIS history capacity (k_update and k_diis_* use the same bound)
 
 // Live per-kernel timing with CUDA events on the launching stream (off unless enabled).
-enum KernelId { KID_MP2 = 0, KID_ENERGY, KID_HH_W, KID_LADDER, KID_MOSAIC_S, KID_MOSAIC_RED, KID_RING_INT,
+enum KernelId { KID_MP2 = 0, KID_ENERGY, KID_HH_W, KID_LADDER, KID_MOSAIC_S, KID_MOSAIC_RED, KID_DRPA_SUMS,
                 KID_UPDATE, KID_REDUCE, KID_RINGS, KID_LADDER_TC, KID_RING_STAGE,
                 KID_COUNT };
 struct KernelTimer {
@@ -198,9 +205,12 @@ struct TermFlags {
 void launch_mp2(const DevBatch &d, cudaStream_t st);
 void launch_reduce(const DevBatch &d, cudaStream_t st);
 void launch_energy(const DevBatch &d, int kind, double csosex, cudaStream_t st);
-// d.t_new = T2aaaa of d.t (t(ij,a) - t(ij,b))
+// d.t <- T2aaaa of d.t (t(ij,a) - t(ij,b))
 void launch_to_aaaa(const DevBatch &d, cudaStream_t st);
-// Residual of the selected terms for d.t; mode 0 also updates into d.t_new.  Returns launches.
+// drows and colpos (pre-set to -1) of the dRPA sums from the blocks
+void launch_drpa_tables(const DevBatch &d, cudaStream_t st);
+// Residual of the selected terms for d.t; mode 0 also updates d.t (with DIIS: the history).
+// Returns launches.
 struct CtlBuffers;
 // diis/ndiis (mode 0 only): fuse the Pulay DIIS push into the update kernel
 int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_out, cudaStream_t st,

@@ -157,12 +157,17 @@ __global__ void k_energy(const ChunkDev *__restrict__ chunks, const SolveDev *__
     if (threadIdx.x == 0) { part_e[blockIdx.x] = e; part_a[blockIdx.x] = mx; part_b[blockIdx.x] = 0.0; }
 }
 
-// t'(ij,a) = t(ij,a) - t(ij,b): T2aaaa of spin-adapted amplitudes (MP2.f90:70), the dRPA start.
-__global__ void k_to_aaaa(int64_t n, const int32_t *__restrict__ partner, const double *__restrict__ t,
-                          double *__restrict__ out)
+// t'(ij,a) = t(ij,a) - t(ij,b): T2aaaa of spin-adapted amplitudes (MP2.f90:70), the dRPA
+// start, in place: the thread of the smaller index of a partner pair forms both values.
+__global__ void k_to_aaaa(int64_t n, const int32_t *__restrict__ partner, double *__restrict__ t)
 {
     int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-    if (p < n) out[p] = t[p] + (-t[partner[p]]);
+    if (p >= n) return;
+    const int32_t q = partner[p];
+    if (q < p) return;
+    const double x = t[p], y = t[q];
+    t[p] = x + (-y);
+    if (q != p) t[q] = y + (-x);
 }
 
 // Per-solve reduction of the chunk partials in chunk order.
@@ -542,7 +547,7 @@ static int launch_ladder3(const DevBatch &d, const LadderTile *tiles, const int 
 //   s(k,l,c) = v(c-k) (T2aaaa + T2abab)(kl,c) - v(c-l) (T2aaaa + T2abba)(kl,c)
 //            = v(c-k) (2t(kl,c) - t(kl,d)) - v(c-l) (t(kl,c) - 2t(kl,d))
 //   Jvv(c) = sum_{k,l} s(k,l,c),  Joo(k) = sum_{l,c} s(k,l,c)
-// dRPA (dRPA.f90:415-431): s(k,l,c) = 2 v(c-k) t(kl,c).
+// (dRPA's own mosaics, dRPA.f90:415-431, come from k_drpa_sums.)
 // s lives only in registers: one CTA per K block forms it row by row (d = K - c is
 // in the same row) and writes the block's row sums (-> Joo of the row's k) and
 // column sums (-> Jvv of the column's c); k_mosaic_sum adds the partials of each
@@ -567,7 +572,7 @@ __global__ void __launch_bounds__(kMosThreads) k_mosaic_blk(const BlockDev *__re
                                                            const int *__restrict__ nvp,
                                                            const double *__restrict__ vtab,
                                                            const double *__restrict__ t,
-                                                           const int16_t *__restrict__ pcol, int drpa,
+                                                           const int16_t *__restrict__ pcol,
                                                            double *__restrict__ mpart,
                                                            const uint8_t *__restrict__ active, int vt_n)
 {
@@ -620,24 +625,19 @@ __global__ void __launch_bounds__(kMosThreads) k_mosaic_blk(const BlockDev *__re
         }
         for (int c = tid; c < v; c += kMosThreads) {
             const int ncv = nvc[c];
-            const int pcc = drpa ? c : pc[c];
+            const int pcc = pc[c];
             double x[kR], y[kR];
 #pragma unroll
             for (int q = 0; q < kR; q++) {
                 x[q] = q < nr ? row[q][c] : 0.0;
-                y[q] = (q < nr && !drpa) ? row[q][pcc] : 0.0;   // t(kl, d), same row
+                y[q] = q < nr ? row[q][pcc] : 0.0;   // t(kl, d), same row
             }
 #pragma unroll
             for (int q = 0; q < kR; q++) {
                 if (q >= nr) continue;
                 const double vck = V(q2p(ncv, rk[q]));
-                double sval;
-                if (drpa) {
-                    sval = 2.0 * vck * x[q];
-                } else {
-                    const double vcl = V(q2p(ncv, rl[q]));
-                    sval = vck * (2.0 * x[q] - y[q]) - vcl * (x[q] - 2.0 * y[q]);
-                }
+                const double vcl = V(q2p(ncv, rl[q]));
+                const double sval = vck * (2.0 * x[q] - y[q]) - vcl * (x[q] - 2.0 * y[q]);
                 rs[q] += sval;
                 if (r0 + q >= B.nd) cdg[c] = sval;
                 else coff[c] += sval;
@@ -752,33 +752,101 @@ void set_mosaic_smem_limit(size_t bytes)
 }
 
 // ----------------------------------------------------------------------------
-// dRPA ring intermediate (dRPA.f90:517-535), for every (i, x, l) with x virtual:
-//   J1 = sum_k 2 t(ik,x) v(i-x).
-// The reference skips (i,x,l) when d = n_l + n_x - n_i is not a virtual; the apply
-// step in k_update makes the same test, so J1 is formed for every l.
-// Layout: J1[ph0 + (i*V + x)*O + l].  (The CCD rings use k_rings.)
+// dRPA rings and mosaics (dRPA.f90:377-551) from two sums per particle-hole pair (i, x):
+//   S1(i,x) = sum_k t(ik,x),   S2(i,x) = sum_k t(ki,d), d = n_k + n_x' the column whose partner
+//                              is x in row (k,i)
+// The quadratic sum J(i,a,l) = sum_k 2 t(ik,a) v(i-a) (dRPA.f90:517-535) does not depend on l
+// -- the reference's test that d is a virtual is the test that (l,j,b) is allowed, which the
+// apply makes again -- so with U = 2 v(i-a) S1 and v(j-b) = v(i-a) every ring term of one
+// amplitude is
+//   U(i,a) + U(j,b) + 2 U(i,a) S2(j,b)                      (dRPA.f90:476-545)
+// and the mosaics s(k,l,c) = 2 v(c-k) t(kl,c) (dRPA.f90:415-431) add up to
+//   Joo(k) = sum_c U(k,c),   Jvv(c) = sum_k U(k,c).
+// k_update then reads three values per amplitude where it walked 3 NOcc of them.
+//
+// One CTA per (solve, i), a thread per virtual x: each k adds one value of row (i,k) and one
+// of its mirror (k,i), at the column of x in that row's block (colpos), in ascending k.  The
+// last CTA of a solve to finish adds the columns of U up for Jvv.
+// Bound by memory latency: every amplitude read twice, near-coalesced (18 bytes with the column
+// index).  30 twists of N=54, 485 plane waves, per iteration: 0.052 ms here and 0.072 ms in
+// k_update, against 0.489 ms for the (i, x, l) intermediate, 0.048 ms of mosaic kernels and
+// 0.645 ms in k_update.
 // ----------------------------------------------------------------------------
-__global__ void k_ring_int(const ChunkDev *__restrict__ rchunks, const SolveDev *__restrict__ solves,
-                           const int32_t *__restrict__ pos, const int4 *__restrict__ nv4,
-                           const double *__restrict__ vtab, const double *__restrict__ t,
-                           double *__restrict__ J1, const uint8_t *__restrict__ active)
+constexpr int kDrpaThreads = 256;
+constexpr int kMaxOcc = 64;   // NOcc limit of a batch
+
+// Row and column lookups, one CTA per K block: drows[(i,j)] = {first packed index of row
+// (i,j), block, nvd, nvd + sd}; colpos[block][x] = column of virtual x (both pre-set to -1).
+__global__ void k_drpa_tables(const BlockDev *__restrict__ blocks, const SolveDev *__restrict__ solves,
+                              const DrpaSolveDev *__restrict__ ds, const int16_t *__restrict__ pair_i,
+                              const int16_t *__restrict__ pair_j, const int16_t *__restrict__ vir,
+                              int4 *__restrict__ drows, int16_t *__restrict__ colpos)
 {
-    const ChunkDev ch = rchunks[blockIdx.x];
-    if (!active[ch.solve]) return;
-    const SolveDev s = solves[ch.solve];
-    const int O = s.O, V = s.V;
-    const int e = ch.start + threadIdx.x;
-    if (e >= O * V * O) return;
-    const int ix = e / O;
-    const int x = ix % V + O;
-    const int i = ix / V;
-    const double vd = vpq(s, nv4, vtab, i, x);
-    double j1 = 0.0;
-    for (int k = 0; k < O; k++) {
-        const int p1 = posmap(s, pos, i, k, x);
-        if (p1 >= 0) j1 += 2.0 * t[p1] * vd;
+    const BlockDev B = blocks[blockIdx.x];
+    const SolveDev s = solves[B.solve];
+    const DrpaSolveDev D = ds[B.solve];
+    const int bl = blockIdx.x - s.blk0;
+    for (int r = threadIdx.x; r < B.o; r += blockDim.x)
+        drows[D.rij0 + (int64_t)pair_i[B.pair0 + r] * s.O + pair_j[B.pair0 + r]] =
+            make_int4((int)(B.t0 + (int64_t)r * B.v), bl, B.nvd, B.nvd + B.sd);
+    for (int c = threadIdx.x; c < B.v; c += blockDim.x)
+        colpos[D.cp0 + (int64_t)bl * s.V + (vir[B.vir0 + c] - s.O)] = (int16_t)c;
+}
+
+__global__ void __launch_bounds__(kDrpaThreads)
+    k_drpa_sums(const int2 *__restrict__ list, const SolveDev *__restrict__ solves,
+                const DrpaSolveDev *__restrict__ ds, const int4 *__restrict__ drows,
+                const int16_t *__restrict__ colpos, const int4 *__restrict__ nv4, const double *__restrict__ vtab,
+                const double *__restrict__ t, double *u, double *__restrict__ s2, double *__restrict__ jvv,
+                double *__restrict__ joo, int *__restrict__ done, const uint8_t *__restrict__ active)
+{
+    const int2 L = list[blockIdx.x];
+    if (!active[L.x]) return;
+    const SolveDev s = solves[L.x];
+    const DrpaSolveDev D = ds[L.x];
+    const int O = s.O, V = s.V, i = L.y;
+    __shared__ int4 row[kMaxOcc];
+    __shared__ int mrow[kMaxOcc];
+    __shared__ bool last;
+    for (int k = threadIdx.x; k < O; k += kDrpaThreads) {
+        row[k] = drows[D.rij0 + (int64_t)i * O + k];
+        mrow[k] = drows[D.rij0 + (int64_t)k * O + i].x;
     }
-    J1[s.ph0 + e] = j1;
+    __syncthreads();
+    const int16_t *cp = colpos + D.cp0;
+    double usum = 0.0;
+    for (int x = threadIdx.x; x < V; x += kDrpaThreads) {
+        double a1 = 0.0, a2 = 0.0;
+#pragma unroll 4
+        for (int k = 0; k < O; k++) {
+            const int4 r = row[k];
+            const int c = r.x >= 0 ? __ldg(&cp[(int64_t)r.y * V + x]) : -1;
+            if (c >= 0) {
+                const int pc = c < r.z ? c + r.w : c < r.w ? c : c - r.w;
+                a1 += __ldg(&t[r.x + c]);
+                a2 += __ldg(&t[mrow[k] + pc]);
+            }
+        }
+        const double y = 2.0 * vpq(s, nv4, vtab, i, s.O + x) * a1;
+        u[s.phr0 + (int64_t)i * V + x] = y;
+        s2[s.phr0 + (int64_t)i * V + x] = a2;
+        usum += y;
+    }
+    usum = block_sum<kDrpaThreads>(usum);
+    if (threadIdx.x == 0) joo[s.joo0 + i] = usum;
+    // Jvv by the solve's last CTA: its reads of u follow every other CTA's fence and count
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) last = atomicAdd(&done[L.x], 1) == O - 1;
+    __syncthreads();
+    if (!last) return;
+    __threadfence();
+    for (int x = threadIdx.x; x < V; x += kDrpaThreads) {
+        double a = 0.0;
+        for (int k = 0; k < O; k++) a += __ldcg(&u[s.phr0 + (int64_t)k * V + x]);
+        jvv[s.jvv0 + x] = a;
+    }
+    if (threadIdx.x == 0) done[L.x] = 0;
 }
 
 // ----------------------------------------------------------------------------
@@ -1234,23 +1302,19 @@ size_t rings_smem_bytes(int O, int R)
 //   t' = (G/D - (1-f) t)/f                (SolveCC, CCD.f90:380)
 //   dT = max |t' - t|                     (CnvrgCC, CCD.f90:452-454)
 //   E  = sum t' (2 v(i-a) - v(a-j))       (CCEnergy, CCD.f90:225-227 re-indexed)
-// mode 0: update (writes t_new, partials e/dT/|R|); mode 1: residual only (|R|).
+// mode 0: update (in place, or with DIIS into the history; partials e/dT/|R|); mode 1:
+// residual only (|R|).
 // ----------------------------------------------------------------------------
 struct UpdateArgs {
     const HChunkDev *chunks;
     const SolveDev *solves;
     const AmpInfo *amps;
-    const int32_t *partner;
     const int32_t *mirror;
-    const int32_t *pos;
-    const int4 *nv4;
     const double *eigen;
-    const double *vtab;
-    const double *t;
-    double *t_new;
+    double *t;                    // each amplitude i <= j reads its own value only: updated in place
     const double *g_ladder;
     const double *jvv, *joo;
-    const double *J1;             // dRPA ring intermediate
+    const double *dru, *drs2;     // dRPA: U and S2 of k_drpa_sums
     double *part_e, *part_dt, *part_r;
     double *g_out;            // optional: full G per amplitude (term checks)
     const double *rx;                          // ring and crossed-ring G, particle-hole layout
@@ -1424,12 +1488,7 @@ __global__ void __launch_bounds__(kChunk, 8) k_update(UpdateArgs A)
     // each amplitude with i < j also updates its mirror (j,i,b); every term of G shares the
     // symmetry.
     const bool valid = loc < ch.end;
-    const int32_t mirv = valid ? A.mirror[s.amp0 + loc] : -2;
-    if (!on && A.mode == 0 && valid) {
-        A.t_new[s.amp0 + loc] = A.t[s.amp0 + loc];
-        if (mirv >= 0) A.t_new[mirv] = A.t[mirv];
-    }
-    const int32_t mir = on ? mirv : -2;
+    const int32_t mir = on && valid ? A.mirror[s.amp0 + loc] : -2;
     const double wgt = mir >= 0 ? 2.0 : 1.0;   // energy and DIIS dot weight: this amplitude and its mirror
     if (mir != -2) {
         const int64_t p = s.amp0 + loc;
@@ -1444,23 +1503,10 @@ __global__ void __launch_bounds__(kChunk, 8) k_update(UpdateArgs A)
         if (A.do_mosaic)
             g -= 0.5 * (A.jvv[s.jvv0 + a - O] + A.jvv[s.jvv0 + b - O] + A.joo[s.joo0 + i] + A.joo[s.joo0 + j]) * told;
         if (A.drpa) {
-            if (A.do_ring) {
-                // linear (dRPA.f90:476-513): 2 v(i-a) sum_k t(ik,a) + 2 v(j-b) sum_k t(jk,b)
-                double s1 = 0.0, s2 = 0.0;
-                for (int k = 0; k < O; k++) {
-                    int p1 = posmap(s, A.pos, i, k, a);
-                    if (p1 >= 0) s1 += A.t[p1];
-                    int p2 = posmap(s, A.pos, j, k, b);
-                    if (p2 >= 0) s2 += A.t[p2];
-                }
-                g += 2.0 * via * s1 + 2.0 * vpq(s, A.nv4, A.vtab, j, b) * s2;
-                // quadratic (dRPA.f90:539-545): sum_l 2 J(i,a,l) t(lj,d), d = n_l + n_a - n_i
-                const double *Jr = A.J1 + s.ph0 + ((int64_t)i * s.V + (a - O)) * O;
-                for (int l = 0; l < O; l++) {
-                    int pb = posmap(s, A.pos, l, j, b);  // exists iff d is a virtual
-                    if (pb < 0) continue;
-                    g += 2.0 * Jr[l] * A.t[A.partner[pb]];
-                }
+            if (A.do_ring) {   // linear and quadratic rings (k_drpa_sums)
+                const int64_t ia = s.phr0 + (int64_t)i * s.V + (a - O), jb = s.phr0 + (int64_t)j * s.V + (b - O);
+                const double u = A.dru[ia];
+                g += u + A.dru[jb] + 2.0 * u * A.drs2[jb];
             }
         } else if (A.do_ring || A.do_xring) {
             // the ring G (rings, linear + quadratic, CCD.f90:716-811) and the crossed-ring G
@@ -1486,8 +1532,8 @@ __global__ void __launch_bounds__(kChunk, 8) k_update(UpdateArgs A)
             const double f = s.denom_factor;
             const double tn = (g / denom - (1.0 - f) * told) / f;
             if (A.ndiis == 0) {  // with DIIS the history slot holds t'
-                A.t_new[p] = tn;
-                if (mir >= 0) A.t_new[mir] = tn;
+                A.t[p] = tn;
+                if (mir >= 0) A.t[mir] = tn;
             }
             dtmax = fabs(tn - told);
             if (A.drpa) esum = via * tn * 2.0;  // SOSEX part added by k_drpa_energy at the end
@@ -1659,23 +1705,6 @@ __global__ void k_active_swap(int nsolves, uint8_t *__restrict__ active, const u
     }
 }
 
-// t <- t_new for the solves still iterating this round (replay mode)
-__global__ void k_commit(const HChunkDev *__restrict__ chunks, const SolveDev *__restrict__ solves,
-                         const int32_t *__restrict__ mirror, const double *__restrict__ t_new,
-                         double *__restrict__ t, const uint8_t *__restrict__ active)
-{
-    const HChunkDev ch = chunks[blockIdx.x];
-    if (!active[ch.solve]) return;
-    const SolveDev s = solves[ch.solve];
-    const int loc = ch.start + threadIdx.x;
-    if (loc >= ch.end) return;
-    const int64_t p = s.amp0 + loc;
-    const double x = t_new[p];
-    t[p] = x;
-    const int32_t mir = mirror[p];
-    if (mir >= 0) t[mir] = x;
-}
-
 __global__ void k_diis_rows2(const int *__restrict__ chunk_begin, const IterState *__restrict__ st, int ndiis,
                              const double *__restrict__ part, double *__restrict__ brow,
                              const uint8_t *__restrict__ active)
@@ -1741,7 +1770,7 @@ void launch_active_swap(const DevBatch &d, const CtlBuffers &c, cudaStream_t st)
     k_active_swap<<<1, 1024, 0, st>>>(d.nsolves, d.active, c.active_next, c.count);
 }
 
-// One iteration: residual + update, reduction, [DIIS], control, commit, swap.  Returns launches.
+// One iteration: residual + update, reduction, [DIIS], control, swap.  Returns launches.
 int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f, double tol, int max_iter,
                      int ndiis, cudaStream_t st, KernelTimer *kt)
 {
@@ -1755,10 +1784,8 @@ int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f,
     if (ndiis > 0)
         k_diis_extrap2<<<d.nhchunks, kChunk, 0, st>>>(d.hchunks, d.solves, d.namp, c.hist_t, c.coef, ndiis, d.mirror,
                                                      d.t, d.active);
-    else
-        k_commit<<<d.nhchunks, kChunk, 0, st>>>(d.hchunks, d.solves, d.mirror, d.t_new, d.t, d.active);
     launch_active_swap(d, c, st);
-    return n + 3;
+    return n + (ndiis > 0 ? 3 : 2);
 }
 
 // ----------------------------------------------------------------------------
@@ -1938,13 +1965,20 @@ void launch_energy(const DevBatch &d, int kind, double csosex, cudaStream_t st)
                                            d.part_r);
 }
 
+void launch_drpa_tables(const DevBatch &d, cudaStream_t st)
+{
+    if (d.nblocks > 0)
+        k_drpa_tables<<<d.nblocks, 256, 0, st>>>(d.blocks, d.solves, d.drsolves, d.pair_i, d.pair_j, d.vir, d.drows,
+                                                 d.colpos);
+}
+
 void launch_to_aaaa(const DevBatch &d, cudaStream_t st)
 {
-    k_to_aaaa<<<(unsigned)((d.namp + 255) / 256), 256, 0, st>>>(d.namp, d.partner, d.t, d.t_new);
+    k_to_aaaa<<<(unsigned)((d.namp + 255) / 256), 256, 0, st>>>(d.namp, d.partner, d.t);
 }
 
 const char *kKernelNames[KID_COUNT] = {"k_mp2",      "k_energy",   "k_ladder_hh", "k_ladder",
-                                      "k_mosaic_blk", "k_mosaic_sum", "k_ring_int", "k_update",
+                                      "k_mosaic_blk", "k_mosaic_sum", "k_drpa_sums", "k_update",
                                       "k_reduce_solves", "k_rings",
                                       "k_ladder_tc", "k_ring_stage"};
 
@@ -2074,10 +2108,10 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
             n += (d.ntc16 > 0) + (d.ntc32 > 0) + (d.ntc64 > 0);
         }
     }
-    if (f.do_mosaic) {
+    if (f.do_mosaic && !f.drpa) {
         kt->begin(KID_MOSAIC_S, st);
         k_mosaic_blk<<<d.nblocks, kMosThreads, d.mosaic_smem, st>>>(d.blocks, d.solves, d.pair_i, d.pair_j, d.vir,
-                                                                   d.nvp, d.vtab, d.t, d.pcol, f.drpa, d.mpart,
+                                                                   d.nvp, d.vtab, d.t, d.pcol, d.mpart,
                                                                    d.active, d.mosaic_vt);
         kt->end(st);
         kt->begin(KID_MOSAIC_RED, st);
@@ -2086,9 +2120,10 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         kt->end(st);
         n += 2;
     }
-    if ((f.do_ring || f.do_xring) && f.drpa) {
-        kt->begin(KID_RING_INT, st);
-        k_ring_int<<<d.nrchunks, kChunk, 0, st>>>(d.rchunks, d.solves, d.pos, d.nv4, d.vtab, d.t, d.J1, d.active);
+    if ((f.do_ring || f.do_mosaic) && f.drpa) {
+        kt->begin(KID_DRPA_SUMS, st);
+        k_drpa_sums<<<d.ndrlist, kDrpaThreads, 0, st>>>(d.drlist, d.solves, d.drsolves, d.drows, d.colpos, d.nv4,
+                                                        d.vtab, d.t, d.dru, d.drs2, d.jvv, d.joo, d.drdone, d.active);
         kt->end(st);
         n++;
     }
@@ -2119,9 +2154,9 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         kt->end(st);
     }
     UpdateArgs A;
-    A.chunks = d.hchunks; A.solves = d.solves; A.amps = d.amps; A.partner = d.partner; A.mirror = d.mirror; A.pos = d.pos;
-    A.nv4 = d.nv4; A.eigen = d.eigen; A.vtab = d.vtab; A.t = d.t; A.t_new = d.t_new; A.g_ladder = d.g;
-    A.jvv = d.jvv; A.joo = d.joo; A.J1 = d.J1;
+    A.chunks = d.hchunks; A.solves = d.solves; A.amps = d.amps; A.mirror = d.mirror;
+    A.eigen = d.eigen; A.t = d.t; A.g_ladder = d.g;
+    A.jvv = d.jvv; A.joo = d.joo; A.dru = d.dru; A.drs2 = d.drs2;
     A.part_e = d.part_e; A.part_dt = d.part_dt; A.part_r = d.part_r; A.g_out = g_out; A.active = d.active;
     A.do_ladder = f.do_ladder; A.do_mosaic = f.do_mosaic; A.do_ring = f.do_ring; A.do_xring = f.do_xring;
     A.do_driver = f.do_driver; A.drpa = f.drpa; A.mode = mode;

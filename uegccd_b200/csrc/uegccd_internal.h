@@ -99,6 +99,12 @@ struct RingPairDev {
     int32_t xy0;
 };
 
+// Where a solve's dRPA lookups start: rows of its pairs (O*O entries), columns of its blocks
+// (nblk*V entries).
+struct DrpaSolveDev {
+    int64_t rij0, cp0;
+};
+
 struct ChunkDev {
     int solve;
     int32_t start;          // first amplitude of the chunk, local to the solve
