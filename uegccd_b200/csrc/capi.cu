@@ -1148,9 +1148,9 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
     if (!c.state) {
         const UegccdBatch::Mark m = b.mark();
         CtlBuffers x = c;
-        if ((rc = b.alloc(x.state, n)) || (rc = b.alloc(x.active_next, n)) || (rc = b.alloc(x.count, 1)) ||
+        if ((rc = b.alloc(x.state, n)) || (rc = b.alloc(x.applied, n)) || (rc = b.alloc(x.count, 1)) ||
             (rc = b.alloc(x.Bm, (size_t)n * kDiisMax * kDiisMax)) || (rc = b.alloc(x.coef, (size_t)n * kDiisMax)) ||
-            (rc = b.alloc(x.brow, (size_t)n * kDiisMax)) || (rc = b.alloc(x.part, (size_t)b.d.nhchunks * kDiisMax))) {
+            (rc = b.alloc(x.part, (size_t)b.d.nhchunks * kDiisMax))) {
             b.rollback(m);
             return rc;
         }
@@ -1303,10 +1303,8 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
     CU(cudaEventRecord(b.ev0, b.stream));
     // CCEnergy of the start amplitudes and dT = max|T| (CCD.f90:63-64, dRPA.f90:68-69)
     launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
-    launch_reduce(d, b.stream);
-    launch_control(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
-    launch_active_swap(d, b.ctl, b.stream);
-    b.launches += 4;
+    launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
+    b.launches += 2;
     int count = n, rounds = 0;
     const int max_rounds = opt->max_iter / kPoll + 2;
     // mixed precision: tensor-core ladder of t - t_ref, t_ref refreshed (FP64) each round,
@@ -1323,6 +1321,7 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
             CU(cudaMemcpyAsync(b.ctl.state, st1.data(), n * sizeof(IterState), cudaMemcpyHostToDevice, b.stream));
             if ((rc = set_active_all(b, 1))) return rc;
             count = n;
+            CU(cudaMemcpyAsync(b.ctl.count, &count, sizeof(int), cudaMemcpyHostToDevice, b.stream));
             rounds = 0;
         }
         if ((rc = capture_iteration(b, f, opt->tol, opt->max_iter, ndiis))) return rc;
@@ -1441,10 +1440,8 @@ int session_start(UegccdBatch &b, const UegccdOptions *opt, int drpa)
     if (drpa && (rc = drpa_alloc(b))) return rc;
     if (!b.rings_tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch_rings(b))) return rc;
     launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
-    launch_reduce(d, b.stream);
-    launch_control(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
-    launch_active_swap(d, b.ctl, b.stream);
-    b.launches += 4;
+    launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
+    b.launches += 2;
     if ((rc = capture_iteration(b, f, opt->tol, opt->max_iter, ndiis))) return rc;
     CU(cudaStreamSynchronize(b.stream));
     S.opt = *opt;

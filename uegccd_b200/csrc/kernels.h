@@ -140,7 +140,7 @@ constexpr int kDiisMax = 16;   // DIIS history capacity (k_update and k_diis_* u
 // Live per-kernel timing with CUDA events on the launching stream (off unless enabled).
 enum KernelId { KID_MP2 = 0, KID_ENERGY, KID_HH_W, KID_LADDER, KID_MOSAIC_S, KID_MOSAIC_RED, KID_DRPA_SUMS,
                 KID_UPDATE, KID_REDUCE, KID_RINGS, KID_LADDER_TC, KID_RING_STAGE,
-                KID_COUNT };
+                KID_TAIL, KID_EXTRAP, KID_COUNT };
 struct KernelTimer {
     bool on = false;
     cudaEvent_t ev[2 * 64];
@@ -177,7 +177,7 @@ struct KernelTimer {
 };
 extern const char *kKernelNames[KID_COUNT];
 
-// Per-solve iteration state kept on the device (see k_control).
+// Per-solve iteration state kept on the device (see k_tail).
 struct IterState {
     int niter;      // NIter of the reference (1 before the first update)
     int status;     // 0 running, 1 converged, 2 MaxIter reached, 3 non-finite
@@ -187,9 +187,9 @@ struct IterState {
 // Buffers of the device-side iteration control.
 struct CtlBuffers {
     IterState *state = nullptr;
-    uint8_t *active_next = nullptr;
-    int *count = nullptr;
-    double *Bm = nullptr, *coef = nullptr, *brow = nullptr, *part = nullptr;
+    uint8_t *applied = nullptr;  // the solves the iteration in flight updated
+    int *count = nullptr;        // solves still iterating
+    double *Bm = nullptr, *coef = nullptr, *part = nullptr;
     double *hist_t = nullptr;   // DIIS history: updated amplitudes t' (FP64)
     float *hist_e = nullptr;    // and error vectors e = t' - t (FP32: they only enter the B-matrix dots)
     double *rec_e = nullptr, *rec_dt = nullptr;
@@ -238,9 +238,8 @@ void launch_w16_build(const DevBatch &d, cudaStream_t st);
 // Refresh point: t_ref <- t and g_ref <- FP64 particle-particle ladder of t_ref
 void launch_refresh(const DevBatch &d, cudaStream_t st);
 // Device-side iteration control
-void launch_control(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
-                    cudaStream_t st);
-void launch_active_swap(const DevBatch &d, const CtlBuffers &c, cudaStream_t st);
+void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
+                 cudaStream_t st);
 int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f, double tol, int max_iter,
                      int ndiis, cudaStream_t st, KernelTimer *kt);
 void launch_unpack(const DevBatch &d, int s, int namp, const double *t, double *ab, double *ba, double *aa,

@@ -1584,80 +1584,135 @@ __global__ void __launch_bounds__(kChunk, 8) k_update(UpdateArgs A)
 // builds a singular matrix and never extrapolates).  Error vector e = t' - t of
 // the (damped) Jacobi step; history of ndiis (t', e) pairs per solve.
 // k_update stores the solve's current slot and forms the dot products e . e_j of
-// every stored j (per-chunk partials); k_diis_rows2 reduces them per solve in chunk order.
+// every stored j (per-chunk partials); k_tail reduces them per solve in chunk order.
 // ----------------------------------------------------------------------------
 constexpr int kMaxDiis = 16;
 // ----------------------------------------------------------------------------
 // Device-side iteration control.  Every solve of a batch carries its own state;
-// one iteration is a fixed sequence of launches (residual terms -> update ->
-// per-solve reduction -> [DIIS push] -> k_control -> commit -> k_active_swap),
-// so it can be captured once as a CUDA graph and replayed.  Converged solves stop
-// being updated (their CTAs return at once) while the others continue.
+// one iteration is a fixed sequence of launches (residual terms -> update -> k_tail ->
+// [DIIS extrapolation]), so it can be captured once as a CUDA graph and replayed.
+// Converged solves stop being updated (their CTAs return at once) while the others continue.
 // ----------------------------------------------------------------------------
 // Pulay system [B 1; 1 0][c; l] = [0; 1] over nvec vectors, B scaled by its max
-// diagonal; Gaussian elimination with partial pivoting.  Returns false if singular.
-__device__ bool pulay_device(const double *B, int nvec, double *c)
+// diagonal; Gaussian elimination with partial pivoting, one lane per row (nvec + 1 <= 17), the
+// matrix in shared memory.  Returns false if singular (the same in every lane).
+__device__ bool pulay_warp(const double *B, int nvec, double *c, double (*A)[kMaxDiis + 2])
 {
-    constexpr int N = kMaxDiis + 1;
-    double A[N][N + 1];
-    const int n = nvec + 1;
-    double scale = 0.0;
-    for (int j = 0; j < nvec; j++) scale = fmax(scale, B[j * kMaxDiis + j]);
+    const int lane = threadIdx.x & 31, n = nvec + 1;
+    double scale = lane < nvec ? B[lane * kMaxDiis + lane] : 0.0;
+    scale = fmax(0.0, scale);
+    for (int o = 16; o > 0; o >>= 1) scale = fmax(scale, __shfl_xor_sync(0xffffffffu, scale, o));
     if (!(scale > 0.0) || !isfinite(scale)) return false;
-    for (int j = 0; j < n; j++)
-        for (int k = 0; k <= n; k++) A[j][k] = 0.0;
-    for (int j = 0; j < nvec; j++) {
-        for (int k = 0; k < nvec; k++) A[j][k] = B[j * kMaxDiis + k] / scale;
-        A[j][nvec] = 1.0;
-        A[nvec][j] = 1.0;
-    }
-    A[nvec][n] = 1.0;
-    for (int k = 0; k < n; k++) {
-        int piv = k;
-        for (int i = k + 1; i < n; i++)
-            if (fabs(A[i][k]) > fabs(A[piv][k])) piv = i;
-        if (fabs(A[piv][k]) < 1e-14) return false;
-        if (piv != k)
-            for (int j = 0; j <= n; j++) {
-                double tmp = A[k][j];
-                A[k][j] = A[piv][j];
-                A[piv][j] = tmp;
-            }
-        for (int i = k + 1; i < n; i++) {
-            const double f = A[i][k] / A[k][k];
-            for (int j = k; j <= n; j++) A[i][j] -= f * A[k][j];
+    if (lane < n)
+        for (int k = 0; k <= n; k++) {
+            double x = 0.0;
+            if (lane < nvec) x = k < nvec ? B[lane * kMaxDiis + k] / scale : k == nvec ? 1.0 : 0.0;
+            else x = k < nvec ? 1.0 : k == n ? 1.0 : 0.0;
+            A[lane][k] = x;
         }
+    __syncwarp();
+    for (int k = 0; k < n; k++) {
+        double best = lane >= k && lane < n ? fabs(A[lane][k]) : -1.0;
+        int piv = lane;
+        for (int o = 16; o > 0; o >>= 1) {   // the first row of the largest entry
+            const double x = __shfl_xor_sync(0xffffffffu, best, o);
+            const int r = __shfl_xor_sync(0xffffffffu, piv, o);
+            if (x > best || (x == best && r < piv)) {
+                best = x;
+                piv = r;
+            }
+        }
+        if (best < 1e-14) return false;
+        if (piv != k && lane <= n) {
+            const double x = A[k][lane];
+            A[k][lane] = A[piv][lane];
+            A[piv][lane] = x;
+        }
+        __syncwarp();
+        if (lane > k && lane < n) {
+            const double f = A[lane][k] / A[k][k];
+            for (int j = k; j <= n; j++) A[lane][j] -= f * A[k][j];
+        }
+        __syncwarp();
     }
-    for (int k = n - 1; k >= 0; k--) {
-        double x = A[k][n];
-        for (int j = k + 1; j < n; j++) x -= A[k][j] * A[j][n];
-        A[k][n] = x / A[k][k];
+    bool ok = true;
+    if (lane == 0) {
+        for (int k = n - 1; k >= 0; k--) {
+            double x = A[k][n];
+            for (int j = k + 1; j < n; j++) x -= A[k][j] * A[j][n];
+            A[k][n] = x / A[k][k];
+        }
+        for (int j = 0; j < nvec; j++) ok = ok && isfinite(A[j][n]);
+        if (ok)
+            for (int j = 0; j < nvec; j++) c[j] = A[j][n];
     }
-    for (int j = 0; j < nvec; j++) {
-        if (!isfinite(A[j][n])) return false;
-        c[j] = A[j][n];
-    }
-    return true;
+    return __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
 }
 
-// One thread per solve.  init = 1: record the start energy and decide whether to iterate.
-__global__ void k_control(int nsolves, const double *__restrict__ red, const double *__restrict__ brow,
-                          IterState *__restrict__ st, double *__restrict__ Bm, double *__restrict__ coef,
-                          double *__restrict__ rec_e, double *__restrict__ rec_dt, int max_rec,
-                          const uint8_t *__restrict__ active, uint8_t *__restrict__ active_next, double tol,
-                          int max_iter, int ndiis, int init)
+// The end of an iteration, one CTA per solve: the energy and max|dT| from the chunk partials in
+// chunk order, the new row of the Pulay matrix from the dot-product partials, the convergence
+// decision and the Pulay coefficients.  init = 1: the start amplitudes' energy, recorded, and
+// whether to iterate.  applied = the solves this iteration updated (k_diis_extrap2 runs on
+// those); active = the ones that go on, *count their number.
+// One launch with the elimination spread over a warp in shared memory, where the reduction, the
+// row reduction, a one-thread-per-solve control (its 17 x 18 matrix in local memory) and the
+// swap of the active flags were four launches: 22 -> 10.5 us an iteration on one N=54 solve,
+// 58 -> 26 us on four of N=114.
+__global__ void __launch_bounds__(256)
+    k_tail(const int *__restrict__ chunk_begin, const double *__restrict__ part_e, const double *__restrict__ part_dt,
+           const double *__restrict__ part_r, const double *__restrict__ dpart, IterState *__restrict__ st,
+           double *__restrict__ Bm, double *__restrict__ coef, double *__restrict__ rec_e,
+           double *__restrict__ rec_dt, int max_rec, uint8_t *active, uint8_t *__restrict__ applied,
+           int *__restrict__ count, double tol, int max_iter, int ndiis, int init)
 {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= nsolves) return;
-    IterState S = st[s];
+    const int s = blockIdx.x;
     if (!init && !active[s]) {
-        active_next[s] = 0;
+        if (threadIdx.x == 0) applied[s] = 0;
         return;
     }
-    const double e = red[3 * s], dt = red[3 * s + 1];
+    __shared__ double sd[8][kMaxDiis], brow[kMaxDiis], A[kMaxDiis + 1][kMaxDiis + 2];
+    IterState S = st[s];
+    const int c0 = chunk_begin[s], c1 = chunk_begin[s + 1];
+    // this iteration pushed slot (niter - 1) % ndiis and has nvec = min(niter, ndiis) vectors
+    const int nvec = !init && ndiis > 0 ? min(S.niter, ndiis) : 0, slot = nvec > 0 ? (S.niter - 1) % ndiis : 0;
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    if (nvec > 0) {
+        double acc[kMaxDiis];
+#pragma unroll
+        for (int j = 0; j < kMaxDiis; j++) acc[j] = 0.0;
+        for (int c = c0 + threadIdx.x; c < c1; c += 256) {
+#pragma unroll
+            for (int j = 0; j < kMaxDiis; j++)
+                if (j < nvec) acc[j] += dpart[(int64_t)c * kMaxDiis + j];
+        }
+#pragma unroll
+        for (int j = 0; j < kMaxDiis; j++)
+            if (j < nvec) {
+                double v = acc[j];
+                for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+                if (l == 0) sd[w][j] = v;
+            }
+        __syncthreads();
+        for (int j = w; j < nvec; j += 8) {
+            double v = l < 8 ? sd[l][j] : 0.0;
+            for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
+            if (l == 0) brow[j] = v;
+        }
+    }
+    double e = 0.0, dt = 0.0, mr = 0.0;
+    for (int c = c0 + threadIdx.x; c < c1; c += 256) {
+        e += part_e[c];
+        dt = fmax(dt, part_dt[c]);
+        mr = fmax(mr, part_r[c]);
+    }
+    block_reduce3<256>(e, dt, mr);
+    __syncthreads();   // brow
+    if (w != 0) return;
+    e = __shfl_sync(0xffffffffu, e, 0);
+    dt = __shfl_sync(0xffffffffu, dt, 0);
     if (!init) S.niter += 1;
     const int r = S.niter - 1;
-    if (r >= 0 && r < max_rec) {
+    if (l == 0 && r >= 0 && r < max_rec) {
         rec_e[(int64_t)s * max_rec + r] = e;
         rec_dt[(int64_t)s * max_rec + r] = dt;
     }
@@ -1666,59 +1721,22 @@ __global__ void k_control(int nsolves, const double *__restrict__ red, const dou
     const bool finite = isfinite(e) && isfinite(dt);
     const bool go = finite && dt >= tol && S.niter < max_iter;
     if (!finite) S.status = 3;
-    if (!init && ndiis > 0) {
-        // this iteration pushed slot (niter_before - 1) % ndiis with nvec = min(niter_before, ndiis)
-        const int nb = S.niter - 1;
-        const int slot = (nb - 1) % ndiis, nvec = min(nb, ndiis);
+    if (nvec > 0) {
         double *B = Bm + (int64_t)s * kMaxDiis * kMaxDiis;
-        for (int j = 0; j < nvec; j++) B[slot * kMaxDiis + j] = B[j * kMaxDiis + slot] = brow[s * kMaxDiis + j];
         double *c = coef + s * kMaxDiis;
-        for (int j = 0; j < kMaxDiis; j++) c[j] = 0.0;
-        if (!go || nvec < 2 || !pulay_device(B, nvec, c)) {
-            for (int j = 0; j < kMaxDiis; j++) c[j] = 0.0;
-            c[slot] = 1.0;
-        }
+        if (l < nvec) B[slot * kMaxDiis + l] = B[l * kMaxDiis + slot] = brow[l];
+        if (l < kMaxDiis) c[l] = 0.0;
+        __syncwarp();
+        const bool solved = go && nvec >= 2 && pulay_warp(B, nvec, c, A);
+        if (!solved && l == 0) c[slot] = 1.0;
     }
     if (!go && S.status == 0) S.status = (finite && dt >= tol) ? 2 : 1;
-    active_next[s] = go ? 1 : 0;
-    st[s] = S;
-}
-
-// active <- active_next; count of active solves for the host's poll.
-__global__ void k_active_swap(int nsolves, uint8_t *__restrict__ active, const uint8_t *__restrict__ active_next,
-                              int *__restrict__ count)
-{
-    int c = 0;
-    for (int s = threadIdx.x; s < nsolves; s += blockDim.x) {
-        const uint8_t a = active_next[s];
-        active[s] = a;
-        c += a;
-    }
-    for (int o = 16; o > 0; o >>= 1) c += __shfl_down_sync(0xffffffffu, c, o);
-    __shared__ int w[32];
-    if ((threadIdx.x & 31) == 0) w[threadIdx.x >> 5] = c;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        int tot = 0;
-        for (int k = 0; k < (int)(blockDim.x >> 5); k++) tot += w[k];
-        *count = tot;
-    }
-}
-
-__global__ void k_diis_rows2(const int *__restrict__ chunk_begin, const IterState *__restrict__ st, int ndiis,
-                             const double *__restrict__ part, double *__restrict__ brow,
-                             const uint8_t *__restrict__ active)
-{
-    const int s = blockIdx.x;
-    if (!active[s]) return;
-    const int nvec = min(st[s].niter, ndiis);
-    const int c0 = chunk_begin[s], c1 = chunk_begin[s + 1];
-    for (int jv = 0; jv < nvec; jv++) {
-        double acc = 0.0;
-        for (int c = c0 + threadIdx.x; c < c1; c += blockDim.x) acc += part[(int64_t)c * kMaxDiis + jv];
-        acc = block_sum<256>(acc);
-        if (threadIdx.x == 0) brow[s * kMaxDiis + jv] = acc;
-        __syncthreads();
+    if (l == 0) {
+        st[s] = S;
+        applied[s] = init ? 0 : 1;
+        active[s] = go ? 1 : 0;
+        if (init) atomicAdd(count, go ? 1 : 0);
+        else if (!go) atomicSub(count, 1);
     }
 }
 
@@ -1726,10 +1744,10 @@ __global__ void k_diis_rows2(const int *__restrict__ chunk_begin, const IterStat
 __global__ void k_diis_extrap2(const HChunkDev *__restrict__ chunks, const SolveDev *__restrict__ solves,
                                int64_t namp, const double *__restrict__ hist_t, const double *__restrict__ coef,
                                int ndiis, const int32_t *__restrict__ mirror, double *__restrict__ t,
-                               const uint8_t *__restrict__ active)
+                               const uint8_t *__restrict__ applied)
 {
     const HChunkDev ch = chunks[blockIdx.x];
-    if (!active[ch.solve]) return;
+    if (!applied[ch.solve]) return;
     const SolveDev s = solves[ch.solve];
     const int loc = ch.start + threadIdx.x;
     if (loc >= ch.end) return;
@@ -1757,35 +1775,33 @@ void launch_refresh(const DevBatch &d, cudaStream_t st)
     launch_ladder3(d, d.tiles, d.ntile_cls, d.t_ref, 0, 1, 0, d.g_ref, st);
 }
 
-void launch_control(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
-                    cudaStream_t st)
+void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
+                 cudaStream_t st)
 {
-    k_control<<<(d.nsolves + 127) / 128, 128, 0, st>>>(d.nsolves, d.red, c.brow, c.state, c.Bm, c.coef, c.rec_e,
-                                                       c.rec_dt, c.max_rec, d.active, c.active_next, tol,
-                                                       max_iter, ndiis, init);
+    if (init) cudaMemsetAsync(c.count, 0, sizeof(int), st);
+    k_tail<<<d.nsolves, 256, 0, st>>>(init ? d.chunk_begin : d.hchunk_begin, d.part_e, d.part_dt, d.part_r, c.part,
+                                      c.state, c.Bm, c.coef, c.rec_e, c.rec_dt, c.max_rec, d.active, c.applied,
+                                      c.count, tol, max_iter, ndiis, init);
 }
 
-void launch_active_swap(const DevBatch &d, const CtlBuffers &c, cudaStream_t st)
-{
-    k_active_swap<<<1, 1024, 0, st>>>(d.nsolves, d.active, c.active_next, c.count);
-}
-
-// One iteration: residual + update, reduction, [DIIS], control, swap.  Returns launches.
+// One iteration: residual + update, control, [DIIS extrapolation].  Returns launches.
 int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f, double tol, int max_iter,
                      int ndiis, cudaStream_t st, KernelTimer *kt)
 {
     // the DIIS push (history slot and e . e_j partials) happens inside k_update
     int n = launch_residual(d, f, 0, nullptr, st, kt, &c, ndiis);
+    if (kt) kt->begin(KID_TAIL, st);
+    launch_tail(d, c, tol, max_iter, ndiis, 0, st);
+    if (kt) kt->end(st);
+    n++;
     if (ndiis > 0) {
-        k_diis_rows2<<<d.nsolves, 256, 0, st>>>(d.hchunk_begin, c.state, ndiis, c.part, c.brow, d.active);
-        n += 1;
-    }
-    launch_control(d, c, tol, max_iter, ndiis, 0, st);
-    if (ndiis > 0)
+        if (kt) kt->begin(KID_EXTRAP, st);
         k_diis_extrap2<<<d.nhchunks, kChunk, 0, st>>>(d.hchunks, d.solves, d.namp, c.hist_t, c.coef, ndiis, d.mirror,
-                                                     d.t, d.active);
-    launch_active_swap(d, c, st);
-    return n + (ndiis > 0 ? 3 : 2);
+                                                     d.t, c.applied);
+        if (kt) kt->end(st);
+        n++;
+    }
+    return n;
 }
 
 // ----------------------------------------------------------------------------
@@ -1980,7 +1996,7 @@ void launch_to_aaaa(const DevBatch &d, cudaStream_t st)
 const char *kKernelNames[KID_COUNT] = {"k_mp2",      "k_energy",   "k_ladder_hh", "k_ladder",
                                       "k_mosaic_blk", "k_mosaic_sum", "k_drpa_sums", "k_update",
                                       "k_reduce_solves", "k_rings",
-                                      "k_ladder_tc", "k_ring_stage"};
+                                      "k_ladder_tc", "k_ring_stage", "k_tail", "k_diis_extrap2"};
 
 int tune_rings(DevBatch &d, cudaStream_t st)
 {
@@ -2169,10 +2185,12 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
     k_update<<<d.nhchunks, kChunk, 0, st>>>(A);
     kt->end(st);
     n++;
-    kt->begin(KID_REDUCE, st);
-    k_reduce_solves<<<d.nsolves, 256, 0, st>>>(d.hchunk_begin, d.part_e, d.part_dt, d.part_r, d.red);
-    kt->end(st);
-    n++;
+    if (mode != 0) {   // in an iteration k_tail reduces the partials
+        kt->begin(KID_REDUCE, st);
+        k_reduce_solves<<<d.nsolves, 256, 0, st>>>(d.hchunk_begin, d.part_e, d.part_dt, d.part_r, d.red);
+        kt->end(st);
+        n++;
+    }
     return n;
 }
 
