@@ -480,6 +480,56 @@ struct PhaseTrace {
     }
 };
 
+// The FP64 ladder's tiles (ladder.cu), the longest first so that the last wave is short.  A
+// block of up to 4 rows is one tile (or one per 256 columns); a larger one is cut into row tiles
+// of at most 16, and those into column tiles of so many passes that the batch makes at least
+// about four tiles per SM -- every column tile forms the block's H again, so a large batch keeps
+// a row tile whole.
+std::vector<LadderTile64> ladder_tiles(const std::vector<BlockDev> &blocks, int &max_rows)
+{
+    constexpr int kSms = 148;
+    int64_t passes = 0;
+    auto row_tiles = [](int rows) { return (rows + kLadderMmaRows - 1) / kLadderMmaRows; };
+    for (const auto &B : blocks) {
+        const int rows = B.nd + B.dg, h = B.nvd + B.sd;
+        max_rows = std::max(max_rows, rows);
+        if (rows <= kLadderFmaRows) continue;
+        const int nt = row_tiles(rows), pc = ladder_pass_cols((rows + nt - 1) / nt);
+        passes += (int64_t)nt * ((h + rows + pc - 1) / pc);
+    }
+    const int per_tile = (int)std::max<int64_t>(1, std::min<int64_t>(passes / (4 * kSms), 1 << 16));
+    std::vector<LadderTile64> tiles;
+    std::vector<std::pair<float, int>> cost;
+    for (size_t k = 0; k < blocks.size(); k++) {
+        const BlockDev &B = blocks[k];
+        const int rows = B.nd + B.dg, h = B.nvd + B.sd;
+        if (rows <= kLadderFmaRows) {
+            const int w = kLadderFmaCols - rows;
+            for (int a0 = 0; a0 < h; a0 += w) {
+                const int a1 = std::min(h, a0 + w);
+                cost.emplace_back((float)h * ((rows + a1 - a0 + 31) / 32) * std::max(5, 1 + rows), (int)tiles.size());
+                tiles.push_back(LadderTile64{(int)k, a0, a1, 0, (int16_t)rows});
+            }
+            continue;
+        }
+        const int nt = row_tiles(rows), np = (rows + nt - 1) / nt, pc = ladder_pass_cols(np);
+        const int w = per_tile * pc - rows;
+        for (int p0 = 0; p0 < rows; p0 += np)
+            for (int a0 = 0; a0 < h; a0 += w) {
+                const int a1 = std::min(h, a0 + w), n = std::min(np, rows - p0);
+                cost.emplace_back((float)h * ((rows + a1 - a0 + 31) / 32) * (np <= 8 ? 8 : 16), (int)tiles.size());
+                tiles.push_back(LadderTile64{(int)k, a0, a1, (int16_t)p0, (int16_t)n});
+            }
+    }
+    std::sort(cost.begin(), cost.end(), [](const auto &x, const auto &y) {
+        return x.first != y.first ? x.first > y.first : x.second < y.second;
+    });
+    std::vector<LadderTile64> out;
+    out.reserve(tiles.size());
+    for (const auto &c : cost) out.push_back(tiles[c.second]);
+    return out;
+}
+
 int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch> &out)
 {
     PhaseTrace trace;
@@ -517,7 +567,7 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
 
     std::vector<SolveDev> solves(n);
     std::vector<BlockDev> blocks;
-    std::vector<LadderTile> tiles, htiles, tc16, tc32, tc64;
+    std::vector<LadderTile> tc16, tc32, tc64;
     std::vector<TcTileDev> tcx16, tcx32, tcx64;   // beside tc16/32/64: FP16 operand offsets
     std::vector<WSlabDev> wslabs;
     std::vector<DTileDev> dtiles;
@@ -550,9 +600,8 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     eigen.clear();
     std::vector<int> chunk_begin(n + 1, 0);
     std::vector<double> vtab;
-    std::vector<int64_t> hh0;
     std::vector<RingPairDev> rpairs, spairs;
-    int64_t amp0 = 0, pos0 = 0, ph0 = 0, hhoff = 0, phr0 = 0, mrows = 0, mcols = 0;
+    int64_t amp0 = 0, pos0 = 0, ph0 = 0, phr0 = 0, mrows = 0, mcols = 0;
     std::vector<int> s_t0(n);   // first mosaic target of each solve
     int orb0 = 0, vtab0 = 0, jvv0 = 0, joo0 = 0, max_o = 0, max_v = 0, max_occ = 0;
     // offsets of each solve in the large concatenated arrays (filled in parallel below)
@@ -602,28 +651,9 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
             mcols += B.v;
             int bi = (int)blocks.size();
             blocks.push_back(bd);
-            hh0.push_back(hhoff);
-            hhoff += (int64_t)B.o * B.o;
             max_o = std::max(max_o, B.o);
             max_v = std::max(max_v, B.v);
-            // FP64 ladder tiles cover the rows up to the diagonal pair (oc = nd + dg); k_ladder3
-            // writes each mirror row from its pair (i,j) with the pair symmetry.  Row tiles of 32
-            // pairs, the last one the remainder rounded up to 8 (8, 16, 24 or 32): at most 7
-            // padded rows per block; columns in tiles of 128 (4 warps x 32)
-            // Blocks with at most kPairedRows such rows run paired tiles (pad 4): each 8-wide
-            // fragment holds the rows and their partner-column images, over the columns
-            // a <= pcol a (mode 0) and the pairs q <= q' (mode 1).
             const int oc = B.nd + B.dg;
-            auto row_tile = [&](int p0) { return std::min(32, (oc - p0 + 7) & ~7); };
-            if (oc <= kPairedRows) {
-                for (int a0 = 0; a0 < B.nvd + B.sd; a0 += 128) tiles.push_back(LadderTile{bi, a0, 0, 4});
-                htiles.push_back(LadderTile{bi, 0, 0, 4});
-            } else {
-                for (int a0 = 0; a0 < B.v; a0 += 128)
-                    for (int p0 = 0; p0 < oc; p0 += 32) tiles.push_back(LadderTile{bi, a0, p0, row_tile(p0)});
-                for (int q0 = 0; q0 < B.o; q0 += 128)
-                    for (int p0 = 0; p0 < oc; p0 += 32) htiles.push_back(LadderTile{bi, q0, p0, row_tile(p0)});
-            }
             // tensor-core tiles: 128 virtuals x (16, 32 or 64) rows over the rows i <= j (the
             // update reads G there only); their FP16 operands: one Coulomb slab per 128
             // virtuals, one d tile per row tile, each over all K chunks
@@ -717,41 +747,12 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     DevBatch &d = b->d;
     d.nsolves = n;
     d.nblocks = (int)blocks.size();
-    // ladder tiles by row-tile class (stable: block order within a class)
-    auto by_class = [](std::vector<LadderTile> &v, int *cnt) {
-        std::vector<LadderTile> out;
-        out.reserve(v.size());
-        for (int c = 0; c < kLadderClasses; c++) {
-            cnt[c] = 0;
-            for (const auto &x : v)
-                if (x.pad == (c == 0 ? 4 : 8 * c)) {
-                    out.push_back(x);
-                    cnt[c]++;
-                }
-        }
-        v.swap(out);
-    };
-    const size_t ntl = tiles.size(), nhtl = htiles.size();
-    by_class(tiles, d.ntile_cls);
-    by_class(htiles, d.nhtile_cls);
-    if (tiles.size() != ntl || htiles.size() != nhtl) return fail(UEGCCD_ERR_UNSUPPORTED, "ladder row tile outside the 4/8/16/24/32 classes");
-    d.ntiles = (int)tiles.size();
-    d.nhtiles = (int)htiles.size();
-    // the second tile order the launch-shape tuner may pick: within each class, the tiles of
-    // the blocks with the most virtuals (the longest c loops) first
-    auto longest_first = [&](const std::vector<LadderTile> &v, const int *cnt) {
-        std::vector<LadderTile> out(v);
-        size_t off = 0;
-        for (int c = 0; c < kLadderClasses; c++) {
-            std::stable_sort(out.begin() + off, out.begin() + off + cnt[c], [&](const LadderTile &x, const LadderTile &y) {
-                return blocks[x.blk].v > blocks[y.blk].v;
-            });
-            off += cnt[c];
-        }
-        return out;
-    };
-    const std::vector<LadderTile> tiles_lpt = longest_first(tiles, d.ntile_cls),
-                                  htiles_lpt = longest_first(htiles, d.nhtile_cls);
+    int q2m = 0;
+    for (const auto &P : b->plans) q2m = std::max(q2m, P.q2max);
+    d.q2max = q2m;
+    int max_rows = 0;
+    const std::vector<LadderTile64> ltiles = ladder_tiles(blocks, max_rows);
+    d.nltiles = (int)ltiles.size();
     d.ntc16 = (int)tc16.size();
     d.ntc32 = (int)tc32.size();
     d.ntc64 = (int)tc64.size();
@@ -772,16 +773,12 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     d.nhchunks = (int)hchunks.size();
     d.nrchunks = (int)rchunks.size();
     d.ntargets = (int)targets.size();
-    d.max_o = max_o;
     d.max_v = max_v;
-    if (ladder_smem_bytes(max_v, 32) > 227 * 1024) return fail(UEGCCD_ERR_UNSUPPORTED, "ladder block exceeds shared memory");
-    set_ladder_smem_limit(max_v);
-    {   // the |q|^2 table the mosaic kernel stages: the batch's largest (tables beyond 1024
-        // entries stay in global memory)
-        int q2m = 0;
-        for (const auto &P : b->plans) q2m = std::max(q2m, P.q2max);
-        d.mosaic_vt = std::min(q2m + 1, kVtabSmemEntries);
-    }
+    d.ladder_smem = ladder_smem_bytes(q2m, max_rows);
+    set_ladder_smem_limit(d.ladder_smem);
+    // the |q|^2 table the mosaic kernel stages: the batch's largest (tables beyond 1024 entries
+    // stay in global memory)
+    d.mosaic_vt = std::min(q2m + 1, kVtabSmemEntries);
     d.mosaic_smem = mosaic_smem_bytes(max_v, max_o, d.mosaic_vt);
     if (d.mosaic_smem > 227 * 1024) return fail(UEGCCD_ERR_UNSUPPORTED, "mosaic block exceeds shared memory");
     set_mosaic_smem_limit(d.mosaic_smem);
@@ -837,10 +834,7 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     trace.mark("host-tables");
     if ((rc = b->upload(d.solves, solves))) return rc;
     if ((rc = b->upload(d.blocks, blocks))) return rc;
-    if ((rc = b->upload(d.tiles, tiles))) return rc;
-    if ((rc = b->upload(d.htiles, htiles))) return rc;
-    if ((rc = b->upload(d.tiles_lpt, tiles_lpt))) return rc;
-    if ((rc = b->upload(d.htiles_lpt, htiles_lpt))) return rc;
+    if ((rc = b->upload(d.ltiles, ltiles))) return rc;
     if ((rc = b->upload(d.tctiles, tct))) return rc;
     if ((rc = b->upload(d.tcx, tcx))) return rc;
     if ((rc = b->upload(d.wslabs, wslabs))) return rc;
@@ -871,7 +865,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->upload(d.eigen, eigen))) return rc;
     if ((rc = b->upload(d.vtab, vtab))) return rc;
     b->vtab_base = vtab;
-    if ((rc = b->upload(d.hh0, hh0))) return rc;
     if ((rc = b->upload(d.rpairs, rpairs))) return rc;
     if ((rc = b->upload(d.spairs, spairs))) return rc;
     if ((rc = b->upload(d.ph_i, ph_i))) return rc;
@@ -889,7 +882,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->alloc(d.g, amp0))) return rc;
     if ((rc = b->alloc(d.jvv, jvv0))) return rc;
     if ((rc = b->alloc(d.joo, joo0))) return rc;
-    if ((rc = b->alloc(d.hh, hhoff))) return rc;
     const size_t npart = std::max(chunks.size(), hchunks.size());   // per full or half chunk
     if ((rc = b->alloc(d.part_e, npart))) return rc;
     if ((rc = b->alloc(d.part_dt, npart))) return rc;
@@ -1202,12 +1194,11 @@ int capture_iteration(UegccdBatch &b, const TermFlags &f, double tol, int max_it
     return 0;
 }
 
-// The launch shapes of a batch (k_rings CTA sizes, k_ring_stage CTA size, ladder tile
-// order): measured once per batch shape in this process (the shape: pair count and shared
-// memory of every ring class, ladder tiles per class, largest block), on the first CCD
-// solve, before the iteration graph is captured.
+// The launch shapes of a batch (k_rings CTA sizes, k_ring_stage CTA size): measured once per
+// batch shape in this process (the shape: pair count and shared memory of every ring class), on
+// the first CCD solve, before the iteration graph is captured.
 std::mutex g_tune_mu;
-std::map<std::vector<int64_t>, std::array<int, kRingClasses + 3>> g_ring_tuning;
+std::map<std::vector<int64_t>, std::array<int, kRingClasses + 1>> g_ring_tuning;
 
 int tune_batch_rings(UegccdBatch &b)
 {
@@ -1217,30 +1208,21 @@ int tune_batch_rings(UegccdBatch &b)
         key.push_back(d.nring[c]);
         key.push_back((int64_t)d.ring_smem[c]);
     }
-    for (int c = 0; c < kLadderClasses; c++) {
-        key.push_back(d.ntile_cls[c]);
-        key.push_back(d.nhtile_cls[c]);
-    }
-    key.push_back(d.max_v);
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
         auto it = g_ring_tuning.find(key);
         if (it != g_ring_tuning.end()) {
             for (int c = 0; c < kRingClasses; c++) d.ring_threads[c] = it->second[c];
             d.stage_threads = it->second[kRingClasses];
-            d.ladder_sched = it->second[kRingClasses + 1];
-            d.hh_kc = it->second[kRingClasses + 2];
             b.rings_tuned = true;
             return 0;
         }
     }
     const int e = tune_rings(d, b.stream);
     if (e != 0) return fail(UEGCCD_ERR_CUDA, std::string("launch-shape tuning: ") + cudaGetErrorString((cudaError_t)e));
-    std::array<int, kRingClasses + 3> th;
+    std::array<int, kRingClasses + 1> th;
     for (int c = 0; c < kRingClasses; c++) th[c] = d.ring_threads[c];
     th[kRingClasses] = d.stage_threads;
-    th[kRingClasses + 1] = d.ladder_sched;
-    th[kRingClasses + 2] = d.hh_kc;
     std::lock_guard<std::mutex> lock(g_tune_mu);
     g_ring_tuning[key] = th;
     b.rings_tuned = true;
@@ -2064,8 +2046,8 @@ int32_t uegccd_batch_launch_shapes(UegccdBatch *b, int32_t *vals, int32_t max)
     int32_t v[kRingClasses + 3];
     for (int c = 0; c < kRingClasses; c++) v[c] = b->d.ring_threads[c];
     v[kRingClasses] = b->d.stage_threads;
-    v[kRingClasses + 1] = b->d.ladder_sched;
-    v[kRingClasses + 2] = b->d.hh_kc;
+    v[kRingClasses + 1] = 1;    // ladder tiles: always the longest first
+    v[kRingClasses + 2] = 32;   // virtuals per staged chunk of the ladder
     const int n = std::min<int>(max, kRingClasses + 3);
     for (int k = 0; k < n; k++) vals[k] = v[k];
     return n;
@@ -2109,8 +2091,7 @@ int uegccd_footprint(const UegccdSystem *sys, int32_t ndiis, int32_t mixed, int6
     std::string msg = build_solve_plan(h, P);
     if (!msg.empty()) return fail(UEGCCD_ERR_ARG, msg);
     const int64_t A = P.namp, O = P.O, V = P.V, M = P.M;
-    int64_t hh = 0, nblk = (int64_t)P.blocks.size();
-    for (const auto &B : P.blocks) hh += (int64_t)B.o * B.o;
+    const int64_t nblk = (int64_t)P.blocks.size();
     int64_t b = 0;
     int64_t sum_ov = 0;
     for (const auto &B : P.blocks) sum_ov += B.o + B.v;
@@ -2129,7 +2110,7 @@ int uegccd_footprint(const UegccdSystem *sys, int32_t ndiis, int32_t mixed, int6
     }
     b += xy * 8 * 2 + O * V * 4 * 2;                 // xy, rx; ph_a, ph_b
     b += O * V * O * 4 * 2;                          // ring gather indices
-    b += hh * 8 + nblk * (sizeof(BlockDev) + 8) + M * (16 + 8) + (P.q2max + 1) * 8;
+    b += nblk * (sizeof(BlockDev) + sizeof(LadderTile64)) + M * (16 + 8) + (P.q2max + 1) * 8;
     b += A * (8 + 4) * (int64_t)std::max(0, (int)ndiis);  // DIIS history (t' FP64, e FP32)
     if (mixed) {
         b += A * 8 * 2;                              // t_ref, g_ref

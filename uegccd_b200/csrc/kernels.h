@@ -13,22 +13,21 @@ constexpr int kVtabSmemEntries = 1024;   // |q|^2 table entries a kernel stages 
 
 struct DevBatch {
     int nsolves = 0, nblocks = 0, ntiles = 0, nchunks = 0, nrchunks = 0, ntargets = 0;
-    int max_o = 0;      // largest o_K
     int max_v = 0;      // largest v_K
     // mosaics: block row and column sums, and per target the list of partials to add
     double *mpart = nullptr;
     int32_t *mt_start = nullptr, *mt_list = nullptr;
     size_t mosaic_smem = 0;
     int mosaic_vt = 0;  // |q|^2 table entries k_mosaic_blk stages: the batch's largest, at most kVtabSmemEntries
-    int ntile_cls[5] = {0, 0, 0, 0, 0};   // ladder tiles per class: paired 8, then 8, 16, 24, 32 pairs
-    int nhtile_cls[5] = {0, 0, 0, 0, 0};  // hole-hole intermediate tiles per class
+    // FP64 ladder tiles (ladder.cu), longest first
+    LadderTile64 *ltiles = nullptr;
+    int nltiles = 0;
+    int q2max = 0;      // largest |q|^2 of the solves' tables
+    size_t ladder_smem = 0;
     int max_occ = 0;    // largest NOcc
     int64_t namp = 0;
     SolveDev *solves = nullptr;
     BlockDev *blocks = nullptr;
-    LadderTile *tiles = nullptr;     // particle-particle (+hole-hole apply) tiles; pad = row tile NP (8/16/24/32)
-    LadderTile *htiles = nullptr;    // hole-hole intermediate tiles
-    int nhtiles = 0;
     ChunkDev *chunks = nullptr;      // amplitude chunks
     ChunkDev *rchunks = nullptr;     // ring-intermediate chunks over (i, x, l)
     int *chunk_begin = nullptr;      // nsolves+1: first chunk of each solve
@@ -57,8 +56,6 @@ struct DevBatch {
     int16_t *colpos = nullptr;
     double *dru = nullptr, *drs2 = nullptr;
     int *drdone = nullptr;
-    int64_t *hh0 = nullptr;          // per block: offset of H_K in hh
-    double *hh = nullptr;
     double *part_e = nullptr, *part_dt = nullptr, *part_r = nullptr;
     double *red = nullptr;           // 3 per solve: sum e, max dt, max |r|
     uint8_t *active = nullptr;       // per solve
@@ -100,24 +97,24 @@ struct DevBatch {
     size_t ring_smem[5] = {0, 0, 0, 0, 0};
     int ring_threads[4] = {32, 128, 256, 256};  // CTA size per k_rings class: defaults, then tune_rings
     int stage_threads = 128;                    // CTA size of k_ring_stage (tune_rings)
-    // ladder tiles in a second order: within each row-tile class the blocks with the most
-    // virtuals (the longest c loops) first; ladder_sched picks the order the launches use
-    LadderTile *tiles_lpt = nullptr, *htiles_lpt = nullptr;
-    int ladder_sched = 0;                       // 0: block order, 1: longest first (tune_rings)
-    int hh_kc = 64;                             // the hole-hole intermediate's column chunk: 64 or 32 (tune_rings)
 };
 // dynamic shared memory of k_rings_wide for NOcc = O and R rows of a group pair
 size_t rings_smem_bytes(int O, int R);
 // dynamic shared memory of k_mosaic_blk for blocks of at most max_v virtuals
 size_t mosaic_smem_bytes(int max_v, int max_o, int vt_n);
 void set_mosaic_smem_limit(size_t bytes);
-// dynamic shared memory of k_ladder3<np> for blocks of at most max_v virtuals
-// row-tile classes: paired 8 (blocks with at most kPairedRows rows i <= j, pad = 4 in
-// LadderTile), then 8, 16, 24 and 32 pairs
-constexpr int kLadderClasses = 5;
-constexpr int kPairedRows = 4;
-size_t ladder_smem_bytes(int max_v, int np);
-void set_ladder_smem_limit(int max_v);
+// FP64 ladders (ladder.cu): blocks with at most kLadderFmaRows rows i <= j take the FMA form,
+// larger ones the DMMA form in tiles of at most kLadderMmaRows rows
+constexpr int kLadderFmaRows = 4, kLadderMmaRows = 16;
+// the FMA form's columns a tile (pairs of H included); the DMMA form's columns a pass for tiles
+// of np rows
+constexpr int kLadderFmaCols = 256;
+constexpr int ladder_pass_cols(int np) { return np <= 8 ? 128 : 64; }
+// dynamic shared memory for |q|^2 tables up to q2max and blocks of at most max_rows rows i <= j
+size_t ladder_smem_bytes(int q2max, int max_rows);
+void set_ladder_smem_limit(size_t bytes);
+// G of the rows i <= j: the particle-particle ladder of t (do_pp), the hole-hole one (do_hh)
+void launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st);
 // dynamic shared memory of k_rings for NOcc = O and groups of n1 and n2 rows
 size_t rings_dmma_smem_bytes(int O, int n1, int n2, int q2max);
 // k_rings classes by padded pair size N1 + N2 (up to kRingClassRows), each with its
@@ -128,17 +125,15 @@ constexpr int kRingClassRows[kRingClasses] = {16, 32, 48, 1 << 30};
 constexpr size_t kRingSmemMax = 200 * 1024;
 void set_rings_smem_limit(int wide, size_t bytes);
 // Launch-shape autotuner, on the batch's current amplitudes: times k_rings of every pair
-// class with 32, 64, 128 and 256 threads per CTA (d.ring_threads), k_ring_stage with 64,
-// 128 and 256 (d.stage_threads), and the particle-particle ladder with its tiles in block
-// order and longest first (d.ladder_sched); keeps the fastest of each.  None of these
-// changes a sum's order: results are bitwise the same.  Not inside a stream capture.
-// Returns a cudaError_t value.
+// class with 32, 64, 128 and 256 threads per CTA (d.ring_threads) and k_ring_stage with 64,
+// 128 and 256 (d.stage_threads); keeps the fastest of each.  Neither changes a sum's order:
+// results are bitwise the same.  Not inside a stream capture.  Returns a cudaError_t value.
 int tune_rings(DevBatch &d, cudaStream_t st);
 
 constexpr int kDiisMax = 16;   // DIIS history capacity (k_update and k_diis_* use the same bound)
 
 // Live per-kernel timing with CUDA events on the launching stream (off unless enabled).
-enum KernelId { KID_MP2 = 0, KID_ENERGY, KID_HH_W, KID_LADDER, KID_MOSAIC_S, KID_MOSAIC_RED, KID_DRPA_SUMS,
+enum KernelId { KID_MP2 = 0, KID_ENERGY, KID_LADDER, KID_MOSAIC_S, KID_MOSAIC_RED, KID_DRPA_SUMS,
                 KID_UPDATE, KID_REDUCE, KID_RINGS, KID_LADDER_TC, KID_RING_STAGE,
                 KID_TAIL, KID_EXTRAP, KID_COUNT };
 struct KernelTimer {

@@ -188,30 +188,13 @@ __global__ void k_reduce_solves(const int *__restrict__ chunk_begin, const doubl
     if (threadIdx.x == 0) { out[3 * s + 0] = e; out[3 * s + 1] = ma; out[3 * s + 2] = mb; }
 }
 
-// ----------------------------------------------------------------------------
-// Ladders (GetG2Ladders, CCD.f90:588-686), per K block, written as
-//   G_K = t_K W_K + H_K t_K
-// particle-particle (CCD.f90:660-681): W_K[c][a] = v(c-a) over the block's virtuals;
-// hole-hole (CCD.f90:611-657): H_K[p][q] = v(i_p - k_q) + sum_c t_K[p][c] v(c - k_q),
-// p = (i,j), q = (k,l), after the pair-swap re-indexing t(kl,b) = t(lk,a).
-// k_ladder3 in mode 1 builds H_K; in mode 0 it writes G (overwriting, so it runs first).
-// Both run over the rows p = (i,j) with i <= j only: by the pair symmetry
-// t(ij,a) = t(ji,b) (T2abab(ij,ab) = T2abab(ji,ba)) the ladder G of the mirror row (j,i)
-// at column b = K - a equals that of (i,j) at a, and k_update reads G only on the rows
-// i <= j (it updates each mirror from its pair).  The reference forms both rows
-// (CCD.f90:617-681); the two agree to rounding.
-// ----------------------------------------------------------------------------
+// (The ladders, CCD.f90:588-686, are in ladder.cu; they write G first, before k_update adds
+// the other terms.)
 constexpr int kVtabSmem = kVtabSmemEntries;  // |q|^2 table entries staged in shared memory
 
-// Ladder tiles v3: FP64 tensor-core MMA (mma.sync m8n8k4 f64; tcgen05 has no f64
-// kind).  One warp owns a 32 (a) x NP (p) output tile as 4 x NP/8 fragments of 8x8;
-// a CTA of 4 warps covers 128 columns.  Each lane generates its own element of the
-// Coulomb fragment, A[a][c] = v(n_a - n_c), from the |q|^2 table, so the Coulomb
-// tile never passes through shared memory; the t fragment is read from L1/L2.
-//   mode 0: G^T[a][p] = sum_c v(a-c) t[p][c] (+ sum_q t[q][a] H[p][q] when do_hh)
-//   mode 1: H^T[q][p] = v(i_p - k_q) + sum_c v(k_q - c) t[p][c]   (columns = pairs)
-// Fragment layouts (PTX ISA, m8n8k4 .f64): A row = lane/4, col = lane%4;
-// B row (k) = lane%4, col = lane/4; C row = lane/4, cols 2*(lane%4) + {0,1}.
+// FP64 tensor-core MMA (tcgen05 has no f64 kind).  Fragment layouts (PTX ISA, m8n8k4 .f64):
+// A row = lane/4, col = lane%4; B row (k) = lane%4, col = lane/4; C row = lane/4, cols
+// 2*(lane%4) + {0,1}.
 __device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
 {
     asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -219,328 +202,11 @@ __device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, doubl
                  : "d"(a), "d"(b));
 }
 
-// The t rows of the tile pass through shared memory in chunks of kLadKC columns,
-// double-buffered with cp.async (8-byte copies: rows of odd length are not 16-byte
-// aligned); the block's virtual n-vectors and the |q|^2 table are staged once.
-constexpr int kLadKC = 32;            // c columns per chunk (mode 0)
-constexpr int kLadLd = kLadKC + 4;    // chunk row stride: = 4 mod 16 doubles, conflict-free fragments
-// The hole-hole intermediate (mode 1) has little work per column: wider chunks, fewer of the
-// round trips that bound it
-constexpr int kLadKC1 = 64;   // the default; the launch-shape tuner may pick 32 (DevBatch::hh_kc)
-
-__device__ __forceinline__ void cp_async8(double *dst, const double *src)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
-
-size_t ladder_smem_bytes(int max_v, int np)
-{
-    return sizeof(double) * (2 * (size_t)np * kLadLd + kVtabSmem) + sizeof(int) * (size_t)max_v;
-}
-size_t ladder1_smem_bytes(int max_v, int np, int kc)
-{
-    return sizeof(double) * (2 * (size_t)np * (kc + 4) + kVtabSmem) + sizeof(int) * (size_t)max_v;
-}
-
-// PAIRED (blocks with at most 4 rows i <= j, NP = 8): the fragment's 8 columns hold the
-// rows p and, after them, the same rows with the c columns swapped to their partners
-// (t[p][pcol c]).  The block's Coulomb kernel is invariant under (a, c) -> (pcol a, pcol c),
-// so the second half gives G[p][pcol a] from the same Coulomb fragment: the tile runs over
-// the columns a <= pcol a only, half the fragments.  The hole-hole intermediate pairs its
-// columns q with their mirror pairs q' the same way (v(k_q' - pcol c) = v(k_q - c)), and the
-// hole-hole apply reads H[p][q'] for the second half (t[q][pcol a] = t[q'][a]).
-template <int NP, bool KS, bool PAIRED, int KC = kLadKC>
-__device__ __forceinline__ void ladder3_tile(const LadderTile &T, const BlockDev &B, const SolveDev &s,
-                                             const int16_t *__restrict__ vir, const int16_t *__restrict__ pair_i,
-                                             const int *__restrict__ nvp, const double *__restrict__ vtab,
-                                             const double *__restrict__ t, const double *__restrict__ H, int mode,
-                                             int do_pp, int do_hh, double *__restrict__ out, const double *sv,
-                                             bool vsm, double *ts, const int *nvc)
-{
-    constexpr int NN = NP / 8;  // n fragments
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const int gid = lane >> 2, tig = lane & 3;
-    const int v = B.v, o = B.o;
-    const int orow = B.nd + B.dg;   // rows computed: pairs i < j and the diagonal pair
-    const int vc = B.nvd + B.sd;    // columns a <= pcol a
-    const int ncol = mode == 0 ? (PAIRED ? vc : v) : (PAIRED ? orow : o);
-    // partner column of a virtual column, mirror of a pair row (both involutions)
-    auto pcolv = [&](int c) { return c < B.nvd ? c + vc : c < vc ? c : c - vc; };
-    auto mirq = [&](int q) { return q < B.nd ? q + orow : q < orow ? q : q - orow; };
-    // hole-hole intermediate with at most 32 columns left: the 4 warps share the columns
-    // and split the c sum instead (each takes every 4th k step), then reduce
-    const bool ksplit = KS && ncol - T.a0 <= 32;
-    const int colbase = ksplit ? T.a0 : T.a0 + warp * 32;
-    const bool wact = colbase < ncol;  // warps past the last column only help with the copies
-    // packed n-vectors of this lane's A-fragment rows (one per m fragment)
-    int na[4];
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        int col = colbase + m * 8 + gid;
-        na[m] = 0;
-        if (col < ncol) na[m] = nvp[s.orb0 + (mode == 0 ? vir[B.vir0 + col] : pair_i[B.pair0 + col])];
-    }
-    double acc[4][NN][2];
-#pragma unroll
-    for (int m = 0; m < 4; m++)
-#pragma unroll
-        for (int n = 0; n < NN; n++) acc[m][n][0] = acc[m][n][1] = 0.0;
-    if (do_pp || mode == 1) {
-        constexpr int LD = KC + 4;
-        const int nchunk = (v + KC - 1) / KC;
-        const double *trow0 = t + B.t0;
-        // chunk j of the tile's t rows -> buffer b
-        auto issue = [&](int j, int b) {
-            double *dst = ts + b * (NP * LD);
-            const int c0 = j * KC;
-            for (int e = threadIdx.x; e < NP * KC; e += blockDim.x) {
-                const int r = e / KC, c = e - r * KC;
-                const int cc = c0 + c;
-                if (PAIRED) {
-                    // rows [0, orow): t[p][c]; rows [orow, 2 orow): t[p][pcol c]
-                    const bool second = r >= orow;
-                    const int p = second ? r - orow : r;
-                    if (r < 2 * orow && cc < v)
-                        cp_async8(dst + r * LD + c, trow0 + (int64_t)p * v + (second ? pcolv(cc) : cc));
-                    else dst[r * LD + c] = 0.0;
-                } else {
-                    const int p = T.p0 + r;
-                    if (p < orow && cc < v) cp_async8(dst + r * LD + c, trow0 + (int64_t)p * v + cc);
-                    else dst[r * LD + c] = 0.0;
-                }
-            }
-            cp_async_commit();
-        };
-        issue(0, 0);
-        for (int j = 0; j < nchunk; j++) {
-            if (j + 1 < nchunk) {
-                issue(j + 1, (j + 1) & 1);
-                cp_async_wait<1>();
-            } else {
-                cp_async_wait<0>();
-            }
-            __syncthreads();
-            if (wact) {
-                const double *tb = ts + (j & 1) * (NP * LD);
-                const int c0 = j * KC;
-                const int kstart = KS && ksplit ? 4 * warp : 0, kstep = KS && ksplit ? 16 : 4;
-#pragma unroll 2
-                for (int kk = kstart; kk < KC; kk += kstep) {
-                    const int c = min(c0 + kk + tig, v - 1);  // beyond v the t column is zero
-                    const int nc = nvc[c];
-                    double bf[NN];
-#pragma unroll
-                    for (int n = 0; n < NN; n++) bf[n] = tb[(n * 8 + gid) * LD + kk + tig];
-#pragma unroll
-                    for (int m = 0; m < 4; m++) {
-                        const int q2 = q2p(na[m], nc);
-                        const double af = vsm ? sv[q2] : __ldg(&vtab[s.vtab0 + q2]);
-#pragma unroll
-                        for (int n = 0; n < NN; n++) dmma_884(acc[m][n][0], acc[m][n][1], af, bf[n]);
-                    }
-                }
-            }
-            __syncthreads();
-        }
-    }
-    if (KS && ksplit) {
-        // acc of warps 2, 3 into warps 0, 1, then warp 1 into warp 0 (through the idle chunk buffer)
-        constexpr int kPart = 4 * NN * 2 * 32;
-        for (int round = 0; round < 2; round++) {
-            const int lo = round == 0 ? 2 : 1, nw = round == 0 ? 2 : 1;
-            if (warp >= lo && warp < lo + nw) {
-                double *dst = ts + (warp - lo) * kPart;
-#pragma unroll
-                for (int m = 0; m < 4; m++)
-#pragma unroll
-                    for (int n = 0; n < NN; n++)
-#pragma unroll
-                        for (int h = 0; h < 2; h++) dst[((m * NN + n) * 2 + h) * 32 + lane] = acc[m][n][h];
-            }
-            __syncthreads();
-            if (warp < nw) {
-                const double *src = ts + warp * kPart;
-#pragma unroll
-                for (int m = 0; m < 4; m++)
-#pragma unroll
-                    for (int n = 0; n < NN; n++)
-#pragma unroll
-                        for (int h = 0; h < 2; h++) acc[m][n][h] += src[((m * NN + n) * 2 + h) * 32 + lane];
-            }
-            __syncthreads();
-        }
-        if (warp != 0) return;
-    }
-    if (!wact) return;  // no barriers below
-    if (mode == 0 && do_hh) {
-        // acc[a][p] += sum_q t[q][a] H[p][q]
-        for (int q0 = 0; q0 < o; q0 += 4) {
-            const int q = q0 + tig;
-            const bool qok = q < o;
-            double bf[NN];
-#pragma unroll
-            for (int n = 0; n < NN; n++) {
-                if (PAIRED) {
-                    const int nn = n * 8 + gid;
-                    const bool second = nn >= orow;
-                    const int p = second ? nn - orow : nn;
-                    bf[n] = (qok && nn < 2 * orow) ? H[(int64_t)p * o + (second ? mirq(q) : q)] : 0.0;
-                } else {
-                    int p = T.p0 + n * 8 + gid;
-                    bf[n] = (qok && p < orow) ? H[(int64_t)p * o + q] : 0.0;
-                }
-            }
-#pragma unroll
-            for (int m = 0; m < 4; m++) {
-                int col = colbase + m * 8 + gid;
-                double af = (qok && col < v) ? __ldg(&t[B.t0 + (int64_t)q * v + col]) : 0.0;
-#pragma unroll
-                for (int n = 0; n < NN; n++) dmma_884(acc[m][n][0], acc[m][n][1], af, bf[n]);
-            }
-        }
-    }
-#pragma unroll
-    for (int m = 0; m < 4; m++) {
-        const int col = colbase + m * 8 + gid;
-        if (col >= ncol) continue;
-#pragma unroll
-        for (int n = 0; n < NN; n++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                int p = T.p0 + n * 8 + 2 * tig + h, oc = col;
-                int nq = na[m];
-                if (PAIRED) {
-                    const int nn = n * 8 + 2 * tig + h;
-                    if (nn >= 2 * orow) continue;
-                    if (nn >= orow) {
-                        // the partner column (mode 0) or mirror pair (mode 1); once on self-partners
-                        p = nn - orow;
-                        oc = mode == 0 ? pcolv(col) : mirq(col);
-                        if (oc == col) continue;
-                        if (mode == 1) nq = nvp[s.orb0 + pair_i[B.pair0 + oc]];
-                    }
-                }
-                if (p >= orow) continue;
-                if (mode == 0) {
-                    out[B.t0 + (int64_t)p * v + oc] = acc[m][n][h];
-                } else {
-                    const int ni = nvp[s.orb0 + pair_i[B.pair0 + p]];
-                    const int q2 = q2p(ni, nq);
-                    out[(int64_t)p * o + oc] = (vsm ? sv[q2] : vtab[s.vtab0 + q2]) + acc[m][n][h];
-                }
-            }
-    }
-}
-
-// One kernel per row tile NP (8, 16, 24, 32 pairs): the small tiles need fewer registers
-// and less shared memory, so more CTAs fit on an SM to hide the lookup latency.
-// KC1: the hole-hole intermediate's column chunk (mode 1), 64 or 32 (the launch-shape tuner's pick)
-template <int NP, bool PAIRED, int KC1 = kLadKC1>
-__global__ void __launch_bounds__(128, NP <= 8 ? 8 : NP <= 16 ? 6 : 4)
-    k_ladder3(const LadderTile *__restrict__ tiles, const BlockDev *__restrict__ blocks,
-              const SolveDev *__restrict__ solves, const int16_t *__restrict__ vir,
-              const int16_t *__restrict__ pair_i, const int *__restrict__ nvp,
-              const double *__restrict__ vtab, const double *__restrict__ t, const int64_t *__restrict__ hh0,
-              double *__restrict__ hh, int mode, int do_pp, int do_hh, double *__restrict__ g,
-              const uint8_t *__restrict__ active)
-{
-    const LadderTile T = tiles[blockIdx.x];
-    const BlockDev B = blocks[T.blk];
-    if (!active[B.solve]) return;
-    const SolveDev s = solves[B.solve];
-    extern __shared__ double lsm[];
-    double *ts = lsm;                              // 2 x NP x (chunk width + 4)
-    double *sv = ts + 2 * NP * (mode == 1 ? KC1 + 4 : kLadLd);   // kVtabSmem
-    int *nvc = (int *)(sv + kVtabSmem);            // v_K packed n-vectors of the block's virtuals
-    const bool vsm = s.q2max < kVtabSmem;
-    if (vsm)
-        for (int q = threadIdx.x; q <= s.q2max; q += blockDim.x) sv[q] = vtab[s.vtab0 + q];
-    for (int c = threadIdx.x; c < B.v; c += blockDim.x) nvc[c] = nvp[s.orb0 + vir[B.vir0 + c]];
-    __syncthreads();
-    double *H = hh + hh0[T.blk];
-    double *out = mode == 0 ? g : H;
-    // the hole-hole intermediate (mode 1) may split its c sum across the warps
-    if (mode == 1)
-        ladder3_tile<NP, true, PAIRED, KC1>(T, B, s, vir, pair_i, nvp, vtab, t, H, mode, do_pp, do_hh, out, sv,
-                                                vsm, ts, nvc);
-    else
-        ladder3_tile<NP, false, PAIRED>(T, B, s, vir, pair_i, nvp, vtab, t, H, mode, do_pp, do_hh, out, sv, vsm, ts,
-                                        nvc);
-}
-
 // The dynamic shared-memory limits only grow (batches of different sizes coexist), under
 // one lock: batches are created from several host threads while others solve.  Kernel
 // attributes belong to a device, so each device keeps its own limits (the caller has made
 // the batch's device current).
 static std::mutex g_smem_limit_mu;
-
-void set_ladder_smem_limit(int max_v)
-{
-    std::lock_guard<std::mutex> lock(g_smem_limit_mu);
-    static int current_by_dev[kMaxDevices] = {};   // attributes are per device
-    const int dev = current_device() % kMaxDevices;
-    int &current = current_by_dev[dev];
-    if (max_v > current) {
-        auto lb = [&](int np) {
-            return (int)std::max(ladder_smem_bytes(max_v, np), ladder1_smem_bytes(max_v, np, kLadKC1));
-        };
-        const int b8 = lb(8);
-        cudaFuncSetAttribute(k_ladder3<8, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, b8);
-        cudaFuncSetAttribute(k_ladder3<8, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, b8);
-        cudaFuncSetAttribute(k_ladder3<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb(16));
-        cudaFuncSetAttribute(k_ladder3<24, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb(24));
-        cudaFuncSetAttribute(k_ladder3<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb(32));
-        cudaFuncSetAttribute(k_ladder3<8, true, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, b8);
-        cudaFuncSetAttribute(k_ladder3<8, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, b8);
-        cudaFuncSetAttribute(k_ladder3<16, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb(16));
-        cudaFuncSetAttribute(k_ladder3<24, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb(24));
-        cudaFuncSetAttribute(k_ladder3<32, false, 32>, cudaFuncAttributeMaxDynamicSharedMemorySize, lb(32));
-        current = max_v;
-    }
-}
-
-// Ladder tiles in row-tile classes (sorted: paired 8, then 8, 16, 24, 32 pairs; counts in
-// ncls): one launch per non-empty class.  Returns the launches.
-static int launch_ladder3(const DevBatch &d, const LadderTile *tiles, const int *ncls, const double *t, int mode,
-                          int do_pp, int do_hh, double *g, cudaStream_t st)
-{
-    int off = 0, n = 0;
-    for (int c = 0; c < kLadderClasses; c++) {
-        const int cnt = ncls[c];
-        if (cnt <= 0) continue;
-        const int np = c == 0 ? 8 : 8 * c;
-        const bool kc32 = mode == 1 && d.hh_kc == 32;
-        const size_t sm = mode == 1 ? ladder1_smem_bytes(d.max_v, np, kc32 ? 32 : kLadKC1) : ladder_smem_bytes(d.max_v, np);
-#define UEGCCD_LADDER_ARGS                                                                                  \
-    tiles + off, d.blocks, d.solves, d.vir, d.pair_i, d.nvp, d.vtab, t, d.hh0, d.hh, mode, do_pp, do_hh, \
-        g, d.active
-        if (kc32) {
-            switch (c) {
-            case 0: k_ladder3<8, true, 32><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            case 1: k_ladder3<8, false, 32><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            case 2: k_ladder3<16, false, 32><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            case 3: k_ladder3<24, false, 32><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            default: k_ladder3<32, false, 32><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            }
-        } else {
-            switch (c) {
-            case 0: k_ladder3<8, true><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            case 1: k_ladder3<8, false><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            case 2: k_ladder3<16, false><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            case 3: k_ladder3<24, false><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            default: k_ladder3<32, false><<<cnt, 128, sm, st>>>(UEGCCD_LADDER_ARGS); break;
-            }
-        }
-#undef UEGCCD_LADDER_ARGS
-        off += cnt;
-        n++;
-    }
-    return n;
-}
 
 // ----------------------------------------------------------------------------
 // Mosaics (GetG2Mosaics, CCD.f90:548-582):
@@ -1772,7 +1438,7 @@ __global__ void k_copy(int64_t n, const double *__restrict__ src, double *__rest
 void launch_refresh(const DevBatch &d, cudaStream_t st)
 {
     k_copy<<<(unsigned)((d.namp + 255) / 256), 256, 0, st>>>(d.namp, d.t, d.t_ref);
-    launch_ladder3(d, d.tiles, d.ntile_cls, d.t_ref, 0, 1, 0, d.g_ref, st);
+    launch_ladder(d, d.t_ref, 1, 0, d.g_ref, st);
 }
 
 void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
@@ -1993,7 +1659,7 @@ void launch_to_aaaa(const DevBatch &d, cudaStream_t st)
     k_to_aaaa<<<(unsigned)((d.namp + 255) / 256), 256, 0, st>>>(d.namp, d.partner, d.t);
 }
 
-const char *kKernelNames[KID_COUNT] = {"k_mp2",      "k_energy",   "k_ladder_hh", "k_ladder",
+const char *kKernelNames[KID_COUNT] = {"k_mp2",      "k_energy",   "k_ladder",
                                       "k_mosaic_blk", "k_mosaic_sum", "k_drpa_sums", "k_update",
                                       "k_reduce_solves", "k_rings",
                                       "k_ladder_tc", "k_ring_stage", "k_tail", "k_diis_extrap2"};
@@ -2053,47 +1719,6 @@ int tune_rings(DevBatch &d, cudaStream_t st)
             }
         }
     }
-    // the ladder tiles' order (particle-particle part alone; it writes only d.g)
-    if (err == cudaSuccess && d.nblocks > 0 && d.tiles_lpt) {
-        float best = 1e30f;
-        for (int sched = 0; sched < 2 && err == cudaSuccess; sched++) {
-            const LadderTile *tl = sched ? d.tiles_lpt : d.tiles;
-            launch_ladder3(d, tl, d.ntile_cls, d.t, 0, 1, 0, d.g, st);
-            cudaEventRecord(e0, st);
-            launch_ladder3(d, tl, d.ntile_cls, d.t, 0, 1, 0, d.g, st);
-            launch_ladder3(d, tl, d.ntile_cls, d.t, 0, 1, 0, d.g, st);
-            cudaEventRecord(e1, st);
-            if ((err = cudaEventSynchronize(e1)) != cudaSuccess) break;
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (ms < best) {
-                best = ms;
-                d.ladder_sched = sched;
-            }
-        }
-    }
-    // the hole-hole intermediate's column chunk (mode 1 alone; it writes only d.hh)
-    if (err == cudaSuccess && d.nblocks > 0) {
-        float best = 1e30f;
-        int pick = 64;
-        const LadderTile *tl = d.ladder_sched ? d.htiles_lpt : d.htiles;
-        for (int kc : {64, 32}) {
-            d.hh_kc = kc;
-            launch_ladder3(d, tl, d.nhtile_cls, d.t, 1, 1, 1, d.g, st);
-            cudaEventRecord(e0, st);
-            launch_ladder3(d, tl, d.nhtile_cls, d.t, 1, 1, 1, d.g, st);
-            launch_ladder3(d, tl, d.nhtile_cls, d.t, 1, 1, 1, d.g, st);
-            cudaEventRecord(e1, st);
-            if ((err = cudaEventSynchronize(e1)) != cudaSuccess) break;
-            float ms = 0.f;
-            cudaEventElapsedTime(&ms, e0, e1);
-            if (ms < best) {
-                best = ms;
-                pick = kc;
-            }
-        }
-        d.hh_kc = pick;
-    }
     if (err == cudaSuccess) err = cudaGetLastError();
     if (e0) cudaEventDestroy(e0);
     if (e1) cudaEventDestroy(e1);
@@ -2107,16 +1732,10 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
     if (!kt) kt = &dummy;
     int n = 0;
     if (f.do_ladder && d.nblocks > 0) {
-        if (f.do_hh) {
-            kt->begin(KID_HH_W, st);
-            n += launch_ladder3(d, d.ladder_sched ? d.htiles_lpt : d.htiles, d.nhtile_cls, d.t, 1, f.do_pp, f.do_hh,
-                                d.g, st);
-            kt->end(st);
-        }
-        const int pp64 = (f.do_pp && !f.mixed) ? 1 : 0;
         kt->begin(KID_LADDER, st);
-        n += launch_ladder3(d, d.ladder_sched ? d.tiles_lpt : d.tiles, d.ntile_cls, d.t, 0, pp64, f.do_hh, d.g, st);
+        launch_ladder(d, d.t, (f.do_pp && !f.mixed) ? 1 : 0, f.do_hh, d.g, st);
         kt->end(st);
+        n++;
         if (f.do_pp && f.mixed) {
             kt->begin(KID_LADDER_TC, st);
             launch_ladder_tc(d, d.t_ref, d.g_ref, d.tc_err, st);

@@ -1,0 +1,525 @@
+// ladder.cu -- the FP64 ladders (GetG2Ladders, CCD.f90:588-686) of the spin-adapted residual.
+//
+// Per K block, written as G_K = t_K W_K + H_K t_K:
+//   particle-particle (CCD.f90:660-681): W_K[c][a] = v(c-a) over the block's virtuals;
+//   hole-hole (CCD.f90:611-657): H_K[p][q] = v(i_p - k_q) + sum_c t_K[p][c] v(c - k_q),
+//   p = (i,j), q = (k,l), after the pair-swap re-indexing t(kl,b) = t(lk,a).
+// Only the rows p = (i,j) with i <= j are formed: by the pair symmetry t(ij,a) = t(ji,b)
+// (T2abab(ij,ab) = T2abab(ji,ba)) the mirror row (j,i) at column b = K - a has the value of
+// (i,j) at a, and k_update reads G on the rows i <= j only.
+//
+// Even and odd halves.  The partner map a -> K - a of a block leaves its Coulomb kernel as it
+// is, v(Ka - Kc) = v(a - c), so over the columns c <= pc (pc the partner of c, h of them)
+//   s_c = (t_c + t_pc)/2,  d_c = (t_c - t_pc)/2     (self-partner: s = t/2, d = 0)
+//   P_a = sum_c (v(a-c) + v(a-pc)) s_c,   M_a = sum_c (v(a-c) - v(a-pc)) d_c
+//   G_a = P_a + M_a,   G_pa = P_a - M_a
+// -- half the multiply-adds of the full product, and half the Coulomb elements for a block's
+// rows.  The columns q <= q' of H (q' the mirror pair) split the same way, v(k_q' - c) =
+// v(k_q - pc), and so does the product H t, t(q',a) = t(q,pa).  So one pass over the columns c
+// forms the particle-particle sums of the columns a and the sums of H together; H stays in
+// shared memory and its product with t follows in the same CTA.
+//
+// Coulomb elements.  v(a-c) is a table lookup by |n_a - n_c|^2 = |a|^2 + |c|^2 - 2 a.c: one byte
+// dot product of packed vectors (a scaled by -2) on top of |c|^2, and one shift-add.  32 lanes
+// look up 32 different entries, and on one copy of the table those reads met about 5-way bank
+// conflicts, which bounded the kernel.  The table is therefore kept in 16 copies, one per pair
+// of banks (entry q at 128 q + 8 (lane mod 16) bytes): every lookup is conflict-free, for 12 KB
+// at N=54.  Tables beyond 256 entries (32 KB of copies) keep one copy, beyond 1,024 stay in
+// global memory.
+//
+// Two forms, by the rows i <= j of a block (one launch runs both, longest tiles first; a tile is
+// one CTA of 128 threads):
+//   1-4 rows    FP64 FMAs: a lane owns columns a, all rows; the s and d of a column c are
+//               broadcast reads.  Per 32 columns and c: two lookups (4 shared-memory cycles),
+//               2 + 2 rows FMA-pipe instructions (1 + rows cycles).  A DMMA tile would spend 8
+//               cycles however few rows fill its 8-wide fragment.
+//   5 and more  DMMA (mma.sync m8n8k4 f64; tcgen05 has no f64 kind), up to 16 rows a tile: each
+//               lane makes its own element of the two Coulomb fragments.  8 cycles per 8 rows.
+// Measured on 100 twists of N=54 (485 plane waves), the residual's ladders and hole-hole
+// intermediate together: LADDER_MS_AFTER against LADDER_MS_BEFORE for DMMA tiles over full
+// products with a separate hole-hole launch.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+#include <mutex>
+
+#include "kernels.h"
+#include "uegccd_internal.h"
+
+namespace uegccd {
+
+namespace {
+
+constexpr int kThreads = 128;
+constexpr int kKC = 32;            // columns c per staged chunk
+constexpr int kLd = kKC + 4;       // row stride of the DMMA operands: = 4 mod 16 doubles, conflict-free
+constexpr int kHLd = 36;           // row stride of H (at most 32 pairs q <= q'): likewise
+
+__device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+// Table forms: 16 copies or one in shared memory, or global memory.
+enum { kTab16 = 0, kTab1 = 1, kTabGlobal = 2 };
+
+// One orbital as the row side of a lookup: its packed vector times -2 and where |n|^2 puts it.
+struct Col {
+    int m2, base;
+};
+
+template <int TAB>
+__device__ __forceinline__ Col make_col(int packed)
+{
+    const int x = (int8_t)packed, y = (int8_t)(packed >> 8), z = (int8_t)(packed >> 16);
+    const int n2 = x * x + y * y + z * z;
+    Col c;
+    c.m2 = ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16);   // |n_d| <= 63
+    c.base = TAB == kTab16 ? (n2 << 7) + ((threadIdx.x & 15) << 3) : TAB == kTab1 ? n2 << 3 : n2;
+    return c;
+}
+
+// v(a - c): packed c and |c|^2
+template <int TAB>
+__device__ __forceinline__ double lookup(const char *tab, const double *__restrict__ gtab, const Col &a, int c, int c2)
+{
+    const int d = __dp4a(a.m2, c, c2);
+    if (TAB == kTab16) return *reinterpret_cast<const double *>(tab + (a.base + (d << 7)));
+    if (TAB == kTab1) return *reinterpret_cast<const double *>(tab + (a.base + (d << 3)));
+    return __ldg(gtab + a.base + d);
+}
+
+struct Args {
+    const LadderTile64 *tiles;
+    const BlockDev *blocks;
+    const SolveDev *solves;
+    const int16_t *vir, *pair_i, *pair_j;
+    const int *nvp;
+    const double *vtab, *t;
+    double *g;
+    const uint8_t *active;
+    int do_pp, do_hh, tab_bytes;
+};
+
+// What both forms use of a tile's block.
+struct Blk {
+    LadderTile64 T;
+    BlockDev B;
+    int orow, h;             // rows i <= j; columns c <= pc
+    int nh, ncol;            // the tile's columns: nh pairs q <= q' of H, then the virtuals a0 .. a1
+    const double *t;         // the block's amplitudes
+    const int *nvp;          // the solve's packed vectors
+    const double *gtab;      // the solve's |q|^2 table
+    const int16_t *vir, *pi, *pj;
+};
+
+__device__ __forceinline__ int packed_col(const Blk &K, int e)
+{
+    e = min(e, K.ncol - 1);   // lanes past the tile repeat its last column
+    return e < K.nh ? K.nvp[K.pi[e]] : K.nvp[K.vir[K.T.a0 + e - K.nh]];
+}
+
+// One column c <= pc as both forms stage it: {c, |c|^2, pc, |pc|^2}, packed vectors.
+__device__ __forceinline__ int4 chunk_col(const Blk &K, int c)
+{
+    c = min(c, K.h - 1);   // past the end the staged amplitudes are zero
+    const int n = K.nvp[K.vir[c]], p = K.nvp[K.vir[c < K.B.nvd ? c + K.h : c]];
+    return make_int4(n, __dp4a(n, n, 0), p, __dp4a(p, p, 0));
+}
+
+__device__ __forceinline__ void load_pair(const Blk &K, int row, int c, double &x, double &y)
+{
+    const double *r = K.t + (int64_t)row * K.B.v;
+    x = c < K.h ? __ldg(r + c) : 0.0;
+    y = c < K.B.nvd ? __ldg(r + c + K.h) : 0.0;
+}
+
+// ---- 1 to 4 rows ------------------------------------------------------------------------
+template <int TAB, int R, int U>
+__device__ __forceinline__ void fma_cols(double (&P)[2][R], double (&M)[2][R], const Col (&a)[2], const char *tab,
+                                         const double *gtab, const int4 *cl, const double2 *sd, int k0, int step,
+                                         int n)
+{
+#pragma unroll 2
+    for (int k = k0; k < n; k += step) {
+        const int4 c = cl[k];
+        double2 x[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) x[r] = sd[k * R + r];
+#pragma unroll
+        for (int m = 0; m < U; m++) {
+            const double v = lookup<TAB>(tab, gtab, a[m], c.x, c.y), w = lookup<TAB>(tab, gtab, a[m], c.z, c.w);
+            const double wp = v + w, wm = v - w;
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                P[m][r] = fma(wp, x[r].x, P[m][r]);
+                M[m][r] = fma(wm, x[r].y, M[m][r]);
+            }
+        }
+    }
+}
+
+// smem: 2 x kKC int4 column records, 2 x kKC x R double2 amplitudes, H, then the reduction area
+template <int TAB, int R>
+__device__ void ladder_fma(const Args &A, const Blk &K, const char *tab, char *smem)
+{
+    int4 *cl = reinterpret_cast<int4 *>(smem);
+    double2 *sd = reinterpret_cast<double2 *>(smem + 2 * kKC * sizeof(int4));
+    double2 *hs = sd + 2 * kKC * R;
+    double *red = reinterpret_cast<double *>(hs + R * R);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    // units of 32 columns, two a warp; with one or two such groups the warps split the columns c
+    const int groups = (K.ncol + 63) >> 6;
+    const int ks = groups == 1 ? 4 : groups == 2 ? 2 : 1;
+    const int grp = warp / ks, split = warp - grp * ks;
+    const bool on = grp < groups && (A.do_pp || grp == 0);
+    const bool two = grp * 64 + 32 < K.ncol;
+    Col a[2];
+    a[0] = make_col<TAB>(packed_col(K, grp * 64 + lane));
+    a[1] = make_col<TAB>(packed_col(K, grp * 64 + 32 + lane));
+    double P[2][R], M[2][R];
+#pragma unroll
+    for (int m = 0; m < 2; m++)
+#pragma unroll
+        for (int r = 0; r < R; r++) P[m][r] = M[m][r] = 0.0;
+    const int nchunk = (K.h + kKC - 1) / kKC;
+    double x = 0.0, y = 0.0;
+    int4 rec = make_int4(0, 0, 0, 0);
+    auto fetch = [&](int j) {
+        if (warp < R) load_pair(K, warp, j * kKC + lane, x, y);
+        if (warp == 3) rec = chunk_col(K, j * kKC + lane);
+    };
+    fetch(0);
+    for (int j = 0; j < nchunk; j++) {
+        const int b = (j & 1) * kKC, c = j * kKC + lane;
+        if (warp < R) sd[(b + lane) * R + warp] = make_double2(0.5 * (x + y), c < K.B.nvd ? 0.5 * (x - y) : 0.0);
+        if (warp == 3) cl[b + lane] = rec;
+        __syncthreads();
+        if (j + 1 < nchunk) fetch(j + 1);
+        if (on) {
+            const int n = min(kKC, K.h - j * kKC);
+            if (two) fma_cols<TAB, R, 2>(P, M, a, tab, K.gtab, cl + b, sd + b * R, split, ks, n);
+            else fma_cols<TAB, R, 1>(P, M, a, tab, K.gtab, cl + b, sd + b * R, split, ks, n);
+        }
+    }
+    if (ks > 1) {
+        // the splits' sums into the first one's, in order
+        auto at = [&](int sp, int m, int r, int q) -> double & {
+            return red[((((sp - 1) * 2 + grp) * 2 + m) * R + r) * 64 + q * 32 + lane];
+        };
+        if (split > 0 && grp < groups)
+#pragma unroll
+            for (int m = 0; m < 2; m++)
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    at(split, m, r, 0) = P[m][r];
+                    at(split, m, r, 1) = M[m][r];
+                }
+        __syncthreads();
+        if (split == 0 && grp < groups)
+            for (int sp = 1; sp < ks; sp++)
+#pragma unroll
+                for (int m = 0; m < 2; m++)
+#pragma unroll
+                    for (int r = 0; r < R; r++) {
+                        P[m][r] += at(sp, m, r, 0);
+                        M[m][r] += at(sp, m, r, 1);
+                    }
+    }
+    const bool lead = split == 0 && grp < groups;
+    if (K.nh > 0) {
+        // halves of H: (H[p][q] +- H[p][q'])/2
+        if (lead && grp == 0 && lane < K.nh) {
+            const Col kq = make_col<TAB>(K.nvp[K.pi[lane]]), lq = make_col<TAB>(K.nvp[K.pj[lane]]);
+#pragma unroll
+            for (int r = 0; r < R; r++) {
+                const int n = K.nvp[K.pi[r]], n2 = __dp4a(n, n, 0);
+                const double v = lookup<TAB>(tab, K.gtab, kq, n, n2), w = lookup<TAB>(tab, K.gtab, lq, n, n2);
+                hs[r * R + lane] = make_double2(P[0][r] + 0.5 * (v + w), M[0][r] + 0.5 * (v - w));
+            }
+        }
+        __syncthreads();
+    }
+    if (!lead) return;
+#pragma unroll
+    for (int m = 0; m < 2; m++) {
+        const int e = grp * 64 + m * 32 + lane, c = K.T.a0 + e - K.nh;
+        if (e < K.nh || e >= K.ncol) continue;
+        const bool pair = c < K.B.nvd;
+        double p[R], q[R];
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            p[r] = A.do_pp ? P[m][r] : 0.0;
+            q[r] = A.do_pp ? M[m][r] : 0.0;
+        }
+        if (K.nh > 0)
+#pragma unroll
+            for (int k = 0; k < R; k++) {
+                const double *row = K.t + (int64_t)k * K.B.v;
+                const double u = __ldg(row + c), w = pair ? __ldg(row + c + K.h) : u;
+                const double f = k < K.B.nd ? 1.0 : 0.5;   // the pair and its mirror, or the diagonal pair
+                const double s = f * (u + w), d = f * (u - w);
+#pragma unroll
+                for (int r = 0; r < R; r++) {
+                    const double2 H = hs[r * R + k];
+                    p[r] = fma(H.x, s, p[r]);
+                    q[r] = fma(H.y, d, q[r]);
+                }
+            }
+        double *out = A.g + K.B.t0 + c;
+#pragma unroll
+        for (int r = 0; r < R; r++) {
+            out[(int64_t)r * K.B.v] = p[r] + q[r];
+            if (pair) out[(int64_t)r * K.B.v + K.h] = p[r] - q[r];
+        }
+    }
+}
+
+// ---- 5 rows and more --------------------------------------------------------------------
+// NN fragments of 8 rows; a warp covers MF fragments of 8 columns, the CTA 4 warps of them a
+// pass.  Fragment layouts (PTX ISA, m8n8k4 .f64): A row = lane/4, col = lane%4; B row (k) =
+// lane%4, col = lane/4; C row = lane/4, cols 2*(lane%4) + {0,1}.
+// smem: 2 x kKC int4 column records, s and d of 2 x 8 NN rows, the halves of H (16 rows each)
+template <int TAB, int NN>
+__device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *smem)
+{
+    constexpr int MF = NN == 1 ? 4 : 2, WC = 8 * MF, PC = 4 * WC, NR = 8 * NN;
+    int4 *cl = reinterpret_cast<int4 *>(smem);
+    double *S = reinterpret_cast<double *>(smem + 2 * kKC * sizeof(int4)), *D = S + 2 * NR * kLd;
+    double *hs = D + 2 * NR * kLd, *hd = hs + NR * kHLd;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
+    const int nchunk = (K.h + kKC - 1) / kKC, np = K.T.np, p0 = K.T.p0;
+    for (int e0 = 0; e0 < K.ncol; e0 += PC) {
+        const int base = e0 + warp * WC;
+        const bool loop = A.do_pp || (e0 == 0 && K.nh > 0);
+        const bool on = base < K.ncol && (A.do_pp || base < K.nh);
+        Col a[MF];
+#pragma unroll
+        for (int m = 0; m < MF; m++) a[m] = make_col<TAB>(packed_col(K, base + m * 8 + gid));
+        double P[MF][NN][2], M[MF][NN][2];
+#pragma unroll
+        for (int m = 0; m < MF; m++)
+#pragma unroll
+            for (int n = 0; n < NN; n++) P[m][n][0] = P[m][n][1] = M[m][n][0] = M[m][n][1] = 0.0;
+        if (loop) {
+            double x[2 * NN], y[2 * NN];
+            int4 rec = make_int4(0, 0, 0, 0);
+            auto fetch = [&](int j) {
+#pragma unroll
+                for (int k = 0; k < 2 * NN; k++) {
+                    const int r = warp + 4 * k;
+                    x[k] = y[k] = 0.0;
+                    if (r < np) load_pair(K, p0 + r, j * kKC + lane, x[k], y[k]);
+                }
+                if (warp == 0) rec = chunk_col(K, j * kKC + lane);
+            };
+            fetch(0);
+            for (int j = 0; j < nchunk; j++) {
+                const int b = j & 1, c = j * kKC + lane;
+#pragma unroll
+                for (int k = 0; k < 2 * NN; k++) {
+                    const int r = warp + 4 * k;
+                    S[(b * NR + r) * kLd + lane] = 0.5 * (x[k] + y[k]);
+                    D[(b * NR + r) * kLd + lane] = c < K.B.nvd ? 0.5 * (x[k] - y[k]) : 0.0;
+                }
+                if (warp == 0) cl[b * kKC + lane] = rec;
+                __syncthreads();
+                if (j + 1 < nchunk) fetch(j + 1);
+                if (on) {
+                    const double *sb = S + (b * NR + gid) * kLd + tig, *db = D + (b * NR + gid) * kLd + tig;
+                    const int n4 = min(kKC, K.h - j * kKC);
+#pragma unroll 2
+                    for (int k = 0; k < n4; k += 4) {
+                        const int4 cc = cl[b * kKC + k + tig];
+                        double bs[NN], bd[NN];
+#pragma unroll
+                        for (int n = 0; n < NN; n++) {
+                            bs[n] = sb[n * 8 * kLd + k];
+                            bd[n] = db[n * 8 * kLd + k];
+                        }
+#pragma unroll
+                        for (int m = 0; m < MF; m++) {
+                            const double v = lookup<TAB>(tab, K.gtab, a[m], cc.x, cc.y);
+                            const double w = lookup<TAB>(tab, K.gtab, a[m], cc.z, cc.w);
+                            const double wp = v + w, wm = v - w;
+#pragma unroll
+                            for (int n = 0; n < NN; n++) {
+                                dmma_884(P[m][n][0], P[m][n][1], wp, bs[n]);
+                                dmma_884(M[m][n][0], M[m][n][1], wm, bd[n]);
+                            }
+                        }
+                    }
+                }
+            }
+        }
+        if (K.nh > 0 && e0 == 0) {
+            // halves of H: (H[p][q] +- H[p][q'])/2; all of a block's q lie in the first pass
+#pragma unroll
+            for (int m = 0; m < MF; m++) {
+                const int q = base + m * 8 + gid;
+                if (q >= K.nh) continue;
+                const Col kq = make_col<TAB>(K.nvp[K.pi[q]]), lq = make_col<TAB>(K.nvp[K.pj[q]]);
+#pragma unroll
+                for (int n = 0; n < NN; n++)
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int r = n * 8 + 2 * tig + u;
+                        double hp = 0.0, hm = 0.0;
+                        if (r < np) {
+                            const int nn = K.nvp[K.pi[p0 + r]], n2 = __dp4a(nn, nn, 0);
+                            const double v = lookup<TAB>(tab, K.gtab, kq, nn, n2);
+                            const double w = lookup<TAB>(tab, K.gtab, lq, nn, n2);
+                            hp = P[m][n][u] + 0.5 * (v + w);
+                            hm = M[m][n][u] + 0.5 * (v - w);
+                        }
+                        hs[r * kHLd + q] = hp;
+                        hd[r * kHLd + q] = hm;
+                    }
+            }
+            __syncthreads();
+        }
+        if (base < K.ncol) {
+            if (!A.do_pp)
+#pragma unroll
+                for (int m = 0; m < MF; m++)
+#pragma unroll
+                    for (int n = 0; n < NN; n++) P[m][n][0] = P[m][n][1] = M[m][n][0] = M[m][n][1] = 0.0;
+            if (K.nh > 0) {
+                for (int q0 = 0; q0 < K.orow; q0 += 4) {
+                    const int q = q0 + tig;
+                    const bool qok = q < K.orow;
+                    const double *row = K.t + (int64_t)(qok ? q : 0) * K.B.v;
+                    const double f = q < K.B.nd ? 1.0 : 0.5;   // the pair and its mirror, or the diagonal pair
+                    double bs[NN], bd[NN];
+#pragma unroll
+                    for (int n = 0; n < NN; n++) {
+                        bs[n] = qok ? hs[(n * 8 + gid) * kHLd + q] : 0.0;
+                        bd[n] = qok ? hd[(n * 8 + gid) * kHLd + q] : 0.0;
+                    }
+#pragma unroll
+                    for (int m = 0; m < MF; m++) {
+                        const int e = base + m * 8 + gid, c = K.T.a0 + e - K.nh;
+                        double s = 0.0, d = 0.0;
+                        if (qok && e >= K.nh && e < K.ncol) {
+                            const double u = __ldg(row + c), w = c < K.B.nvd ? __ldg(row + c + K.h) : u;
+                            s = f * (u + w);
+                            d = f * (u - w);
+                        }
+#pragma unroll
+                        for (int n = 0; n < NN; n++) {
+                            dmma_884(P[m][n][0], P[m][n][1], s, bs[n]);
+                            dmma_884(M[m][n][0], M[m][n][1], d, bd[n]);
+                        }
+                    }
+                }
+            }
+#pragma unroll
+            for (int m = 0; m < MF; m++) {
+                const int e = base + m * 8 + gid, c = K.T.a0 + e - K.nh;
+                if (e < K.nh || e >= K.ncol) continue;
+                double *out = A.g + K.B.t0 + c;
+#pragma unroll
+                for (int n = 0; n < NN; n++)
+#pragma unroll
+                    for (int u = 0; u < 2; u++) {
+                        const int r = n * 8 + 2 * tig + u;
+                        if (r >= np) continue;
+                        double *o = out + (int64_t)(p0 + r) * K.B.v;
+                        o[0] = P[m][n][u] + M[m][n][u];
+                        if (c < K.B.nvd) o[K.h] = P[m][n][u] - M[m][n][u];
+                    }
+            }
+        }
+        __syncthreads();   // the next pass stages its first chunk
+    }
+}
+
+template <int TAB>
+__global__ void __launch_bounds__(kThreads, 5) k_ladder(Args A)
+{
+    Blk K;
+    K.T = A.tiles[blockIdx.x];
+    K.B = A.blocks[K.T.blk];
+    if (!A.active[K.B.solve]) return;
+    const SolveDev &s = A.solves[K.B.solve];
+    K.orow = K.B.nd + K.B.dg;
+    K.h = K.B.nvd + K.B.sd;
+    K.nh = A.do_hh ? K.orow : 0;
+    K.ncol = K.nh + K.T.a1 - K.T.a0;
+    K.t = A.t + K.B.t0;
+    K.nvp = A.nvp + s.orb0;
+    K.gtab = A.vtab + s.vtab0;
+    K.vir = A.vir + K.B.vir0;
+    K.pi = A.pair_i + K.B.pair0;
+    K.pj = A.pair_j + K.B.pair0;
+    extern __shared__ __align__(16) char lsm[];
+    if (TAB == kTab16) {
+        double *tab = reinterpret_cast<double *>(lsm);
+        for (int e = threadIdx.x; e < (s.q2max + 1) * 16; e += kThreads) tab[e] = __ldg(K.gtab + (e >> 4));
+    } else if (TAB == kTab1) {
+        double *tab = reinterpret_cast<double *>(lsm);
+        for (int e = threadIdx.x; e <= s.q2max; e += kThreads) tab[e] = __ldg(K.gtab + e);
+    }
+    __syncthreads();
+    char *sm = lsm + A.tab_bytes;
+    if (K.orow > kLadderFmaRows) {
+        if (K.T.np <= 8) ladder_mma<TAB, 1>(A, K, lsm, sm);
+        else ladder_mma<TAB, 2>(A, K, lsm, sm);
+        return;
+    }
+    switch (K.orow) {
+    case 1: ladder_fma<TAB, 1>(A, K, lsm, sm); break;
+    case 2: ladder_fma<TAB, 2>(A, K, lsm, sm); break;
+    case 3: ladder_fma<TAB, 3>(A, K, lsm, sm); break;
+    default: ladder_fma<TAB, 4>(A, K, lsm, sm); break;
+    }
+}
+
+int tab_form(int q2max) { return q2max < 256 ? kTab16 : q2max < 1024 ? kTab1 : kTabGlobal; }
+int tab_bytes(int q2max)
+{
+    const int f = tab_form(q2max);
+    return f == kTab16 ? (q2max + 1) * 128 : f == kTab1 ? ((q2max + 1) * 8 + 15) / 16 * 16 : 0;
+}
+
+}  // namespace
+
+size_t ladder_smem_bytes(int q2max, int max_rows)
+{
+    const size_t cols = 2 * kKC * sizeof(int4);
+    const int r = std::min(max_rows, kLadderFmaRows), nr = max_rows <= 8 ? 8 : 16;
+    // the FMA form's reduction area: 3 splits of one group of 64 columns, or 1 of two
+    size_t b = cols + sizeof(double2) * (2 * kKC * r + r * r) + sizeof(double) * (3 * 2 * 2 * r * 64);
+    if (max_rows > kLadderFmaRows) b = std::max(b, cols + sizeof(double) * (2 * 2 * (size_t)nr * kLd + 2 * (size_t)nr * kHLd));
+    return tab_bytes(q2max) + b;
+}
+
+void set_ladder_smem_limit(size_t bytes)
+{
+    static std::mutex mu;
+    static size_t current_by_dev[kMaxDevices] = {};   // attributes are per device
+    std::lock_guard<std::mutex> lock(mu);
+    size_t &current = current_by_dev[current_device() % kMaxDevices];
+    if (bytes <= std::max(current, (size_t)48 * 1024)) return;
+    cudaFuncSetAttribute(k_ladder<kTab16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaFuncSetAttribute(k_ladder<kTab1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    cudaFuncSetAttribute(k_ladder<kTabGlobal>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    current = bytes;
+}
+
+void launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st)
+{
+    if (d.nltiles <= 0) return;
+    const Args A{d.ltiles, d.blocks, d.solves, d.vir, d.pair_i, d.pair_j, d.nvp, d.vtab, t, g, d.active,
+                 do_pp, do_hh, tab_bytes(d.q2max)};
+    switch (tab_form(d.q2max)) {
+    case kTab16: k_ladder<kTab16><<<d.nltiles, kThreads, d.ladder_smem, st>>>(A); break;
+    case kTab1: k_ladder<kTab1><<<d.nltiles, kThreads, d.ladder_smem, st>>>(A); break;
+    default: k_ladder<kTabGlobal><<<d.nltiles, kThreads, d.ladder_smem, st>>>(A); break;
+    }
+}
+
+}  // namespace uegccd

@@ -56,7 +56,14 @@ struct BlockDev {
                             // virtual a = K - a if sd = 1, column c + nvd + sd the partner of c < nvd
 };
 
-// One tile of the particle-particle ladder: rows [p0, p0+P) x columns [a0, a0+A) of block blk.
+// One tile of the FP64 ladders: rows [p0, p0+np) of block blk, the columns a0 <= a < a1 among
+// the columns a <= pcol a and, from the partner map, their partners.
+struct LadderTile64 {
+    int blk, a0, a1;
+    int16_t p0, np;
+};
+
+// One tile of the tensor-core ladder: rows [p0, p0+P) x columns [a0, a0+A) of block blk.
 struct LadderTile {
     int blk, a0, p0, pad;
 };
