@@ -1615,7 +1615,7 @@ int make_two_channel(UegccdBatch &b, int s, std::unique_ptr<uegccd::TwoChannel> 
     al.begin = [ar]() { ar->m = ar->b->mark(); };
     al.rollback = [ar]() { ar->b->rollback(ar->m); };
     auto tc = std::make_unique<uegccd::TwoChannel>();
-    const int rc = tc->init(b.sys[s], b.stream, al);
+    const int rc = tc->init(b.sys[s], b.plans[s], b.stream, al);
     if (rc) return rc;
     out = std::move(tc);
     return 0;

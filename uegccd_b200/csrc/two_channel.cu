@@ -26,7 +26,13 @@
 //               mosaics, hole-hole then particle-particle ladder, rings, crossed rings
 // and per iteration k2_update (GetRes, SolveCC, CnvrgCC and CCEnergy).  Each sum has a fixed
 // order and every reduction a fixed tree, so results do not depend on the launch.
+//
+// The CCD residual takes the form of two_channel_mm.cu (matrix products, about an eighth of the
+// time) when the integrals allow it; the kernels here serve dRPA, core orbitals, tables with an
+// excluded integral, and systems whose ring groups exceed its shared memory.
 #include "two_channel.h"
+
+#include "two_channel_mm.h"
 
 #include <algorithm>
 #include <cmath>
@@ -702,6 +708,8 @@ int tc_pick_routine(const UegccdRangeTerms &fl, int safe_eri, int core_n, double
     return TC_BASE;
 }
 
+TwoChannel::TwoChannel() = default;
+
 TwoChannel::~TwoChannel()
 {
     if (ev0_) cudaEventDestroy(ev0_);
@@ -715,7 +723,7 @@ int TwoChannel::alloc(void **p, size_t bytes)
     return rc;
 }
 
-int TwoChannel::init(const SystemHost &sys, cudaStream_t stream, TcAlloc al)
+int TwoChannel::init(const SystemHost &sys, const SolvePlan &plan, cudaStream_t stream, TcAlloc al)
 {
     O_ = sys.O;
     M_ = sys.M;
@@ -743,6 +751,16 @@ int TwoChannel::init(const SystemHost &sys, cudaStream_t stream, TcAlloc al)
         if (c == 0) c = p + 1;   // the first orbital with this vector
     }
     nblk_ = blocks_of(n_);
+    occ_.assign(sys.n.begin(), sys.n.begin() + O_);
+    for (size_t r = 0; r < plan.ph_i.size(); r++) ph_.push_back(plan.ph_i[r] | (int)plan.ph_x[r] << 16);
+    for (size_t g = 0; g < plan.groups.size(); g++) {
+        const auto &G = plan.groups[g];
+        if (G.partner < (int)g) continue;   // each {Q, -Q} once
+        pairs_.push_back(make_int4(G.r0, G.n, plan.groups[G.partner].r0, plan.groups[G.partner].n));
+    }
+    // the largest pairs first: one CTA each, and the small ones fill the end of the launch
+    std::stable_sort(pairs_.begin(), pairs_.end(),
+                     [](const int4 &a, const int4 &b) { return (int64_t)a.y * a.w > (int64_t)b.y * b.w; });
     int *cube_d = nullptr;
     int rc = 0;
     al_.begin();
@@ -825,7 +843,80 @@ int TwoChannel::set_integrals(int routine, const UegccdRangeTerms &fl, int core_
     f.xr_lin_x = m3(fl.xring, fl.exchange_rings, fl.lin_rings);
     f.xr_quad_d = m3(fl.xring, fl.direct_rings, fl.quad_rings);
     f.xr_quad_x = m3(fl.xring, fl.exchange_rings, fl.quad_rings);
+    plain_ = core_n == 0;
+    for (const int flag : {f.drv_d, f.drv_x, f.mosaic, f.lad_lin_d, f.lad_lin_x, f.lad_quad_d, f.lad_quad_x,
+                           f.ring_lin_d, f.ring_lin_x, f.ring_quad_d, f.ring_quad_x, f.xr_lin_d, f.xr_lin_x,
+                           f.xr_quad_d, f.xr_quad_x})
+        for (int q2 = 0; q2 < nq_ && plain_; q2++) plain_ = vt[(size_t)flag * nq_ + q2] >= -80.0;
+    weights_ = false;
     return 0;
+}
+
+// Whether the residual can take the form of two_channel_mm.cu; its arrays on the first call, as
+// long as memory holds them (the loops serve the system otherwise).
+bool TwoChannel::mm_ready()
+{
+    if (mm_state_ != 0) return mm_state_ > 0;
+    mm_state_ = -1;
+    auto m = std::make_unique<TcMm>();
+    TcMm &D = *m;
+    const int O2 = O_ * O_;
+    D.O = O_, D.V = V_, D.n = (int)n_, D.nq = nq_;
+    D.F = F_, D.nv = nv_, D.vt = vt_;
+    D.ring_smem = 0;
+    for (const auto &P : pairs_) D.ring_smem = std::max(D.ring_smem, tc_mm_ring_smem(P.y, P.w));
+    if (D.ring_smem > kTcMmSmemMax || tc_mm_stage_smem(O_) > kTcMmSmemMax) return false;
+    auto up = [](int64_t x, int64_t k) { return (x + k - 1) / k * k; };
+    const int64_t ldw = up(2 * (int64_t)(V_ + O_), 64), ldt = up(2 * (int64_t)O2, 64);
+    D.ldw = (int)ldw, D.ldt = (int)ldt, D.kdim = (int)up(V_, 16);
+    std::vector<int> kl0(O2 + 1, 0), kl, kl_ij;
+    for (int ij = 0; ij < O2; ij++) {
+        const auto &a = occ_[ij % O_], &b = occ_[ij / O_];
+        for (int k = 0; k < O_; k++)
+            for (int l = 0; l < O_; l++)
+                if (a[0] + b[0] == occ_[k][0] + occ_[l][0] && a[1] + b[1] == occ_[k][1] + occ_[l][1] &&
+                    a[2] + b[2] == occ_[k][2] + occ_[l][2]) {
+                    kl.push_back(k | l << 16);
+                    kl_ij.push_back(ij);
+                }
+        kl0[ij + 1] = (int)kl.size();
+    }
+    D.nkl = (int)kl.size();
+    D.npairs = (int)pairs_.size();
+    int *kl0_d = nullptr, *kl_d = nullptr, *klij_d = nullptr, *ph_d = nullptr;
+    int4 *pairs_d = nullptr;
+    al_.begin();
+    if (alloc((void **)&D.w, D.kdim * ldw * sizeof(double)) || alloc((void **)&D.t, D.kdim * ldt * sizeof(double)) ||
+        alloc((void **)&D.c, ldw * ldt * sizeof(double)) || alloc((void **)&D.jpart, (size_t)V_ * O_ * sizeof(double)) ||
+        alloc((void **)&D.done, sizeof(int)) || alloc((void **)&kl0_d, kl0.size() * sizeof(int)) ||
+        alloc((void **)&kl_d, kl.size() * sizeof(int)) || alloc((void **)&klij_d, kl.size() * sizeof(int)) ||
+        alloc((void **)&D.h2, kl.size() * sizeof(double)) || alloc((void **)&D.h3, kl.size() * sizeof(double)) ||
+        alloc((void **)&pairs_d, pairs_.size() * sizeof(int4)) || alloc((void **)&ph_d, ph_.size() * sizeof(int))) {
+        al_.rollback();
+        return false;
+    }
+    D.kl0 = kl0_d, D.kl = kl_d, D.kl_ij = klij_d, D.pairs = pairs_d, D.ph = ph_d;
+    D.gr[0] = r_[0], D.gr[1] = r_[1], D.gx[0] = x_[0], D.gx[1] = x_[1];
+    cudaError_t e = tc_mm_limits(D);
+    auto copy = [&](void *dst, const void *src, size_t bytes) {
+        if (e == cudaSuccess && bytes > 0) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st_);
+    };
+    copy(kl0_d, kl0.data(), kl0.size() * sizeof(int));
+    copy(kl_d, kl.data(), kl.size() * sizeof(int));
+    copy(klij_d, kl_ij.data(), kl_ij.size() * sizeof(int));
+    copy(pairs_d, pairs_.data(), pairs_.size() * sizeof(int4));
+    copy(ph_d, ph_.data(), ph_.size() * sizeof(int));
+    if (e == cudaSuccess) e = cudaMemsetAsync(D.w, 0, D.kdim * ldw * sizeof(double), st_);   // the padding stays 0
+    if (e == cudaSuccess) e = cudaMemsetAsync(D.t, 0, D.kdim * ldt * sizeof(double), st_);
+    if (e == cudaSuccess) e = cudaMemsetAsync(D.done, 0, sizeof(int), st_);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
+    if (e != cudaSuccess) {
+        al_.rollback();
+        return false;
+    }
+    mm_ = std::move(m);
+    mm_state_ = 1;
+    return true;
 }
 
 int TwoChannel::upload_t(const double *h, double *d)
@@ -844,6 +935,14 @@ int TwoChannel::read_out(int k, double *h)
 // One residual G of the terms in mask from t_ into g_.
 int TwoChannel::residual(bool drpa, int mask)
 {
+    if (!drpa && plain_ && mm_ready()) {
+        mm_->sets = f_.lad_lin_d == f_.lad_lin_x && f_.lad_quad_d == f_.lad_quad_x ? 1 : 2;
+        if (!weights_) tc_mm_weights(*mm_, f_, st_);
+        weights_ = true;
+        launches_ += tc_mm_residual(*mm_, f_, mask, t_[0], t_[1], jvv_, joo_, g_[0], g_[1], st_);
+        TCU(cudaGetLastError());
+        return 0;
+    }
     View2 D{O_, M_, V_, nq_, core_n_, (int)n_, F_, nv_, vt_, eig_, f_};
     Inter J{jvv_, joo_, h_[0], h_[1], r_[0], r_[1], r_[2], x_[0], x_[1], x_[2]};
     if (mask & 2) {

@@ -3,8 +3,10 @@
 #pragma once
 #include <cuda_runtime.h>
 
+#include <array>
 #include <cstdint>
 #include <functional>
+#include <memory>
 #include <vector>
 
 #include "plan.h"
@@ -36,11 +38,14 @@ struct TcFlags {
     int xr_lin_d, xr_lin_x, xr_quad_d, xr_quad_x;
 };
 
+struct TcMm;
+
 class TwoChannel {
 public:
+    TwoChannel();
     ~TwoChannel();
     // Device tables of one system (the FindIndex table, plane-wave vectors, work arrays).
-    int init(const SystemHost &sys, cudaStream_t stream, TcAlloc alloc);
+    int init(const SystemHost &sys, const SolvePlan &plan, cudaStream_t stream, TcAlloc alloc);
     // The integrals of every later call: routine (TcRoutine), the fifteen flags, CoreN, GapII
     // and the screening distance of CasedERI.
     int set_integrals(int routine, const UegccdRangeTerms &flags, int core_n, double gapii, double screening);
@@ -82,12 +87,22 @@ private:
     double *ht_[2] = {nullptr, nullptr}, *hr_[2] = {nullptr, nullptr};
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
     int launches_ = 0;
+    // the residual as matrix products (two_channel_mm.cu): device arrays on the first CCD residual
+    // that can take that form; mm_state_ 0 not tried, 1 ready, -1 not for this system
+    std::unique_ptr<TcMm> mm_;
+    int mm_state_ = 0;
+    bool plain_ = false;        // no integral excluded, no core orbital
+    bool weights_ = false;      // mm_'s W holds the current integrals
+    std::vector<std::array<int, 3>> occ_;
+    std::vector<int4> pairs_;   // {Q, -Q} pairs of particle-hole groups: first row and rows of each
+    std::vector<int> ph_;       // rows i | x << 16
 
     int alloc(void **p, size_t bytes);
     int upload_t(const double *h, double *d);
     int residual(bool drpa, int mask);
     int read_out(int k, double *h);
     int diis_alloc(int ndiis);
+    bool mm_ready();
 };
 
 }  // namespace uegccd
