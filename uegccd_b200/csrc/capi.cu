@@ -288,6 +288,8 @@ struct UegccdBatch {
     std::vector<DevChunk> big;       // chunks of one large array each
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_solve0 = nullptr, ev_solve1 = nullptr;
+    Fork fork;                       // side streams of a small batch's residual (on first use)
+    bool fork_made = false;
     std::vector<double> red;         // host copy: 3 per solve
     std::vector<uint8_t> active;     // host copy
     double *dense[3] = {nullptr, nullptr, nullptr};  // reference-layout scratch of the largest solve
@@ -359,6 +361,11 @@ struct UegccdBatch {
         if (ev1) cudaEventDestroy(ev1);
         if (ev_solve0) cudaEventDestroy(ev_solve0);
         if (ev_solve1) cudaEventDestroy(ev_solve1);
+        if (fork.start) cudaEventDestroy(fork.start);
+        for (auto &e : fork.done)
+            if (e) cudaEventDestroy(e);
+        for (auto &x : fork.s)
+            if (x) cudaStreamDestroy(x);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -480,12 +487,14 @@ struct PhaseTrace {
     }
 };
 
-// The FP64 ladder's tiles (ladder.cu), the longest first so that the last wave is short.  A
-// block of up to 4 rows is one tile (or one per 256 columns); a larger one is cut into row tiles
-// of at most 16, and those into column tiles of so many passes that the batch makes at least
-// about four tiles per SM -- every column tile forms the block's H again, so a large batch keeps
-// a row tile whole.
-std::vector<LadderTile64> ladder_tiles(const std::vector<BlockDev> &blocks, int &max_rows)
+// The FP64 ladder's tiles (ladder.cu), form by form, those of one row count together (they run the
+// same code: CTAs of different ones evict each other's instructions) and the longest first, so
+// that the last wave is short.  A block of up to 4 rows is one tile (or one per 256 columns); a larger one is cut into
+// row tiles of at most 16, and those into column tiles of so many passes that the batch makes at
+// least about four tiles per SM -- every column tile forms the block's H again, so a large batch
+// keeps a row tile whole.
+std::vector<LadderTile64> ladder_tiles(const std::vector<BlockDev> &blocks, const std::vector<SolveDev> &solves,
+                                       int (&count)[2], int &max_rows)
 {
     constexpr int kSms = 148;
     int64_t passes = 0;
@@ -498,35 +507,31 @@ std::vector<LadderTile64> ladder_tiles(const std::vector<BlockDev> &blocks, int 
         passes += (int64_t)nt * ((h + rows + pc - 1) / pc);
     }
     const int per_tile = (int)std::max<int64_t>(1, std::min<int64_t>(passes / (4 * kSms), 1 << 16));
-    std::vector<LadderTile64> tiles;
-    std::vector<std::pair<float, int>> cost;
-    for (size_t k = 0; k < blocks.size(); k++) {
-        const BlockDev &B = blocks[k];
+    std::vector<LadderTile64> tiles[2];
+    std::vector<std::pair<float, int>> cost[2];
+    for (const BlockDev &B : blocks) {
         const int rows = B.nd + B.dg, h = B.nvd + B.sd;
-        if (rows <= kLadderFmaRows) {
-            const int w = kLadderFmaCols - rows;
-            for (int a0 = 0; a0 < h; a0 += w) {
-                const int a1 = std::min(h, a0 + w);
-                cost.emplace_back((float)h * ((rows + a1 - a0 + 31) / 32) * std::max(5, 1 + rows), (int)tiles.size());
-                tiles.push_back(LadderTile64{(int)k, a0, a1, 0, (int16_t)rows});
-            }
-            continue;
-        }
-        const int nt = row_tiles(rows), np = (rows + nt - 1) / nt, pc = ladder_pass_cols(np);
-        const int w = per_tile * pc - rows;
+        const SolveDev &S = solves[B.solve];
+        const int f = rows <= kLadderFmaRows ? 0 : 1, nt = f ? row_tiles(rows) : 1, np = (rows + nt - 1) / nt;
+        const int w = (f ? per_tile * ladder_pass_cols(np) : kLadderFmaCols) - rows;
         for (int p0 = 0; p0 < rows; p0 += np)
             for (int a0 = 0; a0 < h; a0 += w) {
                 const int a1 = std::min(h, a0 + w), n = std::min(np, rows - p0);
-                cost.emplace_back((float)h * ((rows + a1 - a0 + 31) / 32) * (np <= 8 ? 8 : 16), (int)tiles.size());
-                tiles.push_back(LadderTile64{(int)k, a0, a1, (int16_t)p0, (int16_t)n});
+                cost[f].emplace_back((f ? (n <= 8 ? 0 : 1) : rows) * 1e7f + (float)h * ((rows + a1 - a0 + 31) / 32),
+                                     (int)tiles[f].size());
+                tiles[f].push_back(LadderTile64{(int)B.t0, B.vir0, B.pair0, S.vtab0, B.solve, S.q2max, a0, a1, B.v,
+                                                B.nvd, B.sd, B.nd, B.dg, p0, n, 0});
             }
     }
-    std::sort(cost.begin(), cost.end(), [](const auto &x, const auto &y) {
-        return x.first != y.first ? x.first > y.first : x.second < y.second;
-    });
     std::vector<LadderTile64> out;
-    out.reserve(tiles.size());
-    for (const auto &c : cost) out.push_back(tiles[c.second]);
+    out.reserve(tiles[0].size() + tiles[1].size());
+    for (int f = 0; f < 2; f++) {
+        std::sort(cost[f].begin(), cost[f].end(), [](const auto &x, const auto &y) {
+            return x.first != y.first ? x.first > y.first : x.second < y.second;
+        });
+        for (const auto &c : cost[f]) out.push_back(tiles[f][c.second]);
+        count[f] = (int)tiles[f].size();
+    }
     return out;
 }
 
@@ -747,12 +752,13 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     DevBatch &d = b->d;
     d.nsolves = n;
     d.nblocks = (int)blocks.size();
-    int q2m = 0;
+    int q2m = 0, n2m = 0;
     for (const auto &P : b->plans) q2m = std::max(q2m, P.q2max);
+    for (const auto &v : nv4) n2m = std::max(n2m, v.x * v.x + v.y * v.y + v.z * v.z);
     d.q2max = q2m;
+    d.n2max = n2m;
     int max_rows = 0;
-    const std::vector<LadderTile64> ltiles = ladder_tiles(blocks, max_rows);
-    d.nltiles = (int)ltiles.size();
+    const std::vector<LadderTile64> ltiles = ladder_tiles(blocks, solves, d.nltiles, max_rows);
     d.ntc16 = (int)tc16.size();
     d.ntc32 = (int)tc32.size();
     d.ntc64 = (int)tc64.size();
@@ -774,8 +780,10 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     d.nrchunks = (int)rchunks.size();
     d.ntargets = (int)targets.size();
     d.max_v = max_v;
-    d.ladder_smem = ladder_smem_bytes(q2m, max_rows);
-    set_ladder_smem_limit(d.ladder_smem);
+    for (int f = 0; f < 2; f++) {
+        d.ladder_smem[f] = ladder_smem_bytes(q2m, n2m, max_rows, f);
+        set_ladder_smem_limit(d.ladder_smem[f]);
+    }
     // the |q|^2 table the mosaic kernel stages: the batch's largest (tables beyond 1024 entries
     // stay in global memory)
     d.mosaic_vt = std::min(q2m + 1, kVtabSmemEntries);
@@ -856,6 +864,8 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->upload(d.pair_i, pair_i))) return rc;
     if ((rc = b->upload(d.pair_j, pair_j))) return rc;
     if ((rc = b->upload(d.vir, vir))) return rc;
+    if ((rc = b->alloc(d.vpk, vir.size()))) return rc;
+    if ((rc = b->alloc(d.ppk, pair_i.size()))) return rc;
     if ((rc = b->alloc(d.pos, pos0))) return rc;
     if ((rc = b->alloc(d.partner, amp0))) return rc;
     if ((rc = b->alloc(d.mirror, amp0))) return rc;
@@ -1174,15 +1184,38 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
     return 0;
 }
 
+// The side streams on which a batch's rings, mosaics and DMMA ladders run beside its FMA
+// ladders: the kernels of a small batch leave most of the GPU idle, and the launches of a
+// residual only wait for one another.  A large batch fills the GPU with each kernel, and run
+// together they contend for the SMs and L2.  Solve times, one stream and side streams: one N=54
+// system 1.59 and 1.05 ms, 16 of them 4.60 and 4.41, 32 (7 M amplitudes) 7.87 and 7.77, 64
+// (14 M) 13.9 and 14.3; four N=114 systems (8.5 M) 15.0 and 14.1.
+constexpr int64_t kForkAmps = 9000000;
+const Fork *fork_of(UegccdBatch &b)
+{
+    if (b.d.namp > kForkAmps) return nullptr;
+    if (!b.fork_made) {
+        b.fork_made = true;
+        Fork &f = b.fork;
+        bool ok = cudaEventCreateWithFlags(&f.start, cudaEventDisableTiming) == cudaSuccess;
+        for (int k = 0; k < 3; k++)
+            ok = ok && cudaStreamCreateWithFlags(&f.s[k], cudaStreamNonBlocking) == cudaSuccess &&
+                 cudaEventCreateWithFlags(&f.done[k], cudaEventDisableTiming) == cudaSuccess;
+        if (!ok) cudaGetLastError();   // one stream then serves all
+    }
+    return b.fork.done[2] ? &b.fork : nullptr;
+}
+
 // Captures one iteration as a CUDA graph.
 int capture_iteration(UegccdBatch &b, const TermFlags &f, double tol, int max_iter, int ndiis)
 {
     UegccdBatch::GraphKey key{f.do_ring, f.do_xring, f.do_ladder, f.do_mosaic, f.drpa, ndiis, max_iter, f.mixed, tol};
     if (b.have_graph && b.gkey == key) return 0;
     if (b.gexec) { cudaGraphExecDestroy(b.gexec); b.gexec = nullptr; }
+    const Fork *fork = fork_of(b);
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal));
-    int nl = launch_iteration(b.d, b.ctl, f, tol, max_iter, ndiis, b.stream, nullptr);
+    int nl = launch_iteration(b.d, b.ctl, f, tol, max_iter, ndiis, b.stream, nullptr, fork);
     cudaError_t e = cudaStreamEndCapture(b.stream, &g);
     if (e != cudaSuccess) return fail(UEGCCD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
     e = cudaGraphInstantiate(&b.gexec, g, 0);
@@ -2110,7 +2143,7 @@ int uegccd_footprint(const UegccdSystem *sys, int32_t ndiis, int32_t mixed, int6
     }
     b += xy * 8 * 2 + O * V * 4 * 2;                 // xy, rx; ph_a, ph_b
     b += O * V * O * 4 * 2;                          // ring gather indices
-    b += nblk * (sizeof(BlockDev) + sizeof(LadderTile64)) + M * (16 + 8) + (P.q2max + 1) * 8;
+    b += sum_ov * 8 + nblk * (sizeof(BlockDev) + 2 * sizeof(LadderTile64)) + M * (16 + 8) + (P.q2max + 1) * 8;
     b += A * (8 + 4) * (int64_t)std::max(0, (int)ndiis);  // DIIS history (t' FP64, e FP32)
     if (mixed) {
         b += A * 8 * 2;                              // t_ref, g_ref

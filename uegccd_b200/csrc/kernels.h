@@ -19,11 +19,13 @@ struct DevBatch {
     int32_t *mt_start = nullptr, *mt_list = nullptr;
     size_t mosaic_smem = 0;
     int mosaic_vt = 0;  // |q|^2 table entries k_mosaic_blk stages: the batch's largest, at most kVtabSmemEntries
-    // FP64 ladder tiles (ladder.cu), longest first
+    // FP64 ladder tiles (ladder.cu): the FMA form's, then the DMMA form's, longest first
     LadderTile64 *ltiles = nullptr;
-    int nltiles = 0;
-    int q2max = 0;      // largest |q|^2 of the solves' tables
-    size_t ladder_smem = 0;
+    int nltiles[2] = {0, 0};
+    size_t ladder_smem[2] = {0, 0};
+    int q2max = 0, n2max = 0;   // largest |q|^2 of the solves' tables, largest |n|^2
+    int *vpk = nullptr;         // beside vir: the virtual's packed vector
+    int2 *ppk = nullptr;        // beside pair_i / pair_j: theirs
     int max_occ = 0;    // largest NOcc
     int64_t namp = 0;
     SolveDev *solves = nullptr;
@@ -110,11 +112,14 @@ constexpr int kLadderFmaRows = 4, kLadderMmaRows = 16;
 // of np rows
 constexpr int kLadderFmaCols = 256;
 constexpr int ladder_pass_cols(int np) { return np <= 8 ? 128 : 64; }
-// dynamic shared memory for |q|^2 tables up to q2max and blocks of at most max_rows rows i <= j
-size_t ladder_smem_bytes(int q2max, int max_rows);
+// dynamic shared memory for |q|^2 tables up to q2max, |n|^2 up to n2max and blocks of at most
+// max_rows rows i <= j; form 0 FMA, 1 DMMA
+size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form);
 void set_ladder_smem_limit(size_t bytes);
-// G of the rows i <= j: the particle-particle ladder of t (do_pp), the hole-hole one (do_hh)
-void launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st);
+// G of the rows i <= j: the particle-particle ladder of t (do_pp), the hole-hole one (do_hh); the
+// DMMA form on st_mma.  Returns the launches.
+int launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st,
+                  cudaStream_t st_mma);
 // dynamic shared memory of k_rings for NOcc = O and groups of n1 and n2 rows
 size_t rings_dmma_smem_bytes(int O, int n1, int n2, int q2max);
 // k_rings classes by padded pair size N1 + N2 (up to kRingClassRows), each with its
@@ -204,12 +209,18 @@ void launch_energy(const DevBatch &d, int kind, double csosex, cudaStream_t st);
 void launch_to_aaaa(const DevBatch &d, cudaStream_t st);
 // drows and colpos (pre-set to -1) of the dRPA sums from the blocks
 void launch_drpa_tables(const DevBatch &d, cudaStream_t st);
+// Side streams for the independent terms of a residual (nullptr: all on one stream).
+struct Fork {
+    cudaStream_t s[3] = {nullptr, nullptr, nullptr};   // rings, mosaics, DMMA ladders
+    cudaEvent_t start = nullptr, done[3] = {nullptr, nullptr, nullptr};
+};
 // Residual of the selected terms for d.t; mode 0 also updates d.t (with DIIS: the history).
-// Returns launches.
+// fork: the rings and the mosaics run beside the ladders.  Returns launches.
 struct CtlBuffers;
 // diis/ndiis (mode 0 only): fuse the Pulay DIIS push into the update kernel
 int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_out, cudaStream_t st,
-                    KernelTimer *kt = nullptr, const CtlBuffers *diis = nullptr, int ndiis = 0);
+                    KernelTimer *kt = nullptr, const CtlBuffers *diis = nullptr, int ndiis = 0,
+                    const Fork *fork = nullptr);
 void launch_pack(const DevBatch &d, int s, int namp, const double *dense, cudaStream_t st);
 void launch_vcoef(const DevBatch &d, cudaStream_t st);
 void launch_unpack_all(const DevBatch &d, const int64_t *dense_off, const double *t, double *out, cudaStream_t st);
@@ -236,7 +247,7 @@ void launch_refresh(const DevBatch &d, cudaStream_t st);
 void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
                  cudaStream_t st);
 int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f, double tol, int max_iter,
-                     int ndiis, cudaStream_t st, KernelTimer *kt);
+                     int ndiis, cudaStream_t st, KernelTimer *kt, const Fork *fork = nullptr);
 void launch_unpack(const DevBatch &d, int s, int namp, const double *t, double *ab, double *ba, double *aa,
                    cudaStream_t st);
 

@@ -1001,16 +1001,21 @@ struct UpdateArgs {
 // amplitude record (i, j, a, b), the position map entry (i, j, a) -> packed index, the
 // packed index of the partner (i, j, b), b in column pcol[c] of the same block, and the
 // mirror: (j, i, b) in row r + nd + dg for the rows r < nd (i < j); -1 on the diagonal
-// pair's row, -2 on the mirror rows.
+// pair's row, -2 on the mirror rows.  Beside them the packed vectors of the block's virtuals and
+// pairs.
 __global__ void k_block_tables(const BlockDev *__restrict__ blocks, const SolveDev *__restrict__ solves,
                                const int16_t *__restrict__ pair_i, const int16_t *__restrict__ pair_j,
                                const int16_t *__restrict__ vir, const int16_t *__restrict__ pcol,
-                               AmpInfo *__restrict__ amps, int32_t *__restrict__ pos, int32_t *__restrict__ partner,
-                               int32_t *__restrict__ mirror)
+                               const int *__restrict__ nvp, AmpInfo *__restrict__ amps, int32_t *__restrict__ pos,
+                               int32_t *__restrict__ partner, int32_t *__restrict__ mirror, int *__restrict__ vpk,
+                               int2 *__restrict__ ppk)
 {
     const BlockDev B = blocks[blockIdx.x];
     const SolveDev s = solves[B.solve];
     const int n = B.o * B.v;
+    for (int c = threadIdx.x; c < B.v; c += blockDim.x) vpk[B.vir0 + c] = nvp[s.orb0 + vir[B.vir0 + c]];
+    for (int r = threadIdx.x; r < B.o; r += blockDim.x)
+        ppk[B.pair0 + r] = make_int2(nvp[s.orb0 + pair_i[B.pair0 + r]], nvp[s.orb0 + pair_j[B.pair0 + r]]);
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
         const int r = e / B.v, c = e - r * B.v;
         const int i = pair_i[B.pair0 + r], j = pair_j[B.pair0 + r];
@@ -1111,8 +1116,8 @@ __global__ void k_rx_pos(const HChunkDev *__restrict__ chunks, const SolveDev *_
 void launch_block_tables(const DevBatch &d, cudaStream_t st)
 {
     if (d.nblocks > 0)
-        k_block_tables<<<d.nblocks, 256, 0, st>>>(d.blocks, d.solves, d.pair_i, d.pair_j, d.vir, d.pcol, d.amps,
-                                                  d.pos, d.partner, d.mirror);
+        k_block_tables<<<d.nblocks, 256, 0, st>>>(d.blocks, d.solves, d.pair_i, d.pair_j, d.vir, d.pcol, d.nvp,
+                                                  d.amps, d.pos, d.partner, d.mirror, d.vpk, d.ppk);
     if (d.nrpairs > 0) k_ph_tables<<<d.nrpairs, 128, 0, st>>>(d.rpairs, d.solves, d.ph_i, d.ph_x, d.ph_a, d.ph_b);
     if (d.nrpairs > 0 && d.nhchunks > 0)
         k_rx_pos<<<d.nhchunks, kChunk, 0, st>>>(d.hchunks, d.solves, d.amps, d.ph_a, d.ph_b, d.rpos);
@@ -1438,7 +1443,7 @@ __global__ void k_copy(int64_t n, const double *__restrict__ src, double *__rest
 void launch_refresh(const DevBatch &d, cudaStream_t st)
 {
     k_copy<<<(unsigned)((d.namp + 255) / 256), 256, 0, st>>>(d.namp, d.t, d.t_ref);
-    launch_ladder(d, d.t_ref, 1, 0, d.g_ref, st);
+    launch_ladder(d, d.t_ref, 1, 0, d.g_ref, st, st);
 }
 
 void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
@@ -1452,10 +1457,10 @@ void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_ite
 
 // One iteration: residual + update, control, [DIIS extrapolation].  Returns launches.
 int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f, double tol, int max_iter,
-                     int ndiis, cudaStream_t st, KernelTimer *kt)
+                     int ndiis, cudaStream_t st, KernelTimer *kt, const Fork *fork)
 {
     // the DIIS push (history slot and e . e_j partials) happens inside k_update
-    int n = launch_residual(d, f, 0, nullptr, st, kt, &c, ndiis);
+    int n = launch_residual(d, f, 0, nullptr, st, kt, &c, ndiis, fork);
     if (kt) kt->begin(KID_TAIL, st);
     launch_tail(d, c, tol, max_iter, ndiis, 0, st);
     if (kt) kt->end(st);
@@ -1726,16 +1731,21 @@ int tune_rings(DevBatch &d, cudaStream_t st)
 }
 
 int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_out, cudaStream_t st,
-                    KernelTimer *kt, const CtlBuffers *diis, int ndiis)
+                    KernelTimer *kt, const CtlBuffers *diis, int ndiis, const Fork *fork)
 {
     KernelTimer dummy;
     if (!kt) kt = &dummy;
     int n = 0;
+    const bool side = fork && !kt->on && !f.drpa && f.do_ladder && !f.mixed;
+    const cudaStream_t rs = side ? fork->s[0] : st, ms = side ? fork->s[1] : st, ls = side ? fork->s[2] : st;
+    if (side) {
+        cudaEventRecord(fork->start, st);
+        for (cudaStream_t x : fork->s) cudaStreamWaitEvent(x, fork->start, 0);
+    }
     if (f.do_ladder && d.nblocks > 0) {
         kt->begin(KID_LADDER, st);
-        launch_ladder(d, d.t, (f.do_pp && !f.mixed) ? 1 : 0, f.do_hh, d.g, st);
+        n += launch_ladder(d, d.t, (f.do_pp && !f.mixed) ? 1 : 0, f.do_hh, d.g, st, ls);
         kt->end(st);
-        n++;
         if (f.do_pp && f.mixed) {
             kt->begin(KID_LADDER_TC, st);
             launch_ladder_tc(d, d.t_ref, d.g_ref, d.tc_err, st);
@@ -1744,15 +1754,15 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         }
     }
     if (f.do_mosaic && !f.drpa) {
-        kt->begin(KID_MOSAIC_S, st);
-        k_mosaic_blk<<<d.nblocks, kMosThreads, d.mosaic_smem, st>>>(d.blocks, d.solves, d.pair_i, d.pair_j, d.vir,
+        kt->begin(KID_MOSAIC_S, ms);
+        k_mosaic_blk<<<d.nblocks, kMosThreads, d.mosaic_smem, ms>>>(d.blocks, d.solves, d.pair_i, d.pair_j, d.vir,
                                                                    d.nvp, d.vtab, d.t, d.pcol, d.mpart,
                                                                    d.active, d.mosaic_vt);
-        kt->end(st);
-        kt->begin(KID_MOSAIC_RED, st);
-        k_mosaic_sum<<<(d.ntargets + 7) / 8, 256, 0, st>>>(d.targets, d.ntargets, d.solves, d.mt_start, d.mt_list,
+        kt->end(ms);
+        kt->begin(KID_MOSAIC_RED, ms);
+        k_mosaic_sum<<<(d.ntargets + 7) / 8, 256, 0, ms>>>(d.targets, d.ntargets, d.solves, d.mt_start, d.mt_list,
                                                            d.mpart, d.jvv, d.joo, d.active);
-        kt->end(st);
+        kt->end(ms);
         n += 2;
     }
     if ((f.do_ring || f.do_mosaic) && f.drpa) {
@@ -1763,17 +1773,17 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         n++;
     }
     if ((f.do_ring || f.do_xring) && !f.drpa) {
-        kt->begin(KID_RING_STAGE, st);
-        k_ring_stage<<<d.nrpairs, d.stage_threads, 0, st>>>(d.spairs, d.solves, d.ph_i, d.ridx_x, d.ridx_y, d.t, d.xy,
+        kt->begin(KID_RING_STAGE, rs);
+        k_ring_stage<<<d.nrpairs, d.stage_threads, 0, rs>>>(d.spairs, d.solves, d.ph_i, d.ridx_x, d.ridx_y, d.t, d.xy,
                                                             d.active);
-        kt->end(st);
+        kt->end(rs);
         n++;
-        kt->begin(KID_RINGS, st);
+        kt->begin(KID_RINGS, rs);
         // pair classes (sorted in this order): DMMA tiles in two shared-memory sizes, then the FMA form
         int off = 0;
         for (int c = 0; c < kRingClasses; c++) {
             if (d.nring[c] > 0) {
-                k_rings<<<d.nring[c], d.ring_threads[c], d.ring_smem[c], st>>>(
+                k_rings<<<d.nring[c], d.ring_threads[c], d.ring_smem[c], rs>>>(
                     d.rpairs + off, d.solves, d.ph_i, d.ph_x, d.nvp, d.vtab, d.xy, f.do_ring, f.do_xring, d.rx,
                     d.active);
                 n++;
@@ -1781,12 +1791,18 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
             off += d.nring[c];
         }
         if (d.nring[kRingClasses] > 0) {
-            k_rings_wide<<<d.nring[kRingClasses], 256, d.ring_smem[kRingClasses], st>>>(d.rpairs + off, d.solves, d.ph_i, d.ph_x, d.pos,
+            k_rings_wide<<<d.nring[kRingClasses], 256, d.ring_smem[kRingClasses], rs>>>(d.rpairs + off, d.solves, d.ph_i, d.ph_x, d.pos,
                                                                  d.partner, d.nv4, d.vtab, d.t, f.do_ring,
                                                                  f.do_xring, d.rx, d.active);
             n++;
         }
-        kt->end(st);
+        kt->end(rs);
+    }
+    if (side) {
+        for (int k = 0; k < 3; k++) {
+            cudaEventRecord(fork->done[k], fork->s[k]);
+            cudaStreamWaitEvent(st, fork->done[k], 0);
+        }
     }
     UpdateArgs A;
     A.chunks = d.hchunks; A.solves = d.solves; A.amps = d.amps; A.mirror = d.mirror;

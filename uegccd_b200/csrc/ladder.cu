@@ -27,17 +27,18 @@
 // at N=54.  Tables beyond 256 entries (32 KB of copies) keep one copy, beyond 1,024 stay in
 // global memory.
 //
-// Two forms, by the rows i <= j of a block (one launch runs both, longest tiles first; a tile is
-// one CTA of 128 threads):
-//   1-4 rows    FP64 FMAs: a lane owns columns a, all rows; the s and d of a column c are
-//               broadcast reads.  Per 32 columns and c: two lookups (4 shared-memory cycles),
+// Two forms, by the rows i <= j of a block, one launch each (a tile is one CTA of 128 threads, the
+// longest tiles first):
+//   1-4 rows    FP64 FMAs: a lane owns two columns a, all rows; the s and d of a column c are
+//               broadcast reads (2 cycles a row).  Per 32 columns and c: two lookups (4 shared-memory cycles),
 //               2 + 2 rows FMA-pipe instructions (1 + rows cycles).  A DMMA tile would spend 8
 //               cycles however few rows fill its 8-wide fragment.
 //   5 and more  DMMA (mma.sync m8n8k4 f64; tcgen05 has no f64 kind), up to 16 rows a tile: each
 //               lane makes its own element of the two Coulomb fragments.  8 cycles per 8 rows.
-// Measured on 100 twists of N=54 (485 plane waves), the residual's ladders and hole-hole
-// intermediate together: LADDER_MS_AFTER against LADDER_MS_BEFORE for DMMA tiles over full
-// products with a separate hole-hole launch.
+// Measured per residual, ladders and hole-hole sums together, against DMMA tiles over the full
+// products with a separate hole-hole launch: 100 twists of N=54 (485 plane waves) 0.79 -> 0.38 ms
+// (FMA form 0.20, bound by its shared-memory reads: 0.15 ms of wavefronts; DMMA form 0.17, its
+// pipe 46% busy), four N=114 systems 0.70 -> 0.25 ms, 100 twists of N=14 21 -> 10.5 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -52,7 +53,8 @@ namespace uegccd {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kKC = 32;            // columns c per staged chunk
+constexpr int kKC = 32;            // columns c per staged chunk, DMMA form (double-buffered)
+constexpr int kFC = 256;           // the same, FMA form
 constexpr int kLd = kKC + 4;       // row stride of the DMMA operands: = 4 mod 16 doubles, conflict-free
 constexpr int kHLd = 36;           // row stride of H (at most 32 pairs q <= q'): likewise
 
@@ -71,6 +73,8 @@ struct Col {
     int m2, base;
 };
 
+// With 16 copies every |n|^2 is at most 127 (launch_ladder's rule): the column side carries it
+// in its fourth byte, against a 1 on the row side.
 template <int TAB>
 __device__ __forceinline__ Col make_col(int packed)
 {
@@ -78,26 +82,35 @@ __device__ __forceinline__ Col make_col(int packed)
     const int n2 = x * x + y * y + z * z;
     Col c;
     c.m2 = ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16);   // |n_d| <= 63
+    if (TAB == kTab16) c.m2 |= 1 << 24;
     c.base = TAB == kTab16 ? (n2 << 7) + ((threadIdx.x & 15) << 3) : TAB == kTab1 ? n2 << 3 : n2;
     return c;
 }
+template <int TAB>
+__device__ __forceinline__ int col_side(int packed)
+{
+    return TAB == kTab16 ? packed | (__dp4a(packed, packed, 0) << 24) : packed;
+}
 
-// v(a - c): packed c and |c|^2
+// v(a - c), c a column side; c2 = |c|^2 where it is not in the fourth byte
 template <int TAB>
 __device__ __forceinline__ double lookup(const char *tab, const double *__restrict__ gtab, const Col &a, int c, int c2)
 {
-    const int d = __dp4a(a.m2, c, c2);
+    const int d = __dp4a(a.m2, c, TAB == kTab16 ? 0 : c2);
     if (TAB == kTab16) return *reinterpret_cast<const double *>(tab + (a.base + (d << 7)));
     if (TAB == kTab1) return *reinterpret_cast<const double *>(tab + (a.base + (d << 3)));
     return __ldg(gtab + a.base + d);
 }
+template <int TAB>
+__device__ __forceinline__ double lookup(const char *tab, const double *__restrict__ gtab, const Col &a, int packed)
+{
+    return lookup<TAB>(tab, gtab, a, col_side<TAB>(packed), __dp4a(packed, packed, 0));
+}
 
 struct Args {
     const LadderTile64 *tiles;
-    const BlockDev *blocks;
-    const SolveDev *solves;
-    const int16_t *vir, *pair_i, *pair_j;
-    const int *nvp;
+    const int *vpk;          // packed vectors beside vir
+    const int2 *ppk;         // packed vectors of i and j beside the pairs
     const double *vtab, *t;
     double *g;
     const uint8_t *active;
@@ -107,51 +120,89 @@ struct Args {
 // What both forms use of a tile's block.
 struct Blk {
     LadderTile64 T;
-    BlockDev B;
-    int orow, h;             // rows i <= j; columns c <= pc
+    int h;                   // columns c <= pc
     int nh, ncol;            // the tile's columns: nh pairs q <= q' of H, then the virtuals a0 .. a1
     const double *t;         // the block's amplitudes
-    const int *nvp;          // the solve's packed vectors
     const double *gtab;      // the solve's |q|^2 table
-    const int16_t *vir, *pi, *pj;
+    const int *vpk;
+    const int2 *ppk;
 };
 
 __device__ __forceinline__ int packed_col(const Blk &K, int e)
 {
     e = min(e, K.ncol - 1);   // lanes past the tile repeat its last column
-    return e < K.nh ? K.nvp[K.pi[e]] : K.nvp[K.vir[K.T.a0 + e - K.nh]];
+    return e < K.nh ? __ldg(&K.ppk[e].x) : __ldg(&K.vpk[K.T.a0 + e - K.nh]);
 }
 
-// One column c <= pc as both forms stage it: {c, |c|^2, pc, |pc|^2}, packed vectors.
-__device__ __forceinline__ int4 chunk_col(const Blk &K, int c)
+// One column c <= pc as both forms stage it: the column sides of c and pc.
+template <int TAB>
+__device__ __forceinline__ int2 chunk_col(const Blk &K, int c)
 {
     c = min(c, K.h - 1);   // past the end the staged amplitudes are zero
-    const int n = K.nvp[K.vir[c]], p = K.nvp[K.vir[c < K.B.nvd ? c + K.h : c]];
-    return make_int4(n, __dp4a(n, n, 0), p, __dp4a(p, p, 0));
+    return make_int2(col_side<TAB>(__ldg(&K.vpk[c])), col_side<TAB>(__ldg(&K.vpk[c < K.T.nvd ? c + K.h : c])));
 }
 
 __device__ __forceinline__ void load_pair(const Blk &K, int row, int c, double &x, double &y)
 {
-    const double *r = K.t + (int64_t)row * K.B.v;
+    const double *r = K.t + row * K.T.v;
     x = c < K.h ? __ldg(r + c) : 0.0;
-    y = c < K.B.nvd ? __ldg(r + c + K.h) : 0.0;
+    y = c < K.T.nvd ? __ldg(r + c + K.h) : 0.0;
+}
+
+// The |c|^2 of two column sides that do not carry them
+template <int TAB>
+__device__ __forceinline__ int2 norms(int2 c)
+{
+    return TAB == kTab16 ? make_int2(0, 0) : make_int2(__dp4a(c.x, c.x, 0), __dp4a(c.y, c.y, 0));
+}
+
+// The tile's block; false when its solve is not active.
+__device__ __forceinline__ bool open_tile(const Args &A, Blk &K)
+{
+    const int4 *p = reinterpret_cast<const int4 *>(A.tiles + blockIdx.x);
+    int4 *q = reinterpret_cast<int4 *>(&K.T);
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(LadderTile64) / sizeof(int4)); k++) q[k] = __ldg(p + k);
+    if (!A.active[K.T.solve]) return false;
+    K.h = K.T.nvd + K.T.sd;
+    K.nh = A.do_hh ? K.T.nd + K.T.dg : 0;
+    K.ncol = K.nh + K.T.a1 - K.T.a0;
+    K.t = A.t + K.T.t0;
+    K.gtab = A.vtab + K.T.vtab0;
+    K.vpk = A.vpk + K.T.vir0;
+    K.ppk = A.ppk + K.T.pair0;
+    return true;
+}
+
+template <int TAB>
+__device__ __forceinline__ void fill_table(const Blk &K, char *smem)
+{
+    double *tab = reinterpret_cast<double *>(smem);
+    if (TAB == kTab16)
+        for (int e = threadIdx.x; e < (K.T.q2max + 1) * 16; e += kThreads) tab[e] = __ldg(K.gtab + (e >> 4));
+    else if (TAB == kTab1)
+        for (int e = threadIdx.x; e <= K.T.q2max; e += kThreads) tab[e] = __ldg(K.gtab + e);
 }
 
 // ---- 1 to 4 rows ------------------------------------------------------------------------
+// Units of 32 columns, two a lane: the broadcast reads of s and d serve both.  (Four a lane, more
+// registers and code, measured the same; so did 24 to 32 warps an SM.)
+constexpr int kUnits = 2;
+
 template <int TAB, int R, int U>
-__device__ __forceinline__ void fma_cols(double (&P)[2][R], double (&M)[2][R], const Col (&a)[2], const char *tab,
-                                         const double *gtab, const int4 *cl, const double2 *sd, int k0, int step,
+__device__ __forceinline__ void fma_cols(double (&P)[kUnits][R], double (&M)[kUnits][R], const Col (&a)[kUnits], const char *tab,
+                                         const double *gtab, const int2 *cl, const double2 *sd, int k0, int step,
                                          int n)
 {
-#pragma unroll 2
+#pragma unroll 1
     for (int k = k0; k < n; k += step) {
-        const int4 c = cl[k];
+        const int2 c = cl[k], c2 = norms<TAB>(c);
         double2 x[R];
 #pragma unroll
         for (int r = 0; r < R; r++) x[r] = sd[k * R + r];
 #pragma unroll
         for (int m = 0; m < U; m++) {
-            const double v = lookup<TAB>(tab, gtab, a[m], c.x, c.y), w = lookup<TAB>(tab, gtab, a[m], c.z, c.w);
+            const double v = lookup<TAB>(tab, gtab, a[m], c.x, c2.x), w = lookup<TAB>(tab, gtab, a[m], c.y, c2.y);
             const double wp = v + w, wm = v - w;
 #pragma unroll
             for (int r = 0; r < R; r++) {
@@ -162,82 +213,89 @@ __device__ __forceinline__ void fma_cols(double (&P)[2][R], double (&M)[2][R], c
     }
 }
 
-// smem: 2 x kKC int4 column records, 2 x kKC x R double2 amplitudes, H, then the reduction area
+// smem: H, kFC int2 column records, then kFC x R double2 amplitudes (the reduction area once they
+// are read)
 template <int TAB, int R>
-__device__ void ladder_fma(const Args &A, const Blk &K, const char *tab, char *smem)
+__device__ __forceinline__ void ladder_fma(const Args &A, const Blk &K, const char *tab, char *smem)
 {
-    int4 *cl = reinterpret_cast<int4 *>(smem);
-    double2 *sd = reinterpret_cast<double2 *>(smem + 2 * kKC * sizeof(int4));
-    double2 *hs = sd + 2 * kKC * R;
-    double *red = reinterpret_cast<double *>(hs + R * R);
+    constexpr int UM = kUnits;
+    double2 *hs = reinterpret_cast<double2 *>(smem);
+    int2 *cl = reinterpret_cast<int2 *>(hs + R * R);
+    double2 *sd = reinterpret_cast<double2 *>(cl + kFC);
+    double *red = reinterpret_cast<double *>(sd);
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    // units of 32 columns, two a warp; with one or two such groups the warps split the columns c
-    const int groups = (K.ncol + 63) >> 6;
+    // the units go to the warps in even groups; with one or two groups the warps split the columns c
+    const int units = (K.ncol + 31) >> 5, groups = (units + UM - 1) / UM, upg = (units + groups - 1) / groups;
     const int ks = groups == 1 ? 4 : groups == 2 ? 2 : 1;
-    const int grp = warp / ks, split = warp - grp * ks;
-    const bool on = grp < groups && (A.do_pp || grp == 0);
-    const bool two = grp * 64 + 32 < K.ncol;
-    Col a[2];
-    a[0] = make_col<TAB>(packed_col(K, grp * 64 + lane));
-    a[1] = make_col<TAB>(packed_col(K, grp * 64 + 32 + lane));
-    double P[2][R], M[2][R];
+    const int grp = warp / ks, split = warp - grp * ks, u0 = grp * upg;
+    const int nu = grp < groups ? min(upg, units - u0) : 0;
+    const bool on = nu > 0 && (A.do_pp || grp == 0);
+    // a chunk's amplitudes and column records, all threads; most blocks are one chunk
+    auto stage = [&](int c0, int n) {
 #pragma unroll
-    for (int m = 0; m < 2; m++)
+        for (int r = 0; r < R; r++)
+            for (int k = threadIdx.x; k < n; k += kThreads) {
+                double x, y;
+                load_pair(K, r, c0 + k, x, y);
+                sd[k * R + r] = make_double2(0.5 * (x + y), c0 + k < K.T.nvd ? 0.5 * (x - y) : 0.0);
+            }
+        for (int k = threadIdx.x; k < n; k += kThreads) cl[k] = chunk_col<TAB>(K, c0 + k);
+    };
+    fill_table<TAB>(K, const_cast<char *>(tab));
+    Col a[UM];
+#pragma unroll
+    for (int m = 0; m < UM; m++) a[m] = make_col<TAB>(packed_col(K, (u0 + m) * 32 + lane));
+    double P[UM][R], M[UM][R];
+#pragma unroll
+    for (int m = 0; m < UM; m++)
 #pragma unroll
         for (int r = 0; r < R; r++) P[m][r] = M[m][r] = 0.0;
-    const int nchunk = (K.h + kKC - 1) / kKC;
-    double x = 0.0, y = 0.0;
-    int4 rec = make_int4(0, 0, 0, 0);
-    auto fetch = [&](int j) {
-        if (warp < R) load_pair(K, warp, j * kKC + lane, x, y);
-        if (warp == 3) rec = chunk_col(K, j * kKC + lane);
-    };
-    fetch(0);
-    for (int j = 0; j < nchunk; j++) {
-        const int b = (j & 1) * kKC, c = j * kKC + lane;
-        if (warp < R) sd[(b + lane) * R + warp] = make_double2(0.5 * (x + y), c < K.B.nvd ? 0.5 * (x - y) : 0.0);
-        if (warp == 3) cl[b + lane] = rec;
+    for (int c0 = 0; c0 < K.h; c0 += kFC) {
+        const int n = min(kFC, K.h - c0);
+        if (c0 > 0) __syncthreads();
+        stage(c0, n);
         __syncthreads();
-        if (j + 1 < nchunk) fetch(j + 1);
-        if (on) {
-            const int n = min(kKC, K.h - j * kKC);
-            if (two) fma_cols<TAB, R, 2>(P, M, a, tab, K.gtab, cl + b, sd + b * R, split, ks, n);
-            else fma_cols<TAB, R, 1>(P, M, a, tab, K.gtab, cl + b, sd + b * R, split, ks, n);
-        }
+        if (!on) continue;
+        if (nu == 2) fma_cols<TAB, R, 2>(P, M, a, tab, K.gtab, cl, sd, split, ks, n);
+        else fma_cols<TAB, R, 1>(P, M, a, tab, K.gtab, cl, sd, split, ks, n);
     }
     if (ks > 1) {
         // the splits' sums into the first one's, in order
-        auto at = [&](int sp, int m, int r, int q) -> double & {
-            return red[((((sp - 1) * 2 + grp) * 2 + m) * R + r) * 64 + q * 32 + lane];
-        };
-        if (split > 0 && grp < groups)
-#pragma unroll
-            for (int m = 0; m < 2; m++)
-#pragma unroll
-                for (int r = 0; r < R; r++) {
-                    at(split, m, r, 0) = P[m][r];
-                    at(split, m, r, 1) = M[m][r];
-                }
         __syncthreads();
-        if (split == 0 && grp < groups)
-            for (int sp = 1; sp < ks; sp++)
+        auto at = [&](int sp, int m, int r, int q) -> double & {
+            return red[((((sp - 1) * groups + grp) * UM + m) * R + r) * 64 + q * 32 + lane];
+        };
+        if (split > 0)
 #pragma unroll
-                for (int m = 0; m < 2; m++)
+            for (int m = 0; m < UM; m++)
+                if (m < nu)
 #pragma unroll
                     for (int r = 0; r < R; r++) {
-                        P[m][r] += at(sp, m, r, 0);
-                        M[m][r] += at(sp, m, r, 1);
+                        at(split, m, r, 0) = P[m][r];
+                        at(split, m, r, 1) = M[m][r];
                     }
+        __syncthreads();
+        if (split == 0)
+            for (int sp = 1; sp < ks; sp++)
+#pragma unroll
+                for (int m = 0; m < UM; m++)
+                    if (m < nu)
+#pragma unroll
+                        for (int r = 0; r < R; r++) {
+                            P[m][r] += at(sp, m, r, 0);
+                            M[m][r] += at(sp, m, r, 1);
+                        }
     }
-    const bool lead = split == 0 && grp < groups;
+    const bool lead = split == 0;
     if (K.nh > 0) {
         // halves of H: (H[p][q] +- H[p][q'])/2
         if (lead && grp == 0 && lane < K.nh) {
-            const Col kq = make_col<TAB>(K.nvp[K.pi[lane]]), lq = make_col<TAB>(K.nvp[K.pj[lane]]);
+            const int2 pk = __ldg(&K.ppk[lane]);
+            const Col kq = make_col<TAB>(pk.x), lq = make_col<TAB>(pk.y);
 #pragma unroll
             for (int r = 0; r < R; r++) {
-                const int n = K.nvp[K.pi[r]], n2 = __dp4a(n, n, 0);
-                const double v = lookup<TAB>(tab, K.gtab, kq, n, n2), w = lookup<TAB>(tab, K.gtab, lq, n, n2);
+                const int n = __ldg(&K.ppk[r].x);
+                const double v = lookup<TAB>(tab, K.gtab, kq, n), w = lookup<TAB>(tab, K.gtab, lq, n);
                 hs[r * R + lane] = make_double2(P[0][r] + 0.5 * (v + w), M[0][r] + 0.5 * (v - w));
             }
         }
@@ -245,10 +303,10 @@ __device__ void ladder_fma(const Args &A, const Blk &K, const char *tab, char *s
     }
     if (!lead) return;
 #pragma unroll
-    for (int m = 0; m < 2; m++) {
-        const int e = grp * 64 + m * 32 + lane, c = K.T.a0 + e - K.nh;
-        if (e < K.nh || e >= K.ncol) continue;
-        const bool pair = c < K.B.nvd;
+    for (int m = 0; m < UM; m++) {
+        const int e = (u0 + m) * 32 + lane, c = K.T.a0 + e - K.nh;
+        if (m >= nu || e < K.nh || e >= K.ncol) continue;
+        const bool pair = c < K.T.nvd;
         double p[R], q[R];
 #pragma unroll
         for (int r = 0; r < R; r++) {
@@ -258,9 +316,9 @@ __device__ void ladder_fma(const Args &A, const Blk &K, const char *tab, char *s
         if (K.nh > 0)
 #pragma unroll
             for (int k = 0; k < R; k++) {
-                const double *row = K.t + (int64_t)k * K.B.v;
+                const double *row = K.t + k * K.T.v;
                 const double u = __ldg(row + c), w = pair ? __ldg(row + c + K.h) : u;
-                const double f = k < K.B.nd ? 1.0 : 0.5;   // the pair and its mirror, or the diagonal pair
+                const double f = k < K.T.nd ? 1.0 : 0.5;   // the pair and its mirror, or the diagonal pair
                 const double s = f * (u + w), d = f * (u - w);
 #pragma unroll
                 for (int r = 0; r < R; r++) {
@@ -269,11 +327,11 @@ __device__ void ladder_fma(const Args &A, const Blk &K, const char *tab, char *s
                     q[r] = fma(H.y, d, q[r]);
                 }
             }
-        double *out = A.g + K.B.t0 + c;
+        double *out = A.g + K.T.t0 + c;
 #pragma unroll
         for (int r = 0; r < R; r++) {
-            out[(int64_t)r * K.B.v] = p[r] + q[r];
-            if (pair) out[(int64_t)r * K.B.v + K.h] = p[r] - q[r];
+            out[r * K.T.v] = p[r] + q[r];
+            if (pair) out[r * K.T.v + K.h] = p[r] - q[r];
         }
     }
 }
@@ -282,16 +340,18 @@ __device__ void ladder_fma(const Args &A, const Blk &K, const char *tab, char *s
 // NN fragments of 8 rows; a warp covers MF fragments of 8 columns, the CTA 4 warps of them a
 // pass.  Fragment layouts (PTX ISA, m8n8k4 .f64): A row = lane/4, col = lane%4; B row (k) =
 // lane%4, col = lane/4; C row = lane/4, cols 2*(lane%4) + {0,1}.
-// smem: 2 x kKC int4 column records, s and d of 2 x 8 NN rows, the halves of H (16 rows each)
+// smem: 2 x kKC int2 column records, s and d of 2 x 8 NN rows, the halves of H (8 NN rows each)
 template <int TAB, int NN>
-__device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *smem)
+__device__ __forceinline__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *smem)
 {
     constexpr int MF = NN == 1 ? 4 : 2, WC = 8 * MF, PC = 4 * WC, NR = 8 * NN;
-    int4 *cl = reinterpret_cast<int4 *>(smem);
-    double *S = reinterpret_cast<double *>(smem + 2 * kKC * sizeof(int4)), *D = S + 2 * NR * kLd;
+    int2 *cl = reinterpret_cast<int2 *>(smem);
+    double *S = reinterpret_cast<double *>(cl + 2 * kKC), *D = S + 2 * NR * kLd;
     double *hs = D + 2 * NR * kLd, *hd = hs + NR * kHLd;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, gid = lane >> 2, tig = lane & 3;
-    const int nchunk = (K.h + kKC - 1) / kKC, np = K.T.np, p0 = K.T.p0;
+    const int nchunk = (K.h + kKC - 1) / kKC, np = K.T.np, p0 = K.T.p0, orow = K.T.nd + K.T.dg;
+    fill_table<TAB>(K, const_cast<char *>(tab));
+    __syncthreads();
     for (int e0 = 0; e0 < K.ncol; e0 += PC) {
         const int base = e0 + warp * WC;
         const bool loop = A.do_pp || (e0 == 0 && K.nh > 0);
@@ -306,7 +366,7 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
             for (int n = 0; n < NN; n++) P[m][n][0] = P[m][n][1] = M[m][n][0] = M[m][n][1] = 0.0;
         if (loop) {
             double x[2 * NN], y[2 * NN];
-            int4 rec = make_int4(0, 0, 0, 0);
+            int2 rec = make_int2(0, 0);
             auto fetch = [&](int j) {
 #pragma unroll
                 for (int k = 0; k < 2 * NN; k++) {
@@ -314,7 +374,7 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
                     x[k] = y[k] = 0.0;
                     if (r < np) load_pair(K, p0 + r, j * kKC + lane, x[k], y[k]);
                 }
-                if (warp == 0) rec = chunk_col(K, j * kKC + lane);
+                if (warp == 0) rec = chunk_col<TAB>(K, j * kKC + lane);
             };
             fetch(0);
             for (int j = 0; j < nchunk; j++) {
@@ -323,7 +383,7 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
                 for (int k = 0; k < 2 * NN; k++) {
                     const int r = warp + 4 * k;
                     S[(b * NR + r) * kLd + lane] = 0.5 * (x[k] + y[k]);
-                    D[(b * NR + r) * kLd + lane] = c < K.B.nvd ? 0.5 * (x[k] - y[k]) : 0.0;
+                    D[(b * NR + r) * kLd + lane] = c < K.T.nvd ? 0.5 * (x[k] - y[k]) : 0.0;
                 }
                 if (warp == 0) cl[b * kKC + lane] = rec;
                 __syncthreads();
@@ -333,7 +393,7 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
                     const int n4 = min(kKC, K.h - j * kKC);
 #pragma unroll 2
                     for (int k = 0; k < n4; k += 4) {
-                        const int4 cc = cl[b * kKC + k + tig];
+                        const int2 cc = cl[b * kKC + k + tig], c2 = norms<TAB>(cc);
                         double bs[NN], bd[NN];
 #pragma unroll
                         for (int n = 0; n < NN; n++) {
@@ -342,8 +402,8 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
                         }
 #pragma unroll
                         for (int m = 0; m < MF; m++) {
-                            const double v = lookup<TAB>(tab, K.gtab, a[m], cc.x, cc.y);
-                            const double w = lookup<TAB>(tab, K.gtab, a[m], cc.z, cc.w);
+                            const double v = lookup<TAB>(tab, K.gtab, a[m], cc.x, c2.x);
+                            const double w = lookup<TAB>(tab, K.gtab, a[m], cc.y, c2.y);
                             const double wp = v + w, wm = v - w;
 #pragma unroll
                             for (int n = 0; n < NN; n++) {
@@ -361,7 +421,8 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
             for (int m = 0; m < MF; m++) {
                 const int q = base + m * 8 + gid;
                 if (q >= K.nh) continue;
-                const Col kq = make_col<TAB>(K.nvp[K.pi[q]]), lq = make_col<TAB>(K.nvp[K.pj[q]]);
+                const int2 pk = __ldg(&K.ppk[q]);
+                const Col kq = make_col<TAB>(pk.x), lq = make_col<TAB>(pk.y);
 #pragma unroll
                 for (int n = 0; n < NN; n++)
 #pragma unroll
@@ -369,9 +430,9 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
                         const int r = n * 8 + 2 * tig + u;
                         double hp = 0.0, hm = 0.0;
                         if (r < np) {
-                            const int nn = K.nvp[K.pi[p0 + r]], n2 = __dp4a(nn, nn, 0);
-                            const double v = lookup<TAB>(tab, K.gtab, kq, nn, n2);
-                            const double w = lookup<TAB>(tab, K.gtab, lq, nn, n2);
+                            const int nn = __ldg(&K.ppk[p0 + r].x);
+                            const double v = lookup<TAB>(tab, K.gtab, kq, nn);
+                            const double w = lookup<TAB>(tab, K.gtab, lq, nn);
                             hp = P[m][n][u] + 0.5 * (v + w);
                             hm = M[m][n][u] + 0.5 * (v - w);
                         }
@@ -388,11 +449,11 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
 #pragma unroll
                     for (int n = 0; n < NN; n++) P[m][n][0] = P[m][n][1] = M[m][n][0] = M[m][n][1] = 0.0;
             if (K.nh > 0) {
-                for (int q0 = 0; q0 < K.orow; q0 += 4) {
+                for (int q0 = 0; q0 < orow; q0 += 4) {
                     const int q = q0 + tig;
-                    const bool qok = q < K.orow;
-                    const double *row = K.t + (int64_t)(qok ? q : 0) * K.B.v;
-                    const double f = q < K.B.nd ? 1.0 : 0.5;   // the pair and its mirror, or the diagonal pair
+                    const bool qok = q < orow;
+                    const double *row = K.t + (qok ? q : 0) * K.T.v;
+                    const double f = q < K.T.nd ? 1.0 : 0.5;   // the pair and its mirror, or the diagonal pair
                     double bs[NN], bd[NN];
 #pragma unroll
                     for (int n = 0; n < NN; n++) {
@@ -404,7 +465,7 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
                         const int e = base + m * 8 + gid, c = K.T.a0 + e - K.nh;
                         double s = 0.0, d = 0.0;
                         if (qok && e >= K.nh && e < K.ncol) {
-                            const double u = __ldg(row + c), w = c < K.B.nvd ? __ldg(row + c + K.h) : u;
+                            const double u = __ldg(row + c), w = c < K.T.nvd ? __ldg(row + c + K.h) : u;
                             s = f * (u + w);
                             d = f * (u - w);
                         }
@@ -420,16 +481,16 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
             for (int m = 0; m < MF; m++) {
                 const int e = base + m * 8 + gid, c = K.T.a0 + e - K.nh;
                 if (e < K.nh || e >= K.ncol) continue;
-                double *out = A.g + K.B.t0 + c;
+                double *out = A.g + K.T.t0 + c;
 #pragma unroll
                 for (int n = 0; n < NN; n++)
 #pragma unroll
                     for (int u = 0; u < 2; u++) {
                         const int r = n * 8 + 2 * tig + u;
                         if (r >= np) continue;
-                        double *o = out + (int64_t)(p0 + r) * K.B.v;
+                        double *o = out + (p0 + r) * K.T.v;
                         o[0] = P[m][n][u] + M[m][n][u];
-                        if (c < K.B.nvd) o[K.h] = P[m][n][u] - M[m][n][u];
+                        if (c < K.T.nvd) o[K.h] = P[m][n][u] - M[m][n][u];
                     }
             }
         }
@@ -438,39 +499,13 @@ __device__ void ladder_mma(const Args &A, const Blk &K, const char *tab, char *s
 }
 
 template <int TAB>
-__global__ void __launch_bounds__(kThreads, 5) k_ladder(Args A)
+__global__ void __launch_bounds__(kThreads, 7) k_ladder_fma(Args A)
 {
     Blk K;
-    K.T = A.tiles[blockIdx.x];
-    K.B = A.blocks[K.T.blk];
-    if (!A.active[K.B.solve]) return;
-    const SolveDev &s = A.solves[K.B.solve];
-    K.orow = K.B.nd + K.B.dg;
-    K.h = K.B.nvd + K.B.sd;
-    K.nh = A.do_hh ? K.orow : 0;
-    K.ncol = K.nh + K.T.a1 - K.T.a0;
-    K.t = A.t + K.B.t0;
-    K.nvp = A.nvp + s.orb0;
-    K.gtab = A.vtab + s.vtab0;
-    K.vir = A.vir + K.B.vir0;
-    K.pi = A.pair_i + K.B.pair0;
-    K.pj = A.pair_j + K.B.pair0;
+    if (!open_tile(A, K)) return;
     extern __shared__ __align__(16) char lsm[];
-    if (TAB == kTab16) {
-        double *tab = reinterpret_cast<double *>(lsm);
-        for (int e = threadIdx.x; e < (s.q2max + 1) * 16; e += kThreads) tab[e] = __ldg(K.gtab + (e >> 4));
-    } else if (TAB == kTab1) {
-        double *tab = reinterpret_cast<double *>(lsm);
-        for (int e = threadIdx.x; e <= s.q2max; e += kThreads) tab[e] = __ldg(K.gtab + e);
-    }
-    __syncthreads();
     char *sm = lsm + A.tab_bytes;
-    if (K.orow > kLadderFmaRows) {
-        if (K.T.np <= 8) ladder_mma<TAB, 1>(A, K, lsm, sm);
-        else ladder_mma<TAB, 2>(A, K, lsm, sm);
-        return;
-    }
-    switch (K.orow) {
+    switch (K.T.nd + K.T.dg) {
     case 1: ladder_fma<TAB, 1>(A, K, lsm, sm); break;
     case 2: ladder_fma<TAB, 2>(A, K, lsm, sm); break;
     case 3: ladder_fma<TAB, 3>(A, K, lsm, sm); break;
@@ -478,23 +513,42 @@ __global__ void __launch_bounds__(kThreads, 5) k_ladder(Args A)
     }
 }
 
-int tab_form(int q2max) { return q2max < 256 ? kTab16 : q2max < 1024 ? kTab1 : kTabGlobal; }
-int tab_bytes(int q2max)
+template <int TAB>
+__global__ void __launch_bounds__(kThreads, 5) k_ladder_mma(Args A)
 {
-    const int f = tab_form(q2max);
-    return f == kTab16 ? (q2max + 1) * 128 : f == kTab1 ? ((q2max + 1) * 8 + 15) / 16 * 16 : 0;
+    Blk K;
+    if (!open_tile(A, K)) return;
+    extern __shared__ __align__(16) char lsm[];
+    char *sm = lsm + A.tab_bytes;
+    if (K.T.np <= 8) ladder_mma<TAB, 1>(A, K, lsm, sm);
+    else ladder_mma<TAB, 2>(A, K, lsm, sm);
+}
+
+int tab_form(int q2max, int n2max) { return q2max < 256 && n2max < 128 ? kTab16 : q2max < 1024 ? kTab1 : kTabGlobal; }
+int tab_bytes(int form, int q2max)
+{
+    return form == kTab16 ? (q2max + 1) * 128 : form == kTab1 ? ((q2max + 1) * 8 + 15) / 16 * 16 : 0;
+}
+
+size_t fma_bytes(int r)
+{
+    const int ks_units = 3 * kUnits;   // three splits of one group; two groups in two splits need less
+    return sizeof(double2) * r * r + sizeof(int2) * kFC +
+           std::max(sizeof(double2) * kFC * r, sizeof(double) * ks_units * r * 64);
 }
 
 }  // namespace
 
-size_t ladder_smem_bytes(int q2max, int max_rows)
+size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form)
 {
-    const size_t cols = 2 * kKC * sizeof(int4);
-    const int r = std::min(max_rows, kLadderFmaRows), nr = max_rows <= 8 ? 8 : 16;
-    // the FMA form's reduction area: 3 splits of one group of 64 columns, or 1 of two
-    size_t b = cols + sizeof(double2) * (2 * kKC * r + r * r) + sizeof(double) * (3 * 2 * 2 * r * 64);
-    if (max_rows > kLadderFmaRows) b = std::max(b, cols + sizeof(double) * (2 * 2 * (size_t)nr * kLd + 2 * (size_t)nr * kHLd));
-    return tab_bytes(q2max) + b;
+    const size_t tab = tab_bytes(tab_form(q2max, n2max), q2max);
+    if (form == 0) {
+        size_t b = 0;
+        for (int r = 1; r <= std::min(max_rows, kLadderFmaRows); r++) b = std::max(b, fma_bytes(r));
+        return tab + b;
+    }
+    const int nr = max_rows <= 8 ? 8 : 16;
+    return tab + sizeof(int2) * 2 * kKC + sizeof(double) * (2 * 2 * (size_t)nr * kLd + 2 * (size_t)nr * kHLd);
 }
 
 void set_ladder_smem_limit(size_t bytes)
@@ -504,22 +558,35 @@ void set_ladder_smem_limit(size_t bytes)
     std::lock_guard<std::mutex> lock(mu);
     size_t &current = current_by_dev[current_device() % kMaxDevices];
     if (bytes <= std::max(current, (size_t)48 * 1024)) return;
-    cudaFuncSetAttribute(k_ladder<kTab16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    cudaFuncSetAttribute(k_ladder<kTab1>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    cudaFuncSetAttribute(k_ladder<kTabGlobal>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    for (auto f : {k_ladder_fma<kTab16>, k_ladder_fma<kTab1>, k_ladder_fma<kTabGlobal>, k_ladder_mma<kTab16>,
+                   k_ladder_mma<kTab1>, k_ladder_mma<kTabGlobal>})
+        cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
     current = bytes;
 }
 
-void launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st)
+int launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st,
+                  cudaStream_t st_mma)
 {
-    if (d.nltiles <= 0) return;
-    const Args A{d.ltiles, d.blocks, d.solves, d.vir, d.pair_i, d.pair_j, d.nvp, d.vtab, t, g, d.active,
-                 do_pp, do_hh, tab_bytes(d.q2max)};
-    switch (tab_form(d.q2max)) {
-    case kTab16: k_ladder<kTab16><<<d.nltiles, kThreads, d.ladder_smem, st>>>(A); break;
-    case kTab1: k_ladder<kTab1><<<d.nltiles, kThreads, d.ladder_smem, st>>>(A); break;
-    default: k_ladder<kTabGlobal><<<d.nltiles, kThreads, d.ladder_smem, st>>>(A); break;
+    const int form = tab_form(d.q2max, d.n2max);
+    Args A{d.ltiles, d.vpk, d.ppk, d.vtab, t, g, d.active, do_pp, do_hh, tab_bytes(form, d.q2max)};
+    int n = 0;
+    if (d.nltiles[1] > 0) {   // the longer tiles first
+        Args B = A;
+        B.tiles += d.nltiles[0];
+        const size_t sm = d.ladder_smem[1];
+        if (form == kTab16) k_ladder_mma<kTab16><<<d.nltiles[1], kThreads, sm, st_mma>>>(B);
+        else if (form == kTab1) k_ladder_mma<kTab1><<<d.nltiles[1], kThreads, sm, st_mma>>>(B);
+        else k_ladder_mma<kTabGlobal><<<d.nltiles[1], kThreads, sm, st_mma>>>(B);
+        n++;
     }
+    if (d.nltiles[0] > 0) {
+        const size_t sm = d.ladder_smem[0];
+        if (form == kTab16) k_ladder_fma<kTab16><<<d.nltiles[0], kThreads, sm, st>>>(A);
+        else if (form == kTab1) k_ladder_fma<kTab1><<<d.nltiles[0], kThreads, sm, st>>>(A);
+        else k_ladder_fma<kTabGlobal><<<d.nltiles[0], kThreads, sm, st>>>(A);
+        n++;
+    }
+    return n;
 }
 
 }  // namespace uegccd

@@ -56,11 +56,14 @@ struct BlockDev {
                             // virtual a = K - a if sd = 1, column c + nvd + sd the partner of c < nvd
 };
 
-// One tile of the FP64 ladders: rows [p0, p0+np) of block blk, the columns a0 <= a < a1 among
-// the columns a <= pcol a and, from the partner map, their partners.
-struct LadderTile64 {
-    int blk, a0, a1;
-    int16_t p0, np;
+// One tile of the FP64 ladders: rows [p0, p0+np) of a block, the columns a0 <= a < a1 among the
+// columns a <= pcol a and, from the partner map, their partners.  The block's fields come with
+// it, so that a CTA starts from one load: 64 bytes.
+struct alignas(16) LadderTile64 {
+    int t0, vir0, pair0, vtab0;
+    int solve, q2max, a0, a1;
+    int v, nvd, sd, nd;
+    int dg, p0, np, pad;
 };
 
 // One tile of the tensor-core ladder: rows [p0, p0+P) x columns [a0, a0+A) of block blk.
