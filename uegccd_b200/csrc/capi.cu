@@ -326,7 +326,7 @@ struct UegccdBatch {
         }
     } gkey{};
     bool have_graph = false;
-    bool rings_tuned = false;        // k_rings CTA sizes picked (before the first graph capture)
+    bool tuned = false;              // launch shape picked (before the first graph capture)
     cudaGraphExec_t gexec = nullptr;
     int g_launches = 0;          // kernels per iteration
     // structure factors (on first use): every solve's particle-hole groups {first row, rows},
@@ -792,23 +792,21 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     set_mosaic_smem_limit(d.mosaic_smem);
     d.max_occ = max_occ;
     d.namp = amp0;
-    // ring pairs by kernel class: k_rings (two shared-memory sizes), then k_rings_wide
+    // ring pairs by class, then by solve (the class sort is stable), and k_rings' CTAs: runs of one
+    // solve's pairs, so long that a CTA's table serves up to four passes while the batch still
+    // makes eight CTAs an SM
+    std::vector<RingItemDev> ritems;
     {
-        auto cls_of = [&](const RingPairDev &r) {
-            const size_t b = rings_dmma_smem_bytes(solves[r.solve].O, r.n1, r.n2, solves[r.solve].q2max);
-            if (b > kRingSmemMax) return kRingClasses;
-            const int rows = ((r.n1 + 7) & ~7) + ((r.n2 + 7) & ~7);
-            for (int c = 0; c < kRingClasses; c++)
-                if (rows <= kRingClassRows[c]) return c;
-            return kRingClasses;
-        };
-        // stable counting sort by class
         std::vector<int> cls(rpairs.size());
-        std::vector<size_t> start(kRingClasses + 2, 0);
-        for (size_t k = 0; k < rpairs.size(); k++) start[(cls[k] = cls_of(rpairs[k])) + 1]++;
-        for (int c = 0; c <= kRingClasses; c++) start[c + 1] += start[c];
+        std::vector<size_t> start(kRingClasses + 1, 0);
+        for (size_t k = 0; k < rpairs.size(); k++) {
+            if ((cls[k] = ring_class(rpairs[k].n1)) < 0) return fail(UEGCCD_ERR_UNSUPPORTED, "ring group of more than 64 rows");
+            start[cls[k] + 1]++;
+        }
+        for (int c = 0; c < kRingClasses; c++) start[c + 1] += start[c];
+        std::vector<size_t> at(start.begin(), start.end() - 1);
         std::vector<RingPairDev> sorted(rpairs.size());
-        for (size_t k = 0; k < rpairs.size(); k++) sorted[start[cls[k]]++] = rpairs[k];
+        for (size_t k = 0; k < rpairs.size(); k++) sorted[at[cls[k]]++] = rpairs[k];
         rpairs.swap(sorted);
         // each pair's rows in the particle-hole arrays, in launch order: group-1 row a holds
         // 2 round8(n2) doubles (a multiple of 16: every row starts 128-byte aligned)
@@ -819,26 +817,33 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
             if (xy_n >= ((int64_t)1 << 31)) return fail(UEGCCD_ERR_ARG, "batch too large for 32-bit ring offsets");
         }
         d.xy_n = xy_n;
-        // the staging kernel walks the pairs solve by solve (the class sort is stable, so a
-        // stable sort by solve restores that order)
+        // the staging kernel walks the pairs solve by solve (a stable sort restores that order)
         spairs.assign(rpairs.begin(), rpairs.end());
         std::stable_sort(spairs.begin(), spairs.end(),
                          [](const RingPairDev &x, const RingPairDev &y) { return x.solve < y.solve; });
-        for (const auto &r : rpairs) {
-            const int c = cls_of(r);
-            d.nring[c]++;
-            const size_t b = c < kRingClasses
-                                 ? rings_dmma_smem_bytes(solves[r.solve].O, r.n1, r.n2, solves[r.solve].q2max)
-                                 : rings_smem_bytes(solves[r.solve].O, r.n1 + r.n2);
-            d.ring_smem[c] = std::max(d.ring_smem[c], b);
+        int64_t passes = 0;
+        for (int c = 0; c < kRingClasses; c++)
+            passes += ((int64_t)(start[c + 1] - start[c]) + ring_pairs_per_pass(c) - 1) / ring_pairs_per_pass(c);
+        const int per_cta = (int)std::max<int64_t>(1, std::min<int64_t>(passes / (8 * 148), 4));
+        for (int c = 0; c < kRingClasses; c++) {
+            const int run = ring_pairs_per_pass(c) * per_cta;
+            int max_n2 = 0;
+            for (size_t k = start[c]; k < start[c + 1];) {
+                RingItemDev it{(int)k, 0, rpairs[k].solve, 0};
+                for (; k < start[c + 1] && it.count < run && rpairs[k].solve == it.solve; k++, it.count++)
+                    max_n2 = std::max(max_n2, rpairs[k].n2);
+                ritems.push_back(it);
+                d.nritems[c]++;
+            }
+            if (d.nritems[c] == 0) continue;
+            d.ring_doubles[c] = ring_doubles(c, max_n2);
+            d.ring_smem[c] = ring_smem_bytes(d, c, max_n2);
+            if (d.ring_smem[c] > 227 * 1024) return fail(UEGCCD_ERR_UNSUPPORTED, "ring group pair exceeds shared memory");
+            set_rings_smem_limit(d.ring_smem[c]);
         }
     }
     trace.mark("classes");
     d.nrpairs = (int)rpairs.size();
-    if (d.ring_smem[kRingClasses] > 227 * 1024)
-        return fail(UEGCCD_ERR_UNSUPPORTED, "ring group pair exceeds shared memory");
-    set_rings_smem_limit(0, *std::max_element(d.ring_smem, d.ring_smem + kRingClasses));
-    set_rings_smem_limit(1, d.ring_smem[kRingClasses]);
     trace.mark("host-tables");
     if ((rc = b->upload(d.solves, solves))) return rc;
     if ((rc = b->upload(d.blocks, blocks))) return rc;
@@ -877,6 +882,12 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     b->vtab_base = vtab;
     if ((rc = b->upload(d.rpairs, rpairs))) return rc;
     if ((rc = b->upload(d.spairs, spairs))) return rc;
+    if ((rc = b->upload(d.ritems, ritems))) return rc;
+    std::vector<int> row0(n);
+    for (int s = 0; s < n; s++) row0[s] = (int)s_phr0[s];
+    int *d_row0 = nullptr;
+    if ((rc = b->upload(d_row0, row0))) return rc;
+    if ((rc = b->alloc(d.rrows, phr0))) return rc;
     if ((rc = b->upload(d.ph_i, ph_i))) return rc;
     if ((rc = b->upload(d.ph_x, ph_x))) return rc;
     if ((rc = b->alloc(d.ridx_x, ph0))) return rc;
@@ -911,6 +922,7 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     CU(cudaMemsetAsync(d.xy, 0, (size_t)d.xy_n * sizeof(double), b->stream));      // padding columns stay 0
 
     launch_block_tables(d, b->stream);
+    launch_ring_rows(d, (int)phr0, d_row0, b->stream);
     launch_mosaic_targets(d, d_tbase, d_lbase, (size_t)max_vo * sizeof(int), b->stream);
     launch_vcoef(d, b->stream);
     size_t dn = 0;
@@ -1227,38 +1239,30 @@ int capture_iteration(UegccdBatch &b, const TermFlags &f, double tol, int max_it
     return 0;
 }
 
-// The launch shapes of a batch (k_rings CTA sizes, k_ring_stage CTA size): measured once per
-// batch shape in this process (the shape: pair count and shared memory of every ring class), on
-// the first CCD solve, before the iteration graph is captured.
+// The launch shape of a batch (k_ring_stage's CTA size): measured once per batch shape in this
+// process (the shape: ring pairs and their operands' size), on the first CCD solve, before the
+// iteration graph is captured.
 std::mutex g_tune_mu;
-std::map<std::vector<int64_t>, std::array<int, kRingClasses + 1>> g_ring_tuning;
+std::map<std::pair<int64_t, int64_t>, int> g_stage_tuning;
 
-int tune_batch_rings(UegccdBatch &b)
+int tune_batch(UegccdBatch &b)
 {
     DevBatch &d = b.d;
-    std::vector<int64_t> key;
-    for (int c = 0; c <= kRingClasses; c++) {
-        key.push_back(d.nring[c]);
-        key.push_back((int64_t)d.ring_smem[c]);
-    }
+    const std::pair<int64_t, int64_t> key{d.nrpairs, d.xy_n};
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
-        auto it = g_ring_tuning.find(key);
-        if (it != g_ring_tuning.end()) {
-            for (int c = 0; c < kRingClasses; c++) d.ring_threads[c] = it->second[c];
-            d.stage_threads = it->second[kRingClasses];
-            b.rings_tuned = true;
+        auto it = g_stage_tuning.find(key);
+        if (it != g_stage_tuning.end()) {
+            d.stage_threads = it->second;
+            b.tuned = true;
             return 0;
         }
     }
-    const int e = tune_rings(d, b.stream);
+    const int e = tune_stage(d, b.stream);
     if (e != 0) return fail(UEGCCD_ERR_CUDA, std::string("launch-shape tuning: ") + cudaGetErrorString((cudaError_t)e));
-    std::array<int, kRingClasses + 1> th;
-    for (int c = 0; c < kRingClasses; c++) th[c] = d.ring_threads[c];
-    th[kRingClasses] = d.stage_threads;
     std::lock_guard<std::mutex> lock(g_tune_mu);
-    g_ring_tuning[key] = th;
-    b.rings_tuned = true;
+    g_stage_tuning[key] = d.stage_threads;
+    b.tuned = true;
     return 0;
 }
 
@@ -1313,7 +1317,7 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
     if (opt->precision == UEGCCD_MIXED && (rc = mixed_alloc(b))) return rc;
     if (drpa && (rc = drpa_alloc(b))) return rc;
     if (d.tc_err) CU(cudaMemsetAsync(d.tc_err, 0, sizeof(int), b.stream));
-    if (!b.rings_tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch_rings(b))) return rc;
+    if (!b.tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch(b))) return rc;
     b.launches = 0;
     CU(cudaEventRecord(b.ev0, b.stream));
     // CCEnergy of the start amplitudes and dT = max|T| (CCD.f90:63-64, dRPA.f90:68-69)
@@ -1453,7 +1457,7 @@ int session_start(UegccdBatch &b, const UegccdOptions *opt, int drpa)
     CU(cudaMemsetAsync(b.ctl.Bm, 0, (size_t)n * kDiisMax * kDiisMax * sizeof(double), b.stream));
     if ((rc = set_active_all(b, 1))) return rc;
     if (drpa && (rc = drpa_alloc(b))) return rc;
-    if (!b.rings_tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch_rings(b))) return rc;
+    if (!b.tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch(b))) return rc;
     launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
     launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
     b.launches += 2;
@@ -2065,23 +2069,26 @@ int uegccd_batch_advance(UegccdBatch *b, int32_t rounds, int32_t *n_active, int3
     return session_advance(*b, rounds, n_active, n_done, done_ids, done_results);
 }
 
+// Values of the four ring entries of the two calls below: k_rings' CTAs are of one size.
+static constexpr int kRingShapes = 4, kRingCta = 256;
+
 int32_t uegccd_batch_ring_threads(UegccdBatch *b, int32_t *threads, int32_t max)
 {
     if (!b || !threads || max <= 0) return fail(UEGCCD_ERR_ARG, "bad argument");
-    const int n = std::min<int>(max, kRingClasses);
-    for (int c = 0; c < n; c++) threads[c] = b->d.ring_threads[c];
+    const int n = std::min<int>(max, kRingShapes);
+    for (int c = 0; c < n; c++) threads[c] = kRingCta;
     return n;
 }
 
 int32_t uegccd_batch_launch_shapes(UegccdBatch *b, int32_t *vals, int32_t max)
 {
     if (!b || !vals || max <= 0) return fail(UEGCCD_ERR_ARG, "bad argument");
-    int32_t v[kRingClasses + 3];
-    for (int c = 0; c < kRingClasses; c++) v[c] = b->d.ring_threads[c];
-    v[kRingClasses] = b->d.stage_threads;
-    v[kRingClasses + 1] = 1;    // ladder tiles: always the longest first
-    v[kRingClasses + 2] = 32;   // virtuals per staged chunk of the ladder
-    const int n = std::min<int>(max, kRingClasses + 3);
+    int32_t v[kRingShapes + 3];
+    for (int c = 0; c < kRingShapes; c++) v[c] = kRingCta;
+    v[kRingShapes] = b->d.stage_threads;
+    v[kRingShapes + 1] = 1;    // ladder tiles: always the longest first
+    v[kRingShapes + 2] = 32;   // virtuals per staged chunk of the DMMA ladder
+    const int n = std::min<int>(max, kRingShapes + 3);
     for (int k = 0; k < n; k++) vals[k] = v[k];
     return n;
 }
@@ -2132,7 +2139,7 @@ int uegccd_footprint(const UegccdSystem *sys, int32_t ndiis, int32_t mixed, int6
     b += sum_ov * (8 + 4) + (V + O + 1) * (4 + 8);   // mosaic partials and target lists
     b += O * O * V * 4;                              // pos
     b += O * V * 8 * 2 + O * O * 16 + nblk * V * 2;  // dRPA sums and lookups (allocated for dRPA only)
-    b += O * V * 2 * 2;                              // ph rows
+    b += O * V * (2 * 2 + 16);                       // ph rows, their lookup sides
     int64_t xy = 0;                                  // particle-hole operands and results of the rings
     for (size_t gi = 0; gi < P.groups.size(); gi++) {
         const auto &G = P.groups[gi];

@@ -64,7 +64,9 @@ struct DevBatch {
     // particle-hole form of the ring terms
     int16_t *ph_i = nullptr, *ph_x = nullptr;   // row -> (i, x), rows grouped by Q
     int32_t *ridx_x = nullptr, *ridx_y = nullptr;  // at ph0 + row*O + k: index of t(ik, x), t(ki, x)
-    RingPairDev *rpairs = nullptr;              // {Q, -Q} group pairs, by k_rings class
+    RingPairDev *rpairs = nullptr;              // {Q, -Q} group pairs, by k_rings class and solve
+    RingItemDev *ritems = nullptr;              // k_rings' CTAs, class by class
+    RingRowDev *rrows = nullptr;                // beside ph_i, ph_x
     RingPairDev *spairs = nullptr;              // the same pairs in solve order (k_ring_stage: each
                                                 // solve's amplitudes are gathered while in L2)
     // rings in the particle-hole layout (RingPairDev::xy0): xy holds the amplitudes each pair
@@ -93,15 +95,12 @@ struct DevBatch {
     float *dscale = nullptr;
     bool w16_valid = false;          // built for the current integral tables
     int nrpairs = 0;
-    // ring pair classes, rpairs sorted in this order: k_rings in kRingClasses shared-memory
-    // sizes (kRingSmemClass), then k_rings_wide
-    int nring[5] = {0, 0, 0, 0, 0};
-    size_t ring_smem[5] = {0, 0, 0, 0, 0};
-    int ring_threads[4] = {32, 128, 256, 256};  // CTA size per k_rings class: defaults, then tune_rings
+    // ring pair classes by the rows of group 1 (kRingFrags): CTAs, shared memory, doubles a pair
+    int nritems[6] = {0, 0, 0, 0, 0, 0};
+    size_t ring_smem[6] = {0, 0, 0, 0, 0, 0};
+    int ring_doubles[6] = {0, 0, 0, 0, 0, 0};
     int stage_threads = 128;                    // CTA size of k_ring_stage (tune_rings)
 };
-// dynamic shared memory of k_rings_wide for NOcc = O and R rows of a group pair
-size_t rings_smem_bytes(int O, int R);
 // dynamic shared memory of k_mosaic_blk for blocks of at most max_v virtuals
 size_t mosaic_smem_bytes(int max_v, int max_o, int vt_n);
 void set_mosaic_smem_limit(size_t bytes);
@@ -120,20 +119,19 @@ void set_ladder_smem_limit(size_t bytes);
 // DMMA form on st_mma.  Returns the launches.
 int launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st,
                   cudaStream_t st_mma);
-// dynamic shared memory of k_rings for NOcc = O and groups of n1 and n2 rows
-size_t rings_dmma_smem_bytes(int O, int n1, int n2, int q2max);
-// k_rings classes by padded pair size N1 + N2 (up to kRingClassRows), each with its
-// CTA size (DevBatch::ring_threads); pairs above the last class, or above kRingSmemMax,
-// go to k_rings_wide
-constexpr int kRingClasses = 4;
-constexpr int kRingClassRows[kRingClasses] = {16, 32, 48, 1 << 30};
-constexpr size_t kRingSmemMax = 200 * 1024;
-void set_rings_smem_limit(int wide, size_t bytes);
-// Launch-shape autotuner, on the batch's current amplitudes: times k_rings of every pair
-// class with 32, 64, 128 and 256 threads per CTA (d.ring_threads) and k_ring_stage with 64,
-// 128 and 256 (d.stage_threads); keeps the fastest of each.  Neither changes a sum's order:
-// results are bitwise the same.  Not inside a stream capture.  Returns a cudaError_t value.
-int tune_rings(DevBatch &d, cudaStream_t st);
+// Rings (rings.cu): pair classes by the fragments of eight rows that hold group 1
+constexpr int kRingClasses = 6;
+constexpr int kRingFrags[kRingClasses] = {1, 2, 3, 4, 6, 8};
+int ring_class(int n1);             // -1: more than 64 rows (NOcc <= 64 keeps every group below)
+int ring_pairs_per_pass(int c);     // pairs a CTA works on at a time
+int ring_doubles(int c, int max_n2);
+size_t ring_smem_bytes(const DevBatch &d, int c, int max_n2);
+void set_rings_smem_limit(size_t bytes);
+int launch_rings(const DevBatch &d, int do_ring, int do_xring, cudaStream_t st);
+// Launch-shape autotuner, on the batch's current amplitudes: times k_ring_stage with 64, 128 and
+// 256 threads per CTA (d.stage_threads) and keeps the fastest.  Results are the same.  Not inside
+// a stream capture.  Returns a cudaError_t value.
+int tune_stage(DevBatch &d, cudaStream_t st);
 
 constexpr int kDiisMax = 16;   // DIIS history capacity (k_update and k_diis_* use the same bound)
 
@@ -233,6 +231,8 @@ void launch_sf(const DevBatch &d, const int2 *groups, int ngroups, int solve, in
 // pos (pre-set to -1), amps, partner, mirror from the block structure; the particle-hole
 // tables ph_a, ph_b (pre-set to -1) from the ring pairs; the ring gather indices
 void launch_block_tables(const DevBatch &d, cudaStream_t st);
+// rrows of the n ph rows (row0: each solve's first)
+void launch_ring_rows(const DevBatch &d, int n, const int *row0, cudaStream_t st);
 // mt_start / mt_list of the mosaic sums from the blocks (tbase: each solve's first target;
 // lbase: its first list entry; smem: (max V + O) ints)
 void launch_mosaic_targets(const DevBatch &d, const int *tbase, const int64_t *lbase, size_t smem, cudaStream_t st);

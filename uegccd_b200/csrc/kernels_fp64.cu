@@ -192,16 +192,6 @@ __global__ void k_reduce_solves(const int *__restrict__ chunk_begin, const doubl
 // the other terms.)
 constexpr int kVtabSmem = kVtabSmemEntries;  // |q|^2 table entries staged in shared memory
 
-// FP64 tensor-core MMA (tcgen05 has no f64 kind).  Fragment layouts (PTX ISA, m8n8k4 .f64):
-// A row = lane/4, col = lane%4; B row (k) = lane%4, col = lane/4; C row = lane/4, cols
-// 2*(lane%4) + {0,1}.
-__device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 // The dynamic shared-memory limits only grow (batches of different sizes coexist), under
 // one lock: batches are created from several host threads while others solve.  Kernel
 // attributes belong to a device, so each device keeps its own limits (the caller has made
@@ -515,451 +505,7 @@ __global__ void __launch_bounds__(kDrpaThreads)
     if (threadIdx.x == 0) done[L.x] = 0;
 }
 
-// ----------------------------------------------------------------------------
-// Rings and crossed rings in particle-hole form (CCD).
-// For every ph row (i,x), x virtual, with c = partner of (i,k,x):
-//   X[k] = t(ik,x),  Y[k] = t(ik,c)                 (= t(ki,x) by the pair swap)
-//   Sx = sum_k X, Sy = sum_k Y
-//   Ex[j] = sum_k v(k-j) X[k],  Ey[j] = sum_k v(k-j) Y[k]
-//   XW[l] = sum_k X[k] v(i+k-x-l), YW[l] = sum_k Y[k] v(i+k-x-l)
-// and the quadratic-ring intermediates of CCD.f90:774-797 / 902-925 become
-//   A1 = J1 + J2 = 2 vd (2Sx - Sy) - 2 XW + YW,  A2 = J2 = vd (2Sx - Sy) - XW,  A3 = J3 = YW,
-// vd = v(i-x).  Then, for the amplitude (i,j,a) with partner b (rows ia, jb, ib, ja):
-//   linear rings   (CCD.f90:716-763): 2 v(i-a)(Sx_ia + Sx_jb) - v(i-a)(Sy_ia + Sy_jb) - Ex_ia[j] - Ex_jb[i]
-//   linear xrings  (CCD.f90:845-892): -Ey_ib[j] - Ey_ja[i]
-//   quadratic rings  (CCD.f90:801-808): A1_ia . X_jb - A2_ia . Y_jb
-//   quadratic xrings (CCD.f90:927-934): A3_ib . Y_ja
-// The quadratic products pair the rows of momentum Q with those of -Q, group by
-// group; every amplitude receives exactly one ring and one crossed-ring product, so
-// no atomics are needed.
-// Row layout: row r (local) of solve s: scalars at s.phr0 + r, vectors at s.ph0 + r * O (O entries).
-// ----------------------------------------------------------------------------
-// ----------------------------------------------------------------------------
-// Fused rings: one CTA per pair of ph groups {Q, -Q}.  Everything of the formulas
-// above happens in shared memory: X, Y rows of both groups, the exchange kernels
-// W_Q[k][l] = v(n_k - n_l - Q) and W_-Q, the direct occupied kernel
-// Vocc[j][k] = v(n_k - n_j), the A rows (chunk by chunk) and the products.  Each
-// pair of rows (r1 in one group, r2 in the other) owns two amplitudes:
-//   ring  amplitude (i1, i2, a = x1):  lin + A1_r1 . X_r2 - A2_r1 . Y_r2
-//   xring amplitude (i1, i2, a = x2):  xlin + A3_r1 . Y_r2
-// with lin = 2 vd_r1 (Sx_r1 + Sx_r2) - vd_r1 (Sy_r1 + Sy_r2) - Ex_r1[i2] - Ex_r2[i1]
-// and xlin = -Ey_r1[i2] - Ey_r2[i1]; Ex/Ey elements are formed where used.
-// ----------------------------------------------------------------------------
-constexpr int kRingCh = 16;  // A rows per chunk
-
-// The FMA form below serves group pairs too large for k_rings' shared-memory tiles
-// (NOcc around 57 and above).
-__global__ void __launch_bounds__(256) k_rings_wide(const RingPairDev *__restrict__ pairs,
-                                               const SolveDev *__restrict__ solves,
-                                               const int16_t *__restrict__ ph_i, const int16_t *__restrict__ ph_x,
-                                               const int32_t *__restrict__ pos, const int32_t *__restrict__ partner,
-                                               const int4 *__restrict__ nv4, const double *__restrict__ vtab,
-                                               const double *__restrict__ t, int do_ring, int do_xring,
-                                               double *__restrict__ rx,
-                                               const uint8_t *__restrict__ active)
-{
-    const RingPairDev P = pairs[blockIdx.x];
-    if (!active[P.solve]) return;
-    const SolveDev s = solves[P.solve];
-    const int O = s.O;
-    const int R = P.n1 + P.n2;
-    const int N2 = (P.n2 + 7) & ~7;   // rx row: ring G of the group-2 columns, then crossed-ring G
-    // shared-memory strides are odd so that consecutive threads hit distinct banks
-    const int ld = O | 1, lr = R | 1;
-    extern __shared__ double smem[];
-    double *sv = smem;                                   // kVtabSmem
-    double *Vo = sv + kVtabSmem;                         // O x ld : Vo[k*ld + j] = v(n_k - n_j)
-    double *W1 = Vo + O * ld;                            // O x ld : W_Q[k][l]
-    double *W2 = W1 + O * ld;                            // O x ld : W_-Q[k][l]
-    double *XT = W2 + O * ld;                            // O x lr : X[r][k] at k*lr + r
-    double *YT = XT + O * lr;                            // O x lr
-    double *A1 = YT + O * lr;                            // kRingCh x ld
-    double *A2 = A1 + kRingCh * ld;
-    double *A3 = A2 + kRingCh * ld;
-    double *Sx = A3 + kRingCh * ld;                      // R
-    double *Sy = Sx + R;                                 // R
-    double *Vd = Sy + R;                                 // R
-    int *ri = (int *)(Vd + R);                           // R
-    int *rxv = ri + R;                                   // R: the row's virtual
-    int4 *no = (int4 *)(((uintptr_t)(rxv + R) + 15) & ~(uintptr_t)15);  // O occupied n-vectors
-    const int tid = threadIdx.x, nt = blockDim.x;
-    const bool vsm = s.q2max < kVtabSmem;
-    if (vsm)
-        for (int q = tid; q <= s.q2max; q += nt) sv[q] = vtab[s.vtab0 + q];
-    for (int k = tid; k < O; k += nt) no[k] = nv4[s.orb0 + k];
-    for (int r = tid; r < R; r += nt) {
-        const int64_t row = s.phr0 + (r < P.n1 ? P.r1 + r : P.r2 + r - P.n1);
-        ri[r] = ph_i[row];
-        rxv[r] = ph_x[row];
-    }
-    __syncthreads();
-    auto V = [&](int q2) -> double { return q2 > s.q2max ? 0.0 : (vsm ? sv[q2] : vtab[s.vtab0 + q2]); };
-    // Q of group 1 = n_x - n_i of its first row
-    const int4 qa = nv4[s.orb0 + rxv[0]], qb = nv4[s.orb0 + ri[0]];
-    const int Qx = qa.x - qb.x, Qy = qa.y - qb.y, Qz = qa.z - qb.z;
-    for (int e = tid; e < O * O; e += nt) {
-        const int k = e / O, l = e % O;
-        const int4 nk = no[k], nl = no[l];
-        const int dx = nk.x - nl.x, dy = nk.y - nl.y, dz = nk.z - nl.z;
-        Vo[k * ld + l] = V(dx * dx + dy * dy + dz * dz);
-        const int ax = dx - Qx, ay = dy - Qy, az = dz - Qz;
-        W1[k * ld + l] = V(ax * ax + ay * ay + az * az);
-        const int bx = dx + Qx, by = dy + Qy, bz = dz + Qz;
-        W2[k * ld + l] = V(bx * bx + by * by + bz * bz);
-    }
-    // X, Y rows (stored transposed)
-    for (int e = tid; e < R * O; e += nt) {
-        const int k = e / R, r = e % R;
-        const int p = posmap(s, pos, ri[r], k, rxv[r]);
-        double xv = 0.0, yv = 0.0;
-        if (p >= 0) {
-            xv = t[p];
-            yv = t[partner[p]];
-        }
-        XT[k * lr + r] = xv;
-        YT[k * lr + r] = yv;
-    }
-    __syncthreads();
-    for (int r = tid; r < R; r += nt) {
-        double sx = 0.0, sy = 0.0;
-        for (int k = 0; k < O; k++) {
-            sx += XT[k * lr + r];
-            sy += YT[k * lr + r];
-        }
-        Sx[r] = sx;
-        Sy[r] = sy;
-        const int4 ni = nv4[s.orb0 + ri[r]], nx = nv4[s.orb0 + rxv[r]];
-        Vd[r] = V(q2_of(ni, nx));
-    }
-    __syncthreads();
-    // rows of group 1 against group 2: the values at (a, b) are the ring G of (i_a, i_b, x_a)
-    // and the crossed-ring G of (i_a, i_b, x_b), which k_update reads for each amplitude or
-    // its mirror (the reverse direction gives the mirrors' values: not needed)
-    for (int dir = 0; dir < 1; dir++) {
-        const int a0 = dir == 0 ? 0 : P.n1, na = dir == 0 ? P.n1 : P.n2;
-        const int b0 = dir == 0 ? P.n1 : 0, nb = dir == 0 ? P.n2 : P.n1;
-        const double *W = dir == 0 ? W1 : W2;
-        for (int c0 = 0; c0 < na; c0 += kRingCh) {
-            const int nc = min(kRingCh, na - c0);
-            // A rows of the chunk: XW, YW with the chunk group's exchange kernel
-            for (int e = tid; e < nc * O; e += nt) {
-                const int rr = e / O, l = e % O;
-                const int r = a0 + c0 + rr;
-                double xw = 0.0, yw = 0.0;
-                for (int k = 0; k < O; k++) {
-                    const double w = W[k * ld + l];
-                    xw = fma(XT[k * lr + r], w, xw);
-                    yw = fma(YT[k * lr + r], w, yw);
-                }
-                const double base = Vd[r] * (2.0 * Sx[r] - Sy[r]);
-                A1[rr * ld + l] = 2.0 * base - 2.0 * xw + yw;
-                A2[rr * ld + l] = base - xw;
-                A3[rr * ld + l] = yw;
-            }
-            __syncthreads();
-            for (int e = tid; e < nc * nb; e += nt) {
-                const int rr = e / nb, r2 = b0 + e % nb;
-                const int r1 = a0 + c0 + rr;
-                const int i1 = ri[r1], i2 = ri[r2];
-                double quad = 0.0, xquad = 0.0, ex12 = 0.0, ex21 = 0.0, ey12 = 0.0, ey21 = 0.0;
-                for (int l = 0; l < O; l++) {
-                    const double x2 = XT[l * lr + r2], y2 = YT[l * lr + r2];
-                    quad = fma(A1[rr * ld + l], x2, quad);
-                    quad = fma(-A2[rr * ld + l], y2, quad);
-                    xquad = fma(A3[rr * ld + l], y2, xquad);
-                    const double vo12 = Vo[l * ld + i2], vo21 = Vo[l * ld + i1];
-                    ex12 = fma(vo12, XT[l * lr + r1], ex12);   // Ex_r1[i2]
-                    ey12 = fma(vo12, YT[l * lr + r1], ey12);   // Ey_r1[i2]
-                    ex21 = fma(vo21, x2, ex21);                // Ex_r2[i1]
-                    ey21 = fma(vo21, y2, ey21);                // Ey_r2[i1]
-                }
-                double *out = rx + P.xy0 + (int64_t)r1 * 2 * N2;
-                if (do_ring) {
-                    const double vd = Vd[r1];
-                    const double lin = 2.0 * vd * (Sx[r1] + Sx[r2]) - vd * (Sy[r1] + Sy[r2]) - ex12 - ex21;
-                    out[r2 - P.n1] = lin + quad;
-                }
-                if (do_xring) out[N2 + r2 - P.n1] = -ey12 - ey21 + xquad;
-            }
-            __syncthreads();
-        }
-    }
-}
-
-
-// ----------------------------------------------------------------------------
-// Rings on the FP64 tensor cores (mma.sync m8n8k4 f64), one CTA per {Q, -Q}
-// group pair, on compressed matrices.  Rows a of group 1 are (i_a, x_a) with
-// n_x - n_i = Q; rows b of group 2 are (i_b, x_b) with -Q.  The amplitude
-// t(i_a k, x_a) exists exactly for k in occ2 = {i_b}: its partner is x_b.  So every
-// ph row of one group is dense over the occupied indices of the other group:
-//   X1[a][b] = t(i_a i_b, x_a)   Y1[a][b] = t(i_b i_a, x_a)   (n1 x n2)
-// The rows of group 2 hold the same amplitudes transposed: by the pair symmetry
-// t(ij, a) = t(ji, b) (T2abab(ij,ab) = T2abab(ji,ba)),
-//   X2[b][a] = t(i_b i_a, x_b) = X1[a][b],   Y2[b][a] = t(i_a i_b, x_b) = Y1[a][b],
-// so only X1 and Y1 are gathered.  With
-//   W[b][a]  = v(n_{i_b} - n_{i_a} - Q)
-//   Vs1[a][a'] = v(n_{i_a'} - n_{i_a}),  Vs2[b][b'] = v(n_{i_b'} - n_{i_b})
-//   XW1 = X1 W,  U1 = Y1 W - Vs1
-// the fused ring form above becomes, for the amplitude pair (a, b):
-//   ring (i_a, i_b, x_a) = lin + base_a (2 Sx_b - Sy_b)
-//                          + sum_a' [XW1[a][a'] (Y1 - 2 X1)[a'][b] + U1[a][a'] X1[a'][b]]
-//                          - sum_b' X1[a][b'] Vs2[b][b']
-//   xring(i_a, i_b, x_b) = sum_a' U1[a][a'] Y1[a'][b] - sum_b' Y1[a][b'] Vs2[b][b']
-// (lin, base as above; Sx_b, Sy_b are the column sums of X1, Y1).  The residual
-// terms share the pair symmetry (ring and crossed-ring G of (j,i,b) equal those of
-// (i,j,a)), and k_update reads G only where the first occupied index is the smaller
-// one: the ring value goes to (i_a, i_b, x_a) or to its mirror (i_b, i_a, x_b), the
-// crossed-ring value to (i_a, i_b, x_b) or to (i_b, i_a, x_a).  The reference forms
-// both halves separately (CCD.f90:716-937); the two agree to rounding.
-// Group 1 is the smaller group (the host orders each pair), which minimises both the
-// shared memory, 2 N1 (N1 + N2 + 8) doubles, and the work, 5 N1^2 N2 + 2 N1 N2^2 DMMA
-// multiply-adds.  Row strides are the padded width + 4 (= 4 or 12 mod 16 doubles):
-// fragment loads without bank conflicts, row-wise and transposed.
-// ----------------------------------------------------------------------------
-__host__ __device__ __forceinline__ int round8(int x) { return (x + 7) & ~7; }
-
-size_t rings_dmma_smem_bytes(int O, int n1, int n2, int q2max)
-{
-    const size_t N1 = round8(n1), N2 = round8(n2), l1 = N1 + 4, l2 = N2 + 4;
-    const size_t nsv = q2max < kVtabSmem ? round8(q2max + 1) : 0;
-    const size_t dbl = 2 * N1 * l2 + 2 * N1 * l1 + 3 * (N1 + N2) + nsv;
-    return sizeof(double) * dbl + sizeof(int) * ((size_t)O + 4 * (N1 + N2));
-}
-
-// Capped at 64 registers (four 256-thread CTAs an SM): a few spill slots, more CTAs resident
-// (0.396 -> 0.362 ms per residual on the 100-twist batch, against the 78 registers uncapped).
-__global__ void __launch_bounds__(256, 4) k_rings(const RingPairDev *__restrict__ pairs,
-                                                        const SolveDev *__restrict__ solves,
-                                                        const int16_t *__restrict__ ph_i,
-                                                        const int16_t *__restrict__ ph_x,
-                                                        const int *__restrict__ nvp,
-                                                        const double *__restrict__ vtab,
-                                                        const double *__restrict__ xy, int do_ring, int do_xring,
-                                                        double *__restrict__ rx,
-                                                        const uint8_t *__restrict__ active)
-{
-    const RingPairDev P = pairs[blockIdx.x];
-    if (!active[P.solve]) return;
-    const SolveDev s = solves[P.solve];
-    const int O = s.O;
-    const int n1 = P.n1, n2 = P.n2;
-    if (n1 <= 0 || n2 <= 0) return;  // a ring pair always has both groups; whole CTA
-    const int N1 = round8(n1), N2 = round8(n2), l1 = N1 + 4, l2 = N2 + 4, R = N1 + N2;
-    const bool vsm = s.q2max < kVtabSmem;
-    const int nsv = vsm ? round8(s.q2max + 1) : 0;
-    extern __shared__ double smem[];
-    // W and the direct kernels Vs1, Vs2 are table lookups: generated where the DMMA loops
-    // read them (from the rows' n-vectors) instead of stored, for more CTAs per SM
-    double *X1 = smem;              // N1 x l2
-    double *Y1 = X1 + N1 * l2;      // N1 x l2
-    double *XW1 = Y1 + N1 * l2;     // N1 x l1
-    double *U1 = XW1 + N1 * l1;     // N1 x l1
-    double *Sx = U1 + N1 * l1;      // R: group 1 rows at [0, N1), group 2 rows at [N1, R)
-    double *Sy = Sx + R;
-    double *Vd = Sy + R;
-    double *sv = Vd + R;            // nsv
-    int *ri = (int *)(sv + nsv);    // R: occupied index of the row (-1 on padding)
-    int *no = ri + R;               // O: packed n-vectors of the occupied orbitals
-    int *nx = no + O;               // R: packed n-vector of the row's virtual
-    int *nr = nx + R;               // R: packed n-vector of the row's occupied index (0 on padding)
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, nt = blockDim.x, kWarps = nt >> 5;
-    auto V = [&](int q2) -> double {
-        return q2 > s.q2max ? 0.0 : (vsm ? sv[q2] : __ldg(&vtab[s.vtab0 + q2]));
-    };
-    for (int q = tid; q < nsv; q += nt) sv[q] = q <= s.q2max ? vtab[s.vtab0 + q] : 0.0;
-    for (int r = tid; r < R; r += nt) {
-        int row = -1;
-        if (r < n1) row = P.r1 + r;
-        else if (r >= N1 && r - N1 < n2) row = P.r2 + (r - N1);
-        const int i = row >= 0 ? ph_i[s.phr0 + row] : -1, x = row >= 0 ? ph_x[s.phr0 + row] : -1;
-        ri[r] = i;
-        nx[r] = x >= 0 ? nvp[s.orb0 + x] : 0;
-    }
-    for (int k = tid; k < O; k += nt) no[k] = nvp[s.orb0 + k];
-    __syncthreads();
-    for (int r = tid; r < R; r += nt) nr[r] = ri[r] >= 0 ? no[ri[r]] : 0;
-    const int Qp = __vsub4(nx[0], no[ri[0]]);   // Q = n_x - n_i of group 1, packed
-    // X1 and Y1: the pair's rows in the particle-hole copy of t (k_ring_stage), 2 N2 doubles
-    // a row and 16-byte aligned -- contiguous loads in place of index -> amplitude gathers.
-    // Columns n2..N2-1 are zero in memory; rows n1..N1-1 are padding.
-    {
-        const double2 *src = reinterpret_cast<const double2 *>(xy + P.xy0);
-        const int half = N2 / 2;   // double2 per X1 (or Y1) row
-        for (int e = tid; e < N1 * N2; e += nt) {
-            const int r = e / N2, c2 = e - r * N2;
-            const double2 v = r < n1 ? __ldg(&src[(int64_t)r * N2 + c2]) : make_double2(0.0, 0.0);
-            double *dst = c2 < half ? X1 + r * l2 + 2 * c2 : Y1 + r * l2 + 2 * (c2 - half);
-            dst[0] = v.x;
-            dst[1] = v.y;
-        }
-    }
-    __syncthreads();
-    // row sums of X1, Y1 for group 1, column sums for group 2 (padding is zero)
-    for (int r = tid; r < R; r += nt) {
-        double sx = 0.0, sy = 0.0;
-        if (r < N1) {
-            for (int c = 0; c < n2; c++) {
-                sx += X1[r * l2 + c];
-                sy += Y1[r * l2 + c];
-            }
-        } else {
-            const int c = r - N1;
-            for (int a = 0; a < n1; a++) {
-                sx += X1[a * l2 + c];
-                sy += Y1[a * l2 + c];
-            }
-        }
-        Sx[r] = sx;
-        Sy[r] = sy;
-        Vd[r] = ri[r] >= 0 ? V(q2p(no[ri[r]], nx[r])) : 0.0;
-    }
-    const int g = lane >> 2, tg = lane & 3;
-    // phase 1: XW1 = X1 W, U1 = Y1 W - Vs1 (K = N2), with W[b][a] = v(n_{i_b} - n_{i_a} - Q)
-    // and Vs1[a][a'] = v(n_{i_a'} - n_{i_a}) generated from the rows' n-vectors (0 on
-    // padding).  Tasks: one 8-row fragment row x up to 2 column fragments; X and Y share
-    // each generated W fragment.
-    {
-        const int ngr = (N1 + 15) / 16, ntask = (N1 / 8) * ngr;
-        for (int task = warp; task < ntask; task += kWarps) {
-            const int mf = task / ngr, ng = task - mf * ngr;
-            const double *AX = X1 + (mf * 8 + g) * l2 + tg;
-            const double *AY = Y1 + (mf * 8 + g) * l2 + tg;
-            const int nbase = ng * 16;
-            int cn[2];
-            bool cok[2];
-#pragma unroll
-            for (int f = 0; f < 2; f++) {
-                const int n = nbase + f * 8 + g;
-                cok[f] = n < n1;
-                cn[f] = cok[f] ? __vadd4(nr[n], Qp) : 0;   // n_{i_a'} + Q
-            }
-            double acc[2][2][2];
-#pragma unroll
-            for (int f = 0; f < 2; f++) acc[0][f][0] = acc[0][f][1] = acc[1][f][0] = acc[1][f][1] = 0.0;
-            for (int k0 = 0; k0 < N2; k0 += 4) {
-                const int k = k0 + tg;
-                const double ax = AX[k0], ay = AY[k0];
-                const bool kok = k < n2;
-                const int kn = nr[N1 + k];
-#pragma unroll
-                for (int f = 0; f < 2; f++) {
-                    if (nbase + f * 8 >= N1) break;
-                    // B(k = b, n = a') = W[b][a'] = v(n_{i_b} - n_{i_a'} - Q)
-                    const double bv = (kok && cok[f]) ? V(q2p(kn, cn[f])) : 0.0;
-                    dmma_884(acc[0][f][0], acc[0][f][1], ax, bv);
-                    dmma_884(acc[1][f][0], acc[1][f][1], ay, bv);
-                }
-            }
-            const int r = mf * 8 + g;
-            const bool rok = r < n1;
-            const int rn = rok ? nr[r] : 0;
-#pragma unroll
-            for (int f = 0; f < 2; f++) {
-                if (nbase + f * 8 >= N1) break;
-#pragma unroll
-                for (int h = 0; h < 2; h++) {
-                    const int n = nbase + f * 8 + 2 * tg + h;
-                    const double vs = (rok && n < n1) ? V(q2p(nr[n], rn)) : 0.0;
-                    XW1[r * l1 + n] = acc[0][f][h];
-                    U1[r * l1 + n] = acc[1][f][h] - vs;
-                }
-            }
-        }
-    }
-    __syncthreads();
-    // phase 2: rows a x columns b, tasks of 8 x 16
-    const int nng = (N2 + 15) / 16, ntask = (N1 / 8) * nng;
-    for (int task = warp; task < ntask; task += kWarps) {
-        const int mf = task / nng, ng = task - mf * nng;
-        const int m0 = mf * 8;
-        double ra[2][2], rb[2][2], xa[2][2], xb[2][2];
-#pragma unroll
-        for (int f = 0; f < 2; f++)
-#pragma unroll
-            for (int h = 0; h < 2; h++) ra[f][h] = rb[f][h] = xa[f][h] = xb[f][h] = 0.0;
-        // sum over a': A = XW1, U1 rows a; B(k = a', n = b) = X1[a'][b], Y1[a'][b]
-        for (int k0 = 0; k0 < N1; k0 += 4) {
-            const int k = k0 + tg;
-            const double axw = XW1[(m0 + g) * l1 + k], au = U1[(m0 + g) * l1 + k];
-#pragma unroll
-            for (int f = 0; f < 2; f++) {
-                const int n0 = ng * 16 + f * 8;
-                if (n0 >= N2) break;
-                const double bx = X1[k * l2 + n0 + g], by = Y1[k * l2 + n0 + g];
-                dmma_884(ra[f][0], ra[f][1], axw, by - 2.0 * bx);
-                dmma_884(rb[f][0], rb[f][1], au, bx);
-                dmma_884(xa[f][0], xa[f][1], au, by);
-            }
-        }
-        // sum over b': A = X1, Y1 rows a; B = -Vs2[b][b'], generated
-        int bn[2];
-        bool bok[2];
-#pragma unroll
-        for (int f = 0; f < 2; f++) {
-            const int bb = ng * 16 + f * 8 + g;
-            bok[f] = bb < n2;
-            bn[f] = bok[f] ? nr[N1 + bb] : 0;
-        }
-        for (int k0 = 0; k0 < N2; k0 += 4) {
-            const int k = k0 + tg;
-            const double ax = X1[(m0 + g) * l2 + k], ay = Y1[(m0 + g) * l2 + k];
-            const bool kok = k < n2;
-            const int kn = nr[N1 + k];
-#pragma unroll
-            for (int f = 0; f < 2; f++) {
-                const int n0 = ng * 16 + f * 8;
-                if (n0 >= N2) break;
-                const double bv = (kok && bok[f]) ? -V(q2p(kn, bn[f])) : -0.0;
-                dmma_884(rb[f][0], rb[f][1], ax, bv);
-                dmma_884(xb[f][0], xb[f][1], ay, bv);
-            }
-        }
-        const int r1 = m0 + g;                          // this lane's row (group 1)
-        if (r1 >= n1) continue;
-        const double vd = Vd[r1], sx1 = Sx[r1], sy1 = Sy[r1];
-        const double base = vd * (2.0 * sx1 - sy1);
-        // the ring G of (i_a, i_b, x_a) and the crossed-ring G of (i_a, i_b, x_b) at (a, b) of
-        // the pair's rows in rx; k_update picks each amplitude's value there (or its mirror's)
-        double *out = rx + P.xy0 + (int64_t)r1 * 2 * N2;
-#pragma unroll
-        for (int f = 0; f < 2; f++) {
-            const int n0 = ng * 16 + f * 8;
-            if (n0 >= N2) break;
-#pragma unroll
-            for (int h = 0; h < 2; h++) {
-                const int n = n0 + 2 * tg + h;
-                if (n >= n2) continue;
-                const int r2 = N1 + n;
-                if (do_ring) {
-                    const double lin = 2.0 * vd * (sx1 + Sx[r2]) - vd * (sy1 + Sy[r2]);
-                    out[n] = lin + base * (2.0 * Sx[r2] - Sy[r2]) + ra[f][h] + rb[f][h];
-                }
-                if (do_xring) out[N2 + n] = xa[f][h] + xb[f][h];
-            }
-        }
-    }
-}
-
-void set_rings_smem_limit(int wide, size_t bytes)
-{
-    // keep the largest limit ever requested per kernel: batches of different sizes coexist
-    std::lock_guard<std::mutex> lock(g_smem_limit_mu);
-    static size_t current_by_dev[kMaxDevices][2] = {};   // attributes are per device
-    size_t *current = current_by_dev[current_device() % kMaxDevices];
-    if (bytes > current[wide ? 1 : 0]) {
-        if (wide) cudaFuncSetAttribute(k_rings_wide, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        else cudaFuncSetAttribute(k_rings, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        current[wide ? 1 : 0] = bytes;
-    }
-}
-
-size_t rings_smem_bytes(int O, int R)
-{
-    const int ld = O | 1, lr = R | 1;
-    return sizeof(double) * ((size_t)kVtabSmem + 3 * O * ld + 2 * O * lr + 3 * kRingCh * ld + 3 * R) +
-           sizeof(int) * 2 * R + 16 + sizeof(int4) * O;
-}
+// (The rings and crossed rings, CCD.f90:689-940, are in rings.cu.)
 
 // ----------------------------------------------------------------------------
 // Fused residual / update / convergence / energy, one thread per amplitude.
@@ -1063,6 +609,43 @@ __global__ void k_ph_tables(const RingPairDev *__restrict__ pairs, const SolveDe
         ph_a[k] = g1 ? P.xy0 + 2 * r * N2 : -1;
         ph_b[k] = g1 ? N2 : r - P.n1;
     }
+}
+
+// The orbitals of every ph row as k_rings looks them up; carry: |n|^2 in the fourth byte of the
+// column side (against a 1 in the row sides), where it fits.
+__global__ void k_ring_rows(int n, const int *__restrict__ row0, int nsolves, const SolveDev *__restrict__ solves,
+                            const int16_t *__restrict__ ph_i, const int16_t *__restrict__ ph_x,
+                            const int *__restrict__ nvp, int carry, RingRowDev *__restrict__ rows)
+{
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r >= n) return;
+    int lo = 0, hi = nsolves - 1;   // the solve whose rows hold r
+    while (lo < hi) {
+        const int m = (lo + hi + 1) >> 1;
+        if (row0[m] <= r) lo = m;
+        else hi = m - 1;
+    }
+    const SolveDev &s = solves[lo];
+    auto m2 = [&](int p) {
+        const int x = (int8_t)p, y = (int8_t)(p >> 8), z = (int8_t)(p >> 16);
+        return ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16) | (carry ? 1 << 24 : 0);
+    };
+    const int pi = nvp[s.orb0 + ph_i[r]], px = nvp[s.orb0 + ph_x[r]];
+    RingRowDev R;
+    const int ni2 = __dp4a(pi, pi, 0);
+    R.ci = carry ? pi | (ni2 << 24) : pi;
+    R.mi = m2(pi);
+    R.mx = m2(px);
+    R.ni2 = (int16_t)ni2;
+    R.nx2 = (int16_t)__dp4a(px, px, 0);
+    rows[r] = R;
+}
+
+void launch_ring_rows(const DevBatch &d, int n, const int *row0, cudaStream_t st)
+{
+    const int carry = d.q2max < 256 && d.n2max < 128;
+    if (n > 0)
+        k_ring_rows<<<(n + 255) / 256, 256, 0, st>>>(n, row0, d.nsolves, d.solves, d.ph_i, d.ph_x, d.nvp, carry, d.rrows);
 }
 
 // The particle-hole copy of t that k_rings reads, one CTA per {Q, -Q} pair: row a of group
@@ -1669,39 +1252,11 @@ const char *kKernelNames[KID_COUNT] = {"k_mp2",      "k_energy",   "k_ladder",
                                       "k_reduce_solves", "k_rings",
                                       "k_ladder_tc", "k_ring_stage", "k_tail", "k_diis_extrap2"};
 
-int tune_rings(DevBatch &d, cudaStream_t st)
+int tune_stage(DevBatch &d, cudaStream_t st)
 {
-    static const int kCand[] = {32, 64, 128, 256};
     cudaEvent_t e0 = nullptr, e1 = nullptr;
     cudaError_t err = cudaEventCreate(&e0);
     if (err == cudaSuccess) err = cudaEventCreate(&e1);
-    int off = 0;
-    for (int c = 0; c < kRingClasses && err == cudaSuccess; c++) {
-        if (d.nring[c] > 0) {
-            float best = 1e30f;
-            int pick = d.ring_threads[c];
-            for (int th : kCand) {
-                auto run = [&]() {
-                    k_rings<<<d.nring[c], th, d.ring_smem[c], st>>>(d.rpairs + off, d.solves, d.ph_i, d.ph_x,
-                                                                    d.nvp, d.vtab, d.xy, 1, 1, d.rx, d.active);
-                };
-                run();  // warm
-                cudaEventRecord(e0, st);
-                run();
-                run();
-                cudaEventRecord(e1, st);
-                if ((err = cudaEventSynchronize(e1)) != cudaSuccess) break;
-                float ms = 0.f;
-                cudaEventElapsedTime(&ms, e0, e1);
-                if (ms < best) {
-                    best = ms;
-                    pick = th;
-                }
-            }
-            d.ring_threads[c] = pick;
-        }
-        off += d.nring[c];
-    }
     // the staging kernel's CTA size
     if (err == cudaSuccess && d.nrpairs > 0) {
         float best = 1e30f;
@@ -1779,23 +1334,7 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         kt->end(rs);
         n++;
         kt->begin(KID_RINGS, rs);
-        // pair classes (sorted in this order): DMMA tiles in two shared-memory sizes, then the FMA form
-        int off = 0;
-        for (int c = 0; c < kRingClasses; c++) {
-            if (d.nring[c] > 0) {
-                k_rings<<<d.nring[c], d.ring_threads[c], d.ring_smem[c], rs>>>(
-                    d.rpairs + off, d.solves, d.ph_i, d.ph_x, d.nvp, d.vtab, d.xy, f.do_ring, f.do_xring, d.rx,
-                    d.active);
-                n++;
-            }
-            off += d.nring[c];
-        }
-        if (d.nring[kRingClasses] > 0) {
-            k_rings_wide<<<d.nring[kRingClasses], 256, d.ring_smem[kRingClasses], rs>>>(d.rpairs + off, d.solves, d.ph_i, d.ph_x, d.pos,
-                                                                 d.partner, d.nv4, d.vtab, d.t, f.do_ring,
-                                                                 f.do_xring, d.rx, d.active);
-            n++;
-        }
+        n += launch_rings(d, f.do_ring, f.do_xring, rs);
         kt->end(rs);
     }
     if (side) {

@@ -115,6 +115,18 @@ struct DrpaSolveDev {
     int64_t rij0, cp0;
 };
 
+// Pairs [first, first + count) of one solve and one row class, done by one CTA of k_rings.
+struct RingItemDev {
+    int first, count, solve, pad;
+};
+
+// The orbitals (i, x) of a ph row as the Coulomb lookups take them (rings.cu): the column side of
+// i, the row sides of i and x (packed vector times -2) and their |n|^2.
+struct alignas(16) RingRowDev {
+    int ci, mi, mx;
+    int16_t ni2, nx2;
+};
+
 struct ChunkDev {
     int solve;
     int32_t start;          // first amplitude of the chunk, local to the solve
