@@ -19,7 +19,7 @@ LIB = os.path.join(PKG, "libuegccd.so")
 ZCODE = os.path.join(PKG, "uegccd_zcode")
 OBJDIR = os.path.join(PKG, "_build")
 
-SOURCES = ["capi.cu", "kernels_fp64.cu", "ladder.cu", "rings.cu", "kernels_tc.cu", "plan.cpp", "heg_host.cpp", "zcode.cpp", "mp2_static.cu",
+SOURCES = ["capi.cu", "kernels_fp64.cu", "ladder.cu", "rings.cu", "update.cu", "kernels_tc.cu", "plan.cpp", "heg_host.cpp", "zcode.cpp", "mp2_static.cu",
            "diis_api.cu", "heg_device.cu", "two_channel.cu", "two_channel_mm.cu"]
 # bench.py's FP64 tensor-core peak measurement: a library of its own beside bench.py
 BENCH_PEAK_SRC = os.path.join(ROOT, "bench_peak.cu")

@@ -281,7 +281,6 @@ struct UegccdBatch {
     std::vector<SystemHost> sys;
     std::vector<SolvePlan> plans;
     std::vector<SolveDev> hsolves;
-    std::vector<int> chunk_begin;
     DevBatch d;
     std::vector<DevChunk> chunks;    // device memory of the batch (see chunk_get): arena chunks
     size_t chunk_used = 0;           // bytes used in the last arena chunk
@@ -603,7 +602,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     nv4.clear();
     nvp.clear();
     eigen.clear();
-    std::vector<int> chunk_begin(n + 1, 0);
     std::vector<double> vtab;
     std::vector<RingPairDev> rpairs, spairs;
     int64_t amp0 = 0, pos0 = 0, ph0 = 0, phr0 = 0, mrows = 0, mcols = 0;
@@ -694,7 +692,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
         }
         eigen.insert(eigen.end(), H.eigen.begin(), H.eigen.end());
         vtab.insert(vtab.end(), P.vtab.begin(), P.vtab.end());
-        chunk_begin[s] = (int)chunks.size();
         for (int64_t st = 0; st < P.namp; st += kChunk) chunks.push_back(ChunkDev{s, (int32_t)st});
         for (int64_t st = 0; st < P.ring_entries; st += kChunk) rchunks.push_back(ChunkDev{s, (int32_t)st});
         s_t0[s] = (int)targets.size();
@@ -709,19 +706,31 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
         phr0 += (int64_t)P.O * P.V;
         if (amp0 >= ((int64_t)1 << 31)) return fail(UEGCCD_ERR_ARG, "batch too large for 32-bit packed indices");
     }
-    chunk_begin[n] = (int)chunks.size();
-    // chunks of the amplitudes i <= j: each block's rows up to its diagonal pair
-    std::vector<HChunkDev> hchunks;
-    std::vector<int> hchunk_begin(n + 1, 0);
-    for (int s = 0; s < n; s++) {
-        hchunk_begin[s] = (int)hchunks.size();
-        for (const auto &B : b->plans[s].blocks) {
-            const int64_t lo = B.t0, hi = B.t0 + (int64_t)(B.nd + B.dg) * B.v;
-            for (int64_t st = lo; st < hi; st += kChunk)
-                hchunks.push_back(HChunkDev{s, (int32_t)st, (int32_t)std::min(st + kChunk, hi), 0});
-        }
+    // tiles of the amplitudes i <= j: each block's rows up to its diagonal pair
+    std::vector<UTileDev> utiles;
+    std::vector<int> utile_begin(n + 1, 0);
+    for (const auto &bd : blocks) {
+        const SolveDev &S = solves[bd.solve];
+        struct Emit {
+            std::vector<UTileDev> *out;
+            UTileDev base;
+        } em{&utiles, UTileDev{(int)bd.t0, bd.vir0, bd.pair0, bd.solve, S.orb0, S.vtab0, S.jvv0, S.joo0, (int)S.phr0,
+                               S.q2max, bd.v, bd.nvd, (int16_t)bd.sd, (int16_t)bd.dg, (int16_t)bd.nd, 0, 0, 0, 0,
+                               (int16_t)S.O, S.V, {0, 0, 0}}};
+        update_tiles(bd.nd + bd.dg, bd.v,
+                     [](void *to, int c0, int nc, int r0, int nr) {
+                         auto *e = static_cast<Emit *>(to);
+                         UTileDev t = e->base;
+                         t.c0 = (int16_t)c0;
+                         t.nc = (int16_t)nc;
+                         t.r0 = (int16_t)r0;
+                         t.nr = (int16_t)nr;
+                         e->out->push_back(t);
+                     },
+                     &em);
+        utile_begin[bd.solve + 1] = (int)utiles.size();
     }
-    hchunk_begin[n] = (int)hchunks.size();
+    for (int s = 0; s < n; s++) utile_begin[s + 1] = std::max(utile_begin[s + 1], utile_begin[s]);
     trace.mark("solve-loop");
     ph_i.resize(phr0);
     ph_x.resize(phr0);
@@ -776,7 +785,7 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     d.d16_n = d16_n;
     d.nscale = nscale;
     d.nchunks = (int)chunks.size();
-    d.nhchunks = (int)hchunks.size();
+    d.nutiles = (int)utiles.size();
     d.nrchunks = (int)rchunks.size();
     d.ntargets = (int)targets.size();
     d.max_v = max_v;
@@ -854,9 +863,8 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->upload(d.dtiles, dtiles))) return rc;
     if ((rc = b->upload(d.chunks, chunks))) return rc;
     if ((rc = b->upload(d.rchunks, rchunks))) return rc;
-    if ((rc = b->upload(d.chunk_begin, chunk_begin))) return rc;
-    if ((rc = b->upload(d.hchunks, hchunks))) return rc;
-    if ((rc = b->upload(d.hchunk_begin, hchunk_begin))) return rc;
+    if ((rc = b->upload(d.utiles, utiles))) return rc;
+    if ((rc = b->upload(d.utile_begin, utile_begin))) return rc;
     if ((rc = b->upload(d.targets, targets))) return rc;
     if ((rc = b->upload(d.pcol, pcol))) return rc;
     int *d_tbase = nullptr;
@@ -871,9 +879,9 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->upload(d.vir, vir))) return rc;
     if ((rc = b->alloc(d.vpk, vir.size()))) return rc;
     if ((rc = b->alloc(d.ppk, pair_i.size()))) return rc;
+    if ((rc = b->alloc(d.rowpk, pair_i.size()))) return rc;
     if ((rc = b->alloc(d.pos, pos0))) return rc;
     if ((rc = b->alloc(d.partner, amp0))) return rc;
-    if ((rc = b->alloc(d.mirror, amp0))) return rc;
     if ((rc = b->alloc(d.amps, amp0))) return rc;
     if ((rc = b->upload(d.nv4, nv4))) return rc;
     if ((rc = b->upload(d.nvp, nvp))) return rc;
@@ -892,7 +900,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->upload(d.ph_x, ph_x))) return rc;
     if ((rc = b->alloc(d.ridx_x, ph0))) return rc;
     if ((rc = b->alloc(d.ridx_y, ph0))) return rc;
-    if ((rc = b->alloc(d.vcoef, amp0))) return rc;
     if ((rc = b->alloc(d.xy, d.xy_n))) return rc;
     if ((rc = b->alloc(d.rx, d.xy_n))) return rc;
     if ((rc = b->alloc(d.ph_a, phr0))) return rc;
@@ -903,14 +910,13 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->alloc(d.g, amp0))) return rc;
     if ((rc = b->alloc(d.jvv, jvv0))) return rc;
     if ((rc = b->alloc(d.joo, joo0))) return rc;
-    const size_t npart = std::max(chunks.size(), hchunks.size());   // per full or half chunk
+    const size_t npart = utiles.size();
     if ((rc = b->alloc(d.part_e, npart))) return rc;
     if ((rc = b->alloc(d.part_dt, npart))) return rc;
     if ((rc = b->alloc(d.part_r, npart))) return rc;
     if ((rc = b->alloc(d.red, 3 * (size_t)n))) return rc;
     if ((rc = b->alloc(d.active, n))) return rc;
     b->hsolves = solves;
-    b->chunk_begin = chunk_begin;
     b->red.assign(3 * (size_t)n, 0.0);
     b->active.assign(n, 1);
     CU(cudaMemcpyAsync(d.active, b->active.data(), n, cudaMemcpyHostToDevice, b->stream));
@@ -924,7 +930,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     launch_block_tables(d, b->stream);
     launch_ring_rows(d, (int)phr0, d_row0, b->stream);
     launch_mosaic_targets(d, d_tbase, d_lbase, (size_t)max_vo * sizeof(int), b->stream);
-    launch_vcoef(d, b->stream);
     size_t dn = 0;
     for (int s = 0; s < n; s++) dn = std::max(dn, (size_t)b->plans[s].O * b->plans[s].O * b->plans[s].V);
     b->dense_n = dn;
@@ -991,8 +996,7 @@ int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, doubl
 // Integral options for every later call on the batch (SetPointers, Main.f90:274-318, with
 // no range flags): GapII > 0 zeroes the integrals above GapII (GapERI, HEG.f90:938-940) --
 // the |q|^2 tables are filtered; CoreN > 0 zeroes those with an index p <= CoreN
-// (CoreERI, HEG.f90:882-885) -- the kernels hold core pairs at zero.  The per-amplitude
-// Coulomb factors are rebuilt from the filtered tables.
+// (CoreERI, HEG.f90:882-885) -- the kernels hold core pairs at zero.
 // The |q|^2 tables of every solve for an ERI flag (CasedERI, HEG.f90:725-774; flag 0 is
 // BaseERI's value), with the reference's "< 0 -> -100" guard and the GapII filter applied in
 // its order.  CoreN is not in the tables: the kernels hold core pairs at zero.
@@ -1023,12 +1027,11 @@ std::vector<double> integral_tables(const UegccdBatch &b, int flag, double gapii
     return vt;
 }
 
-// Uploads the tables of an ERI flag and the Coulomb factors that follow them.
+// Uploads the tables of an ERI flag.
 int load_tables(UegccdBatch &b, int flag)
 {
     const std::vector<double> vt = integral_tables(b, flag, b.gapii);
     CU(cudaMemcpyAsync(b.d.vtab, vt.data(), vt.size() * sizeof(double), cudaMemcpyHostToDevice, b.stream));
-    launch_vcoef(b.d, b.stream);
     b.d.w16_valid = false;   // the FP16 Coulomb slabs follow the tables
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(b.stream));
@@ -1051,7 +1054,6 @@ int set_integrals(UegccdBatch &b, int core_n, double gapii)
     for (auto &S : b.hsolves) S.core_n = core_n;
     CU(cudaMemcpyAsync(b.d.solves, b.hsolves.data(), b.hsolves.size() * sizeof(SolveDev), cudaMemcpyHostToDevice,
                        b.stream));
-    launch_vcoef(b.d, b.stream);
     b.d.w16_valid = false;   // the FP16 Coulomb slabs follow the tables
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(b.stream));
@@ -1164,7 +1166,7 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
         CtlBuffers x = c;
         if ((rc = b.alloc(x.state, n)) || (rc = b.alloc(x.applied, n)) || (rc = b.alloc(x.count, 1)) ||
             (rc = b.alloc(x.Bm, (size_t)n * kDiisMax * kDiisMax)) || (rc = b.alloc(x.coef, (size_t)n * kDiisMax)) ||
-            (rc = b.alloc(x.part, (size_t)b.d.nhchunks * kDiisMax))) {
+            (rc = b.alloc(x.part, (size_t)b.d.nutiles * kDiisMax))) {
             b.rollback(m);
             return rc;
         }
@@ -1266,12 +1268,13 @@ int tune_batch(UegccdBatch &b)
     return 0;
 }
 
-// Runs the iteration for all solves of the batch from the amplitudes in d.t.
+// Runs the iteration for all solves of the batch from the amplitudes in d.t (from_mp2: those
+// k_mp2 has just written).
 // Iteration control lives on the device; the host replays a captured iteration
 // graph kPoll times between polls of the number of active solves.  With kernel
 // timing on, the last iteration of each round runs as direct launches between
 // CUDA events: that iteration is the sample the per-kernel times come from.
-int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult *res)
+int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult *res, bool from_mp2 = false)
 {
     constexpr int kPoll = 4;
     DevBatch &d = b.d;
@@ -1320,10 +1323,14 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
     if (!b.tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch(b))) return rc;
     b.launches = 0;
     CU(cudaEventRecord(b.ev0, b.stream));
-    // CCEnergy of the start amplitudes and dT = max|T| (CCD.f90:63-64, dRPA.f90:68-69)
-    launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
+    // CCEnergy of the start amplitudes and dT = max|T| (CCD.f90:63-64, dRPA.f90:68-69).  Those of
+    // the MP2 amplitudes on the plain integrals are k_mp2's own sums.
+    if (!from_mp2 || drpa || table_guard.on) {
+        launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
+        b.launches++;
+    }
     launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
-    b.launches += 2;
+    b.launches++;
     int count = n, rounds = 0;
     const int max_rounds = opt->max_iter / kPoll + 2;
     // mixed precision: tensor-core ladder of t - t_ref, t_ref refreshed (FP64) each round,
@@ -1458,9 +1465,12 @@ int session_start(UegccdBatch &b, const UegccdOptions *opt, int drpa)
     if ((rc = set_active_all(b, 1))) return rc;
     if (drpa && (rc = drpa_alloc(b))) return rc;
     if (!b.tuned && !drpa && (f.do_ring || f.do_xring) && (rc = tune_batch(b))) return rc;
-    launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
+    if (drpa) {   // else k_mp2's own sums are those of the start amplitudes
+        launch_energy(d, 1, 0.0, b.stream);
+        b.launches++;
+    }
     launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
-    b.launches += 2;
+    b.launches++;
     if ((rc = capture_iteration(b, f, opt->tol, opt->max_iter, ndiis))) return rc;
     CU(cudaStreamSynchronize(b.stream));
     S.opt = *opt;
@@ -2021,7 +2031,7 @@ int uegccd_batch_solve(UegccdBatch *b, const UegccdOptions *opt, int32_t drpa, d
         // the reference starts dRPA from T2aaaa of the MP2 step (Main.f90:85-91)
         launch_to_aaaa(b->d, b->stream);
     }
-    int st = two ? run_two_channel_solves(*b, opt, results) : run_solves(*b, opt, drpa, results);
+    int st = two ? run_two_channel_solves(*b, opt, results) : run_solves(*b, opt, drpa, results, true);
     if (st < 0) return st;
     CU(cudaEventRecord(b->ev_solve1, b->stream));
     CU(cudaEventSynchronize(b->ev_solve1));
@@ -2135,7 +2145,7 @@ int uegccd_footprint(const UegccdSystem *sys, int32_t ndiis, int32_t mixed, int6
     int64_t b = 0;
     int64_t sum_ov = 0;
     for (const auto &B : P.blocks) sum_ov += B.o + B.v;
-    b += A * (8 * 3 + 16 + sizeof(AmpInfo) + 4 + 4); // t, t_new, g; Coulomb factors; amps; partner, mirror
+    b += A * (8 * 3 + sizeof(AmpInfo) + 4 + 8);      // t, t_new, g; amps; partner, ring positions
     b += sum_ov * (8 + 4) + (V + O + 1) * (4 + 8);   // mosaic partials and target lists
     b += O * O * V * 4;                              // pos
     b += O * V * 8 * 2 + O * O * 16 + nblk * V * 2;  // dRPA sums and lookups (allocated for dRPA only)

@@ -26,28 +26,26 @@ struct DevBatch {
     int q2max = 0, n2max = 0;   // largest |q|^2 of the solves' tables, largest |n|^2
     int *vpk = nullptr;         // beside vir: the virtual's packed vector
     int2 *ppk = nullptr;        // beside pair_i / pair_j: theirs
+    int4 *rowpk = nullptr;      // the same with i | j << 16 in the third word
     int max_occ = 0;    // largest NOcc
     int64_t namp = 0;
     SolveDev *solves = nullptr;
     BlockDev *blocks = nullptr;
     ChunkDev *chunks = nullptr;      // amplitude chunks
     ChunkDev *rchunks = nullptr;     // ring-intermediate chunks over (i, x, l)
-    int *chunk_begin = nullptr;      // nsolves+1: first chunk of each solve
-    HChunkDev *hchunks = nullptr;    // chunks of the amplitudes i <= j (k_update, DIIS, commit)
-    int nhchunks = 0;
-    int *hchunk_begin = nullptr;     // nsolves+1: first half chunk of each solve
+    UTileDev *utiles = nullptr;      // tiles of the amplitudes i <= j (update.cu), solve after solve
+    int nutiles = 0;
+    int *utile_begin = nullptr;      // nsolves+1: first tile of each solve
     int2 *targets = nullptr;         // mosaic targets (solve, id)
     int16_t *pair_i = nullptr, *pair_j = nullptr, *vir = nullptr;
     int16_t *pcol = nullptr;          // beside vir: column of the partner d = K - c in the same block
     int32_t *pos = nullptr;          // dense (i,j,a) -> global packed index or -1
     int32_t *partner = nullptr;      // packed -> packed index of (i,j,b)
-    int32_t *mirror = nullptr;       // packed (i,j,a): index of (j,i,b) if i < j, -1 if i = j, -2 if i > j
     AmpInfo *amps = nullptr;
     int4 *nv4 = nullptr;
     int *nvp = nullptr;              // the same vectors packed a component per byte (q2p in kernels_fp64.cu)
     double *eigen = nullptr, *vtab = nullptr;
     double *t = nullptr, *t_new = nullptr, *g = nullptr;
-    double2 *vcoef = nullptr;         // per amplitude {v(i-a), v(a-j)} (k_vcoef, once per batch)
     double *jvv = nullptr, *joo = nullptr;
     // dRPA (on the first dRPA solve): k_drpa_sums' CTA list {solve, i}, row and column lookups,
     // and its U, S2 per (i, x) at phr0 + i*V + x - O; per solve the count of finished CTAs
@@ -220,7 +218,6 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
                     KernelTimer *kt = nullptr, const CtlBuffers *diis = nullptr, int ndiis = 0,
                     const Fork *fork = nullptr);
 void launch_pack(const DevBatch &d, int s, int namp, const double *dense, cudaStream_t st);
-void launch_vcoef(const DevBatch &d, cudaStream_t st);
 void launch_unpack_all(const DevBatch &d, const int64_t *dense_off, const double *t, double *out, cudaStream_t st);
 // Structure-factor sums of solve `solve` from d.t: groups = its particle-hole groups
 // {first row, rows}; grid = 5 arrays of (2S+1)^3 (SfSum, SfDSum, SfXSum, contributions,
@@ -228,7 +225,7 @@ void launch_unpack_all(const DevBatch &d, const int64_t *dense_off, const double
 // zeroed by the caller; *err = 1 if a transfer falls outside.
 void launch_sf(const DevBatch &d, const int2 *groups, int ngroups, int solve, int S, double *grid, int *err,
                cudaStream_t st);
-// pos (pre-set to -1), amps, partner, mirror from the block structure; the particle-hole
+// pos (pre-set to -1), amps, partner from the block structure; the particle-hole
 // tables ph_a, ph_b (pre-set to -1) from the ring pairs; the ring gather indices
 void launch_block_tables(const DevBatch &d, cudaStream_t st);
 // rrows of the n ph rows (row0: each solve's first)
@@ -246,6 +243,12 @@ void launch_refresh(const DevBatch &d, cudaStream_t st);
 // Device-side iteration control
 void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
                  cudaStream_t st);
+// The element-wise kernels (update.cu): G, residual and update of the amplitudes i <= j, and the
+// DIIS extrapolation; update_tiles hands (c0, nc, r0, nr) of each tile of a block to emit.
+void launch_update(const DevBatch &d, const TermFlags &f, int mode, double *g_out, const CtlBuffers *diis, int ndiis,
+                   cudaStream_t st);
+void launch_extrap(const DevBatch &d, const CtlBuffers &c, int ndiis, cudaStream_t st);
+void update_tiles(int rows, int v, void (*emit)(void *, int, int, int, int), void *to);
 int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f, double tol, int max_iter,
                      int ndiis, cudaStream_t st, KernelTimer *kt, const Fork *fork = nullptr);
 void launch_unpack(const DevBatch &d, int s, int namp, const double *t, double *ab, double *ba, double *aa,

@@ -95,68 +95,6 @@ __device__ __forceinline__ double block_sum(double v)
     return r;  // valid in thread 0
 }
 
-// ----------------------------------------------------------------------------
-// MP2 (MP2.f90:56-74): t = v(i-a)/D, D = e_i + e_j - e_a - e_b.
-// E(2) = 1/2 sum [T2aaaa (V_ijab - V_ijba) + T2abab V_ijab - T2abba V_ijba]
-//      = sum t(ij,a) (2 v(i-a) - v(i-b))   after the a <-> b re-indexing.
-// ----------------------------------------------------------------------------
-// The integrals come from the per-amplitude Coulomb factors {v(i-a), v(a-j)} (k_vcoef; the
-// same table entries): v(i-b) = v(a-j), since n_i - n_b = n_a - n_j.
-__global__ void k_mp2(const ChunkDev *__restrict__ chunks, const SolveDev *__restrict__ solves,
-                      const AmpInfo *__restrict__ amps, const double2 *__restrict__ vcoef,
-                      const double *__restrict__ eigen, double *__restrict__ t,
-                      double *__restrict__ part_e, double *__restrict__ part_a, double *__restrict__ part_b)
-{
-    const ChunkDev ch = chunks[blockIdx.x];
-    const SolveDev s = solves[ch.solve];
-    const int loc = ch.start + threadIdx.x;
-    double e = 0.0, mx = 0.0;
-    if (loc < s.namp) {
-        const int64_t p = s.amp0 + loc;
-        const AmpInfo q = amps[p];
-        const double *ev = eigen + s.orb0;
-        double denom = ev[q.i] + ev[q.j] - ev[q.a] - ev[q.b];
-        const double2 vc = vcoef[p];
-        double via = vc.x;
-        double vib = vc.y;
-        // a core pair's integrals are zero (CoreERI), so is its amplitude
-        double x = (q.i < s.core_n || q.j < s.core_n) ? 0.0 : via / denom;
-        t[p] = x;
-        e = x * (2.0 * via - vib);
-        mx = fabs(x);
-    }
-    double dummy = 0.0;
-    block_reduce3<kChunk>(e, mx, dummy);
-    if (threadIdx.x == 0) { part_e[blockIdx.x] = e; part_a[blockIdx.x] = mx; part_b[blockIdx.x] = 0.0; }
-}
-
-// Energy of the current amplitudes and max|t| (the dT before the first iteration).
-// kind 0, CCEnergy (CCD.f90:225-227): E = sum t(ij,a) (2 v(i-a) - v(a-j)) after re-indexing;
-// kind 1, dRPA CCEnergy (dRPA.f90:206-210): E = sum t (2 v(a-i) - csosex v(b-i)).
-// The integrals come from the per-amplitude Coulomb factors {v(i-a), v(a-j)} (k_vcoef):
-// v(a-i) = v(i-a), and v(b-i) = v(a-j) since n_b - n_i = n_j - n_a.
-__global__ void k_energy(const ChunkDev *__restrict__ chunks, const SolveDev *__restrict__ solves,
-                         const double2 *__restrict__ vcoef, const double *__restrict__ t, int kind, double csosex,
-                         double *__restrict__ part_e, double *__restrict__ part_a, double *__restrict__ part_b)
-{
-    const ChunkDev ch = chunks[blockIdx.x];
-    const SolveDev s = solves[ch.solve];
-    const int loc = ch.start + threadIdx.x;
-    double e = 0.0, mx = 0.0;
-    if (loc < s.namp) {
-        const int64_t p = s.amp0 + loc;
-        double x = t[p];
-        const double2 vc = vcoef[p];
-        double via = vc.x;
-        if (kind == 0) e = x * (2.0 * via - vc.y);
-        else e = via * x * 2.0 - vc.y * x * csosex;
-        mx = fabs(x);
-    }
-    double dummy = 0.0;
-    block_reduce3<kChunk>(e, mx, dummy);
-    if (threadIdx.x == 0) { part_e[blockIdx.x] = e; part_a[blockIdx.x] = mx; part_b[blockIdx.x] = 0.0; }
-}
-
 // t'(ij,a) = t(ij,a) - t(ij,b): T2aaaa of spin-adapted amplitudes (MP2.f90:70), the dRPA
 // start, in place: the thread of the smaller index of a partner pair forms both values.
 __global__ void k_to_aaaa(int64_t n, const int32_t *__restrict__ partner, double *__restrict__ t)
@@ -190,7 +128,6 @@ __global__ void k_reduce_solves(const int *__restrict__ chunk_begin, const doubl
 
 // (The ladders, CCD.f90:588-686, are in ladder.cu; they write G first, before k_update adds
 // the other terms.)
-constexpr int kVtabSmem = kVtabSmemEntries;  // |q|^2 table entries staged in shared memory
 
 // The dynamic shared-memory limits only grow (batches of different sizes coexist), under
 // one lock: batches are created from several host threads while others solve.  Kernel
@@ -238,7 +175,7 @@ __global__ void __launch_bounds__(kMosThreads) k_mosaic_blk(const BlockDev *__re
     const int v = B.v, oc = B.nd + B.dg;
     constexpr int kW = kMosThreads / 32;
     extern __shared__ double msm[];
-    double *sv = msm;                          // vt_n: the batch's largest |q|^2 table (at most kVtabSmem)
+    double *sv = msm;                          // vt_n: the batch's largest |q|^2 table (at most kVtabSmemEntries)
     double *coff = sv + vt_n;                  // v: column sums over the rows i < j
     double *cdg = coff + v;                    // v: the diagonal pair's row (if any)
     double *wrs = cdg + v;                     // kW x oc: per-warp row sums
@@ -507,61 +444,27 @@ __global__ void __launch_bounds__(kDrpaThreads)
 
 // (The rings and crossed rings, CCD.f90:689-940, are in rings.cu.)
 
-// ----------------------------------------------------------------------------
-// Fused residual / update / convergence / energy, one thread per amplitude.
-//   G = ladders (from k_ladder) + drivers + mosaics + rings + crossed rings
-//   R = -G + D t                          (GetRes, CCD.f90:417)
-//   t' = (G/D - (1-f) t)/f                (SolveCC, CCD.f90:380)
-//   dT = max |t' - t|                     (CnvrgCC, CCD.f90:452-454)
-//   E  = sum t' (2 v(i-a) - v(a-j))       (CCEnergy, CCD.f90:225-227 re-indexed)
-// mode 0: update (in place, or with DIIS into the history; partials e/dT/|R|); mode 1:
-// residual only (|R|).
-// ----------------------------------------------------------------------------
-struct UpdateArgs {
-    const HChunkDev *chunks;
-    const SolveDev *solves;
-    const AmpInfo *amps;
-    const int32_t *mirror;
-    const double *eigen;
-    double *t;                    // each amplitude i <= j reads its own value only: updated in place
-    const double *g_ladder;
-    const double *jvv, *joo;
-    const double *dru, *drs2;     // dRPA: U and S2 of k_drpa_sums
-    double *part_e, *part_dt, *part_r;
-    double *g_out;            // optional: full G per amplitude (term checks)
-    const double *rx;                          // ring and crossed-ring G, particle-hole layout
-    const int2 *rpos;                          // where each amplitude's two values sit in it
-    const uint8_t *active;
-    int do_ladder, do_mosaic, do_ring, do_xring, do_driver, drpa, mode;
-    // Pulay DIIS push fused into the update (mode 0, ndiis > 0): the new (t', e) pair
-    // goes to the solve's history slot and the chunk partials of e . e_j to dpart
-    const IterState *st;
-    int ndiis;
-    int64_t namp;
-    double *hist_t, *dpart;
-    float *hist_e;
-    const double2 *vcoef;     // per amplitude {v(i-a), v(a-j)}
-};
-
 // One CTA per momentum block: for every element (pair r = (i, j), column c = a) the
-// amplitude record (i, j, a, b), the position map entry (i, j, a) -> packed index, the
-// packed index of the partner (i, j, b), b in column pcol[c] of the same block, and the
-// mirror: (j, i, b) in row r + nd + dg for the rows r < nd (i < j); -1 on the diagonal
-// pair's row, -2 on the mirror rows.  Beside them the packed vectors of the block's virtuals and
-// pairs.
+// amplitude record (i, j, a, b), the position map entry (i, j, a) -> packed index and the packed
+// index of the partner (i, j, b), b in column pcol[c] of the same block.  Beside them the packed
+// vectors of the block's virtuals and pairs.
 __global__ void k_block_tables(const BlockDev *__restrict__ blocks, const SolveDev *__restrict__ solves,
                                const int16_t *__restrict__ pair_i, const int16_t *__restrict__ pair_j,
                                const int16_t *__restrict__ vir, const int16_t *__restrict__ pcol,
                                const int *__restrict__ nvp, AmpInfo *__restrict__ amps, int32_t *__restrict__ pos,
-                               int32_t *__restrict__ partner, int32_t *__restrict__ mirror, int *__restrict__ vpk,
-                               int2 *__restrict__ ppk)
+                               int32_t *__restrict__ partner, int *__restrict__ vpk, int2 *__restrict__ ppk,
+                               int4 *__restrict__ rowpk)
 {
     const BlockDev B = blocks[blockIdx.x];
     const SolveDev s = solves[B.solve];
     const int n = B.o * B.v;
     for (int c = threadIdx.x; c < B.v; c += blockDim.x) vpk[B.vir0 + c] = nvp[s.orb0 + vir[B.vir0 + c]];
-    for (int r = threadIdx.x; r < B.o; r += blockDim.x)
-        ppk[B.pair0 + r] = make_int2(nvp[s.orb0 + pair_i[B.pair0 + r]], nvp[s.orb0 + pair_j[B.pair0 + r]]);
+    for (int r = threadIdx.x; r < B.o; r += blockDim.x) {
+        const int i = pair_i[B.pair0 + r], j = pair_j[B.pair0 + r];
+        const int2 n = make_int2(nvp[s.orb0 + i], nvp[s.orb0 + j]);
+        ppk[B.pair0 + r] = n;
+        rowpk[B.pair0 + r] = make_int4(n.x, n.y, i | j << 16, 0);
+    }
     for (int e = threadIdx.x; e < n; e += blockDim.x) {
         const int r = e / B.v, c = e - r * B.v;
         const int i = pair_i[B.pair0 + r], j = pair_j[B.pair0 + r];
@@ -570,8 +473,6 @@ __global__ void k_block_tables(const BlockDev *__restrict__ blocks, const SolveD
         amps[p] = AmpInfo{(int16_t)i, (int16_t)j, (int16_t)a, vir[B.vir0 + pc]};
         pos[s.pos0 + ((int64_t)i * s.O + j) * s.V + (a - s.O)] = (int32_t)p;
         partner[p] = (int32_t)(B.t0 + (int64_t)r * B.v + pc);
-        const int oc = B.nd + B.dg;
-        mirror[p] = r < B.nd ? (int32_t)(B.t0 + (int64_t)(r + oc) * B.v + pc) : r < oc ? -1 : -2;
     }
 }
 
@@ -678,159 +579,35 @@ __global__ void k_ring_stage(const RingPairDev *__restrict__ pairs, const SolveD
 // row (i,a), column (j,b) when (i,a) is in group 1, else at row (j,b), column (i,a) (its
 // mirror's place); its crossed-ring G in the second half of row (i,b) at column (j,a), or of
 // row (j,a) at column (i,b).
-__global__ void k_rx_pos(const HChunkDev *__restrict__ chunks, const SolveDev *__restrict__ solves,
-                         const AmpInfo *__restrict__ amps, const int32_t *__restrict__ ph_a,
-                         const int32_t *__restrict__ ph_b, int2 *__restrict__ rpos)
+__global__ void __launch_bounds__(128) k_rx_pos(const UTileDev *__restrict__ tiles, const SolveDev *__restrict__ solves,
+                                               const AmpInfo *__restrict__ amps, const int32_t *__restrict__ ph_a,
+                                               const int32_t *__restrict__ ph_b, int2 *__restrict__ rpos)
 {
-    const HChunkDev ch = chunks[blockIdx.x];
-    const SolveDev s = solves[ch.solve];
-    const int loc = ch.start + threadIdx.x;
-    if (loc >= ch.end) return;
-    const int64_t p = s.amp0 + loc;
-    const AmpInfo q = amps[p];
-    const int V = s.V, O = s.O;
-    const int32_t *pa = ph_a + s.phr0, *pb = ph_b + s.phr0;
-    const int ia = q.i * V + q.a - O, jb = q.j * V + q.b - O, ib = q.i * V + q.b - O, ja = q.j * V + q.a - O;
-    const int r = pa[ia] >= 0 ? pa[ia] + pb[jb] : pa[jb] + pb[ia];
-    const int x = pa[ib] >= 0 ? pa[ib] + pb[ib] + pb[ja] : pa[ja] + pb[ja] + pb[ib];
-    rpos[p] = make_int2(r, x);
+    const UTileDev T = tiles[blockIdx.x];
+    const SolveDev s = solves[T.solve];
+    for (int e = threadIdx.x; e < T.nr * T.nc; e += blockDim.x) {
+        const int64_t p = T.t0 + (int64_t)(T.r0 + e / T.nc) * T.v + T.c0 + e % T.nc;
+        const AmpInfo q = amps[p];
+        const int V = s.V, O = s.O;
+        const int32_t *pa = ph_a + s.phr0, *pb = ph_b + s.phr0;
+        const int ia = q.i * V + q.a - O, jb = q.j * V + q.b - O, ib = q.i * V + q.b - O, ja = q.j * V + q.a - O;
+        const int r = pa[ia] >= 0 ? pa[ia] + pb[jb] : pa[jb] + pb[ia];
+        const int x = pa[ib] >= 0 ? pa[ib] + pb[ib] + pb[ja] : pa[ja] + pb[ja] + pb[ib];
+        rpos[p] = make_int2(r, x);
+    }
 }
 
 void launch_block_tables(const DevBatch &d, cudaStream_t st)
 {
     if (d.nblocks > 0)
         k_block_tables<<<d.nblocks, 256, 0, st>>>(d.blocks, d.solves, d.pair_i, d.pair_j, d.vir, d.pcol, d.nvp,
-                                                  d.amps, d.pos, d.partner, d.mirror, d.vpk, d.ppk);
+                                                  d.amps, d.pos, d.partner, d.vpk, d.ppk, d.rowpk);
     if (d.nrpairs > 0) k_ph_tables<<<d.nrpairs, 128, 0, st>>>(d.rpairs, d.solves, d.ph_i, d.ph_x, d.ph_a, d.ph_b);
-    if (d.nrpairs > 0 && d.nhchunks > 0)
-        k_rx_pos<<<d.nhchunks, kChunk, 0, st>>>(d.hchunks, d.solves, d.amps, d.ph_a, d.ph_b, d.rpos);
+    if (d.nrpairs > 0 && d.nutiles > 0)
+        k_rx_pos<<<d.nutiles, 128, 0, st>>>(d.utiles, d.solves, d.amps, d.ph_a, d.ph_b, d.rpos);
     if (d.nrchunks > 0)
         k_ring_index<<<d.nrchunks, kChunk, 0, st>>>(d.rchunks, d.solves, d.ph_i, d.ph_x, d.pos, d.ridx_x,
                                                     d.ridx_y);
-}
-
-// Static per-amplitude Coulomb factors of the update: {v(i-a), v(a-j)}.
-__global__ void k_vcoef(const ChunkDev *__restrict__ chunks, const SolveDev *__restrict__ solves,
-                        const AmpInfo *__restrict__ amps, const int4 *__restrict__ nv4,
-                        const double *__restrict__ vtab, double2 *__restrict__ vcoef)
-{
-    const ChunkDev ch = chunks[blockIdx.x];
-    const SolveDev s = solves[ch.solve];
-    const int loc = ch.start + threadIdx.x;
-    if (loc >= s.namp) return;
-    const int64_t p = s.amp0 + loc;
-    const AmpInfo q = amps[p];
-    vcoef[p] = make_double2(vpq(s, nv4, vtab, q.i, q.a), vpq(s, nv4, vtab, q.a, q.j));
-}
-
-void launch_vcoef(const DevBatch &d, cudaStream_t st)
-{
-    k_vcoef<<<d.nchunks, kChunk, 0, st>>>(d.chunks, d.solves, d.amps, d.nv4, d.vtab, d.vcoef);
-}
-
-// Eight CTAs per SM (32 registers, a few spilled): the kernel waits on scattered loads, and
-// full occupancy hides them better than the spills cost (0.70 -> 0.50 ms per residual at
-// 100 twists of N=54, against the 64-register form).
-__global__ void __launch_bounds__(kChunk, 8) k_update(UpdateArgs A)
-{
-    const HChunkDev ch = A.chunks[blockIdx.x];
-    double esum = 0.0, dtmax = 0.0, rmax = 0.0;
-    const bool on = A.active[ch.solve];
-    const SolveDev s = A.solves[ch.solve];
-    const int loc = ch.start + threadIdx.x;
-    // The chunks cover the amplitudes i <= j only: by the pair symmetry t(ij,a) = t(ji,b)
-    // each amplitude with i < j also updates its mirror (j,i,b); every term of G shares the
-    // symmetry.
-    const bool valid = loc < ch.end;
-    const int32_t mir = on && valid ? A.mirror[s.amp0 + loc] : -2;
-    const double wgt = mir >= 0 ? 2.0 : 1.0;   // energy and DIIS dot weight: this amplitude and its mirror
-    if (mir != -2) {
-        const int64_t p = s.amp0 + loc;
-        const AmpInfo q = A.amps[p];
-        const int i = q.i, j = q.j, a = q.a, b = q.b;
-        const int O = s.O;
-        const double told = A.t[p];
-        const double2 vc = A.vcoef[p];
-        const double via = vc.x;
-        double g = A.do_ladder ? A.g_ladder[p] : 0.0;
-        if (A.do_driver) g += via;  // GetG2Drivers: G2abab = V(n_i - n_a)
-        if (A.do_mosaic)
-            g -= 0.5 * (A.jvv[s.jvv0 + a - O] + A.jvv[s.jvv0 + b - O] + A.joo[s.joo0 + i] + A.joo[s.joo0 + j]) * told;
-        if (A.drpa) {
-            if (A.do_ring) {   // linear and quadratic rings (k_drpa_sums)
-                const int64_t ia = s.phr0 + (int64_t)i * s.V + (a - O), jb = s.phr0 + (int64_t)j * s.V + (b - O);
-                const double u = A.dru[ia];
-                g += u + A.dru[jb] + 2.0 * u * A.drs2[jb];
-            }
-        } else if (A.do_ring || A.do_xring) {
-            // the ring G (rings, linear + quadratic, CCD.f90:716-811) and the crossed-ring G
-            // (CCD.f90:845-937) of this amplitude, where k_rings left them (k_rx_pos)
-            const int2 ro = A.rpos[p];
-            if (A.do_ring) g += A.rx[ro.x];
-            if (A.do_xring) g += A.rx[ro.y];
-        }
-        {   // core pair: every term has a zero factor (CoreN read on its own: taken from the
-            // solve record above, it costs this kernel registers)
-            const int cn = __ldg(&A.solves[ch.solve].core_n);
-            if (i < cn || j < cn) g = 0.0;
-        }
-        if (A.g_out) {
-            A.g_out[p] = g;
-            if (mir >= 0) A.g_out[mir] = g;
-        }
-        const double *ev = A.eigen + s.orb0;
-        const double denom = ev[i] + ev[j] - ev[a] - ev[b];
-        const double r = -g + denom * told;
-        rmax = fabs(r);
-        if (A.mode == 0) {
-            const double f = s.denom_factor;
-            const double tn = (g / denom - (1.0 - f) * told) / f;
-            if (A.ndiis == 0) {  // with DIIS the history slot holds t'
-                A.t[p] = tn;
-                if (mir >= 0) A.t[mir] = tn;
-            }
-            dtmax = fabs(tn - told);
-            if (A.drpa) esum = via * tn * 2.0;  // SOSEX part added by k_drpa_energy at the end
-            else esum = tn * (2.0 * via - vc.y);
-            esum *= wgt;
-            if (!(fabs(tn) < 1e300)) dtmax = __longlong_as_double(0x7ff0000000000000LL);  // +Inf marks NaN/Inf
-            if (A.ndiis > 0) {
-                const int slot = (A.st[ch.solve].niter - 1) % A.ndiis;
-                const float e = (float)(tn - told);
-                // the mirrors' history entries are never read: k_diis_extrap2 and the dot
-                // products go through the amplitudes i <= j
-                A.hist_t[(int64_t)slot * A.namp + p] = tn;
-                A.hist_e[(int64_t)slot * A.namp + p] = e;
-            }
-        }
-    }
-    if (A.mode == 0 && A.ndiis > 0 && on) {
-        // e . e_j of every stored j (the chunk belongs to one solve: the loop is uniform)
-        const int nb = A.st[ch.solve].niter;
-        const int slot = (nb - 1) % A.ndiis, nvec = min(nb, A.ndiis);
-        const bool mine = mir != -2;   // the mirrors count through their pair (weight 2)
-        const int64_t p = s.amp0 + loc;
-        const double e0 = mine ? (double)A.hist_e[(int64_t)slot * A.namp + p] : 0.0, e = wgt * e0;
-        __shared__ double sd[kChunk / 32][kDiisMax];
-        const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-        for (int jv = 0; jv < nvec; jv++) {
-            double d = mine ? e * (jv == slot ? e0 : (double)A.hist_e[(int64_t)jv * A.namp + p]) : 0.0;
-            for (int o = 16; o > 0; o >>= 1) d += __shfl_down_sync(0xffffffffu, d, o);
-            if (l == 0) sd[w][jv] = d;
-        }
-        __syncthreads();
-        if (threadIdx.x < nvec) {
-            double d = 0.0;
-            for (int k = 0; k < kChunk / 32; k++) d += sd[k][threadIdx.x];
-            A.dpart[(int64_t)blockIdx.x * kDiisMax + threadIdx.x] = d;
-        }
-    }
-    block_reduce3<kChunk>(esum, dtmax, rmax);
-    if (threadIdx.x == 0) {
-        A.part_e[blockIdx.x] = esum;
-        A.part_dt[blockIdx.x] = dtmax;
-        A.part_r[blockIdx.x] = rmax;
-    }
 }
 
 // ----------------------------------------------------------------------------
@@ -906,7 +683,7 @@ __device__ bool pulay_warp(const double *B, int nvec, double *c, double (*A)[kMa
 // The end of an iteration, one CTA per solve: the energy and max|dT| from the chunk partials in
 // chunk order, the new row of the Pulay matrix from the dot-product partials, the convergence
 // decision and the Pulay coefficients.  init = 1: the start amplitudes' energy, recorded, and
-// whether to iterate.  applied = the solves this iteration updated (k_diis_extrap2 runs on
+// whether to iterate.  applied = the solves this iteration updated (k_diis_extrap runs on
 // those); active = the ones that go on, *count their number.
 // One launch with the elimination spread over a warp in shared memory, where the reduction, the
 // row reduction, a one-thread-per-solve control (its 17 x 18 matrix in local memory) and the
@@ -994,29 +771,6 @@ __global__ void __launch_bounds__(256)
     }
 }
 
-// t = sum_j c_j t'_j over the amplitudes i <= j, each also written to its mirror (j,i,b)
-__global__ void k_diis_extrap2(const HChunkDev *__restrict__ chunks, const SolveDev *__restrict__ solves,
-                               int64_t namp, const double *__restrict__ hist_t, const double *__restrict__ coef,
-                               int ndiis, const int32_t *__restrict__ mirror, double *__restrict__ t,
-                               const uint8_t *__restrict__ applied)
-{
-    const HChunkDev ch = chunks[blockIdx.x];
-    if (!applied[ch.solve]) return;
-    const SolveDev s = solves[ch.solve];
-    const int loc = ch.start + threadIdx.x;
-    if (loc >= ch.end) return;
-    const int64_t p = s.amp0 + loc;
-    const int32_t mir = mirror[p];
-    const double *c = coef + ch.solve * kMaxDiis;
-    double x = 0.0;
-    for (int jv = 0; jv < ndiis; jv++) {
-        const double cj = c[jv];
-        if (cj != 0.0) x = fma(cj, hist_t[(int64_t)jv * namp + p], x);
-    }
-    t[p] = x;
-    if (mir >= 0) t[mir] = x;
-}
-
 __global__ void k_copy(int64_t n, const double *__restrict__ src, double *__restrict__ dst)
 {
     const int64_t p = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1033,7 +787,7 @@ void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_ite
                  cudaStream_t st)
 {
     if (init) cudaMemsetAsync(c.count, 0, sizeof(int), st);
-    k_tail<<<d.nsolves, 256, 0, st>>>(init ? d.chunk_begin : d.hchunk_begin, d.part_e, d.part_dt, d.part_r, c.part,
+    k_tail<<<d.nsolves, 256, 0, st>>>(d.utile_begin, d.part_e, d.part_dt, d.part_r, c.part,
                                       c.state, c.Bm, c.coef, c.rec_e, c.rec_dt, c.max_rec, d.active, c.applied,
                                       c.count, tol, max_iter, ndiis, init);
 }
@@ -1050,8 +804,7 @@ int launch_iteration(const DevBatch &d, const CtlBuffers &c, const TermFlags &f,
     n++;
     if (ndiis > 0) {
         if (kt) kt->begin(KID_EXTRAP, st);
-        k_diis_extrap2<<<d.nhchunks, kChunk, 0, st>>>(d.hchunks, d.solves, d.namp, c.hist_t, c.coef, ndiis, d.mirror,
-                                                     d.t, c.applied);
+        launch_extrap(d, c, ndiis, st);
         if (kt) kt->end(st);
         n++;
     }
@@ -1218,21 +971,9 @@ void launch_sf(const DevBatch &d, const int2 *groups, int ngroups, int solve, in
 // ----------------------------------------------------------------------------
 // Launch wrappers
 // ----------------------------------------------------------------------------
-void launch_mp2(const DevBatch &d, cudaStream_t st)
-{
-    k_mp2<<<d.nchunks, kChunk, 0, st>>>(d.chunks, d.solves, d.amps, d.vcoef, d.eigen, d.t, d.part_e, d.part_dt,
-                                        d.part_r);
-}
-
 void launch_reduce(const DevBatch &d, cudaStream_t st)
 {
-    k_reduce_solves<<<d.nsolves, 256, 0, st>>>(d.chunk_begin, d.part_e, d.part_dt, d.part_r, d.red);
-}
-
-void launch_energy(const DevBatch &d, int kind, double csosex, cudaStream_t st)
-{
-    k_energy<<<d.nchunks, kChunk, 0, st>>>(d.chunks, d.solves, d.vcoef, d.t, kind, csosex, d.part_e, d.part_dt,
-                                           d.part_r);
+    k_reduce_solves<<<d.nsolves, 256, 0, st>>>(d.utile_begin, d.part_e, d.part_dt, d.part_r, d.red);
 }
 
 void launch_drpa_tables(const DevBatch &d, cudaStream_t st)
@@ -1250,7 +991,7 @@ void launch_to_aaaa(const DevBatch &d, cudaStream_t st)
 const char *kKernelNames[KID_COUNT] = {"k_mp2",      "k_energy",   "k_ladder",
                                       "k_mosaic_blk", "k_mosaic_sum", "k_drpa_sums", "k_update",
                                       "k_reduce_solves", "k_rings",
-                                      "k_ladder_tc", "k_ring_stage", "k_tail", "k_diis_extrap2"};
+                                      "k_ladder_tc", "k_ring_stage", "k_tail", "k_diis_extrap"};
 
 int tune_stage(DevBatch &d, cudaStream_t st)
 {
@@ -1343,25 +1084,13 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
             cudaStreamWaitEvent(st, fork->done[k], 0);
         }
     }
-    UpdateArgs A;
-    A.chunks = d.hchunks; A.solves = d.solves; A.amps = d.amps; A.mirror = d.mirror;
-    A.eigen = d.eigen; A.t = d.t; A.g_ladder = d.g;
-    A.jvv = d.jvv; A.joo = d.joo; A.dru = d.dru; A.drs2 = d.drs2;
-    A.part_e = d.part_e; A.part_dt = d.part_dt; A.part_r = d.part_r; A.g_out = g_out; A.active = d.active;
-    A.do_ladder = f.do_ladder; A.do_mosaic = f.do_mosaic; A.do_ring = f.do_ring; A.do_xring = f.do_xring;
-    A.do_driver = f.do_driver; A.drpa = f.drpa; A.mode = mode;
-    A.rx = d.rx; A.rpos = d.rpos;
-    A.st = diis ? diis->state : nullptr; A.ndiis = (diis && mode == 0) ? ndiis : 0; A.namp = d.namp;
-    A.hist_t = diis ? diis->hist_t : nullptr; A.hist_e = diis ? diis->hist_e : nullptr;
-    A.dpart = diis ? diis->part : nullptr;
-    A.vcoef = d.vcoef;
     kt->begin(KID_UPDATE, st);
-    k_update<<<d.nhchunks, kChunk, 0, st>>>(A);
+    launch_update(d, f, mode, g_out, diis, ndiis, st);
     kt->end(st);
     n++;
     if (mode != 0) {   // in an iteration k_tail reduces the partials
         kt->begin(KID_REDUCE, st);
-        k_reduce_solves<<<d.nsolves, 256, 0, st>>>(d.hchunk_begin, d.part_e, d.part_dt, d.part_r, d.red);
+        k_reduce_solves<<<d.nsolves, 256, 0, st>>>(d.utile_begin, d.part_e, d.part_dt, d.part_r, d.red);
         kt->end(st);
         n++;
     }

@@ -132,11 +132,14 @@ struct ChunkDev {
     int32_t start;          // first amplitude of the chunk, local to the solve
 };
 
-// A chunk of the amplitudes i <= j (the rows a block keeps; each mirror row follows from
-// its pair): [start, end) local to the solve, at most kChunk long, inside one block.
-struct HChunkDev {
-    int solve;
-    int32_t start, end, pad;
+// A tile of a block's amplitudes i <= j (update.cu): rows [r0, r0+nr), columns [c0, c0+nc), with
+// the block's and the solve's fields that its kernels use.
+struct alignas(16) UTileDev {
+    int t0, vir0, pair0, solve;
+    int orb0, vtab0, jvv0, joo0;
+    int phr0, q2max, v, nvd;
+    int16_t sd, dg, nd, c0, nc, r0, nr, O;
+    int V, pad[3];
 };
 
 }  // namespace uegccd

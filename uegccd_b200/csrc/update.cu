@@ -1,0 +1,459 @@
+// update.cu -- the element-wise kernels of the spin-adapted solve: MP2 start, energy, the update
+// of one iteration and the DIIS extrapolation, all over the amplitudes i <= j.
+//
+// The amplitudes of a block are rows (pairs) of columns (virtuals).  A tile is up to 128 columns of
+// some rows; a thread owns a column: its orbital energies, mosaic sums and Coulomb row side are
+// loaded once and serve its rows, and the values of a row are the same for the whole warp.  What a
+// thread per amplitude fetched for each one -- the four orbitals, the mirror's index, two Coulomb
+// factors (16 bytes), four orbital energies, four mosaic sums, most of them scattered -- is index
+// arithmetic, two table lookups and a few loads per column.  The sums of a tile, the energy and
+// the DIIS dot products, are reduced together (warp_sums): one after the other they were nearly
+// half of the instructions.
+// Latency decides: all warps resident (32 registers, a few spilled) and the |q|^2 table read through
+// L1 -- no barrier before the arithmetic -- beat fewer warps with more rows in flight, and a table
+// in shared memory.  Per launch, 100 twists of N=54 (485 plane waves), against a thread per
+// amplitude: the update with the DIIS push 0.381 -> 0.294 ms (0.23 ms of it without the push: the
+// ring values), the MP2 start 0.227 -> 0.148 ms; four N=114 systems: update 0.125 -> 0.100 ms.
+#include <cuda_runtime.h>
+
+#include <algorithm>
+#include <cstdint>
+
+#include "kernels.h"
+#include "uegccd_internal.h"
+
+namespace uegccd {
+
+namespace {
+
+constexpr int kThreads = 128;
+constexpr int kRows = 2;      // rows a thread has in flight
+
+// Sum and maxima over the CTA in a fixed order (valid in thread 0).
+__device__ __forceinline__ void reduce3(double &sum, double &mx1, double &mx2)
+{
+    __shared__ double s[3][kThreads / 32];
+    for (int o = 16; o > 0; o >>= 1) {
+        sum += __shfl_down_sync(0xffffffffu, sum, o);
+        mx1 = fmax(mx1, __shfl_down_sync(0xffffffffu, mx1, o));
+        mx2 = fmax(mx2, __shfl_down_sync(0xffffffffu, mx2, o));
+    }
+    const int w = threadIdx.x >> 5;
+    if ((threadIdx.x & 31) == 0) {
+        s[0][w] = sum;
+        s[1][w] = mx1;
+        s[2][w] = mx2;
+    }
+    __syncthreads();
+    if (threadIdx.x == 0)
+        for (int k = 1; k < kThreads / 32; k++) {
+            sum += s[0][k];
+            mx1 = fmax(mx1, s[1][k]);
+            mx2 = fmax(mx2, s[2][k]);
+        }
+}
+
+__device__ __forceinline__ UTileDev load_tile(const UTileDev *__restrict__ tiles)
+{
+    UTileDev T;
+    const int4 *p = reinterpret_cast<const int4 *>(tiles + blockIdx.x);
+    int4 *q = reinterpret_cast<int4 *>(&T);
+#pragma unroll
+    for (int k = 0; k < (int)(sizeof(UTileDev) / sizeof(int4)); k++) q[k] = __ldg(p + k);
+    return T;
+}
+
+// The warp's sums of N values (a power of two) into out[0..N), in a fixed order: the lanes halve
+// the values between them, then the lanes, 2 N - 2 + log2(32 / N) exchanges for what N separate
+// reductions take 5 N.
+template <int N>
+__device__ __forceinline__ void warp_sums(double (&v)[N], double *out)
+{
+    const int l = threadIdx.x & 31;
+    int at = 0;
+#pragma unroll
+    for (int o = 16, n = N / 2; o > 0; o >>= 1, n >>= 1) {
+        const bool up = l & o;
+        if (n > 0) {
+#pragma unroll
+            for (int k = 0; k < N / 2; k++)
+                if (k < n) {
+                    const double give = up ? v[k] : v[k + n], keep = up ? v[k + n] : v[k];
+                    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
+                }
+            at += up ? n : 0;
+        } else {
+            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
+        }
+    }
+    if ((l & (32 / N - 1)) == 0) out[at] = v[0];
+}
+
+// The warp's maximum of non-negative values (a NaN counts as 0).
+__device__ __forceinline__ double warp_max(double x)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(fmax(0.0, x));
+    const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
+    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
+    return __longlong_as_double((long long)((unsigned long long)mh << 32 | ml));
+}
+
+// A tile's threads: groups of `width` lanes (32, 64 or 128, the least that holds the columns), a
+// group per row; thread (grp, lane) makes the rows r0 + grp + k * ngrp.
+struct Place {
+    int grp, ngrp, c, pc;     // row group, groups, column and its partner's column
+    bool ok;
+};
+__device__ __forceinline__ Place place(const UTileDev &T)
+{
+    const int width = T.nc <= 32 ? 32 : T.nc <= 64 ? 64 : 128;
+    Place P;
+    P.grp = threadIdx.x / width;
+    P.ngrp = kThreads / width;
+    const int l = threadIdx.x - P.grp * width, vc = T.nvd + T.sd;
+    P.ok = l < T.nc;
+    P.c = T.c0 + min(l, T.nc - 1);
+    P.pc = P.c < T.nvd ? P.c + vc : P.c < vc ? P.c : P.c - vc;
+    return P;
+}
+
+// |n_a - n_k|^2 from a's packed vector times -2 and norm, and k's packed vector and norm
+__device__ __forceinline__ int neg2(int p)
+{
+    const int x = (int8_t)p, y = (int8_t)(p >> 8), z = (int8_t)(p >> 16);
+    return ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16);
+}
+
+}  // namespace
+
+// ----------------------------------------------------------------------------
+// MP2 (MP2.f90:56-74): t = v(i-a)/D, D = e_i + e_j - e_a - e_b.
+// E(2) = 1/2 sum [T2aaaa (V_ijab - V_ijba) + T2abab V_ijab - T2abba V_ijba]
+//      = sum t(ij,a) (2 v(i-a) - v(i-b))   after the a <-> b re-indexing; v(i-b) = v(a-j).
+// The mirror (j,i,b) has the same integrals; its denominator is summed in its own order.
+// A core pair's integrals are zero (CoreERI), so is its amplitude.
+// ----------------------------------------------------------------------------
+__global__ void __launch_bounds__(kThreads) k_mp2(const UTileDev *__restrict__ tiles,
+                                                  const SolveDev *__restrict__ solves,
+                                                  const int16_t *__restrict__ vir, const int *__restrict__ vpk,
+                                                  const int4 *__restrict__ rowpk, const double *__restrict__ eigen,
+                                                  const double *__restrict__ vtab, double *__restrict__ t,
+                                                  double *__restrict__ part_e, double *__restrict__ part_a,
+                                                  double *__restrict__ part_b)
+{
+    const UTileDev T = load_tile(tiles);
+    const int core = solves[T.solve].core_n;
+    const double *__restrict__ V = vtab + T.vtab0;
+    double e = 0.0, mx = 0.0, none = 0.0;
+    const Place P = place(T);
+    const double *ev = eigen + T.orb0;
+    const double ea = ev[vir[T.vir0 + P.c]], eb = ev[vir[T.vir0 + P.pc]];
+    const int na = vpk[T.vir0 + P.c], m2 = neg2(na), na2 = __dp4a(na, na, 0);
+#pragma unroll 2
+    for (int r = P.ok ? P.grp : T.nr; r < T.nr; r += P.ngrp) {
+        const int q = T.r0 + r;
+        const int4 R = __ldg(&rowpk[T.pair0 + q]);
+        const int i = R.z & 0xffff, j = R.z >> 16;
+        const double via = V[__dp4a(m2, R.x, na2 + __dp4a(R.x, R.x, 0))];
+        const double vaj = V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))];
+        const double eij = ev[i] + ev[j];
+        const bool c = i < core || j < core;
+        const double x = c ? 0.0 : via / (eij - ea - eb);
+        t[T.t0 + q * T.v + P.c] = x;
+        double y = 0.0;
+        if (q < T.nd) {
+            y = c ? 0.0 : via / (eij - eb - ea);
+            t[T.t0 + (q + T.nd + T.dg) * T.v + P.pc] = y;
+        }
+        e += (x + y) * (2.0 * via - vaj);
+        mx = fmax(mx, fmax(fabs(x), fabs(y)));
+    }
+    reduce3(e, mx, none);
+    if (threadIdx.x == 0) {
+        part_e[blockIdx.x] = e;
+        part_a[blockIdx.x] = mx;
+        part_b[blockIdx.x] = 0.0;
+    }
+}
+
+// Energy of the current amplitudes and max|t| (the dT before the first iteration).
+// kind 0, CCEnergy (CCD.f90:225-227): E = sum t(ij,a) (2 v(i-a) - v(a-j)) after re-indexing;
+// kind 1, dRPA CCEnergy (dRPA.f90:206-210): E = sum t (2 v(a-i) - csosex v(b-i)), v(b-i) = v(a-j).
+// A mirror's integrals are those of its pair.
+__global__ void __launch_bounds__(kThreads) k_energy(const UTileDev *__restrict__ tiles,
+                                                     const int *__restrict__ vpk, const int4 *__restrict__ rowpk,
+                                                     const double *__restrict__ vtab, const double *__restrict__ t, int kind, double csosex,
+                                                     double *__restrict__ part_e, double *__restrict__ part_a,
+                                                     double *__restrict__ part_b)
+{
+    const UTileDev T = load_tile(tiles);
+    const double *__restrict__ V = vtab + T.vtab0;
+    double e = 0.0, mx = 0.0, none = 0.0;
+    const Place P = place(T);
+    const int na = vpk[T.vir0 + P.c], m2 = neg2(na), na2 = __dp4a(na, na, 0);
+#pragma unroll 2
+    for (int r = P.ok ? P.grp : T.nr; r < T.nr; r += P.ngrp) {
+        const int q = T.r0 + r;
+        const int4 R = __ldg(&rowpk[T.pair0 + q]);
+        const double x = t[T.t0 + q * T.v + P.c];
+        const double y = q < T.nd ? t[T.t0 + (q + T.nd + T.dg) * T.v + P.pc] : 0.0;
+        const double via = V[__dp4a(m2, R.x, na2 + __dp4a(R.x, R.x, 0))];
+        const double vaj = V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))];
+        if (kind == 0) e += (x + y) * (2.0 * via - vaj);
+        else e += via * (x + y) * 2.0 - vaj * (x + y) * csosex;
+        mx = fmax(mx, fmax(fabs(x), fabs(y)));
+    }
+    reduce3(e, mx, none);
+    if (threadIdx.x == 0) {
+        part_e[blockIdx.x] = e;
+        part_a[blockIdx.x] = mx;
+        part_b[blockIdx.x] = 0.0;
+    }
+}
+
+// ----------------------------------------------------------------------------
+// Fused residual / update / convergence / energy.
+//   G = ladders (from k_ladder) + drivers + mosaics + rings + crossed rings
+//   R = -G + D t                          (GetRes, CCD.f90:417)
+//   t' = (G/D - (1-f) t)/f                (SolveCC, CCD.f90:380)
+//   dT = max |t' - t|                     (CnvrgCC, CCD.f90:452-454)
+//   E  = sum t' (2 v(i-a) - v(a-j))       (CCEnergy, CCD.f90:225-227 re-indexed)
+// By the pair symmetry t(ij,a) = t(ji,b) each amplitude with i < j also updates its mirror
+// (j,i,b); every term of G shares the symmetry.
+// NV: 0 updates in place, or forms the residual only (mode 1: max|R|, and G where g_out is given);
+// else the Pulay DIIS push: the new (t', e) pair goes to the solve's history slot and the partials
+// of e . e_j of every stored j < NV - 1 to dpart.
+// ----------------------------------------------------------------------------
+struct UpdateArgs {
+    const UTileDev *tiles;
+    const SolveDev *solves;
+    const int16_t *vir;
+    const int *vpk;
+    const int4 *rowpk;
+    const double *eigen, *vtab;
+    double *t;                    // each amplitude i <= j reads its own value only: updated in place
+    const double *g_ladder;
+    const double *jvv, *joo;
+    const double *dru, *drs2;     // dRPA: U and S2 of k_drpa_sums
+    double *part_e, *part_dt, *part_r;
+    double *g_out;                // optional: full G per amplitude (term checks)
+    const double *rx;             // ring and crossed-ring G, particle-hole layout
+    const int2 *rpos;             // where each amplitude's two values sit in it
+    const uint8_t *active;
+    int do_ladder, do_mosaic, do_ring, do_xring, do_driver, drpa, mode;
+    const IterState *st;
+    int ndiis;
+    int64_t namp;
+    double *hist_t, *dpart;
+    float *hist_e;
+};
+
+template <int NV>
+__global__ void __launch_bounds__(kThreads, NV <= 8 ? 16 : 6) k_update(UpdateArgs A)
+{
+    const UTileDev T = load_tile(A.tiles);
+    if (!A.active[T.solve]) {
+        if (threadIdx.x == 0) A.part_e[blockIdx.x] = A.part_dt[blockIdx.x] = A.part_r[blockIdx.x] = 0.0;
+        return;
+    }
+    const Place P = place(T);
+    const bool rings = !A.drpa && (A.do_ring || A.do_xring), mos = A.do_mosaic != 0;
+    double told[kRows], g[kRows], s1[kRows], s2[kRows];
+    int2 ro[kRows];
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        const int r = P.grp + k * P.ngrp, p = T.t0 + (T.r0 + r) * T.v + P.c;
+        const bool in = P.ok && r < T.nr;
+        told[k] = in ? A.t[p] : 0.0;
+        g[k] = in && A.do_ladder ? A.g_ladder[p] : 0.0;
+        ro[k] = in && rings ? A.rpos[p] : make_int2(0, 0);
+    }
+    const double *ev = A.eigen + T.orb0;
+    const int a = A.vir[T.vir0 + P.c], b = A.vir[T.vir0 + P.pc];
+    const double ea = ev[a], eb = ev[b];
+    const double jab = mos ? A.jvv[T.jvv0 + a - T.O] + A.jvv[T.jvv0 + b - T.O] : 0.0;
+    const int na = A.vpk[T.vir0 + P.c], m2 = neg2(na), na2 = __dp4a(na, na, 0);
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        const bool in = P.ok && P.grp + k * P.ngrp < T.nr && rings;
+        s1[k] = in && A.do_ring ? __ldg(&A.rx[ro[k].x]) : 0.0;
+        s2[k] = in && A.do_xring ? __ldg(&A.rx[ro[k].y]) : 0.0;
+    }
+    const int core = A.solves[T.solve].core_n;
+    const double f = A.solves[T.solve].denom_factor;
+    const bool pow2 = (__double_as_longlong(f) & 0xfffffffffffffLL) == 0;   // then x / f = x * (1 / f) exactly
+    // the push of iteration niter goes to slot (niter - 1) % ndiis, with min(niter, ndiis) stored
+    const int nb = NV > 0 ? A.st[T.solve].niter : 1;
+    const int slot = NV > 0 ? (nb - 1) % A.ndiis : 0, nvec = NV > 0 ? min(nb, A.ndiis) : 0;
+    const double *__restrict__ V = A.vtab + T.vtab0;
+    double esum = 0.0, mx = 0.0;   // mx: max|dT|, or max|R| in mode 1
+    float err[kRows];
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        err[k] = 0.0f;
+        const int r = P.grp + k * P.ngrp;
+        if (!P.ok || r >= T.nr) continue;
+        const int q = T.r0 + r, p = T.t0 + q * T.v + P.c;
+        const int4 R = __ldg(&A.rowpk[T.pair0 + q]);
+        const int i = R.z & 0xffff, j = R.z >> 16;
+        const bool pair = q < T.nd;
+        const int mir = T.t0 + (q + T.nd + T.dg) * T.v + P.pc;
+        const double via = V[__dp4a(m2, R.x, na2 + __dp4a(R.x, R.x, 0))];
+        double x = g[k];
+        if (A.do_driver) x += via;   // GetG2Drivers: G2abab = V(n_i - n_a)
+        if (mos) x -= 0.5 * (jab + A.joo[T.joo0 + i] + A.joo[T.joo0 + j]) * told[k];
+        if (A.drpa) {
+            if (A.do_ring) {   // linear and quadratic rings (k_drpa_sums)
+                const int ia = T.phr0 + i * T.V + (a - T.O), jb = T.phr0 + j * T.V + (b - T.O);
+                const double u = A.dru[ia];
+                x += u + A.dru[jb] + 2.0 * u * A.drs2[jb];
+            }
+        } else {   // the ring G and the crossed-ring G, where k_rings left them (k_rx_pos)
+            if (A.do_ring) x += s1[k];
+            if (A.do_xring) x += s2[k];
+        }
+        if (i < core || j < core) x = 0.0;   // core pair: every term has a zero factor
+        const double denom = ev[i] + ev[j] - ea - eb;
+        if (NV == 0 && A.mode != 0) {
+            if (A.g_out) {
+                A.g_out[p] = x;
+                if (pair) A.g_out[mir] = x;
+            }
+            mx = fmax(mx, fabs(-x + denom * told[k]));
+            continue;
+        }
+        const double y = x / denom - (1.0 - f) * told[k], tn = pow2 ? y * (1.0 / f) : y / f;
+        double d = fabs(tn - told[k]);
+        if (!(fabs(tn) < 1e300)) d = __longlong_as_double(0x7ff0000000000000LL);  // +Inf marks NaN/Inf
+        mx = fmax(mx, d);
+        double es = via * tn * 2.0;   // dRPA: the SOSEX part at the end
+        if (!A.drpa) es = tn * (2.0 * via - V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))]);
+        esum += pair ? 2.0 * es : es;
+        if (NV == 0) {
+            A.t[p] = tn;
+            if (pair) A.t[mir] = tn;
+        } else {   // the history slot holds t'; the mirrors' entries are never read
+            err[k] = (float)(tn - told[k]);
+            A.hist_t[(int64_t)slot * A.namp + p] = tn;
+            A.hist_e[(int64_t)slot * A.namp + p] = err[k];
+        }
+    }
+    const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+    constexpr int NS = NV == 0 ? 1 : NV;   // sums: the dot products, and the energy in the last place
+    __shared__ double sd[kThreads / 32][NS], sm[kThreads / 32];
+    double v[NS];
+#pragma unroll
+    for (int j = 0; j < NS - 1; j++) {
+        // e . e_j; an amplitude with a mirror counts twice
+        v[j] = 0.0;
+        if (j < nvec)
+#pragma unroll
+            for (int k = 0; k < kRows; k++) {
+                const int r = P.grp + k * P.ngrp, q = T.r0 + r;
+                if (!P.ok || r >= T.nr) continue;
+                const double e0 = err[k];
+                const double h = j == slot ? e0 : (double)A.hist_e[(int64_t)j * A.namp + T.t0 + q * T.v + P.c];
+                v[j] = fma(q < T.nd ? 2.0 * e0 : e0, h, v[j]);
+            }
+    }
+    v[NS - 1] = esum;
+    warp_sums<NS>(v, sd[w]);
+    mx = warp_max(mx);
+    if (l == 0) sm[w] = mx;
+    __syncthreads();
+    if (threadIdx.x < NS) {
+        double d = 0.0;
+        for (int k = 0; k < kThreads / 32; k++) d += sd[k][threadIdx.x];
+        if (threadIdx.x == NS - 1) A.part_e[blockIdx.x] = d;
+        else if (threadIdx.x < kDiisMax) A.dpart[(int64_t)blockIdx.x * kDiisMax + threadIdx.x] = d;
+    }
+    if (threadIdx.x == 32) {
+        for (int k = 1; k < kThreads / 32; k++) sm[0] = fmax(sm[0], sm[k]);
+        A.part_dt[blockIdx.x] = A.mode == 0 ? sm[0] : 0.0;
+        A.part_r[blockIdx.x] = A.mode == 0 ? 0.0 : sm[0];
+    }
+}
+
+// t = sum_j c_j t'_j over the amplitudes i <= j, each also written to its mirror (j,i,b)
+__global__ void __launch_bounds__(kThreads) k_diis_extrap(const UTileDev *__restrict__ tiles, int64_t namp,
+                                                          const double *__restrict__ hist_t,
+                                                          const double *__restrict__ coef, int ndiis,
+                                                          double *__restrict__ t, const uint8_t *__restrict__ applied)
+{
+    const UTileDev T = load_tile(tiles);
+    if (!applied[T.solve]) return;
+    const double *c = coef + T.solve * kDiisMax;
+    const Place P = place(T);
+    double x[kRows];
+#pragma unroll
+    for (int k = 0; k < kRows; k++) x[k] = 0.0;
+    for (int j = 0; j < ndiis; j++) {
+        const double cj = c[j];
+        if (cj == 0.0) continue;   // a slot not yet filled has coefficient 0 and is not read
+        const double *h = hist_t + (int64_t)j * namp;
+#pragma unroll
+        for (int k = 0; k < kRows; k++) {
+            const int r = P.grp + k * P.ngrp;
+            if (P.ok && r < T.nr) x[k] = fma(cj, h[T.t0 + (T.r0 + r) * T.v + P.c], x[k]);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kRows; k++) {
+        const int r = P.grp + k * P.ngrp, q = T.r0 + r;
+        if (!P.ok || r >= T.nr) continue;
+        t[T.t0 + q * T.v + P.c] = x[k];
+        if (q < T.nd) t[T.t0 + (q + T.nd + T.dg) * T.v + P.pc] = x[k];
+    }
+}
+
+void launch_mp2(const DevBatch &d, cudaStream_t st)
+{
+    k_mp2<<<d.nutiles, kThreads, 0, st>>>(d.utiles, d.solves, d.vir, d.vpk, d.rowpk,
+                                                                     d.eigen, d.vtab, d.t, d.part_e,
+                                                                     d.part_dt, d.part_r);
+}
+
+void launch_energy(const DevBatch &d, int kind, double csosex, cudaStream_t st)
+{
+    k_energy<<<d.nutiles, kThreads, 0, st>>>(d.utiles, d.vpk, d.rowpk, d.vtab,
+                                                                        d.t, kind, csosex, d.part_e,
+                                                                        d.part_dt, d.part_r);
+}
+
+void launch_update(const DevBatch &d, const TermFlags &f, int mode, double *g_out, const CtlBuffers *diis, int ndiis,
+                   cudaStream_t st)
+{
+    UpdateArgs A;
+    A.tiles = d.utiles; A.solves = d.solves; A.vir = d.vir; A.vpk = d.vpk; A.rowpk = d.rowpk;
+    A.eigen = d.eigen; A.vtab = d.vtab;
+    A.t = d.t; A.g_ladder = d.g; A.jvv = d.jvv; A.joo = d.joo; A.dru = d.dru; A.drs2 = d.drs2;
+    A.part_e = d.part_e; A.part_dt = d.part_dt; A.part_r = d.part_r; A.g_out = g_out; A.active = d.active;
+    A.do_ladder = f.do_ladder; A.do_mosaic = f.do_mosaic; A.do_ring = f.do_ring; A.do_xring = f.do_xring;
+    A.do_driver = f.do_driver; A.drpa = f.drpa; A.mode = mode;
+    A.rx = d.rx; A.rpos = d.rpos;
+    A.st = diis ? diis->state : nullptr; A.ndiis = (diis && mode == 0) ? ndiis : 0; A.namp = d.namp;
+    A.hist_t = diis ? diis->hist_t : nullptr; A.hist_e = diis ? diis->hist_e : nullptr;
+    A.dpart = diis ? diis->part : nullptr;
+    if (A.ndiis == 0) k_update<0><<<d.nutiles, kThreads, 0, st>>>(A);
+    else if (A.ndiis <= 7) k_update<8><<<d.nutiles, kThreads, 0, st>>>(A);
+    else k_update<32><<<d.nutiles, kThreads, 0, st>>>(A);
+}
+
+void launch_extrap(const DevBatch &d, const CtlBuffers &c, int ndiis, cudaStream_t st)
+{
+    k_diis_extrap<<<d.nutiles, kThreads, 0, st>>>(d.utiles, d.namp, c.hist_t, c.coef, ndiis, d.t, c.applied);
+}
+
+// The tiles of a block of `rows` rows and v columns: column ranges of at most 128, each in ranges
+// that fill the threads' rows.
+void update_tiles(int rows, int v, void (*emit)(void *, int, int, int, int), void *to)
+{
+    const int nt = (v + kThreads - 1) / kThreads, w = (v + nt - 1) / nt;
+    for (int c0 = 0; c0 < v; c0 += w) {
+        const int nc = std::min(w, v - c0), width = nc <= 32 ? 32 : nc <= 64 ? 64 : 128;
+        const int step = kRows * (kThreads / width);
+        for (int r0 = 0; r0 < rows; r0 += step) emit(to, c0, nc, r0, std::min(step, rows - r0));
+    }
+}
+
+}  // namespace uegccd
