@@ -170,12 +170,90 @@ struct DevChunk {
     size_t size;
     int dev;
 };
-// pinned staging buffer of the batch-wide amplitude download (grown on demand, kept; portable:
-// page-locked for every device's context)
-constexpr size_t kStageMin = 8ull << 20;
-std::mutex g_stage_mu;
-char *g_stage = nullptr;
-size_t g_stage_bytes = 0;
+// Page-locked host memory for downloads, in buffers that outlive the calls (portable: page-locked
+// for every device's context): a call takes one, any number of threads theirs, and gives it back;
+// up to kPinnedCap bytes stay for the next call, until uegccd_trim_cache.
+constexpr size_t kPinnedCap = 512ull << 20;
+constexpr size_t kPinnedMin = 64ull << 10;
+struct PinnedBuf {
+    char *p = nullptr;
+    size_t bytes = 0;
+};
+std::mutex g_pinned_mu;
+std::vector<PinnedBuf> g_pinned;
+size_t g_pinned_bytes = 0;
+
+// At least `bytes` (p = nullptr when the host has no more to lock).
+PinnedBuf pinned_get(size_t bytes)
+{
+    bytes = std::max(bytes, kPinnedMin);
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mu);
+        int best = -1;
+        for (size_t k = 0; k < g_pinned.size(); k++)
+            if (g_pinned[k].bytes >= bytes && (best < 0 || g_pinned[k].bytes < g_pinned[best].bytes)) best = (int)k;
+        if (best >= 0) {
+            const PinnedBuf b = g_pinned[best];
+            g_pinned_bytes -= b.bytes;
+            g_pinned.erase(g_pinned.begin() + best);
+            return b;
+        }
+    }
+    PinnedBuf b;
+    if (cudaHostAlloc((void **)&b.p, bytes, cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        b.p = nullptr;
+        return b;
+    }
+    b.bytes = bytes;
+    return b;
+}
+
+void pinned_put(const PinnedBuf &b)
+{
+    if (!b.p) return;
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mu);
+        if (g_pinned_bytes + b.bytes <= kPinnedCap) {
+            g_pinned.push_back(b);
+            g_pinned_bytes += b.bytes;
+            return;
+        }
+    }
+    cudaFreeHost(b.p);
+}
+
+struct PinnedScope {
+    PinnedBuf b;
+    explicit PinnedScope(size_t bytes) : b(pinned_get(bytes)) {}
+    ~PinnedScope() { pinned_put(b); }
+    PinnedScope(const PinnedScope &) = delete;
+    PinnedScope &operator=(const PinnedScope &) = delete;
+};
+
+bool is_pinned(const void *p)
+{
+    cudaPointerAttributes pa;
+    const bool yes = cudaPointerGetAttributes(&pa, p) == cudaSuccess && pa.type == cudaMemoryTypeHost;
+    if (!yes) cudaGetLastError();   // clear the query's status on older drivers
+    return yes;
+}
+
+// memcpy on the host's cores (large copies; the destination's pages are often touched first here)
+void host_copy(char *dst, const char *src, size_t bytes)
+{
+    constexpr size_t kPiece = 256 << 10;
+    if (bytes <= 2 * kPiece) {
+        std::memcpy(dst, src, bytes);
+        return;
+    }
+    const int n = (int)((bytes + kPiece - 1) / kPiece);
+    const int nth = std::max(1, std::min({16, n, (int)std::thread::hardware_concurrency()}));
+    parallel_for(n, nth, [&](int k) {
+        const size_t a = (size_t)k * kPiece;
+        std::memcpy(dst + a, src + a, std::min(kPiece, bytes - a));
+    });
+}
 // g_pool_mu guards the cache, the per-device byte counts and the limit
 std::mutex g_pool_mu;
 std::vector<DevChunk> g_pool;
@@ -287,11 +365,13 @@ struct UegccdBatch {
     std::vector<DevChunk> big;       // chunks of one large array each
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_solve0 = nullptr, ev_solve1 = nullptr;
+    PinnedBuf pin;                   // page-locked words the small reads land in (on first use)
+    cudaEvent_t ev_copy[3] = {nullptr, nullptr, nullptr};   // arrays of a download (on first use)
     Fork fork;                       // side streams of a small batch's residual (on first use)
     bool fork_made = false;
     std::vector<double> red;         // host copy: 3 per solve
     std::vector<uint8_t> active;     // host copy
-    double *dense[3] = {nullptr, nullptr, nullptr};  // reference-layout scratch of the largest solve
+    double *dense = nullptr;         // reference-layout scratch: three arrays of the largest solve
     size_t dense_n = 0;
     double *dense_all = nullptr;     // reference layout of every solve, back to back (on first use)
     int64_t *dense_off = nullptr;
@@ -360,6 +440,9 @@ struct UegccdBatch {
         if (ev1) cudaEventDestroy(ev1);
         if (ev_solve0) cudaEventDestroy(ev_solve0);
         if (ev_solve1) cudaEventDestroy(ev_solve1);
+        pinned_put(pin);
+        for (auto &e : ev_copy)
+            if (e) cudaEventDestroy(e);
         if (fork.start) cudaEventDestroy(fork.start);
         for (auto &e : fork.done)
             if (e) cudaEventDestroy(e);
@@ -933,8 +1016,7 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     size_t dn = 0;
     for (int s = 0; s < n; s++) dn = std::max(dn, (size_t)b->plans[s].O * b->plans[s].O * b->plans[s].V);
     b->dense_n = dn;
-    for (int k = 0; k < 3; k++)
-        if ((rc = b->alloc(b->dense[k], dn))) return rc;
+    if ((rc = b->alloc(b->dense, 3 * dn))) return rc;
     trace.mark("device-launch");
     CU(cudaStreamSynchronize(b->stream));
     trace.mark("device-wait");
@@ -950,12 +1032,32 @@ int set_active_all(UegccdBatch &b, uint8_t v)
     return 0;
 }
 
-int read_red(UegccdBatch &b)
+// Where a small device read of `bytes` lands: page-locked, so that the copy is one DMA after the
+// kernels before it; the caller's own memory when there is none.
+void *small_read(UegccdBatch &b, void *own, size_t bytes)
 {
-    CU(cudaMemcpyAsync(b.red.data(), b.d.red, b.red.size() * sizeof(double), cudaMemcpyDeviceToHost, b.stream));
-    b.d2h_bytes += (int64_t)(b.red.size() * sizeof(double));
+    if (b.pin.bytes < bytes) {
+        pinned_put(b.pin);
+        b.pin = pinned_get(bytes);
+    }
+    return b.pin.p ? b.pin.p : own;
+}
+
+int read_back(UegccdBatch &b, void *dst, const void *src, size_t bytes)
+{
+    void *p = small_read(b, dst, bytes);
+    CU(cudaMemcpyAsync(p, src, bytes, cudaMemcpyDeviceToHost, b.stream));
+    b.d2h_bytes += (int64_t)bytes;
     CU(cudaStreamSynchronize(b.stream));
     CU(cudaGetLastError());
+    if (p != dst) std::memcpy(dst, p, bytes);
+    return 0;
+}
+
+int read_red(UegccdBatch &b)
+{
+    const int rc = read_back(b, b.red.data(), b.d.red, b.red.size() * sizeof(double));
+    if (rc) return rc;
     b.kt.collect();
     return 0;
 }
@@ -965,31 +1067,66 @@ int pack_from_host(UegccdBatch &b, int s, const double *host_dense)
 {
     const SolvePlan &P = b.plans[s];
     size_t n = (size_t)P.O * P.O * P.V;
-    CU(cudaMemcpyAsync(b.dense[0], host_dense, n * sizeof(double), cudaMemcpyHostToDevice, b.stream));
+    CU(cudaMemcpyAsync(b.dense, host_dense, n * sizeof(double), cudaMemcpyHostToDevice, b.stream));
     b.h2d_bytes += (int64_t)(n * sizeof(double));
-    launch_pack(b.d, s, (int)P.namp, b.dense[0], b.stream);
+    launch_pack(b.d, s, (int)P.namp, b.dense, b.stream);
     b.launches++;
     CU(cudaGetLastError());
     return 0;
 }
 
-int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, double *ba, double *aa)
+// T2abab / T2abba / T2aaaa of solve s in the reference layout (each may be null) into host
+// arrays; with_red: the batch's reduced sums too, in the same wait.  The arrays leave the device in
+// one run into page-locked memory and go on from there on the host's cores, one while the next is
+// on its way: the driver stages a copy into pageable memory on one thread, 11 GB/s measured with
+// fresh pages, 2.7 MB an array at N=54.
+int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, double *ba, double *aa,
+                   bool with_red = false)
 {
     const SolvePlan &P = b.plans[s];
-    size_t n = (size_t)P.O * P.O * P.V;
-    double *h[3] = {ab, ba, aa};
+    const size_t n = (size_t)P.O * P.O * P.V, bytes = n * sizeof(double);
+    double *out[3] = {ab, ba, aa}, *host[3], *dev[3] = {nullptr, nullptr, nullptr};
+    int m = 0;
     for (int k = 0; k < 3; k++)
-        if (h[k]) CU(cudaMemsetAsync(b.dense[k], 0, n * sizeof(double), b.stream));
-    launch_unpack(b.d, s, (int)P.namp, t_dev, ab ? b.dense[0] : nullptr, ba ? b.dense[1] : nullptr,
-                  aa ? b.dense[2] : nullptr, b.stream);
+        if (out[k]) {
+            dev[k] = b.dense + m * n;
+            host[m++] = out[k];
+        }
+    CU(cudaMemsetAsync(b.dense, 0, m * bytes, b.stream));
+    launch_unpack(b.d, s, (int)P.namp, t_dev, dev[0], dev[1], dev[2], b.stream);
     b.launches++;
     CU(cudaGetLastError());
-    for (int k = 0; k < 3; k++)
-        if (h[k]) {
-            CU(cudaMemcpyAsync(h[k], b.dense[k], n * sizeof(double), cudaMemcpyDeviceToHost, b.stream));
-            b.d2h_bytes += (int64_t)(n * sizeof(double));
+    b.d2h_bytes += (int64_t)(m * bytes);
+    const size_t red = with_red ? b.red.size() * sizeof(double) : 0;
+    if (red) b.d2h_bytes += (int64_t)red;
+    bool direct = true;   // page-locked destinations take the copies themselves
+    for (int k = 0; k < m; k++) direct = direct && is_pinned(host[k]);
+    PinnedScope buf(direct ? red : red + m * bytes);
+    if (!buf.b.p || direct) {
+        for (int k = 0; k < m; k++)
+            CU(cudaMemcpyAsync(host[k], b.dense + k * n, bytes, cudaMemcpyDeviceToHost, b.stream));
+        if (red) CU(cudaMemcpyAsync(b.red.data(), b.d.red, red, cudaMemcpyDeviceToHost, b.stream));
+        CU(cudaStreamSynchronize(b.stream));
+        return 0;
+    }
+    char *arrays = buf.b.p + red;
+    if (red) CU(cudaMemcpyAsync(buf.b.p, b.d.red, red, cudaMemcpyDeviceToHost, b.stream));
+    const bool apart = bytes >= (512 << 10);
+    if (apart) {
+        for (int k = 0; k < m; k++) {
+            if (!b.ev_copy[k]) CU(cudaEventCreateWithFlags(&b.ev_copy[k], cudaEventDisableTiming));
+            CU(cudaMemcpyAsync(arrays + k * bytes, b.dense + k * n, bytes, cudaMemcpyDeviceToHost, b.stream));
+            CU(cudaEventRecord(b.ev_copy[k], b.stream));
         }
-    CU(cudaStreamSynchronize(b.stream));
+    } else {
+        CU(cudaMemcpyAsync(arrays, b.dense, m * bytes, cudaMemcpyDeviceToHost, b.stream));
+        CU(cudaStreamSynchronize(b.stream));
+    }
+    for (int k = 0; k < m; k++) {
+        if (apart) CU(cudaEventSynchronize(b.ev_copy[k]));
+        host_copy((char *)host[k], arrays + k * bytes, bytes);
+    }
+    if (red) std::memcpy(b.red.data(), buf.b.p, red);
     return 0;
 }
 
@@ -1366,10 +1503,7 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
                     b.launches += b.g_launches;
                 }
             }
-            CU(cudaMemcpyAsync(&count, b.ctl.count, sizeof(int), cudaMemcpyDeviceToHost, b.stream));
-            b.d2h_bytes += sizeof(int);
-            CU(cudaStreamSynchronize(b.stream));
-            CU(cudaGetLastError());
+            if ((rc = read_back(b, &count, b.ctl.count, sizeof(int)))) return rc;
             b.kt.collect();
             rounds++;
             if (phase == 1 && mixed && ++sweeps >= std::max(1, opt->refine_sweeps)) break;
@@ -1499,10 +1633,8 @@ int session_advance(UegccdBatch &b, int rounds, int *n_active, int *n_done, int 
             CU(cudaGraphLaunch(b.gexec, b.stream));
             b.launches += b.g_launches;
         }
-        CU(cudaMemcpyAsync(&count, b.ctl.count, sizeof(int), cudaMemcpyDeviceToHost, b.stream));
-        b.d2h_bytes += sizeof(int);
-        CU(cudaStreamSynchronize(b.stream));
-        CU(cudaGetLastError());
+        const int rc = read_back(b, &count, b.ctl.count, sizeof(int));
+        if (rc) return rc;
     }
     std::vector<IterState> st(n);
     CU(cudaMemcpyAsync(st.data(), b.ctl.state, n * sizeof(IterState), cudaMemcpyDeviceToHost, b.stream));
@@ -1839,13 +1971,9 @@ int uegccd_mp2(UegccdCtx *c, double *t_aaaa, double *t_abab, double *t_abba, dou
     launch_mp2(b.d, b.stream);
     launch_reduce(b.d, b.stream);
     CU(cudaGetLastError());
-    int rc = read_red(b);
+    const int rc = t_aaaa || t_abab || t_abba ? unpack_to_host(b, 0, b.d.t, t_abab, t_abba, t_aaaa, true) : read_red(b);
     if (rc) return rc;
     if (e2) *e2 = b.red[0];
-    if (t_aaaa || t_abab || t_abba) {
-        rc = unpack_to_host(b, 0, b.d.t, t_abab, t_abba, t_aaaa);
-        if (rc) return rc;
-    }
     return std::isfinite(b.red[0]) ? 0 : fail(UEGCCD_ERR_NUMERIC, "non-finite MP2 energy");
 }
 
@@ -2210,33 +2338,18 @@ int uegccd_batch_get_all_amplitudes(UegccdBatch *b, double *t_abab)
     CU(cudaGetLastError());
     const size_t bytes = b->dense_all_n * sizeof(double);
     b->d2h_bytes += (int64_t)bytes;
-    // a page-locked destination takes the copy directly
-    cudaPointerAttributes pa;
-    const bool pinned = cudaPointerGetAttributes(&pa, t_abab) == cudaSuccess && pa.type == cudaMemoryTypeHost;
-    if (!pinned) cudaGetLastError();   // clear the query's status on older drivers
-    if (bytes < kStageMin || pinned) {
+    // a page-locked destination takes the copy directly; else through page-locked memory, copied
+    // out on all host cores (a pageable copy is staged by the driver on one thread)
+    const bool direct = is_pinned(t_abab);
+    PinnedScope buf(direct ? 0 : bytes);
+    if (direct || !buf.b.p) {
         CU(cudaMemcpyAsync(t_abab, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
         CU(cudaStreamSynchronize(b->stream));
         return UEGCCD_OK;
     }
-    // large downloads: through a cached pinned buffer, copied out on all host cores
-    // (a pageable copy is staged by the driver on one thread)
-    std::lock_guard<std::mutex> lock(g_stage_mu);
-    if (g_stage_bytes < bytes) {
-        if (g_stage) cudaFreeHost(g_stage);
-        g_stage = nullptr;
-        g_stage_bytes = 0;
-        CU(cudaHostAlloc((void **)&g_stage, bytes, cudaHostAllocPortable));
-        g_stage_bytes = bytes;
-    }
-    CU(cudaMemcpyAsync(g_stage, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
+    CU(cudaMemcpyAsync(buf.b.p, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
     CU(cudaStreamSynchronize(b->stream));
-    const int nth = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
-    const size_t piece = (bytes + nth - 1) / nth;
-    parallel_for(nth, nth, [&](int k) {
-        const size_t a = (size_t)k * piece, e = std::min(bytes, a + piece);
-        if (a < e) std::memcpy((char *)t_abab + a, g_stage + a, e - a);
-    });
+    host_copy((char *)t_abab, buf.b.p, bytes);
     return UEGCCD_OK;
 }
 
@@ -2271,12 +2384,13 @@ int uegccd_batch_structure_factor(UegccdBatch *b, int32_t s, const UegccdSfGrid 
 
 int uegccd_trim_cache(void)
 {
+    std::vector<PinnedBuf> unlock;
     {
-        std::lock_guard<std::mutex> lock(g_stage_mu);
-        if (g_stage) cudaFreeHost(g_stage);
-        g_stage = nullptr;
-        g_stage_bytes = 0;
+        std::lock_guard<std::mutex> lock(g_pinned_mu);
+        unlock.swap(g_pinned);
+        g_pinned_bytes = 0;
     }
+    for (auto &b : unlock) cudaFreeHost(b.p);
     std::vector<DevChunk> drop;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
