@@ -24,7 +24,7 @@ SOURCES = ["capi.cu", "kernels_fp64.cu", "ladder.cu", "rings.cu", "update.cu", "
 # bench.py's FP64 tensor-core peak measurement: a library of its own beside bench.py
 BENCH_PEAK_SRC = os.path.join(ROOT, "bench_peak.cu")
 BENCH_PEAK_LIB = os.path.join(ROOT, "bench_peak.so")
-HEADERS = ["kernels.h", "plan.h", "uegccd_internal.h", "listdir.h", "heg_device.h", "two_channel.h", "two_channel_mm.h"]
+HEADERS = ["kernels.h", "plan.h", "uegccd_internal.h", "listdir.h", "heg_device.h", "two_channel.h", "two_channel_mm.h", "warp.cuh"]
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 NVCC_FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "--expt-relaxed-constexpr"]
 

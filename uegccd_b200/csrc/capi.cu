@@ -876,12 +876,9 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
         d.ladder_smem[f] = ladder_smem_bytes(q2m, n2m, max_rows, f);
         set_ladder_smem_limit(d.ladder_smem[f]);
     }
-    // the |q|^2 table the mosaic kernel stages: the batch's largest (tables beyond 1024 entries
-    // stay in global memory)
-    d.mosaic_vt = std::min(q2m + 1, kVtabSmemEntries);
-    d.mosaic_smem = mosaic_smem_bytes(max_v, max_o, d.mosaic_vt);
-    if (d.mosaic_smem > 227 * 1024) return fail(UEGCCD_ERR_UNSUPPORTED, "mosaic block exceeds shared memory");
-    set_mosaic_smem_limit(d.mosaic_smem);
+    // K blocks of more than some 9000 virtuals are outside what the kernels are checked for
+    if (24 * (size_t)max_v + 40 * (size_t)max_o + 8 * (size_t)std::min(q2m + 1, kVtabSmemEntries) > 227 * 1024)
+        return fail(UEGCCD_ERR_UNSUPPORTED, "momentum block too large");
     d.max_occ = max_occ;
     d.namp = amp0;
     // ring pairs by class, then by solve (the class sort is stable), and k_rings' CTAs: runs of one

@@ -17,8 +17,6 @@ struct DevBatch {
     // mosaics: block row and column sums, and per target the list of partials to add
     double *mpart = nullptr;
     int32_t *mt_start = nullptr, *mt_list = nullptr;
-    size_t mosaic_smem = 0;
-    int mosaic_vt = 0;  // |q|^2 table entries k_mosaic_blk stages: the batch's largest, at most kVtabSmemEntries
     // FP64 ladder tiles (ladder.cu): the FMA form's, then the DMMA form's, longest first
     LadderTile64 *ltiles = nullptr;
     int nltiles[2] = {0, 0};
@@ -43,7 +41,7 @@ struct DevBatch {
     int32_t *partner = nullptr;      // packed -> packed index of (i,j,b)
     AmpInfo *amps = nullptr;
     int4 *nv4 = nullptr;
-    int *nvp = nullptr;              // the same vectors packed a component per byte (q2p in kernels_fp64.cu)
+    int *nvp = nullptr;              // the same vectors packed a component per byte (warp.cuh)
     double *eigen = nullptr, *vtab = nullptr;
     double *t = nullptr, *t_new = nullptr, *g = nullptr;
     double *jvv = nullptr, *joo = nullptr;
@@ -99,9 +97,6 @@ struct DevBatch {
     int ring_doubles[6] = {0, 0, 0, 0, 0, 0};
     int stage_threads = 128;                    // CTA size of k_ring_stage (tune_rings)
 };
-// dynamic shared memory of k_mosaic_blk for blocks of at most max_v virtuals
-size_t mosaic_smem_bytes(int max_v, int max_o, int vt_n);
-void set_mosaic_smem_limit(size_t bytes);
 // FP64 ladders (ladder.cu): blocks with at most kLadderFmaRows rows i <= j take the FMA form,
 // larger ones the DMMA form in tiles of at most kLadderMmaRows rows
 constexpr int kLadderFmaRows = 4, kLadderMmaRows = 16;

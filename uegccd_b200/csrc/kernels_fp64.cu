@@ -20,19 +20,9 @@
 
 #include "kernels.h"
 #include "uegccd_internal.h"
+#include "warp.cuh"
 
 namespace uegccd {
-
-// Plane-wave vectors packed one component per byte (x | y << 8 | z << 16, two's complement;
-// DevBatch::nvp): the squared length of the difference of two orbitals' vectors is then one
-// per-byte subtraction and one 4-way byte dot product.  Every |n_d| <= 63 (checked when the
-// batch is made), so each component difference fits a signed byte; modular byte arithmetic
-// keeps a difference of differences exact as long as the final one does.
-__device__ __forceinline__ int q2p(int a, int c)
-{
-    const int d = __vsub4(a, c);
-    return __dp4a(d, d, 0);
-}
 
 __device__ __forceinline__ int q2_of(int4 x, int4 y)
 {
@@ -129,128 +119,85 @@ __global__ void k_reduce_solves(const int *__restrict__ chunk_begin, const doubl
 // (The ladders, CCD.f90:588-686, are in ladder.cu; they write G first, before k_update adds
 // the other terms.)
 
-// The dynamic shared-memory limits only grow (batches of different sizes coexist), under
-// one lock: batches are created from several host threads while others solve.  Kernel
-// attributes belong to a device, so each device keeps its own limits (the caller has made
-// the batch's device current).
-static std::mutex g_smem_limit_mu;
-
 // ----------------------------------------------------------------------------
 // Mosaics (GetG2Mosaics, CCD.f90:548-582):
 //   s(k,l,c) = v(c-k) (T2aaaa + T2abab)(kl,c) - v(c-l) (T2aaaa + T2abba)(kl,c)
 //            = v(c-k) (2t(kl,c) - t(kl,d)) - v(c-l) (t(kl,c) - 2t(kl,d))
 //   Jvv(c) = sum_{k,l} s(k,l,c),  Joo(k) = sum_{l,c} s(k,l,c)
 // (dRPA's own mosaics, dRPA.f90:415-431, come from k_drpa_sums.)
-// s lives only in registers: one CTA per K block forms it row by row (d = K - c is
-// in the same row) and writes the block's row sums (-> Joo of the row's k) and
-// column sums (-> Jvv of the column's c); k_mosaic_sum adds the partials of each
-// target in a fixed order.
+// v(d-k) = v(c-l) and v(d-l) = v(c-k) for the partner d = K - c of c in the row (k,l), so
+// s(k,l,d) = s(k,l,c), and by the pair symmetry s(l,k,c) is the same again: s is formed on the
+// rows i <= j and the columns c <= d only, an element standing for two or four.
+// s lives only in registers: one CTA per K block writes the block's row sums (-> Joo of the row's
+// k) and column sums (-> Jvv of the column's c); k_mosaic_sum adds the partials of each target in
+// a fixed order.  The threads own the columns, so that all warps stay busy however few rows a
+// block has: a column's sum stays with its thread, four rows are in flight and their sums are
+// reduced together.  Bound by latency (a short chain per block) and, beyond that, by reading half
+// the amplitudes once.  Per iteration, 100 twists of N=54 (485 plane
+// waves): 100 -> 50 us against every column by itself, its partner found through the map and the
+// |q|^2 table staged by each CTA; 100 twists of N=14: 8 -> 5 us.
 // ----------------------------------------------------------------------------
 constexpr int kMosThreads = 128;
+constexpr int kMaxOcc = 64;             // NOcc limit of a batch
+constexpr int kMosRows = kMaxOcc / 2 + 4;   // rows i <= j of a block, rounded up to fours
 
-size_t mosaic_smem_bytes(int max_v, int max_o, int vt_n)
-{
-    return sizeof(double) * ((size_t)vt_n + 2 * (size_t)max_v + (size_t)(kMosThreads / 32) * max_o) +
-           sizeof(int) * (2 * (size_t)max_v + 2 * (size_t)max_o);
-}
-
-// The threads own the columns (c = tid + k * kMosThreads) and walk the rows: all warps stay
-// busy however few rows a block has.  Column sums stay with their thread; row sums are
-// reduced per warp, then over the warps in a fixed order.
-__global__ void __launch_bounds__(kMosThreads) k_mosaic_blk(const BlockDev *__restrict__ blocks,
+__global__ void __launch_bounds__(kMosThreads, 12) k_mosaic_blk(const BlockDev *__restrict__ blocks,
                                                            const SolveDev *__restrict__ solves,
-                                                           const int16_t *__restrict__ pair_i,
-                                                           const int16_t *__restrict__ pair_j,
-                                                           const int16_t *__restrict__ vir,
-                                                           const int *__restrict__ nvp,
+                                                           const int *__restrict__ vpk,
+                                                           const int4 *__restrict__ rowpk,
                                                            const double *__restrict__ vtab,
                                                            const double *__restrict__ t,
-                                                           const int16_t *__restrict__ pcol,
                                                            double *__restrict__ mpart,
-                                                           const uint8_t *__restrict__ active, int vt_n)
+                                                           const uint8_t *__restrict__ active)
 {
+    constexpr int kW = kMosThreads / 32, kR = 4;
+    __shared__ double wrs[kW][kMosRows];   // per-warp row sums
     const BlockDev B = blocks[blockIdx.x];
     if (!active[B.solve]) return;
-    const SolveDev s = solves[B.solve];
-    const int v = B.v, oc = B.nd + B.dg;
-    constexpr int kW = kMosThreads / 32;
-    extern __shared__ double msm[];
-    double *sv = msm;                          // vt_n: the batch's largest |q|^2 table (at most kVtabSmemEntries)
-    double *coff = sv + vt_n;                  // v: column sums over the rows i < j
-    double *cdg = coff + v;                    // v: the diagonal pair's row (if any)
-    double *wrs = cdg + v;                     // kW x oc: per-warp row sums
-    int *nvc = (int *)(wrs + kW * oc);         // v: packed n-vectors of the block's virtuals
-    int *nk = nvc + v, *nl = nk + oc;          // oc: packed n-vectors of each row's k and l
-    int *pc = nl + oc;                         // v: column of the partner d = K - c
+    const double *__restrict__ V = vtab + solves[B.solve].vtab0;
+    const int oc = B.nd + B.dg, h = B.nvd + B.sd;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const bool vsm = s.q2max < vt_n;
-    if (vsm)
-        for (int q = tid; q <= s.q2max; q += kMosThreads) sv[q] = vtab[s.vtab0 + q];
-    for (int c = tid; c < v; c += kMosThreads) {
-        nvc[c] = nvp[s.orb0 + vir[B.vir0 + c]];
-        pc[c] = pcol[B.vir0 + c];
-        coff[c] = cdg[c] = 0.0;
-    }
-    for (int r = tid; r < oc; r += kMosThreads) {
-        nk[r] = nvp[s.orb0 + pair_i[B.pair0 + r]];
-        nl[r] = nvp[s.orb0 + pair_j[B.pair0 + r]];
-    }
-    __syncthreads();
-    auto V = [&](int q2) -> double { return vsm ? sv[q2] : __ldg(&vtab[s.vtab0 + q2]); };
-    // Rows i <= j only: by the pair symmetry s(l,k,d) = s(k,l,c) for the mirror (l,k) of a
-    // row (k,l) and d = K - c, so the mirror row has the same row sum (Joo of l) and adds
-    // the column sums of (k,l) with the columns swapped to their partners.  Four rows at a
-    // time: their loads go out together (most blocks have at most four rows), and each column
-    // sum still takes the rows in order.
-    constexpr int kR = 4;
-    for (int r0 = 0; r0 < oc; r0 += kR) {
-        const int nr = min(kR, oc - r0);
-        const double *row[kR];
-        int rk[kR], rl[kR];
-        double rs[kR];
-#pragma unroll
-        for (int q = 0; q < kR; q++) {
-            const int r = min(r0 + q, oc - 1);
-            row[q] = t + B.t0 + (int64_t)r * v;
-            rk[q] = nk[r];
-            rl[q] = nl[r];
-            rs[q] = 0.0;
-        }
-        for (int c = tid; c < v; c += kMosThreads) {
-            const int ncv = nvc[c];
-            const int pcc = pc[c];
-            double x[kR], y[kR];
+    for (int r = lane; r < kMosRows; r += 32) wrs[warp][r] = 0.0;
+    __syncwarp();
+    for (int cw = warp * 32; cw < h; cw += kMosThreads) {
+        const int c = min(cw + lane, h - 1);
+        const bool ok = cw + lane < h, pair = c < B.nvd;
+        const int na = vpk[B.vir0 + c], m2 = neg2(na), na2 = __dp4a(na, na, 0);
+        const double *col = t + B.t0 + c;
+        const int po = pair ? h : 0;
+        double cs = 0.0;
+        for (int r0 = 0; r0 < oc; r0 += kR) {
+            double x[kR], y[kR], sr[kR];
 #pragma unroll
             for (int q = 0; q < kR; q++) {
-                x[q] = q < nr ? row[q][c] : 0.0;
-                y[q] = q < nr ? row[q][pcc] : 0.0;   // t(kl, d), same row
+                const bool in = ok && r0 + q < oc;
+                x[q] = in ? col[(int64_t)(r0 + q) * B.v] : 0.0;
+                y[q] = in ? col[(int64_t)(r0 + q) * B.v + po] : 0.0;   // t(kl, d), same row
             }
 #pragma unroll
             for (int q = 0; q < kR; q++) {
-                if (q >= nr) continue;
-                const double vck = V(q2p(ncv, rk[q]));
-                const double vcl = V(q2p(ncv, rl[q]));
-                const double sval = vck * (2.0 * x[q] - y[q]) - vcl * (x[q] - 2.0 * y[q]);
-                rs[q] += sval;
-                if (r0 + q >= B.nd) cdg[c] = sval;
-                else coff[c] += sval;
+                const int4 R = __ldg(&rowpk[B.pair0 + min(r0 + q, oc - 1)]);
+                const double vck = V[__dp4a(m2, R.x, na2 + __dp4a(R.x, R.x, 0))];
+                const double vcl = V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))];
+                const double s = vck * (2.0 * x[q] - y[q]) - vcl * (x[q] - 2.0 * y[q]);
+                cs += r0 + q < B.nd ? 2.0 * s : s;
+                sr[q] = pair ? 2.0 * s : s;
             }
+            const int at = warp_sums<kR>(sr);
+            if (at >= 0) wrs[warp][r0 + at] += sr[0];
         }
-#pragma unroll
-        for (int q = 0; q < kR; q++) {
-            double v0 = rs[q];
-            for (int off = 16; off > 0; off >>= 1) v0 += __shfl_down_sync(0xffffffffu, v0, off);
-            if (lane == 0 && q < nr) wrs[warp * oc + r0 + q] = v0;
+        if (ok) {
+            mpart[B.col0 + c] = cs;
+            if (pair) mpart[B.col0 + c + h] = cs;
         }
     }
     __syncthreads();
     for (int r = tid; r < oc; r += kMosThreads) {
         double rs = 0.0;
-        for (int w = 0; w < kW; w++) rs += wrs[w * oc + r];
+        for (int w = 0; w < kW; w++) rs += wrs[w][r];
         mpart[B.row0 + r] = rs;
         if (r < B.nd) mpart[B.row0 + r + oc] = rs;   // the mirror row
     }
-    for (int c = tid; c < v; c += kMosThreads) mpart[B.col0 + c] = coff[c] + coff[pc[c]] + cdg[c];
 }
 
 // One warp per target: targets (s, y < V) are Jvv(c = O + y), (s, y >= V) are Joo(k = y - V).
@@ -332,18 +279,6 @@ __global__ void __launch_bounds__(256) k_mosaic_sum(const int2 *__restrict__ tar
     }
 }
 
-void set_mosaic_smem_limit(size_t bytes)
-{
-    std::lock_guard<std::mutex> lock(g_smem_limit_mu);
-    static size_t current_by_dev[kMaxDevices] = {};   // attributes are per device
-    size_t &current = current_by_dev[current_device() % kMaxDevices];
-    if (current < 48 * 1024) current = 48 * 1024;
-    if (bytes > current) {
-        cudaFuncSetAttribute(k_mosaic_blk, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-        current = bytes;
-    }
-}
-
 // ----------------------------------------------------------------------------
 // dRPA rings and mosaics (dRPA.f90:377-551) from two sums per particle-hole pair (i, x):
 //   S1(i,x) = sum_k t(ik,x),   S2(i,x) = sum_k t(ki,d), d = n_k + n_x' the column whose partner
@@ -366,7 +301,6 @@ void set_mosaic_smem_limit(size_t bytes)
 // 0.645 ms in k_update.
 // ----------------------------------------------------------------------------
 constexpr int kDrpaThreads = 256;
-constexpr int kMaxOcc = 64;   // NOcc limit of a batch
 
 // Row and column lookups, one CTA per K block: drows[(i,j)] = {first packed index of row
 // (i,j), block, nvd, nvd + sd}; colpos[block][x] = column of virtual x (both pre-set to -1).
@@ -1051,9 +985,8 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
     }
     if (f.do_mosaic && !f.drpa) {
         kt->begin(KID_MOSAIC_S, ms);
-        k_mosaic_blk<<<d.nblocks, kMosThreads, d.mosaic_smem, ms>>>(d.blocks, d.solves, d.pair_i, d.pair_j, d.vir,
-                                                                   d.nvp, d.vtab, d.t, d.pcol, d.mpart,
-                                                                   d.active, d.mosaic_vt);
+        k_mosaic_blk<<<d.nblocks, kMosThreads, 0, ms>>>(d.blocks, d.solves, d.vpk, d.rowpk, d.vtab, d.t, d.mpart,
+                                                        d.active);
         kt->end(ms);
         kt->begin(KID_MOSAIC_RED, ms);
         k_mosaic_sum<<<(d.ntargets + 7) / 8, 256, 0, ms>>>(d.targets, d.ntargets, d.solves, d.mt_start, d.mt_list,

@@ -21,6 +21,7 @@
 
 #include "kernels.h"
 #include "uegccd_internal.h"
+#include "warp.cuh"
 
 namespace uegccd {
 
@@ -63,41 +64,6 @@ __device__ __forceinline__ UTileDev load_tile(const UTileDev *__restrict__ tiles
     return T;
 }
 
-// The warp's sums of N values (a power of two) into out[0..N), in a fixed order: the lanes halve
-// the values between them, then the lanes, 2 N - 2 + log2(32 / N) exchanges for what N separate
-// reductions take 5 N.
-template <int N>
-__device__ __forceinline__ void warp_sums(double (&v)[N], double *out)
-{
-    const int l = threadIdx.x & 31;
-    int at = 0;
-#pragma unroll
-    for (int o = 16, n = N / 2; o > 0; o >>= 1, n >>= 1) {
-        const bool up = l & o;
-        if (n > 0) {
-#pragma unroll
-            for (int k = 0; k < N / 2; k++)
-                if (k < n) {
-                    const double give = up ? v[k] : v[k + n], keep = up ? v[k + n] : v[k];
-                    v[k] = keep + __shfl_xor_sync(0xffffffffu, give, o);
-                }
-            at += up ? n : 0;
-        } else {
-            v[0] += __shfl_xor_sync(0xffffffffu, v[0], o);
-        }
-    }
-    if ((l & (32 / N - 1)) == 0) out[at] = v[0];
-}
-
-// The warp's maximum of non-negative values (a NaN counts as 0).
-__device__ __forceinline__ double warp_max(double x)
-{
-    const unsigned long long b = (unsigned long long)__double_as_longlong(fmax(0.0, x));
-    const unsigned hi = (unsigned)(b >> 32), mh = __reduce_max_sync(0xffffffffu, hi);
-    const unsigned ml = __reduce_max_sync(0xffffffffu, hi == mh ? (unsigned)b : 0u);
-    return __longlong_as_double((long long)((unsigned long long)mh << 32 | ml));
-}
-
 // A tile's threads: groups of `width` lanes (32, 64 or 128, the least that holds the columns), a
 // group per row; thread (grp, lane) makes the rows r0 + grp + k * ngrp.
 struct Place {
@@ -115,13 +81,6 @@ __device__ __forceinline__ Place place(const UTileDev &T)
     P.c = T.c0 + min(l, T.nc - 1);
     P.pc = P.c < T.nvd ? P.c + vc : P.c < vc ? P.c : P.c - vc;
     return P;
-}
-
-// |n_a - n_k|^2 from a's packed vector times -2 and norm, and k's packed vector and norm
-__device__ __forceinline__ int neg2(int p)
-{
-    const int x = (int8_t)p, y = (int8_t)(p >> 8), z = (int8_t)(p >> 16);
-    return ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16);
 }
 
 }  // namespace
@@ -357,7 +316,8 @@ __global__ void __launch_bounds__(kThreads, NV <= 8 ? 16 : 6) k_update(UpdateArg
             }
     }
     v[NS - 1] = esum;
-    warp_sums<NS>(v, sd[w]);
+    const int at = warp_sums<NS>(v);
+    if (at >= 0) sd[w][at] = v[0];
     mx = warp_max(mx);
     if (l == 0) sm[w] = mx;
     __syncthreads();
