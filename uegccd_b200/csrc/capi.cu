@@ -393,7 +393,8 @@ struct UegccdBatch {
         TermFlags f;
         std::vector<uint8_t> released;
     } ses;
-    // CUDA graphs of one iteration: plain and with kernel timers, keyed by the options
+    // CUDA graphs of one iteration, in FP64 and with the mixed-precision ladder (a mixed solve runs
+    // both), each kept until other options or buffers are asked for
     struct GraphKey {
         int do_ring, do_xring, do_ladder, do_mosaic, drpa, ndiis, max_iter, mixed;
         double tol;
@@ -403,11 +404,15 @@ struct UegccdBatch {
                    do_mosaic == o.do_mosaic && drpa == o.drpa && ndiis == o.ndiis && max_iter == o.max_iter &&
                    mixed == o.mixed && tol == o.tol;
         }
-    } gkey{};
-    bool have_graph = false;
+    };
+    struct IterGraph {
+        GraphKey key{};
+        cudaGraphExec_t exec = nullptr;
+        bool valid = false;
+        int launches = 0;            // kernels per iteration
+    } graphs[2];
+    void drop_graphs() { graphs[0].valid = graphs[1].valid = false; }
     bool tuned = false;              // launch shape picked (before the first graph capture)
-    cudaGraphExec_t gexec = nullptr;
-    int g_launches = 0;          // kernels per iteration
     // structure factors (on first use): every solve's particle-hole groups {first row, rows},
     // solve s at [sf_g0[s], sf_g0[s+1]); one grid of the largest solve
     int2 *sf_groups = nullptr;
@@ -430,7 +435,8 @@ struct UegccdBatch {
 
     ~UegccdBatch()
     {
-        if (gexec) cudaGraphExecDestroy(gexec);
+        for (auto &g : graphs)
+            if (g.exec) cudaGraphExecDestroy(g.exec);
         if (kt_events)
             for (auto &e : kt.ev) cudaEventDestroy(e);
         if (stream) cudaStreamSynchronize(stream);
@@ -443,7 +449,8 @@ struct UegccdBatch {
         pinned_put(pin);
         for (auto &e : ev_copy)
             if (e) cudaEventDestroy(e);
-        if (fork.start) cudaEventDestroy(fork.start);
+        for (cudaEvent_t e : {fork.start, fork.staged})
+            if (e) cudaEventDestroy(e);
         for (auto &e : fork.done)
             if (e) cudaEventDestroy(e);
         for (auto &x : fork.s)
@@ -1316,6 +1323,7 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
         c.rec_e = re;
         c.rec_dt = rd;
         c.max_rec = max_rec;
+        b.drop_graphs();
     }
     if (ndiis > b.diis_cap) {
         const UegccdBatch::Mark m = b.mark();
@@ -1328,50 +1336,57 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
         c.hist_t = ht;
         c.hist_e = he;
         b.diis_cap = ndiis;
+        b.drop_graphs();
     }
     return 0;
 }
 
-// The side streams on which a batch's rings, mosaics and DMMA ladders run beside its FMA
-// ladders: the kernels of a small batch leave most of the GPU idle, and the launches of a
-// residual only wait for one another.  A large batch fills the GPU with each kernel, and run
-// together they contend for the SMs and L2.  Solve times, one stream and side streams: one N=54
-// system 1.59 and 1.05 ms, 16 of them 4.60 and 4.41, 32 (7 M amplitudes) 7.87 and 7.77, 64
-// (14 M) 13.9 and 14.3; four N=114 systems (8.5 M) 15.0 and 14.1.
+// The side streams of a batch.  The ring classes always run beside each other: each is a launch of
+// its own whose last CTAs leave the GPU idle.  In a small batch the rings, the mosaics and the DMMA
+// ladders also run beside the FMA ladders; in a large one each kernel fills the GPU, and run
+// together they contend for the SMs and L2.  Solve times in ms on one stream, with the ring classes
+// apart, with the terms apart: one N=54 system 1.50, 1.2, 0.93; 8 of them 2.72, 2.53, 2.13;
+// 32 (11 M amplitudes) 6.76, 6.37, 6.30; 48 (16 M) 8.70 and 9.16 apart; 100 (33 M) 17.02, 16.47,
+// 18.46; four N=114 systems (13 M) 11.8, 10.7, 9.7; 8 of them (26 M) 20.9, 18.8, 17.9; 16 of them
+// (51 M) 36.0, 34.2, 34.3.
 constexpr int64_t kForkAmps = 9000000;
+constexpr int kForkSolves = 8;
 const Fork *fork_of(UegccdBatch &b)
 {
-    if (b.d.namp > kForkAmps) return nullptr;
     if (!b.fork_made) {
         b.fork_made = true;
         Fork &f = b.fork;
-        bool ok = cudaEventCreateWithFlags(&f.start, cudaEventDisableTiming) == cudaSuccess;
-        for (int k = 0; k < 3; k++)
+        f.terms = b.d.namp <= kForkAmps || b.d.nsolves <= kForkSolves;
+        bool ok = cudaEventCreateWithFlags(&f.start, cudaEventDisableTiming) == cudaSuccess &&
+                  cudaEventCreateWithFlags(&f.staged, cudaEventDisableTiming) == cudaSuccess;
+        for (int k = 0; k < kSideStreams; k++)
             ok = ok && cudaStreamCreateWithFlags(&f.s[k], cudaStreamNonBlocking) == cudaSuccess &&
                  cudaEventCreateWithFlags(&f.done[k], cudaEventDisableTiming) == cudaSuccess;
         if (!ok) cudaGetLastError();   // one stream then serves all
     }
-    return b.fork.done[2] ? &b.fork : nullptr;
+    return b.fork.done[kSideStreams - 1] ? &b.fork : nullptr;
 }
 
 // Captures one iteration as a CUDA graph.
 int capture_iteration(UegccdBatch &b, const TermFlags &f, double tol, int max_iter, int ndiis)
 {
     UegccdBatch::GraphKey key{f.do_ring, f.do_xring, f.do_ladder, f.do_mosaic, f.drpa, ndiis, max_iter, f.mixed, tol};
-    if (b.have_graph && b.gkey == key) return 0;
-    if (b.gexec) { cudaGraphExecDestroy(b.gexec); b.gexec = nullptr; }
+    UegccdBatch::IterGraph &G = b.graphs[f.mixed ? 1 : 0];
+    if (G.valid && G.key == key) return 0;
+    G.valid = false;
+    if (G.exec) { cudaGraphExecDestroy(G.exec); G.exec = nullptr; }
     const Fork *fork = fork_of(b);
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal));
     int nl = launch_iteration(b.d, b.ctl, f, tol, max_iter, ndiis, b.stream, nullptr, fork);
     cudaError_t e = cudaStreamEndCapture(b.stream, &g);
     if (e != cudaSuccess) return fail(UEGCCD_ERR_CUDA, std::string("graph capture: ") + cudaGetErrorString(e));
-    e = cudaGraphInstantiate(&b.gexec, g, 0);
+    e = cudaGraphInstantiate(&G.exec, g, 0);
     cudaGraphDestroy(g);
     if (e != cudaSuccess) return fail(UEGCCD_ERR_CUDA, std::string("graph instantiate: ") + cudaGetErrorString(e));
-    b.g_launches = nl;
-    b.gkey = key;
-    b.have_graph = true;
+    G.launches = nl;
+    G.key = key;
+    G.valid = true;
     return 0;
 }
 
@@ -1496,8 +1511,9 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
                     // the sampled iteration of the round: direct launches between CUDA events
                     b.launches += launch_iteration(d, b.ctl, f, opt->tol, opt->max_iter, ndiis, b.stream, &b.kt);
                 } else {
-                    CU(cudaGraphLaunch(b.gexec, b.stream));
-                    b.launches += b.g_launches;
+                    const UegccdBatch::IterGraph &G = b.graphs[f.mixed];
+                    CU(cudaGraphLaunch(G.exec, b.stream));
+                    b.launches += G.launches;
                 }
             }
             if ((rc = read_back(b, &count, b.ctl.count, sizeof(int)))) return rc;
@@ -1627,8 +1643,8 @@ int session_advance(UegccdBatch &b, int rounds, int *n_active, int *n_done, int 
     CU(cudaStreamSynchronize(b.stream));
     for (int r = 0; r < rounds && count > 0; r++) {
         for (int k = 0; k < kPoll; k++) {
-            CU(cudaGraphLaunch(b.gexec, b.stream));
-            b.launches += b.g_launches;
+            CU(cudaGraphLaunch(b.graphs[0].exec, b.stream));
+            b.launches += b.graphs[0].launches;
         }
         const int rc = read_back(b, &count, b.ctl.count, sizeof(int));
         if (rc) return rc;
@@ -2238,7 +2254,7 @@ int uegccd_batch_set_profiling(UegccdBatch *b, int32_t on)
     }
     b->kt.on = on != 0;
     for (int k = 0; k < KID_COUNT; k++) { b->kt.ms[k] = 0.0; b->kt.launches[k] = 0; }
-    b->have_graph = false;  // re-capture with (or without) the timer events
+    b->drop_graphs();  // re-capture with (or without) the timer events
     return 0;
 }
 

@@ -120,7 +120,8 @@ int ring_pairs_per_pass(int c);     // pairs a CTA works on at a time
 int ring_doubles(int c, int max_n2);
 size_t ring_smem_bytes(const DevBatch &d, int c, int max_n2);
 void set_rings_smem_limit(size_t bytes);
-int launch_rings(const DevBatch &d, int do_ring, int do_xring, cudaStream_t st);
+// the classes go to the ns streams in turn, the largest first
+int launch_rings(const DevBatch &d, int do_ring, int do_xring, const cudaStream_t *streams, int ns);
 // Launch-shape autotuner, on the batch's current amplitudes: times k_ring_stage with 64, 128 and
 // 256 threads per CTA (d.stage_threads) and keeps the fastest.  Results are the same.  Not inside
 // a stream capture.  Returns a cudaError_t value.
@@ -201,12 +202,14 @@ void launch_to_aaaa(const DevBatch &d, cudaStream_t st);
 // drows and colpos (pre-set to -1) of the dRPA sums from the blocks
 void launch_drpa_tables(const DevBatch &d, cudaStream_t st);
 // Side streams for the independent terms of a residual (nullptr: all on one stream).
+constexpr int kSideStreams = 5;
 struct Fork {
-    cudaStream_t s[3] = {nullptr, nullptr, nullptr};   // rings, mosaics, DMMA ladders
-    cudaEvent_t start = nullptr, done[3] = {nullptr, nullptr, nullptr};
+    cudaStream_t s[kSideStreams] = {};   // rings, mosaics, DMMA ladders, two more for the ring classes
+    bool terms = false;                  // the terms beside each other, not the ring classes only
+    cudaEvent_t start = nullptr, staged = nullptr, done[kSideStreams] = {};
 };
 // Residual of the selected terms for d.t; mode 0 also updates d.t (with DIIS: the history).
-// fork: the rings and the mosaics run beside the ladders.  Returns launches.
+// fork: the ring classes and, with fork->terms, the terms run beside each other.  Returns launches.
 struct CtlBuffers;
 // diis/ndiis (mode 0 only): fuse the Pulay DIIS push into the update kernel
 int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_out, cudaStream_t st,

@@ -965,12 +965,14 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
 {
     KernelTimer dummy;
     if (!kt) kt = &dummy;
-    int n = 0;
-    const bool side = fork && !kt->on && !f.drpa && f.do_ladder && !f.mixed;
-    const cudaStream_t rs = side ? fork->s[0] : st, ms = side ? fork->s[1] : st, ls = side ? fork->s[2] : st;
-    if (side) {
+    int n = 0, classes = 0;
+    for (int k : d.nritems) classes += k > 0;
+    const bool side = fork && !kt->on && !f.drpa, apart = side && fork->terms && f.do_ladder;
+    const cudaStream_t rs = apart ? fork->s[0] : st, ms = apart ? fork->s[1] : st;
+    const cudaStream_t ls = apart && !f.mixed ? fork->s[2] : st;   // (the mixed ladder adds to what both forms leave)
+    if (apart) {
         cudaEventRecord(fork->start, st);
-        for (cudaStream_t x : fork->s) cudaStreamWaitEvent(x, fork->start, 0);
+        for (int k = 0; k < 3; k++) cudaStreamWaitEvent(fork->s[k], fork->start, 0);
     }
     if (f.do_ladder && d.nblocks > 0) {
         kt->begin(KID_LADDER, st);
@@ -1008,10 +1010,18 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         kt->end(rs);
         n++;
         kt->begin(KID_RINGS, rs);
-        n += launch_rings(d, f.do_ring, f.do_xring, rs);
+        const cudaStream_t lanes[3] = {rs, side ? fork->s[3] : rs, side ? fork->s[4] : rs};
+        const int nl = side ? std::min(classes, 3) : 1;
+        if (nl > 1) cudaEventRecord(fork->staged, rs);
+        for (int k = 1; k < nl; k++) cudaStreamWaitEvent(lanes[k], fork->staged, 0);
+        n += launch_rings(d, f.do_ring, f.do_xring, lanes, nl);
+        for (int k = 1; k < nl; k++) {
+            cudaEventRecord(fork->done[k + 2], lanes[k]);
+            cudaStreamWaitEvent(rs, fork->done[k + 2], 0);
+        }
         kt->end(rs);
     }
-    if (side) {
+    if (apart) {
         for (int k = 0; k < 3; k++) {
             cudaEventRecord(fork->done[k], fork->s[k]);
             cudaStreamWaitEvent(st, fork->done[k], 0);

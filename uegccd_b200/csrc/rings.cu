@@ -348,7 +348,7 @@ void set_rings_smem_limit(size_t bytes)
     current = bytes;
 }
 
-int launch_rings(const DevBatch &d, int do_ring, int do_xring, cudaStream_t st)
+int launch_rings(const DevBatch &d, int do_ring, int do_xring, const cudaStream_t *streams, int ns)
 {
     int n = 0, off = 0, offs[kRingClasses];
     for (int c = 0; c < kRingClasses; c++) {
@@ -359,6 +359,7 @@ int launch_rings(const DevBatch &d, int do_ring, int do_xring, cudaStream_t st)
         if (d.nritems[c] <= 0) continue;
         const Args A{d.ritems + offs[c], d.rpairs, d.solves, d.rrows, d.vtab, d.xy, d.rx, d.active, do_ring, do_xring,
                      tab_bytes(d), d.ring_doubles[c]};
+        const cudaStream_t st = streams[n % ns];
         switch (kRingFrags[c]) {
         case 1: launch<1>(d, c, A, st); break;
         case 2: launch<2>(d, c, A, st); break;
