@@ -807,7 +807,7 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
         } em{&utiles, UTileDev{(int)bd.t0, bd.vir0, bd.pair0, bd.solve, S.orb0, S.vtab0, S.jvv0, S.joo0, (int)S.phr0,
                                S.q2max, bd.v, bd.nvd, (int16_t)bd.sd, (int16_t)bd.dg, (int16_t)bd.nd, 0, 0, 0, 0,
                                (int16_t)S.O, S.V, {0, 0, 0}}};
-        update_tiles(bd.nd + bd.dg, bd.v,
+        update_tiles(bd.nd + bd.dg, bd.nvd + bd.sd,
                      [](void *to, int c0, int nc, int r0, int nr) {
                          auto *e = static_cast<Emit *>(to);
                          UTileDev t = e->base;

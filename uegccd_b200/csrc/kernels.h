@@ -69,12 +69,11 @@ struct DevBatch {
     // multiplies, row by row (k_ring_stage gathers t into it before every ring launch); rx
     // the ring and crossed-ring G the pair forms, in the same places (k_update reads them).
     // Per (i, x) at phr0 + i*V + x - O: ph_a = the row's offset in xy/rx when (i, x) is in
-    // its pair's group 1, else -1; ph_b = round8(n2) of its pair in group 1 (where the Y1 /
-    // crossed-ring half of the row starts), its column b in group 2 (-1 without a pair).
+    // its pair's group 1, else -1; ph_b = its column b in group 2, else -1.
     double *xy = nullptr, *rx = nullptr;
     int64_t xy_n = 0;
     int32_t *ph_a = nullptr, *ph_b = nullptr;
-    int2 *rpos = nullptr;            // per amplitude i <= j: its ring G and crossed-ring G in rx
+    int2 *rpos = nullptr;            // per amplitude i <= j, a <= b: where rx holds its and its partner's
     // mixed precision: tensor-core ladder tiles sorted by row tile (16, 32, 64)
     LadderTile *tctiles = nullptr;
     int ntc16 = 0, ntc32 = 0, ntc64 = 0;
@@ -121,7 +120,7 @@ int ring_doubles(int c, int max_n2);
 size_t ring_smem_bytes(const DevBatch &d, int c, int max_n2);
 void set_rings_smem_limit(size_t bytes);
 // the classes go to the ns streams in turn, the largest first
-int launch_rings(const DevBatch &d, int do_ring, int do_xring, const cudaStream_t *streams, int ns);
+int launch_rings(const DevBatch &d, const cudaStream_t *streams, int ns);
 // Launch-shape autotuner, on the batch's current amplitudes: times k_ring_stage with 64, 128 and
 // 256 threads per CTA (d.stage_threads) and keeps the fastest.  Results are the same.  Not inside
 // a stream capture.  Returns a cudaError_t value.

@@ -427,7 +427,7 @@ __global__ void k_ring_index(const ChunkDev *__restrict__ rchunks, const SolveDe
 }
 
 // One CTA per ring pair: where each of its rows (i, x) sits in the particle-hole arrays.
-// Group-1 row a: ph_a = xy0 + 2 a N2 (its X1 row; Y1 follows at + N2), ph_b = N2.  Group-2
+// Group-1 row a: ph_a = xy0 + 2 a N2 (its row of two values a column), ph_b = -1.  Group-2
 // row b: ph_a = -1, ph_b = b.  (Rows of groups without a -Q partner keep -1, -1.)
 __global__ void k_ph_tables(const RingPairDev *__restrict__ pairs, const SolveDev *__restrict__ solves,
                             const int16_t *__restrict__ ph_i, const int16_t *__restrict__ ph_x,
@@ -442,7 +442,7 @@ __global__ void k_ph_tables(const RingPairDev *__restrict__ pairs, const SolveDe
         const int i = ph_i[s.phr0 + row], x = ph_x[s.phr0 + row];
         const int64_t k = s.phr0 + (int64_t)i * s.V + (x - s.O);
         ph_a[k] = g1 ? P.xy0 + 2 * r * N2 : -1;
-        ph_b[k] = g1 ? N2 : r - P.n1;
+        ph_b[k] = g1 ? -1 : r - P.n1;
     }
 }
 
@@ -507,12 +507,12 @@ __global__ void k_ring_stage(const RingPairDev *__restrict__ pairs, const SolveD
     }
 }
 
-// Where k_update finds each amplitude's ring values in rx, once per batch: k_rings leaves at
-// (a, b) of a {Q, -Q} pair the ring G of (i_a, i_b, x_a) and the crossed-ring G of
-// (i_a, i_b, x_b), a in group 1.  Amplitude (i,j,a) (partner b, i <= j) finds its ring G at
-// row (i,a), column (j,b) when (i,a) is in group 1, else at row (j,b), column (i,a) (its
-// mirror's place); its crossed-ring G in the second half of row (i,b) at column (j,a), or of
-// row (j,a) at column (i,b).
+// Where k_update finds the ring values of an amplitude (i,j,a), i <= j and a <= b, and of its partner
+// (i,j,b) in rx, once per batch.  k_rings leaves at (a, b) of a {Q, -Q} pair the ring G of
+// (i_a, i_b, x_a) beside the crossed-ring G of (i_a, i_b, x_b), a in group 1.  The place of (i,a),
+// (j,b) -- row (i,a), column (j,b) when (i,a) is in group 1, else its mirror's, row (j,b), column
+// (i,a) -- holds the ring G of (i,j,a) and the crossed-ring G of (i,j,b); that of (i,b), (j,a) the
+// ring G of (i,j,b) and the crossed-ring G of (i,j,a).
 __global__ void __launch_bounds__(128) k_rx_pos(const UTileDev *__restrict__ tiles, const SolveDev *__restrict__ solves,
                                                const AmpInfo *__restrict__ amps, const int32_t *__restrict__ ph_a,
                                                const int32_t *__restrict__ ph_b, int2 *__restrict__ rpos)
@@ -520,13 +520,13 @@ __global__ void __launch_bounds__(128) k_rx_pos(const UTileDev *__restrict__ til
     const UTileDev T = tiles[blockIdx.x];
     const SolveDev s = solves[T.solve];
     for (int e = threadIdx.x; e < T.nr * T.nc; e += blockDim.x) {
-        const int64_t p = T.t0 + (int64_t)(T.r0 + e / T.nc) * T.v + T.c0 + e % T.nc;
+        const int64_t p = T.t0 + (int64_t)(T.r0 + e / T.nc) * T.v + T.c0 + e % T.nc;   // column a <= b
         const AmpInfo q = amps[p];
         const int V = s.V, O = s.O;
         const int32_t *pa = ph_a + s.phr0, *pb = ph_b + s.phr0;
         const int ia = q.i * V + q.a - O, jb = q.j * V + q.b - O, ib = q.i * V + q.b - O, ja = q.j * V + q.a - O;
-        const int r = pa[ia] >= 0 ? pa[ia] + pb[jb] : pa[jb] + pb[ia];
-        const int x = pa[ib] >= 0 ? pa[ib] + pb[ib] + pb[ja] : pa[ja] + pb[ja] + pb[ib];
+        const int r = pa[ia] >= 0 ? pa[ia] + 2 * pb[jb] : pa[jb] + 2 * pb[ia];
+        const int x = pa[ib] >= 0 ? pa[ib] + 2 * pb[ja] : pa[ja] + 2 * pb[ib];
         rpos[p] = make_int2(r, x);
     }
 }
@@ -1014,7 +1014,7 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         const int nl = side ? std::min(classes, 3) : 1;
         if (nl > 1) cudaEventRecord(fork->staged, rs);
         for (int k = 1; k < nl; k++) cudaStreamWaitEvent(lanes[k], fork->staged, 0);
-        n += launch_rings(d, f.do_ring, f.do_xring, lanes, nl);
+        n += launch_rings(d, lanes, nl);
         for (int k = 1; k < nl; k++) {
             cudaEventRecord(fork->done[k + 2], lanes[k]);
             cudaStreamWaitEvent(rs, fork->done[k + 2], 0);

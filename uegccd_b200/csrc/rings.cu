@@ -25,7 +25,8 @@
 //   ring (i_a, i_b, x_a) = vd (z_a + z_b + z_a z_b)
 //                          + sum_a' [XW[a][a'] (Y - 2X)[a'][b] + U[a][a'] X[a'][b]] - sum_b' X[a][b'] Vs2[b'][b]
 //   xring(i_a, i_b, x_b) = sum_a' U[a][a'] Y[a'][b] - sum_b' Y[a][b'] Vs2[b'][b]
-// k_update reads each amplitude's two values where its row is in group 1 (or its mirror's).
+// k_update reads the two values of a pair (a, b) together: they belong to an amplitude and its
+// partner, whose other two sit at one more place (k_rx_pos).
 // Group 1 is the smaller group: 5 n1^2 n2 + 2 n1 n2^2 multiply-adds.
 //
 // A warp owns eight rows a for the whole pair: its XW and U stay in registers, as the A operand
@@ -108,7 +109,7 @@ struct Args {
     const double *vtab, *xy;
     double *rx;
     const uint8_t *active;
-    int do_ring, do_xring, tab_bytes, pair_doubles;
+    int tab_bytes, pair_doubles;
 };
 
 // Starts the copies of one pair into its buffer: X and Y (8 NF rows, stride N2 + 4; the rows
@@ -135,7 +136,7 @@ __device__ __forceinline__ void fetch_pair(const RingPairDev &P, const double *_
 // FN fragments of columns b from n0 of a warp's rows.
 template <bool TAB16, int NF, int FN>
 __device__ __forceinline__ void do_cols(const Args &A, const double *X, const double *Y, const double *Xr,
-                                        const double *Yr, const RingRowDev *r2, const char *tab, int n0, int n2, int N2,
+                                        const double *Yr, const RingRowDev *r2, const char *tab, int n0, int n2,
                                         int l2, int k2, const double (&xw)[NF][2], const double (&u)[NF][2], double z,
                                         double vd, bool store, double *out)
 {
@@ -187,9 +188,9 @@ __device__ __forceinline__ void do_cols(const Args &A, const double *X, const do
         const double z0 = __shfl_sync(0xffffffffu, zb[f], tig * 8);
         const double z1 = __shfl_sync(0xffffffffu, zb[f], tig * 8 + 4);
         if (!store) continue;
-        double2 *o = reinterpret_cast<double2 *>(out + n0 + f * 8);
-        if (A.do_ring) o[0] = make_double2(vd * (z + z0 + z * z0) + rg[f][0], vd * (z + z1 + z * z1) + rg[f][1]);
-        if (A.do_xring) o[N2 / 2] = make_double2(xr[f][0], xr[f][1]);
+        double2 *o = reinterpret_cast<double2 *>(out) + n0 + f * 8;
+        o[0] = make_double2(vd * (z + z0 + z * z0) + rg[f][0], xr[f][0]);
+        o[1] = make_double2(vd * (z + z1 + z * z1) + rg[f][1], xr[f][1]);
     }
 }
 
@@ -237,10 +238,10 @@ __device__ __forceinline__ void do_pair(const Args &A, const RingPairDev &P, con
             u[f][h] -= lookup<TAB16>(tab, row_side<TAB16>(R.mi, R.ni2), ci_row);
         }
     const double vd = lookup<TAB16>(tab, row_side<TAB16>(r1[0].mx, r1[0].nx2), r1[0].ci);
-    double *out = A.rx + P.xy0 + (int64_t)(m0 + gid) * 2 * N2 + 2 * tig;
+    double *out = A.rx + P.xy0 + (int64_t)(m0 + gid) * 2 * N2 + 4 * tig;
     int n0 = 0;
-    for (; n0 + 8 < N2; n0 += 16) do_cols<TAB16, NF, 2>(A, X, Y, Xr, Yr, r2, tab, n0, n2, N2, l2, k2, xw, u, z, vd, m0 + gid < n1, out);
-    if (n0 < N2) do_cols<TAB16, NF, 1>(A, X, Y, Xr, Yr, r2, tab, n0, n2, N2, l2, k2, xw, u, z, vd, m0 + gid < n1, out);
+    for (; n0 + 8 < N2; n0 += 16) do_cols<TAB16, NF, 2>(A, X, Y, Xr, Yr, r2, tab, n0, n2, l2, k2, xw, u, z, vd, m0 + gid < n1, out);
+    if (n0 < N2) do_cols<TAB16, NF, 1>(A, X, Y, Xr, Yr, r2, tab, n0, n2, l2, k2, xw, u, z, vd, m0 + gid < n1, out);
 }
 
 // NF fragments of eight rows a (n1 <= 8 NF), a warp each; a CTA works on ring_groups(NF) pairs at a
@@ -348,7 +349,7 @@ void set_rings_smem_limit(size_t bytes)
     current = bytes;
 }
 
-int launch_rings(const DevBatch &d, int do_ring, int do_xring, const cudaStream_t *streams, int ns)
+int launch_rings(const DevBatch &d, const cudaStream_t *streams, int ns)
 {
     int n = 0, off = 0, offs[kRingClasses];
     for (int c = 0; c < kRingClasses; c++) {
@@ -357,8 +358,7 @@ int launch_rings(const DevBatch &d, int do_ring, int do_xring, const cudaStream_
     }
     for (int c = kRingClasses - 1; c >= 0; c--) {   // the largest pairs first
         if (d.nritems[c] <= 0) continue;
-        const Args A{d.ritems + offs[c], d.rpairs, d.solves, d.rrows, d.vtab, d.xy, d.rx, d.active, do_ring, do_xring,
-                     tab_bytes(d), d.ring_doubles[c]};
+        const Args A{d.ritems + offs[c], d.rpairs, d.solves, d.rrows, d.vtab, d.xy, d.rx, d.active, tab_bytes(d), d.ring_doubles[c]};
         const cudaStream_t st = streams[n % ns];
         switch (kRingFrags[c]) {
         case 1: launch<1>(d, c, A, st); break;

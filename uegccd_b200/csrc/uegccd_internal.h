@@ -100,8 +100,8 @@ struct AmpInfo {
 // ring and crossed-ring products between the two groups are formed by one CTA.
 // xy0: where the pair's operands and results start (in doubles) in the batch's
 // particle-hole arrays: row a < n1 of group 1 holds 2 round8(n2) doubles -- in xy the
-// amplitudes X1[a][b] = t(i_a i_b, x_a) then Y1[a][b] = t(i_b i_a, x_a), in rx the ring G
-// of (i_a, i_b, x_a) then the crossed-ring G of (i_a, i_b, x_b), b over group 2.
+// amplitudes X1[a][b] = t(i_a i_b, x_a) then Y1[a][b] = t(i_b i_a, x_a), in rx for each b the ring
+// G of (i_a, i_b, x_a) and the crossed-ring G of (i_a, i_b, x_b), b over group 2.
 struct RingPairDev {
     int solve;
     int r1, n1;

@@ -1,19 +1,21 @@
 // update.cu -- the element-wise kernels of the spin-adapted solve: MP2 start, energy, the update
 // of one iteration and the DIIS extrapolation, all over the amplitudes i <= j.
 //
-// The amplitudes of a block are rows (pairs) of columns (virtuals).  A tile is up to 128 columns of
-// some rows; a thread owns a column: its orbital energies, mosaic sums and Coulomb row side are
-// loaded once and serve its rows, and the values of a row are the same for the whole warp.  What a
-// thread per amplitude fetched for each one -- the four orbitals, the mirror's index, two Coulomb
-// factors (16 bytes), four orbital energies, four mosaic sums, most of them scattered -- is index
-// arithmetic, two table lookups and a few loads per column.  The sums of a tile, the energy and
-// the DIIS dot products, are reduced together (warp_sums): one after the other they were nearly
-// half of the instructions.
+// The amplitudes of a block are rows (pairs) of columns (virtuals).  A tile is up to 128 columns
+// c <= K - c of some rows; a thread owns such a column and its partner's, the amplitudes (i,j,a) and
+// (i,j,b): v(i-b) = v(a-j), so both take the same two Coulomb factors, denominator and mosaic sums,
+// and each of the two places in the ring results that hold theirs serves both (16 bytes; k_rx_pos).
+// What a thread per amplitude fetched for each one -- the four orbitals, the mirror's index, two
+// Coulomb factors (16 bytes), four orbital energies, four mosaic sums, two ring values, most of them
+// scattered -- is index arithmetic, two table lookups and a few loads for two.  The sums of a tile,
+// the energy and the DIIS dot products, are reduced together (warp_sums): one after the other they
+// were nearly half of the instructions.
 // Latency decides: all warps resident (32 registers, a few spilled) and the |q|^2 table read through
 // L1 -- no barrier before the arithmetic -- beat fewer warps with more rows in flight, and a table
-// in shared memory.  Per launch, 100 twists of N=54 (485 plane waves), against a thread per
-// amplitude: the update with the DIIS push 0.381 -> 0.294 ms (0.23 ms of it without the push: the
-// ring values), the MP2 start 0.227 -> 0.148 ms; four N=114 systems: update 0.125 -> 0.100 ms.
+// in shared memory.  Per launch, 100 twists of N=54 (485 plane waves), a thread per amplitude, a
+// column of two rows each, a row of two columns: the update with the DIIS push (0.2 ms of DRAM
+// traffic) 0.381, 0.294, 0.239 ms; the MP2 start 0.227, 0.148, 0.133 ms; four N=114 systems: update
+// 0.125, 0.098, 0.075 ms.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -28,7 +30,7 @@ namespace uegccd {
 namespace {
 
 constexpr int kThreads = 128;
-constexpr int kRows = 2;      // rows a thread has in flight
+constexpr int kRows = 1;      // rows a thread has in flight, two columns each
 
 // Sum and maxima over the CTA in a fixed order (valid in thread 0).
 __device__ __forceinline__ void reduce3(double &sum, double &mx1, double &mx2)
@@ -65,10 +67,11 @@ __device__ __forceinline__ UTileDev load_tile(const UTileDev *__restrict__ tiles
 }
 
 // A tile's threads: groups of `width` lanes (32, 64 or 128, the least that holds the columns), a
-// group per row; thread (grp, lane) makes the rows r0 + grp + k * ngrp.
+// group per row; thread (grp, lane) makes the rows r0 + grp + k * ngrp, in each the column c and,
+// where `two`, its partner's column pc.
 struct Place {
     int grp, ngrp, c, pc;     // row group, groups, column and its partner's column
-    bool ok;
+    bool ok, two;
 };
 __device__ __forceinline__ Place place(const UTileDev &T)
 {
@@ -76,10 +79,11 @@ __device__ __forceinline__ Place place(const UTileDev &T)
     Place P;
     P.grp = threadIdx.x / width;
     P.ngrp = kThreads / width;
-    const int l = threadIdx.x - P.grp * width, vc = T.nvd + T.sd;
+    const int l = threadIdx.x - P.grp * width;
     P.ok = l < T.nc;
     P.c = T.c0 + min(l, T.nc - 1);
-    P.pc = P.c < T.nvd ? P.c + vc : P.c < vc ? P.c : P.c - vc;
+    P.two = P.c < T.nvd;
+    P.pc = P.two ? P.c + T.nvd + T.sd : P.c;
     return P;
 }
 
@@ -92,7 +96,7 @@ __device__ __forceinline__ Place place(const UTileDev &T)
 // The mirror (j,i,b) has the same integrals; its denominator is summed in its own order.
 // A core pair's integrals are zero (CoreERI), so is its amplitude.
 // ----------------------------------------------------------------------------
-__global__ void __launch_bounds__(kThreads) k_mp2(const UTileDev *__restrict__ tiles,
+__global__ void __launch_bounds__(kThreads, 12) k_mp2(const UTileDev *__restrict__ tiles,
                                                   const SolveDev *__restrict__ solves,
                                                   const int16_t *__restrict__ vir, const int *__restrict__ vpk,
                                                   const int4 *__restrict__ rowpk, const double *__restrict__ eigen,
@@ -115,17 +119,21 @@ __global__ void __launch_bounds__(kThreads) k_mp2(const UTileDev *__restrict__ t
         const int i = R.z & 0xffff, j = R.z >> 16;
         const double via = V[__dp4a(m2, R.x, na2 + __dp4a(R.x, R.x, 0))];
         const double vaj = V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))];
-        const double eij = ev[i] + ev[j];
-        const bool c = i < core || j < core;
-        const double x = c ? 0.0 : via / (eij - ea - eb);
-        t[T.t0 + q * T.v + P.c] = x;
-        double y = 0.0;
-        if (q < T.nd) {
-            y = c ? 0.0 : via / (eij - eb - ea);
-            t[T.t0 + (q + T.nd + T.dg) * T.v + P.pc] = y;
-        }
+        const double eij = ev[i] + ev[j], dab = eij - ea - eb, dba = eij - eb - ea;
+        const bool z = i < core || j < core, pair = q < T.nd;
+        const int row = T.t0 + q * T.v, mir = row + (T.nd + T.dg) * T.v;
+        const double x = z ? 0.0 : via / dab, y = z || !pair ? 0.0 : via / dba;
+        t[row + P.c] = x;
+        if (pair) t[mir + P.pc] = y;
         e += (x + y) * (2.0 * via - vaj);
         mx = fmax(mx, fmax(fabs(x), fabs(y)));
+        if (P.two) {   // v(i - b) = v(a - j)
+            const double u = z ? 0.0 : vaj / dba, w = z || !pair ? 0.0 : vaj / dab;
+            t[row + P.pc] = u;
+            if (pair) t[mir + P.c] = w;
+            e += (u + w) * (2.0 * vaj - via);
+            mx = fmax(mx, fmax(fabs(u), fabs(w)));
+        }
     }
     reduce3(e, mx, none);
     if (threadIdx.x == 0) {
@@ -154,13 +162,19 @@ __global__ void __launch_bounds__(kThreads) k_energy(const UTileDev *__restrict_
     for (int r = P.ok ? P.grp : T.nr; r < T.nr; r += P.ngrp) {
         const int q = T.r0 + r;
         const int4 R = __ldg(&rowpk[T.pair0 + q]);
-        const double x = t[T.t0 + q * T.v + P.c];
-        const double y = q < T.nd ? t[T.t0 + (q + T.nd + T.dg) * T.v + P.pc] : 0.0;
+        const int row = T.t0 + q * T.v, mir = row + (T.nd + T.dg) * T.v;
+        const bool pair = q < T.nd;
+        const double x = t[row + P.c], y = pair ? t[mir + P.pc] : 0.0;
+        const double u = P.two ? t[row + P.pc] : 0.0, w = P.two && pair ? t[mir + P.c] : 0.0;
         const double via = V[__dp4a(m2, R.x, na2 + __dp4a(R.x, R.x, 0))];
         const double vaj = V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))];
-        if (kind == 0) e += (x + y) * (2.0 * via - vaj);
-        else e += via * (x + y) * 2.0 - vaj * (x + y) * csosex;
-        mx = fmax(mx, fmax(fabs(x), fabs(y)));
+        if (kind == 0) {
+            e += (x + y) * (2.0 * via - vaj) + (u + w) * (2.0 * vaj - via);
+        } else {
+            e += via * (x + y) * 2.0 - vaj * (x + y) * csosex;
+            e += vaj * (u + w) * 2.0 - via * (u + w) * csosex;
+        }
+        mx = fmax(fmax(mx, fmax(fabs(x), fabs(y))), fmax(fabs(u), fabs(w)));
     }
     reduce3(e, mx, none);
     if (threadIdx.x == 0) {
@@ -199,7 +213,7 @@ struct UpdateArgs {
     const double *rx;             // ring and crossed-ring G, particle-hole layout
     const int2 *rpos;             // where each amplitude's two values sit in it
     const uint8_t *active;
-    int do_ladder, do_mosaic, do_ring, do_xring, do_driver, drpa, mode;
+    int do_ladder, do_mosaic, do_ring, do_xring, do_driver, mode;
     const IterState *st;
     int ndiis;
     int64_t namp;
@@ -207,7 +221,7 @@ struct UpdateArgs {
     float *hist_e;
 };
 
-template <int NV>
+template <int NV, bool DRPA>
 __global__ void __launch_bounds__(kThreads, NV <= 8 ? 16 : 6) k_update(UpdateArgs A)
 {
     const UTileDev T = load_tile(A.tiles);
@@ -216,16 +230,19 @@ __global__ void __launch_bounds__(kThreads, NV <= 8 ? 16 : 6) k_update(UpdateArg
         return;
     }
     const Place P = place(T);
-    const bool rings = !A.drpa && (A.do_ring || A.do_xring), mos = A.do_mosaic != 0;
-    double told[kRows], g[kRows], s1[kRows], s2[kRows];
+    const bool rings = !DRPA && (A.do_ring || A.do_xring), mos = A.do_mosaic != 0;
+    // index 0: the column c, 1: its partner's
+    double told[kRows][2], g[kRows][2], s1[kRows][2], s2[kRows][2];
     int2 ro[kRows];
 #pragma unroll
     for (int k = 0; k < kRows; k++) {
-        const int r = P.grp + k * P.ngrp, p = T.t0 + (T.r0 + r) * T.v + P.c;
-        const bool in = P.ok && r < T.nr;
-        told[k] = in ? A.t[p] : 0.0;
-        g[k] = in && A.do_ladder ? A.g_ladder[p] : 0.0;
-        ro[k] = in && rings ? A.rpos[p] : make_int2(0, 0);
+        const int r = P.grp + k * P.ngrp, row = T.t0 + (T.r0 + r) * T.v;
+        const bool in = P.ok && r < T.nr, two = in && P.two;
+        told[k][0] = in ? A.t[row + P.c] : 0.0;
+        told[k][1] = two ? A.t[row + P.pc] : 0.0;
+        g[k][0] = in && A.do_ladder ? A.g_ladder[row + P.c] : 0.0;
+        g[k][1] = two && A.do_ladder ? A.g_ladder[row + P.pc] : 0.0;
+        ro[k] = in && rings ? A.rpos[row + P.c] : make_int2(0, 0);
     }
     const double *ev = A.eigen + T.orb0;
     const int a = A.vir[T.vir0 + P.c], b = A.vir[T.vir0 + P.pc];
@@ -234,9 +251,16 @@ __global__ void __launch_bounds__(kThreads, NV <= 8 ? 16 : 6) k_update(UpdateArg
     const int na = A.vpk[T.vir0 + P.c], m2 = neg2(na), na2 = __dp4a(na, na, 0);
 #pragma unroll
     for (int k = 0; k < kRows; k++) {
+        // the place of (ia, jb) holds the ring G of (ij, a) and the crossed-ring G of (ij, b), that
+        // of (ib, ja) the ring G of (ij, b) and the crossed-ring G of (ij, a)
         const bool in = P.ok && P.grp + k * P.ngrp < T.nr && rings;
-        s1[k] = in && A.do_ring ? __ldg(&A.rx[ro[k].x]) : 0.0;
-        s2[k] = in && A.do_xring ? __ldg(&A.rx[ro[k].y]) : 0.0;
+        const double2 zero = make_double2(0.0, 0.0);
+        const double2 u = in ? __ldg(reinterpret_cast<const double2 *>(A.rx + ro[k].x)) : zero;
+        const double2 w = in ? P.two ? __ldg(reinterpret_cast<const double2 *>(A.rx + ro[k].y)) : u : zero;
+        s1[k][0] = A.do_ring ? u.x : 0.0;
+        s1[k][1] = A.do_ring ? w.x : 0.0;
+        s2[k][0] = A.do_xring ? w.y : 0.0;
+        s2[k][1] = A.do_xring ? u.y : 0.0;
     }
     const int core = A.solves[T.solve].core_n;
     const double f = A.solves[T.solve].denom_factor;
@@ -246,55 +270,64 @@ __global__ void __launch_bounds__(kThreads, NV <= 8 ? 16 : 6) k_update(UpdateArg
     const int slot = NV > 0 ? (nb - 1) % A.ndiis : 0, nvec = NV > 0 ? min(nb, A.ndiis) : 0;
     const double *__restrict__ V = A.vtab + T.vtab0;
     double esum = 0.0, mx = 0.0;   // mx: max|dT|, or max|R| in mode 1
-    float err[kRows];
+    float err[kRows][2];
 #pragma unroll
     for (int k = 0; k < kRows; k++) {
-        err[k] = 0.0f;
+        err[k][0] = err[k][1] = 0.0f;
         const int r = P.grp + k * P.ngrp;
         if (!P.ok || r >= T.nr) continue;
-        const int q = T.r0 + r, p = T.t0 + q * T.v + P.c;
+        const int q = T.r0 + r, row = T.t0 + q * T.v;
         const int4 R = __ldg(&A.rowpk[T.pair0 + q]);
         const int i = R.z & 0xffff, j = R.z >> 16;
         const bool pair = q < T.nd;
-        const int mir = T.t0 + (q + T.nd + T.dg) * T.v + P.pc;
+        const int mir = row + (T.nd + T.dg) * T.v;
         const double via = V[__dp4a(m2, R.x, na2 + __dp4a(R.x, R.x, 0))];
-        double x = g[k];
-        if (A.do_driver) x += via;   // GetG2Drivers: G2abab = V(n_i - n_a)
-        if (mos) x -= 0.5 * (jab + A.joo[T.joo0 + i] + A.joo[T.joo0 + j]) * told[k];
-        if (A.drpa) {
-            if (A.do_ring) {   // linear and quadratic rings (k_drpa_sums)
-                const int ia = T.phr0 + i * T.V + (a - T.O), jb = T.phr0 + j * T.V + (b - T.O);
-                const double u = A.dru[ia];
-                x += u + A.dru[jb] + 2.0 * u * A.drs2[jb];
-            }
-        } else {   // the ring G and the crossed-ring G, where k_rings left them (k_rx_pos)
-            if (A.do_ring) x += s1[k];
-            if (A.do_xring) x += s2[k];
-        }
-        if (i < core || j < core) x = 0.0;   // core pair: every term has a zero factor
+        const double vaj = V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))];   // = v(i - b)
+        const double jj = mos ? 0.5 * (jab + A.joo[T.joo0 + i] + A.joo[T.joo0 + j]) : 0.0;
         const double denom = ev[i] + ev[j] - ea - eb;
-        if (NV == 0 && A.mode != 0) {
-            if (A.g_out) {
-                A.g_out[p] = x;
-                if (pair) A.g_out[mir] = x;
+#pragma unroll
+        for (int m = 0; m < 2; m++) {
+            if (m == 1 && !P.two) continue;
+            const double v1 = m == 0 ? via : vaj, v2 = m == 0 ? vaj : via, t0 = told[k][m];
+            const int p = row + (m == 0 ? P.c : P.pc), pm = mir + (m == 0 ? P.pc : P.c);
+            double x = g[k][m];
+            if (A.do_driver) x += v1;   // GetG2Drivers: G2abab = V(n_i - n_a)
+            if (mos) x -= jj * t0;
+            if (DRPA) {
+                if (A.do_ring) {   // linear and quadratic rings (k_drpa_sums)
+                    const int xa = (m == 0 ? a : b) - T.O, xb = (m == 0 ? b : a) - T.O;
+                    const int ia = T.phr0 + i * T.V + xa, jb = T.phr0 + j * T.V + xb;
+                    const double u = A.dru[ia];
+                    x += u + A.dru[jb] + 2.0 * u * A.drs2[jb];
+                }
+            } else {   // the ring G and the crossed-ring G, where k_rings left them (k_rx_pos)
+                if (A.do_ring) x += s1[k][m];
+                if (A.do_xring) x += s2[k][m];
             }
-            mx = fmax(mx, fabs(-x + denom * told[k]));
-            continue;
-        }
-        const double y = x / denom - (1.0 - f) * told[k], tn = pow2 ? y * (1.0 / f) : y / f;
-        double d = fabs(tn - told[k]);
-        if (!(fabs(tn) < 1e300)) d = __longlong_as_double(0x7ff0000000000000LL);  // +Inf marks NaN/Inf
-        mx = fmax(mx, d);
-        double es = via * tn * 2.0;   // dRPA: the SOSEX part at the end
-        if (!A.drpa) es = tn * (2.0 * via - V[__dp4a(m2, R.y, na2 + __dp4a(R.y, R.y, 0))]);
-        esum += pair ? 2.0 * es : es;
-        if (NV == 0) {
-            A.t[p] = tn;
-            if (pair) A.t[mir] = tn;
-        } else {   // the history slot holds t'; the mirrors' entries are never read
-            err[k] = (float)(tn - told[k]);
-            A.hist_t[(int64_t)slot * A.namp + p] = tn;
-            A.hist_e[(int64_t)slot * A.namp + p] = err[k];
+            if (i < core || j < core) x = 0.0;   // core pair: every term has a zero factor
+            if (NV == 0 && A.mode != 0) {
+                if (A.g_out) {
+                    A.g_out[p] = x;
+                    if (pair) A.g_out[pm] = x;
+                }
+                mx = fmax(mx, fabs(-x + denom * t0));
+                continue;
+            }
+            const double y = x / denom - (1.0 - f) * t0, tn = pow2 ? y * (1.0 / f) : y / f;
+            double d = fabs(tn - t0);
+            if (!(fabs(tn) < 1e300)) d = __longlong_as_double(0x7ff0000000000000LL);  // +Inf marks NaN/Inf
+            mx = fmax(mx, d);
+            // dRPA: the SOSEX part at the end
+            const double es = DRPA ? v1 * tn * 2.0 : tn * (2.0 * v1 - v2);
+            esum += pair ? 2.0 * es : es;
+            if (NV == 0) {
+                A.t[p] = tn;
+                if (pair) A.t[pm] = tn;
+            } else {   // the history slot holds t'; the mirrors' entries are never read
+                err[k][m] = (float)(tn - t0);
+                A.hist_t[(int64_t)slot * A.namp + p] = tn;
+                A.hist_e[(int64_t)slot * A.namp + p] = err[k][m];
+            }
         }
     }
     const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
@@ -310,9 +343,11 @@ __global__ void __launch_bounds__(kThreads, NV <= 8 ? 16 : 6) k_update(UpdateArg
             for (int k = 0; k < kRows; k++) {
                 const int r = P.grp + k * P.ngrp, q = T.r0 + r;
                 if (!P.ok || r >= T.nr) continue;
-                const double e0 = err[k];
-                const double h = j == slot ? e0 : (double)A.hist_e[(int64_t)j * A.namp + T.t0 + q * T.v + P.c];
-                v[j] = fma(q < T.nd ? 2.0 * e0 : e0, h, v[j]);
+                const float *h = A.hist_e + (int64_t)j * A.namp + T.t0 + q * T.v;
+                const double h0 = j == slot ? err[k][0] : h[P.c], h1 = j == slot ? err[k][1] : P.two ? h[P.pc] : 0.0f;
+                const double e0 = err[k][0], e1 = err[k][1];
+                v[j] = fma(q < T.nd ? 2.0 * e0 : e0, h0, v[j]);
+                v[j] = fma(q < T.nd ? 2.0 * e1 : e1, h1, v[j]);
             }
     }
     v[NS - 1] = esum;
@@ -344,25 +379,32 @@ __global__ void __launch_bounds__(kThreads) k_diis_extrap(const UTileDev *__rest
     if (!applied[T.solve]) return;
     const double *c = coef + T.solve * kDiisMax;
     const Place P = place(T);
-    double x[kRows];
+    double x[kRows][2];
 #pragma unroll
-    for (int k = 0; k < kRows; k++) x[k] = 0.0;
+    for (int k = 0; k < kRows; k++) x[k][0] = x[k][1] = 0.0;
     for (int j = 0; j < ndiis; j++) {
         const double cj = c[j];
         if (cj == 0.0) continue;   // a slot not yet filled has coefficient 0 and is not read
         const double *h = hist_t + (int64_t)j * namp;
 #pragma unroll
         for (int k = 0; k < kRows; k++) {
-            const int r = P.grp + k * P.ngrp;
-            if (P.ok && r < T.nr) x[k] = fma(cj, h[T.t0 + (T.r0 + r) * T.v + P.c], x[k]);
+            const int r = P.grp + k * P.ngrp, row = T.t0 + (T.r0 + r) * T.v;
+            if (P.ok && r < T.nr) {
+                x[k][0] = fma(cj, h[row + P.c], x[k][0]);
+                if (P.two) x[k][1] = fma(cj, h[row + P.pc], x[k][1]);
+            }
         }
     }
 #pragma unroll
     for (int k = 0; k < kRows; k++) {
-        const int r = P.grp + k * P.ngrp, q = T.r0 + r;
+        const int r = P.grp + k * P.ngrp, q = T.r0 + r, row = T.t0 + q * T.v, mir = row + (T.nd + T.dg) * T.v;
         if (!P.ok || r >= T.nr) continue;
-        t[T.t0 + q * T.v + P.c] = x[k];
-        if (q < T.nd) t[T.t0 + (q + T.nd + T.dg) * T.v + P.pc] = x[k];
+        t[row + P.c] = x[k][0];
+        if (P.two) t[row + P.pc] = x[k][1];
+        if (q < T.nd) {
+            t[mir + P.pc] = x[k][0];
+            if (P.two) t[mir + P.c] = x[k][1];
+        }
     }
 }
 
@@ -389,14 +431,14 @@ void launch_update(const DevBatch &d, const TermFlags &f, int mode, double *g_ou
     A.t = d.t; A.g_ladder = d.g; A.jvv = d.jvv; A.joo = d.joo; A.dru = d.dru; A.drs2 = d.drs2;
     A.part_e = d.part_e; A.part_dt = d.part_dt; A.part_r = d.part_r; A.g_out = g_out; A.active = d.active;
     A.do_ladder = f.do_ladder; A.do_mosaic = f.do_mosaic; A.do_ring = f.do_ring; A.do_xring = f.do_xring;
-    A.do_driver = f.do_driver; A.drpa = f.drpa; A.mode = mode;
+    A.do_driver = f.do_driver; A.mode = mode;
     A.rx = d.rx; A.rpos = d.rpos;
     A.st = diis ? diis->state : nullptr; A.ndiis = (diis && mode == 0) ? ndiis : 0; A.namp = d.namp;
     A.hist_t = diis ? diis->hist_t : nullptr; A.hist_e = diis ? diis->hist_e : nullptr;
     A.dpart = diis ? diis->part : nullptr;
-    if (A.ndiis == 0) k_update<0><<<d.nutiles, kThreads, 0, st>>>(A);
-    else if (A.ndiis <= 7) k_update<8><<<d.nutiles, kThreads, 0, st>>>(A);
-    else k_update<32><<<d.nutiles, kThreads, 0, st>>>(A);
+    auto *k = f.drpa ? A.ndiis == 0 ? k_update<0, true> : A.ndiis <= 7 ? k_update<8, true> : k_update<32, true>
+                     : A.ndiis == 0 ? k_update<0, false> : A.ndiis <= 7 ? k_update<8, false> : k_update<32, false>;
+    k<<<d.nutiles, kThreads, 0, st>>>(A);
 }
 
 void launch_extrap(const DevBatch &d, const CtlBuffers &c, int ndiis, cudaStream_t st)
@@ -404,8 +446,8 @@ void launch_extrap(const DevBatch &d, const CtlBuffers &c, int ndiis, cudaStream
     k_diis_extrap<<<d.nutiles, kThreads, 0, st>>>(d.utiles, d.namp, c.hist_t, c.coef, ndiis, d.t, c.applied);
 }
 
-// The tiles of a block of `rows` rows and v columns: column ranges of at most 128, each in ranges
-// that fill the threads' rows.
+// The tiles of a block of `rows` rows and v columns c <= K - c: column ranges of at most 128, each in
+// ranges that fill the threads' rows.
 void update_tiles(int rows, int v, void (*emit)(void *, int, int, int, int), void *to)
 {
     const int nt = (v + kThreads - 1) / kThreads, w = (v + nt - 1) / nt;
