@@ -239,19 +239,21 @@ bool is_pinned(const void *p)
     return yes;
 }
 
-// memcpy on the host's cores (large copies; the destination's pages are often touched first here)
-void host_copy(char *dst, const char *src, size_t bytes)
+// memcpy, on the host's cores from kCoresMin bytes on, each a range of its own.  The destination's
+// pages are often touched first here, and threads that fault pages in contend: three arrays of
+// 2.7 MB take 0.35 ms by one thread and 0.9 ms by 16, of 28 MB 12 and 5 ms.
+constexpr size_t kCoresMin = 8ull << 20;
+void host_copy(char *dst, const char *src, size_t bytes, bool cores)
 {
-    constexpr size_t kPiece = 256 << 10;
-    if (bytes <= 2 * kPiece) {
+    if (!cores) {
         std::memcpy(dst, src, bytes);
         return;
     }
-    const int n = (int)((bytes + kPiece - 1) / kPiece);
-    const int nth = std::max(1, std::min({16, n, (int)std::thread::hardware_concurrency()}));
-    parallel_for(n, nth, [&](int k) {
-        const size_t a = (size_t)k * kPiece;
-        std::memcpy(dst + a, src + a, std::min(kPiece, bytes - a));
+    const int nth = std::max(1, std::min(16, (int)std::thread::hardware_concurrency()));
+    const size_t piece = (bytes + nth - 1) / nth;
+    parallel_for(nth, nth, [&](int k) {
+        const size_t a = (size_t)k * piece, e = std::min(bytes, a + piece);
+        if (a < e) std::memcpy(dst + a, src + a, e - a);
     });
 }
 // g_pool_mu guards the cache, the per-device byte counts and the limit
@@ -1081,9 +1083,10 @@ int pack_from_host(UegccdBatch &b, int s, const double *host_dense)
 
 // T2abab / T2abba / T2aaaa of solve s in the reference layout (each may be null) into host
 // arrays; with_red: the batch's reduced sums too, in the same wait.  The arrays leave the device in
-// one run into page-locked memory and go on from there on the host's cores, one while the next is
-// on its way: the driver stages a copy into pageable memory on one thread, 11 GB/s measured with
-// fresh pages, 2.7 MB an array at N=54.
+// one run into page-locked memory and go on from there, one copied while the next is on its way: a
+// pageable copy waits for the one before it.  MP2 with its three arrays: N=38 (0.7 MB each) 0.48 ->
+// 0.24 ms, N=54 (3.3 MB) 1.28 -> 0.82, N=114 (28 MB) 16 -> 6.5; one array, the residual, of 17 MB
+// 3.9 -> 3.4 ms, but of 28 MB 5.7 -> 7.4: a single one above kAloneMax is left to the driver.
 int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, double *ba, double *aa,
                    bool with_red = false)
 {
@@ -1103,8 +1106,10 @@ int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, doubl
     b.d2h_bytes += (int64_t)(m * bytes);
     const size_t red = with_red ? b.red.size() * sizeof(double) : 0;
     if (red) b.d2h_bytes += (int64_t)red;
+    constexpr size_t kAloneMax = 24ull << 20;
     bool direct = true;   // page-locked destinations take the copies themselves
     for (int k = 0; k < m; k++) direct = direct && is_pinned(host[k]);
+    direct = direct || (m == 1 && bytes > kAloneMax);
     PinnedScope buf(direct ? red : red + m * bytes);
     if (!buf.b.p || direct) {
         for (int k = 0; k < m; k++)
@@ -1128,7 +1133,7 @@ int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, doubl
     }
     for (int k = 0; k < m; k++) {
         if (apart) CU(cudaEventSynchronize(b.ev_copy[k]));
-        host_copy((char *)host[k], arrays + k * bytes, bytes);
+        host_copy((char *)host[k], arrays + k * bytes, bytes, m * bytes > 2 * kCoresMin);
     }
     if (red) std::memcpy(b.red.data(), buf.b.p, red);
     return 0;
@@ -2362,7 +2367,7 @@ int uegccd_batch_get_all_amplitudes(UegccdBatch *b, double *t_abab)
     }
     CU(cudaMemcpyAsync(buf.b.p, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
     CU(cudaStreamSynchronize(b->stream));
-    host_copy((char *)t_abab, buf.b.p, bytes);
+    host_copy((char *)t_abab, buf.b.p, bytes, bytes >= kCoresMin);
     return UEGCCD_OK;
 }
 
