@@ -368,6 +368,8 @@ struct UegccdBatch {
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_solve0 = nullptr, ev_solve1 = nullptr;
     PinnedBuf pin;                   // page-locked words the small reads land in (on first use)
+    PinnedBuf flag;                  // CtlBuffers::done (with the control buffers)
+    cudaEvent_t ev_iter[2] = {nullptr, nullptr};            // the two latest iterations
     cudaEvent_t ev_copy[3] = {nullptr, nullptr, nullptr};   // arrays of a download (on first use)
     Fork fork;                       // side streams of a small batch's residual (on first use)
     bool fork_made = false;
@@ -449,6 +451,9 @@ struct UegccdBatch {
         if (ev_solve0) cudaEventDestroy(ev_solve0);
         if (ev_solve1) cudaEventDestroy(ev_solve1);
         pinned_put(pin);
+        pinned_put(flag);
+        for (auto &e : ev_iter)
+            if (e) cudaEventDestroy(e);
         for (auto &e : ev_copy)
             if (e) cudaEventDestroy(e);
         for (cudaEvent_t e : {fork.start, fork.staged})
@@ -1307,10 +1312,16 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
     CtlBuffers &c = b.ctl;
     const int n = b.d.nsolves;
     int rc = 0;
+    if (!c.done) {
+        b.flag = pinned_get(sizeof(int));
+        if (!b.flag.p) return fail(UEGCCD_ERR_ALLOC, "no page-locked host memory");
+        c.done = reinterpret_cast<int *>(b.flag.p);
+        for (auto &e : b.ev_iter) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    }
     if (!c.state) {
         const UegccdBatch::Mark m = b.mark();
         CtlBuffers x = c;
-        if ((rc = b.alloc(x.state, n)) || (rc = b.alloc(x.applied, n)) || (rc = b.alloc(x.count, 1)) ||
+        if ((rc = b.alloc(x.state, n)) || (rc = b.alloc(x.applied, n)) || (rc = b.alloc(x.stopped, 1)) ||
             (rc = b.alloc(x.Bm, (size_t)n * kDiisMax * kDiisMax)) || (rc = b.alloc(x.coef, (size_t)n * kDiisMax)) ||
             (rc = b.alloc(x.part, (size_t)b.d.nutiles * kDiisMax))) {
             b.rollback(m);
@@ -1483,9 +1494,13 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
         launch_energy(d, drpa ? 1 : 0, 0.0, b.stream);
         b.launches++;
     }
+    *(volatile int *)b.ctl.done = 0;
     launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
     b.launches++;
-    int count = n, rounds = 0;
+    // The iterations go in rounds of kPoll.  The host keeps one queued behind the one whose end it
+    // waits for, and looks at the flag of k_tail: the GPU does not wait for the host, and a solve
+    // that has stopped costs one empty iteration.  (A copy of the count and a wait every four
+    // iterations left the GPU idle for 22 us and up to three iterations empty.)
     const int max_rounds = opt->max_iter / kPoll + 2;
     // mixed precision: tensor-core ladder of t - t_ref, t_ref refreshed (FP64) each round,
     // then FP64 iterations from where the mixed phase stopped (refinement)
@@ -1495,37 +1510,47 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
         if (phase == 1 && mixed) {
             // reopen every solve for the FP64 sweeps
             std::vector<IterState> st1(n);
-            CU(cudaMemcpyAsync(st1.data(), b.ctl.state, n * sizeof(IterState), cudaMemcpyDeviceToHost, b.stream));
-            CU(cudaStreamSynchronize(b.stream));
+            if ((rc = read_back(b, st1.data(), b.ctl.state, n * sizeof(IterState)))) return rc;
             for (auto &x : st1) x.status = 0;
             CU(cudaMemcpyAsync(b.ctl.state, st1.data(), n * sizeof(IterState), cudaMemcpyHostToDevice, b.stream));
             if ((rc = set_active_all(b, 1))) return rc;
-            count = n;
-            CU(cudaMemcpyAsync(b.ctl.count, &count, sizeof(int), cudaMemcpyHostToDevice, b.stream));
-            rounds = 0;
+            CU(cudaMemsetAsync(b.ctl.stopped, 0, sizeof(int), b.stream));
+            *(volatile int *)b.ctl.done = 0;
         }
         if ((rc = capture_iteration(b, f, opt->tol, opt->max_iter, ndiis))) return rc;
-        int sweeps = 0;
-        while (count > 0 && rounds < max_rounds) {
+        const UegccdBatch::IterGraph &G = b.graphs[f.mixed];
+        auto stopped = [&](int it) {   // 1 when no solve iterates after iteration `it`, -1: failed
+            if (cudaEventSynchronize(b.ev_iter[it & 1]) != cudaSuccess) return -1;
+            return (int)*(volatile int *)b.ctl.done;
+        };
+        const int most = phase == 1 && mixed ? std::min(max_rounds, std::max(1, opt->refine_sweeps)) : max_rounds;
+        int it = 0, stop = 0;
+        for (int round = 0; round < most && stop == 0; round++) {
+            // the refresh is not queued ahead: it costs as much as an iteration
+            if (f.mixed && it > 0 && (stop = stopped(it - 1)) != 0) break;
             if (f.mixed) {
                 launch_refresh(d, b.stream);
                 b.launches += 2;
             }
-            for (int k = 0; k < kPoll; k++) {
+            for (int k = 0; k < kPoll && stop == 0; k++, it++) {
                 if (b.kt.on && k == kPoll - 1) {
                     // the sampled iteration of the round: direct launches between CUDA events
                     b.launches += launch_iteration(d, b.ctl, f, opt->tol, opt->max_iter, ndiis, b.stream, &b.kt);
                 } else {
-                    const UegccdBatch::IterGraph &G = b.graphs[f.mixed];
                     CU(cudaGraphLaunch(G.exec, b.stream));
                     b.launches += G.launches;
                 }
+                CU(cudaEventRecord(b.ev_iter[it & 1], b.stream));
+                if (it > 0) stop = stopped(it - 1);
             }
-            if ((rc = read_back(b, &count, b.ctl.count, sizeof(int)))) return rc;
-            b.kt.collect();
-            rounds++;
-            if (phase == 1 && mixed && ++sweeps >= std::max(1, opt->refine_sweeps)) break;
+            if (b.kt.on) {
+                CU(cudaStreamSynchronize(b.stream));
+                b.kt.collect();
+            }
         }
+        if (stop < 0) CU(cudaStreamSynchronize(b.stream));
+        CU(cudaGetLastError());
+        // (the iteration queued behind may still run: what follows is on its stream)
     }
     if (mixed) {
         int err = 0;
@@ -1621,6 +1646,7 @@ int session_start(UegccdBatch &b, const UegccdOptions *opt, int drpa)
         launch_energy(d, 1, 0.0, b.stream);
         b.launches++;
     }
+    *(volatile int *)b.ctl.done = 0;
     launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
     b.launches++;
     if ((rc = capture_iteration(b, f, opt->tol, opt->max_iter, ndiis))) return rc;
@@ -1643,20 +1669,18 @@ int session_advance(UegccdBatch &b, int rounds, int *n_active, int *n_done, int 
     auto &S = b.ses;
     const int n = d.nsolves;
     const UegccdOptions &opt = S.opt;
-    int count = 0;
-    CU(cudaMemcpyAsync(&count, b.ctl.count, sizeof(int), cudaMemcpyDeviceToHost, b.stream));
-    CU(cudaStreamSynchronize(b.stream));
-    for (int r = 0; r < rounds && count > 0; r++) {
+    for (int r = 0; r < rounds && *(volatile int *)b.ctl.done == 0; r++) {
         for (int k = 0; k < kPoll; k++) {
             CU(cudaGraphLaunch(b.graphs[0].exec, b.stream));
             b.launches += b.graphs[0].launches;
         }
-        const int rc = read_back(b, &count, b.ctl.count, sizeof(int));
-        if (rc) return rc;
+        if (r + 1 < rounds) CU(cudaStreamSynchronize(b.stream));
     }
     std::vector<IterState> st(n);
-    CU(cudaMemcpyAsync(st.data(), b.ctl.state, n * sizeof(IterState), cudaMemcpyDeviceToHost, b.stream));
-    CU(cudaStreamSynchronize(b.stream));
+    {
+        const int rc = read_back(b, st.data(), b.ctl.state, n * sizeof(IterState));
+        if (rc) return rc;
+    }
     std::vector<int> fresh;
     for (int s = 0; s < n; s++)
         if (st[s].status != 0 && !S.released[s]) fresh.push_back(s);

@@ -179,7 +179,8 @@ struct IterState {
 struct CtlBuffers {
     IterState *state = nullptr;
     uint8_t *applied = nullptr;  // the solves the iteration in flight updated
-    int *count = nullptr;        // solves still iterating
+    int *stopped = nullptr;      // solves no longer iterating
+    int *done = nullptr;         // host memory (page-locked): 1 when none is
     double *Bm = nullptr, *coef = nullptr, *part = nullptr;
     double *hist_t = nullptr;   // DIIS history: updated amplitudes t' (FP64)
     float *hist_e = nullptr;    // and error vectors e = t' - t (FP32: they only enter the B-matrix dots)

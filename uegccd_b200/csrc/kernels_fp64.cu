@@ -618,7 +618,8 @@ __device__ bool pulay_warp(const double *B, int nvec, double *c, double (*A)[kMa
 // chunk order, the new row of the Pulay matrix from the dot-product partials, the convergence
 // decision and the Pulay coefficients.  init = 1: the start amplitudes' energy, recorded, and
 // whether to iterate.  applied = the solves this iteration updated (k_diis_extrap runs on
-// those); active = the ones that go on, *count their number.
+// those); active = the ones that go on.  *stopped counts the others; the last of them sets *done,
+// in host memory, so that the host learns of it without a copy.
 // One launch with the elimination spread over a warp in shared memory, where the reduction, the
 // row reduction, a one-thread-per-solve control (its 17 x 18 matrix in local memory) and the
 // swap of the active flags were four launches: 22 -> 10.5 us an iteration on one N=54 solve,
@@ -628,7 +629,7 @@ __global__ void __launch_bounds__(256)
            const double *__restrict__ part_r, const double *__restrict__ dpart, IterState *__restrict__ st,
            double *__restrict__ Bm, double *__restrict__ coef, double *__restrict__ rec_e,
            double *__restrict__ rec_dt, int max_rec, uint8_t *active, uint8_t *__restrict__ applied,
-           int *__restrict__ count, double tol, int max_iter, int ndiis, int init)
+           int *__restrict__ stopped, int *done, double tol, int max_iter, int ndiis, int init)
 {
     const int s = blockIdx.x;
     if (!init && !active[s]) {
@@ -700,8 +701,10 @@ __global__ void __launch_bounds__(256)
         st[s] = S;
         applied[s] = init ? 0 : 1;
         active[s] = go ? 1 : 0;
-        if (init) atomicAdd(count, go ? 1 : 0);
-        else if (!go) atomicSub(count, 1);
+        if (!go && atomicAdd(stopped, 1) + 1 == (int)gridDim.x) {
+            *(volatile int *)done = 1;
+            __threadfence_system();
+        }
     }
 }
 
@@ -720,10 +723,10 @@ void launch_refresh(const DevBatch &d, cudaStream_t st)
 void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
                  cudaStream_t st)
 {
-    if (init) cudaMemsetAsync(c.count, 0, sizeof(int), st);
+    if (init) cudaMemsetAsync(c.stopped, 0, sizeof(int), st);
     k_tail<<<d.nsolves, 256, 0, st>>>(d.utile_begin, d.part_e, d.part_dt, d.part_r, c.part,
                                       c.state, c.Bm, c.coef, c.rec_e, c.rec_dt, c.max_rec, d.active, c.applied,
-                                      c.count, tol, max_iter, ndiis, init);
+                                      c.stopped, c.done, tol, max_iter, ndiis, init);
 }
 
 // One iteration: residual + update, control, [DIIS extrapolation].  Returns launches.

@@ -712,6 +712,8 @@ TwoChannel::TwoChannel() = default;
 
 TwoChannel::~TwoChannel()
 {
+    if (out_) cudaFreeHost(out_);
+    if (evo_) cudaEventDestroy(evo_);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
 }
@@ -769,7 +771,7 @@ int TwoChannel::init(const SystemHost &sys, const SolvePlan &plan, cudaStream_t 
         (rc = alloc((void **)&eig_, M_ * sizeof(double))) || (rc = alloc((void **)&cube_d, cube.size() * sizeof(int))) ||
         (rc = alloc((void **)&jvv_, V_ * sizeof(double))) || (rc = alloc((void **)&joo_, O_ * sizeof(double))) ||
         (rc = alloc((void **)&part_, (size_t)2 * std::max(nblk_, 1) * kMaxDiis * sizeof(double))) ||
-        (rc = alloc((void **)&out_, 2 * kMaxDiis * sizeof(double)))) {
+        (rc = host_words())) {
         al_.rollback();
         return rc;
     }
@@ -925,10 +927,30 @@ int TwoChannel::upload_t(const double *h, double *d)
     return 0;
 }
 
+// Where the reductions' results land: page-locked host memory, written by the kernels.
+int TwoChannel::host_words()
+{
+    if (!out_ && cudaHostAlloc((void **)&out_, 2 * kMaxDiis * sizeof(double), cudaHostAllocPortable) != cudaSuccess) {
+        cudaGetLastError();
+        out_ = nullptr;
+        return set_last_error(UEGCCD_ERR_ALLOC, "no page-locked host memory");
+    }
+    if (!evo_) TCU(cudaEventCreateWithFlags(&evo_, cudaEventDisableTiming));
+    return 0;
+}
+
+// The reductions of the kernels before note_out(), which left them in host memory.
+int TwoChannel::note_out()
+{
+    TCU(cudaEventRecord(evo_, st_));
+    return 0;
+}
+
 int TwoChannel::read_out(int k, double *h)
 {
-    TCU(cudaMemcpyAsync(h, out_, k * sizeof(double), cudaMemcpyDeviceToHost, st_));
-    TCU(cudaStreamSynchronize(st_));
+    TCU(cudaEventSynchronize(evo_));
+    TCU(cudaGetLastError());
+    for (int q = 0; q < k; q++) h[q] = ((volatile double *)out_)[q];
     return 0;
 }
 
@@ -1058,6 +1080,10 @@ int TwoChannel::solve(const UegccdOptions &opt, bool drpa, const std::vector<dou
         k2_stats<false><<<nblk_, kThreads, 0, st_>>>(D, 0.0, t_[0], t_[1], nullptr, nullptr, part_);
     k2_finish<<<1, kThreads, 0, st_>>>(part_, nblk_, out_);
     launches_ += 2;
+    // The residual of the new amplitudes is queued before the host waits for their energy and dT: it
+    // is the next iteration's, or the final one.  Only an extrapolation that is due comes before it.
+    bool fresh = true;
+    if ((rc = note_out()) || (rc = residual(drpa, mask))) return rc;
     double o[2];
     if ((rc = read_out(2, o))) return rc;
     double dt = o[0], e = o[1];
@@ -1093,7 +1119,7 @@ int TwoChannel::solve(const UegccdOptions &opt, bool drpa, const std::vector<dou
                 launches_++;
             }
         }
-        if ((rc = residual(drpa, mask))) return rc;
+        if (!fresh && (rc = residual(drpa, mask))) return rc;
         const int slot = nd > 0 ? pushed % nd : 0;
         double *rab = nd > 0 ? hr_[0] + (int64_t)slot * n_ : nullptr;
         double *rba = nd > 0 && !drpa ? hr_[1] + (int64_t)slot * n_ : nullptr;
@@ -1111,6 +1137,8 @@ int TwoChannel::solve(const UegccdOptions &opt, bool drpa, const std::vector<dou
             k2_dots_finish<<<1, kThreads, 0, st_>>>(part_ + 2 * nblk_, nb, nd, out_ + 2);
             launches_ += 2;
         }
+        fresh = nd == 0 || niter + 1 < nd + 5 || pushed + 1 < nd;
+        if ((rc = note_out()) || (fresh && (rc = residual(drpa, mask)))) return rc;
         double ob[2 + kMaxDiis];
         if ((rc = read_out(2 + nd, ob))) return rc;
         dt = ob[0];
@@ -1124,14 +1152,14 @@ int TwoChannel::solve(const UegccdOptions &opt, bool drpa, const std::vector<dou
     }
     if (status == 0 && (!std::isfinite(dt) || !std::isfinite(e))) status = UEGCCD_ERR_NUMERIC;
     // the final residual (CCD.f90:103-107; dRPA.f90:98-101)
-    if ((rc = residual(drpa, mask))) return rc;
+    if (!fresh && (rc = residual(drpa, mask))) return rc;
     if (drpa)
         k2_stats<true><<<nblk_, kThreads, 0, st_>>>(D, 1.0, t_[0], t_[1], g_[0], g_[1], part_);
     else
         k2_stats<false><<<nblk_, kThreads, 0, st_>>>(D, 0.0, t_[0], t_[1], g_[0], g_[1], part_);
     k2_finish<<<1, kThreads, 0, st_>>>(part_, nblk_, out_);
     launches_ += 2;
-    if ((rc = read_out(2, o))) return rc;
+    if ((rc = note_out()) || (rc = read_out(2, o))) return rc;
     const double maxres = o[0];
     TCU(cudaEventRecord(ev1_, st_));
     TCU(cudaEventSynchronize(ev1_));

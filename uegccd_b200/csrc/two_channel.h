@@ -80,12 +80,12 @@ private:
     double *h_[2] = {nullptr, nullptr};          // hole-hole intermediates, O^3 each
     double *r_[3] = {nullptr, nullptr, nullptr}; // quadratic ring intermediates, O*O*V each
     double *x_[3] = {nullptr, nullptr, nullptr}; // quadratic crossed-ring intermediates
-    double *part_ = nullptr, *out_ = nullptr;    // reduction partials and results
+    double *part_ = nullptr, *out_ = nullptr;    // reduction partials; results, in host memory
     int nblk_ = 0;
     // DIIS history (T after the update, R of the amplitudes before it), per channel
     int ndiis_cap_ = 0;
     double *ht_[2] = {nullptr, nullptr}, *hr_[2] = {nullptr, nullptr};
-    cudaEvent_t ev0_ = nullptr, ev1_ = nullptr;
+    cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, evo_ = nullptr;
     int launches_ = 0;
     // the residual as matrix products (two_channel_mm.cu): device arrays on the first CCD residual
     // that can take that form; mm_state_ 0 not tried, 1 ready, -1 not for this system
@@ -100,6 +100,8 @@ private:
     int alloc(void **p, size_t bytes);
     int upload_t(const double *h, double *d);
     int residual(bool drpa, int mask);
+    int host_words();
+    int note_out();
     int read_out(int k, double *h);
     int diis_alloc(int ndiis);
     bool mm_ready();
