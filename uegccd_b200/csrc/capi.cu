@@ -1227,6 +1227,7 @@ int mixed_alloc(UegccdBatch &b)
         uint16_t *w = nullptr, *dd = nullptr;
         if ((rc = b.alloc(w, (size_t)d.w16_n))) return rc;
         if ((rc = b.alloc(dd, (size_t)d.d16_n))) return rc;
+        CU(cudaMemsetAsync(dd, 0, (size_t)d.d16_n * sizeof(uint16_t), b.stream));   // the tiles' padding
         if ((rc = b.alloc(d.dscale, (size_t)d.nscale))) return rc;
         d.w16 = w;
         d.d16 = dd;

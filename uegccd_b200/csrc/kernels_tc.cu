@@ -183,50 +183,52 @@ __global__ void __launch_bounds__(128) k_w16_build(const WSlabDev *__restrict__ 
     }
 }
 
-// Scaled FP16 d = t - t_ref of one row tile: the scale of row p is max_c |d[p][c]| (1 if
-// zero); chunk ch holds B[n][k] = d[p0 + n][32 ch + k] / scale, in the canonical layout.
-__global__ void __launch_bounds__(128) k_delta16(const DTileDev *__restrict__ dt,
+// Scaled FP16 d = t - t_ref of the rows i <= j of one row tile: the scale of row p is
+// max_c |d[p][c]| (1 if zero); chunk ch holds B[n][k] = d[p0 + n][32 ch + k] / scale, in the
+// canonical layout.  The tile's padding, rows and columns, is zero from the start.  A warp has a row:
+// its d, up to kHeld columns of them, stay in registers between the maximum and the division, so
+// that t and t_ref are read once.  Bound by those reads.  Per launch, 100 twists of N=54 (485 plane
+// waves): 204 -> 72 us (every padded row, t and t_ref twice, a division of the index an element).
+__global__ void __launch_bounds__(128, 8) k_delta16(const DTileDev *__restrict__ dt,
                                                 const BlockDev *__restrict__ blocks,
                                                 const double *__restrict__ t, const double *__restrict__ t_ref,
                                                 __half *__restrict__ d16, float *__restrict__ dscale,
                                                 const uint8_t *__restrict__ active)
 {
-    __shared__ float rs[64];
+    constexpr int kHeldChunks = 16, kHeld = kHeldChunks * kTcK;
     const DTileDev D = dt[blockIdx.x];
     const BlockDev B = blocks[D.blk];
     if (!active[B.solve]) return;
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31, v = B.v, o = B.o, np = D.np;
-    for (int pp = warp; pp < np; pp += 4) {
-        const int p = D.p0 + pp;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, v = B.v, np = D.np;
+    const int nr = min(np, B.nd + B.dg - D.p0);
+    for (int pp = warp; pp < nr; pp += 4) {
+        const double *x = t + B.t0 + (int64_t)(D.p0 + pp) * v, *y = t_ref + B.t0 + (int64_t)(D.p0 + pp) * v;
+        double d[kHeldChunks];
         float m = 0.f;
-        if (p < o)
-            for (int c = lane; c < v; c += 32) {
-                const int64_t idx = B.t0 + (int64_t)p * v + c;
-                m = fmaxf(m, fabsf((float)(t[idx] - t_ref[idx])));
-            }
+#pragma unroll
+        for (int q = 0; q < kHeldChunks; q++) {
+            const int c = q * kTcK + lane;
+            d[q] = c < v ? x[c] - y[c] : 0.0;
+            m = fmaxf(m, fabsf((float)d[q]));
+        }
+        for (int c = kHeld + lane; c < v; c += 32) m = fmaxf(m, fabsf((float)(x[c] - y[c])));
         for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
-        if (lane == 0) {
-            rs[pp] = m > 0.f ? m : 1.f;
-            dscale[D.soff + pp] = rs[pp];
-        }
-    }
-    __syncthreads();
-    const int nch = (v + kTcK - 1) / kTcK;
-    for (int e = tid; e < nch * np * kTcK; e += blockDim.x) {
-        const int ch = e / (np * kTcK), r = e - ch * (np * kTcK);
-        const int pp = r / kTcK, k = r - pp * kTcK;
-        const int p = D.p0 + pp, c = ch * kTcK + k;
-        float x = 0.f;
-        if (p < o && c < v) {
-            const int64_t idx = B.t0 + (int64_t)p * v + c;
-            x = (float)((t[idx] - t_ref[idx]) / (double)rs[pp]);
-        }
-        d16[D.doff + (int64_t)ch * np * kTcK + cm_off(pp, k)] = __float2half_rn(x);
+        const float rs = m > 0.f ? m : 1.f;
+        if (lane == 0) dscale[D.soff + pp] = rs;
+        __half *dst = d16 + D.doff + cm_off(pp, lane);
+#pragma unroll
+        for (int q = 0; q < kHeldChunks; q++)
+            if (q * kTcK + lane < v) dst[q * np * kTcK] = __float2half_rn((float)(d[q] / (double)rs));
+        for (int c = kHeld + lane; c < v; c += 32)
+            dst[(int64_t)(c / kTcK) * np * kTcK] = __float2half_rn((float)((x[c] - y[c]) / (double)rs));
     }
 }
 
 // One CTA per (block, 128-virtual tile).  g[...] += g_ref[...] + sum_c v(a-c) (t - t_ref)[p][c]
-// for every (p, a) of the tile (g already holds the hole-hole part).
+// for every (p, a) of the tile with p a row i <= j (g already holds the hole-hole part; the update
+// reads those rows only).  Bound by the reads of the Coulomb slabs, of which a tile fetches the
+// eight-row groups it has: per launch, 100 twists of N=54, 474 -> 430 us (the mirrors' rows
+// of g and g_ref too, and 128 rows of every slab).
 template <int NP>
 __global__ void __launch_bounds__(128) k_ladder_tc(const LadderTile *__restrict__ tiles,
                                                   const TcTileDev *__restrict__ tcx,
@@ -250,7 +252,7 @@ __global__ void __launch_bounds__(128) k_ladder_tc(const LadderTile *__restrict_
     const BlockDev B = blocks[T.blk];
     if (!active[B.solve]) return;
     const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    const int v = B.v, o = B.o;
+    const int v = B.v, o = B.nd + B.dg;
 
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_base)),
@@ -274,14 +276,17 @@ __global__ void __launch_bounds__(128) k_ladder_tc(const LadderTile *__restrict_
     const int nchunks = (v + kTcK - 1) / kTcK;
     bool ok = true;
     if (tid == 0) {
-        // chunk c of the Coulomb slab (8 KB) and of the d tile (NP x 64 B) into stage c % kStages:
+        // chunk c of the Coulomb slab (up to 8 KB) and of the d tile (NP x 64 B) into stage c % kStages:
         // one bulk copy each, both completing on full[stage]
-        constexpr uint32_t kWBytes = kTcM * kTcK * 2, kDBytes = NP * kTcK * 2;
+        // (a slab's eight-row groups are 512 bytes apart; what the last tile of a block leaves of
+        // the stage enters accumulator rows that nothing reads)
+        constexpr uint32_t kDBytes = NP * kTcK * 2;
+        const uint32_t wbytes = (uint32_t)(min(kTcM, v - T.a0) + 7) / 8 * (8 * kTcK * 2);
         int issued = 0;
         auto issue = [&](int c) {
             const int b = c % kStages;
-            mbar_expect_tx(&full[b], kWBytes + kDBytes);
-            bulk_g2s(&As[b][0], w16 + X.woff + (int64_t)c * kTcM * kTcK, kWBytes, &full[b]);
+            mbar_expect_tx(&full[b], wbytes + kDBytes);
+            bulk_g2s(&As[b][0], w16 + X.woff + (int64_t)c * kTcM * kTcK, wbytes, &full[b]);
             bulk_g2s(&Bs[b][0], d16 + X.doff + (int64_t)c * NP * kTcK, kDBytes, &full[b]);
             issued = c + 1;
         };
