@@ -109,10 +109,10 @@ def _measured_peaks():
 
 HBM_PEAK, BF16_PEAK = _measured_peaks()
 # DRAM bytes of one launch per solve: dram__bytes_read.sum + dram__bytes_write.sum of every class
-# launch of one residual, from one ncu capture of the 100-twist batch itself (a one-pass
-# metric set), divided by the 100 solves of a launch.
-TRAFFIC_PER_SOLVE = {"k_ladder": 193.4e6 / 100, "k_ladder_hh": 101.5e6 / 100, "k_mosaic_blk": 116.7e6 / 100,
-                     "k_rings": 310.0e6 / 100, "k_ring_stage": 496.8e6 / 100, "k_update": 968.7e6 / 100}
+# launch of one residual, from one ncu capture of a 100-twist N=54 batch (a one-pass metric
+# set), divided by the 100 solves of a launch.
+TRAFFIC_PER_SOLVE = {"k_ladder": 121.2e6 / 100, "k_mosaic_blk": 111.6e6 / 100, "k_rings": 301.1e6 / 100,
+                     "k_ring_stage": 506.3e6 / 100, "k_update": 766.3e6 / 100}
 
 
 def twists(n: int, seed: int = SEED, rank: int = 0):
@@ -280,9 +280,9 @@ def kernel_units(st):
     A = st["A"]
     ndiis = SOLVE_OPTS["ndiis"]
     return {
-        # rows i <= j: pp ladder sum_c v(a-c) t(p,c) and hole-hole apply sum_q H(p,q) t(q,a)
-        "k_ladder": ("flop", 2 * (st["ov2_half"] + st["o2v_half"])),
-        "k_ladder_hh": ("flop", 2 * st["o2v_half"]),
+        # rows i <= j: pp ladder sum_c v(a-c) t(p,c), the hole-hole intermediate sum_c v t and its
+        # apply sum_q H(p,q) t(q,a), both forms of the kernel
+        "k_ladder": ("flop", 2 * (st["ov2_half"] + 2 * st["o2v_half"])),
         # pp ladder on the tensor cores (FP16 operands)
         "k_ladder_tc": ("tflop16", 2 * st["ov2"]),
         # per {Q, -Q} group pair, n1 <= n2 rows: X W and Y W of the smaller group, 4 n1^2 n2,
@@ -294,10 +294,9 @@ def kernel_units(st):
         # the particle-hole copy: every amplitude read once through a 4-byte index and written
         # once (the pairs' X1 and Y1 hold A entries between them)
         "k_ring_stage": ("byte", (8 + 4 + 8) * A),
-        # every amplitude: the mirror index (4 B); the amplitudes i <= j: t, the ladder G and the
-        # two ring G, the Pulay push (t' FP64 and e FP32 to the history) and the other ndiis - 1
-        # error vectors (FP32)
-        "k_update": ("byte", 4 * A + (4 * 8 + 8 + 4 + (ndiis - 1) * 4) * st["A_half"]),
+        # the amplitudes i <= j: t, the ladder G and the two ring G with 4 bytes of their places, the
+        # Pulay push (t' FP64 and e FP32 to the history) and the other ndiis - 1 error vectors (FP32)
+        "k_update": ("byte", (4 * 8 + 4 + 8 + 4 + (ndiis - 1) * 4) * st["A_half"]),
     }
 
 
@@ -376,7 +375,7 @@ def run_gpu(args, rank, world):
         batch.solve(**opts)
     stats = batch.kernel_stats()
     batch.set_profiling(False)
-    ring_threads = batch.launch_shapes()  # the tuner's picks, from the first CCD solve
+    ring_threads = batch.launch_shapes()  # the staging size is the tuner's pick
     fp64_peak = probe_fp64_peak()           # the FP64 tensor-core roofline denominator, measured
     niters = [r["niter"] for r in res]
     fails = sum(r["fail"] for r in res)
@@ -653,7 +652,7 @@ def main(argv=None):
     tr = TRAFFIC_PER_SOLVE.get(top)
     roof["traffic"] = tr * nsys if tr else None
     flops_pp = sum(ps["ov2_half"] * 2 for ps in per_solve) / len(per_solve) * nsys
-    config["launch_shapes"] = g["ring_threads"]   # picked by the launch-shape tuner on the batch
+    config["launch_shapes"] = g["ring_threads"]   # (the staging size timed on the batch)
     if args.precision == "mixed":
         config["precision"] = "particle-particle ladder FP16 tensor cores (FP32 accumulate), rest FP64"
     line = {"metric": metric, "value": g["value"], "unit": "solves/s", "n_gpus": world, "steps": args.steps,

@@ -314,17 +314,15 @@ int uegccd_trim_cache(void);
 int uegccd_batch_history(UegccdBatch *b, int32_t s, double *energies, double *dts, int32_t max_rec,
                          int32_t *n_recorded);
 
-/* CTA sizes of the ring kernel's pair classes (by padded pair size: <= 16, 32, 48 rows,
- * larger), as the launch-shape tuner picked them on the batch's first CCD solve (timed
- * on the batch itself, once per batch shape in a process; the CTA size leaves every
- * result bitwise the same).  Writes at most max values; returns how many. */
+/* CTA sizes of the ring kernel's pair classes: up to 256 threads each, the same for every batch
+ * (eight, four or two small pairs, or one large one, a CTA).  Writes at most max values; returns
+ * how many. */
 int32_t uegccd_batch_ring_threads(UegccdBatch *b, int32_t *threads, int32_t max);
-/* Every launch shape the tuner picked on the batch's first CCD solve (new; the reference has
- * no launches): the four ring CTA sizes above, the CTA size of the ring staging kernel (64,
- * 128 or 256), the ladder tile order (0: block order, 1: the blocks with the most virtuals
- * first, within each row-tile class), and the column chunk of the hole-hole intermediate (64
- * or 32 virtuals per shared-memory stage).  None changes a result.  Writes at most max values;
- * returns how many. */
+/* The launch shapes of a batch (new; the reference has no launches): the four ring CTA sizes
+ * above, the CTA size of the ring staging kernel (64, 128 or 256: picked by timing on the batch's
+ * first CCD solve, once per batch shape in a process), the ladder tile order (1: the longest
+ * first) and the column chunk of the ladder on the FP64 tensor cores (32 virtuals per stage).  None changes a
+ * result.  Writes at most max values; returns how many. */
 int32_t uegccd_batch_launch_shapes(UegccdBatch *b, int32_t *vals, int32_t max);
 
 /* Live kernel timing: when on, every kernel of a batch solve is bracketed by CUDA

@@ -1363,9 +1363,9 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
 // ladders also run beside the FMA ladders; in a large one each kernel fills the GPU, and run
 // together they contend for the SMs and L2.  Solve times in ms on one stream, with the ring classes
 // apart, with the terms apart: one N=54 system 1.50, 1.2, 0.93; 8 of them 2.72, 2.53, 2.13;
-// 32 (11 M amplitudes) 6.76, 6.37, 6.30; 48 (16 M) 8.70 and 9.16 apart; 100 (33 M) 17.02, 16.47,
-// 18.46; four N=114 systems (13 M) 11.8, 10.7, 9.7; 8 of them (26 M) 20.9, 18.8, 17.9; 16 of them
-// (51 M) 36.0, 34.2, 34.3.
+// 32 (7 M packed amplitudes) 6.76, 6.37, 6.30; 48 (10.5 M) 8.70 and 9.16 apart; 100 (22 M) 17.02,
+// 16.47, 18.46; four N=114 systems (8.5 M) 11.8, 10.7, 9.7; 8 of them (17 M) 20.9, 18.8, 17.9; 16 of
+// them (34 M) 36.0, 34.2, 34.3.
 constexpr int64_t kForkAmps = 9000000;
 constexpr int kForkSolves = 8;
 const Fork *fork_of(UegccdBatch &b)

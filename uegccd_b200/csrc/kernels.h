@@ -94,7 +94,7 @@ struct DevBatch {
     int nritems[6] = {0, 0, 0, 0, 0, 0};
     size_t ring_smem[6] = {0, 0, 0, 0, 0, 0};
     int ring_doubles[6] = {0, 0, 0, 0, 0, 0};
-    int stage_threads = 128;                    // CTA size of k_ring_stage (tune_rings)
+    int stage_threads = 128;                    // CTA size of k_ring_stage (tune_stage)
 };
 // FP64 ladders (ladder.cu): blocks with at most kLadderFmaRows rows i <= j take the FMA form,
 // larger ones the DMMA form in tiles of at most kLadderMmaRows rows

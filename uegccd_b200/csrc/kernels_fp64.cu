@@ -1,4 +1,6 @@
-// kernels_fp64.cu -- FP64 kernels of the spin-adapted CCD / MP2 / dRPA residual.
+// kernels_fp64.cu -- the spin-adapted CCD / MP2 / dRPA iteration: mosaics, dRPA sums, the staging of the
+// rings, index tables, the iteration's tail and its launch order.  (The ladders are in ladder.cu, the rings
+// in rings.cu, the element-wise kernels in update.cu.)
 //
 // Storage (uegccd_internal.h): t(ij,a) = T2abab(i,j,a), block-packed by
 // K = n_i + n_j.  The reference's abba and aaaa channels are recovered from
