@@ -210,7 +210,9 @@ __global__ void __launch_bounds__(kMosThreads, 12) k_mosaic_blk(const BlockDev *
 // occupied k the first index of one row at most (l = K - k), so within a block the targets
 // are distinct and the block's entries go in at once.  mt_start[tbase[s] + y] is the first
 // entry of target y of solve s (entries from lbase[s] on); the last solve also writes the
-// end sentinel.  cnt: V + O ints of dynamic shared memory.
+// end sentinel.  cnt: V + O ints of dynamic shared memory.  Bound by the latency of the chain block ->
+// orbitals -> place, block after block: 30 twists of N=54, 197 -> 70 us with four blocks'
+// orbitals in flight and the places in shared memory.
 __global__ void k_mosaic_targets(const SolveDev *__restrict__ solves, const BlockDev *__restrict__ blocks,
                                  const int16_t *__restrict__ vir, const int16_t *__restrict__ pair_i,
                                  const int *__restrict__ tbase, const int64_t *__restrict__ lbase,
@@ -222,40 +224,69 @@ __global__ void k_mosaic_targets(const SolveDev *__restrict__ solves, const Bloc
     const int nt = S.V + S.O, t0 = tbase[sv];
     for (int y = threadIdx.x; y < nt; y += blockDim.x) cnt[y] = 0;
     __syncthreads();
-    for (int bi = 0; bi < S.nblk; bi++) {
-        const BlockDev B = blocks[S.blk0 + bi];
-        for (int c = threadIdx.x; c < B.v; c += blockDim.x) atomicAdd(&cnt[vir[B.vir0 + c] - S.O], 1);
-        for (int r = threadIdx.x; r < B.o; r += blockDim.x) atomicAdd(&cnt[S.V + pair_i[B.pair0 + r]], 1);
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+    for (int bi = warp; bi < S.nblk; bi += nw) {
+        const BlockDev &B = blocks[S.blk0 + bi];
+#pragma unroll 4
+        for (int c = lane; c < B.v; c += 32) atomicAdd(&cnt[vir[B.vir0 + c] - S.O], 1);
+        for (int r = lane; r < B.o; r += 32) atomicAdd(&cnt[S.V + pair_i[B.pair0 + r]], 1);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        int64_t run = lbase[sv];
-        for (int y = 0; y < nt; y++) {
-            mt_start[t0 + y] = (int32_t)run;
-            run += cnt[y];
-            cnt[y] = 0;
+    if (warp == 0) {   // cnt becomes the place of each target's next entry; a lane has a run of targets
+        const int per = (nt + 31) / 32, y0 = min(lane * per, nt), y1 = min(y0 + per, nt);
+        int sum = 0;
+        for (int y = y0; y < y1; y++) sum += cnt[y];
+        int run = sum;
+        for (int o = 1; o < 32; o <<= 1) {
+            const int x = __shfl_up_sync(0xffffffffu, run, o);
+            if (lane >= o) run += x;
         }
-        mt_start[t0 + nt] = (int32_t)run;   // the next solve's first entry, or the end sentinel
+        run += (int)lbase[sv] - sum;
+        for (int y = y0; y < y1; y++) {
+            const int k = cnt[y];
+            mt_start[t0 + y] = run;
+            cnt[y] = run;
+            run += k;
+        }
+        if (lane == 31) mt_start[t0 + nt] = run;   // the next solve's first entry, or the end sentinel
     }
     __syncthreads();
-    for (int bi = 0; bi < S.nblk; bi++) {
-        const BlockDev B = blocks[S.blk0 + bi];
-        for (int c = threadIdx.x; c < B.v; c += blockDim.x) {
-            const int y = vir[B.vir0 + c] - S.O;
-            mt_list[mt_start[t0 + y] + cnt[y]++] = (int32_t)(B.col0 + c);
+    // four blocks' orbitals are fetched together, then entered block by block
+    constexpr int kAhead = 4;
+    for (int b0 = 0; b0 < S.nblk; b0 += kAhead) {
+        int v[kAhead], o[kAhead], vir0[kAhead], col0[kAhead], row0[kAhead], y[kAhead], r[kAhead];
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            const bool in = b0 + k < S.nblk;
+            const BlockDev &B = blocks[S.blk0 + min(b0 + k, S.nblk - 1)];
+            v[k] = in ? B.v : 0;
+            o[k] = in ? B.o : 0;
+            vir0[k] = B.vir0;
+            col0[k] = (int)B.col0;
+            row0[k] = (int)B.row0;
+            r[k] = B.pair0;
         }
-        for (int r = threadIdx.x; r < B.o; r += blockDim.x) {
-            const int y = S.V + pair_i[B.pair0 + r];
-            mt_list[mt_start[t0 + y] + cnt[y]++] = (int32_t)(B.row0 + r);
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            y[k] = (int)threadIdx.x < v[k] ? vir[vir0[k] + threadIdx.x] - S.O : 0;
+            r[k] = (int)threadIdx.x < o[k] ? S.V + pair_i[r[k] + threadIdx.x] : 0;   // o <= 64 threads
         }
-        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kAhead; k++) {
+            for (int c = threadIdx.x; c < v[k]; c += blockDim.x) {
+                const int z = c == (int)threadIdx.x ? y[k] : vir[vir0[k] + c] - S.O;
+                mt_list[cnt[z]++] = col0[k] + c;
+            }
+            if ((int)threadIdx.x < o[k]) mt_list[cnt[r[k]]++] = row0[k] + (int)threadIdx.x;
+            __syncthreads();
+        }
     }
 }
 
 void launch_mosaic_targets(const DevBatch &d, const int *tbase, const int64_t *lbase, size_t smem, cudaStream_t st)
 {
     if (smem > 48 * 1024) cudaFuncSetAttribute(k_mosaic_targets, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_mosaic_targets<<<d.nsolves, 256, smem, st>>>(d.solves, d.blocks, d.vir, d.pair_i, tbase, lbase, d.mt_start,
+    k_mosaic_targets<<<d.nsolves, 512, smem, st>>>(d.solves, d.blocks, d.vir, d.pair_i, tbase, lbase, d.mt_start,
                                                    d.mt_list);
 }
 
