@@ -170,9 +170,11 @@ struct DevChunk {
     size_t size;
     int dev;
 };
-// Page-locked host memory for downloads, in buffers that outlive the calls (portable: page-locked
-// for every device's context): a call takes one, any number of threads theirs, and gives it back;
-// up to kPinnedCap bytes stay for the next call, until uegccd_trim_cache.
+// Page-locked host memory (portable: page-locked for every device's context).  Downloads take
+// buffers that outlive the calls: any number of threads theirs, given back for the next call, until
+// uegccd_trim_cache.  At most kPinnedCap bytes are locked at a time, idle or in use; past that a
+// call goes on without one.  A buffer of more than about twice the size asked for stays where it
+// is: a large one would be out of reach of the downloads it was made for.
 constexpr size_t kPinnedCap = 512ull << 20;
 constexpr size_t kPinnedMin = 64ull << 10;
 struct PinnedBuf {
@@ -180,56 +182,128 @@ struct PinnedBuf {
     size_t bytes = 0;
 };
 std::mutex g_pinned_mu;
-std::vector<PinnedBuf> g_pinned;
-size_t g_pinned_bytes = 0;
+std::vector<PinnedBuf> g_pinned;   // idle, the longest idle first
+size_t g_pinned_bytes = 0;         // locked, idle or in use
 
-// At least `bytes` (p = nullptr when the host has no more to lock).
+char *lock_host(size_t bytes)
+{
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, bytes, cudaHostAllocPortable) == cudaSuccess) return (char *)p;
+    cudaGetLastError();
+    return nullptr;
+}
+
+// At least `bytes` > 0 (p = nullptr: past the cap, or the host has no more to lock).
 PinnedBuf pinned_get(size_t bytes)
 {
-    bytes = std::max(bytes, kPinnedMin);
+    PinnedBuf b;
+    b.bytes = (bytes + kPinnedMin - 1) / kPinnedMin * kPinnedMin;
+    std::vector<PinnedBuf> drop;
     {
         std::lock_guard<std::mutex> lock(g_pinned_mu);
         int best = -1;
         for (size_t k = 0; k < g_pinned.size(); k++)
-            if (g_pinned[k].bytes >= bytes && (best < 0 || g_pinned[k].bytes < g_pinned[best].bytes)) best = (int)k;
+            if (g_pinned[k].bytes >= bytes && g_pinned[k].bytes <= 2 * b.bytes &&
+                (best < 0 || g_pinned[k].bytes < g_pinned[best].bytes))
+                best = (int)k;
         if (best >= 0) {
-            const PinnedBuf b = g_pinned[best];
-            g_pinned_bytes -= b.bytes;
+            b = g_pinned[best];
             g_pinned.erase(g_pinned.begin() + best);
             return b;
         }
+        while (g_pinned_bytes + b.bytes > kPinnedCap && !g_pinned.empty()) {   // idle ones make room
+            drop.push_back(g_pinned.front());
+            g_pinned_bytes -= g_pinned.front().bytes;
+            g_pinned.erase(g_pinned.begin());
+        }
+        if (g_pinned_bytes + b.bytes > kPinnedCap) b.bytes = 0;
+        g_pinned_bytes += b.bytes;
     }
-    PinnedBuf b;
-    if (cudaHostAlloc((void **)&b.p, bytes, cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        b.p = nullptr;
-        return b;
-    }
-    b.bytes = bytes;
-    return b;
+    for (auto &x : drop) cudaFreeHost(x.p);
+    if (b.bytes == 0 || (b.p = lock_host(b.bytes))) return b;
+    std::lock_guard<std::mutex> lock(g_pinned_mu);
+    g_pinned_bytes -= b.bytes;
+    return PinnedBuf{};
 }
 
 void pinned_put(const PinnedBuf &b)
 {
     if (!b.p) return;
-    {
-        std::lock_guard<std::mutex> lock(g_pinned_mu);
-        if (g_pinned_bytes + b.bytes <= kPinnedCap) {
-            g_pinned.push_back(b);
-            g_pinned_bytes += b.bytes;
-            return;
-        }
-    }
-    cudaFreeHost(b.p);
+    std::lock_guard<std::mutex> lock(g_pinned_mu);
+    g_pinned.push_back(b);
 }
 
+// A buffer of one call, none for 0 bytes.  A call that returns early with copies in flight waits
+// for them before another may have it.
 struct PinnedScope {
     PinnedBuf b;
-    explicit PinnedScope(size_t bytes) : b(pinned_get(bytes)) {}
-    ~PinnedScope() { pinned_put(b); }
+    cudaStream_t st;
+    bool settled = false;   // no copy in flight
+    PinnedScope(size_t bytes, cudaStream_t stream) : st(stream)
+    {
+        if (bytes > 0) b = pinned_get(bytes);
+    }
+    ~PinnedScope()
+    {
+        if (b.p && !settled) cudaStreamSynchronize(st);
+        pinned_put(b);
+    }
     PinnedScope(const PinnedScope &) = delete;
     PinnedScope &operator=(const PinnedScope &) = delete;
 };
+
+// Page-locked words an object keeps for its life (the flag of an iteration, small reads): kWords
+// bytes each, cut from slabs of their own.
+constexpr size_t kWords = 4096, kSlab = 64ull << 10;
+constexpr size_t kFlagBytes = 64;   // of a batch's words, for CtlBuffers::done
+std::vector<char *> g_slabs, g_words;   // slabs, and their free pieces (under g_pinned_mu)
+
+char *words_get()
+{
+    std::lock_guard<std::mutex> lock(g_pinned_mu);
+    if (g_words.empty()) {
+        char *s = lock_host(kSlab);
+        if (!s) return nullptr;
+        g_slabs.push_back(s);
+        for (size_t k = kSlab; k > 0; k -= kWords) g_words.push_back(s + k - kWords);
+    }
+    char *p = g_words.back();
+    g_words.pop_back();
+    return p;
+}
+
+void words_put(char *p)
+{
+    if (!p) return;
+    std::lock_guard<std::mutex> lock(g_pinned_mu);
+    g_words.push_back(p);
+}
+
+// The idle buffers and the slabs nothing uses, back to the host.
+void pinned_trim()
+{
+    std::vector<char *> drop;
+    {
+        std::lock_guard<std::mutex> lock(g_pinned_mu);
+        for (auto &b : g_pinned) {
+            drop.push_back(b.p);
+            g_pinned_bytes -= b.bytes;
+        }
+        g_pinned.clear();
+        for (size_t k = 0; k < g_slabs.size();) {
+            char *s = g_slabs[k];
+            auto in = [s](char *w) { return w >= s && w < s + kSlab; };
+            if (std::count_if(g_words.begin(), g_words.end(), in) < (int)(kSlab / kWords)) {
+                k++;
+                continue;
+            }
+            g_words.erase(std::remove_if(g_words.begin(), g_words.end(), in), g_words.end());
+            g_slabs.erase(g_slabs.begin() + k);
+            drop.push_back(s);
+        }
+    }
+    for (char *p : drop) cudaFreeHost(p);
+}
 
 bool is_pinned(const void *p)
 {
@@ -367,8 +441,8 @@ struct UegccdBatch {
     std::vector<DevChunk> big;       // chunks of one large array each
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_solve0 = nullptr, ev_solve1 = nullptr;
-    PinnedBuf pin;                   // page-locked words the small reads land in (on first use)
-    PinnedBuf flag;                  // CtlBuffers::done (with the control buffers)
+    char *words = nullptr;           // page-locked words (on first use): CtlBuffers::done, then small reads
+    PinnedBuf pin;                   // where small reads land that the words do not hold
     cudaEvent_t ev_iter[2] = {nullptr, nullptr};            // the two latest iterations
     cudaEvent_t ev_copy[3] = {nullptr, nullptr, nullptr};   // arrays of a download (on first use)
     Fork fork;                       // side streams of a small batch's residual (on first use)
@@ -451,7 +525,7 @@ struct UegccdBatch {
         if (ev_solve0) cudaEventDestroy(ev_solve0);
         if (ev_solve1) cudaEventDestroy(ev_solve1);
         pinned_put(pin);
-        pinned_put(flag);
+        words_put(words);
         for (auto &e : ev_iter)
             if (e) cudaEventDestroy(e);
         for (auto &e : ev_copy)
@@ -1047,6 +1121,10 @@ int set_active_all(UegccdBatch &b, uint8_t v)
 // kernels before it; the caller's own memory when there is none.
 void *small_read(UegccdBatch &b, void *own, size_t bytes)
 {
+    if (bytes <= kWords - kFlagBytes) {
+        if (!b.words) b.words = words_get();
+        return b.words ? b.words + kFlagBytes : own;
+    }
     if (b.pin.bytes < bytes) {
         pinned_put(b.pin);
         b.pin = pinned_get(bytes);
@@ -1110,37 +1188,37 @@ int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, doubl
     CU(cudaGetLastError());
     b.d2h_bytes += (int64_t)(m * bytes);
     const size_t red = with_red ? b.red.size() * sizeof(double) : 0;
-    if (red) b.d2h_bytes += (int64_t)red;
+    void *sums = red ? small_read(b, b.red.data(), red) : nullptr;
+    if (red) {
+        CU(cudaMemcpyAsync(sums, b.d.red, red, cudaMemcpyDeviceToHost, b.stream));
+        b.d2h_bytes += (int64_t)red;
+    }
     constexpr size_t kAloneMax = 24ull << 20;
     bool direct = true;   // page-locked destinations take the copies themselves
     for (int k = 0; k < m; k++) direct = direct && is_pinned(host[k]);
     direct = direct || (m == 1 && bytes > kAloneMax);
-    PinnedScope buf(direct ? red : red + m * bytes);
-    if (!buf.b.p || direct) {
+    PinnedScope buf(direct ? 0 : m * bytes, b.stream);
+    const bool apart = bytes >= (512 << 10);
+    if (!buf.b.p) {
         for (int k = 0; k < m; k++)
             CU(cudaMemcpyAsync(host[k], b.dense + k * n, bytes, cudaMemcpyDeviceToHost, b.stream));
-        if (red) CU(cudaMemcpyAsync(b.red.data(), b.d.red, red, cudaMemcpyDeviceToHost, b.stream));
         CU(cudaStreamSynchronize(b.stream));
-        return 0;
-    }
-    char *arrays = buf.b.p + red;
-    if (red) CU(cudaMemcpyAsync(buf.b.p, b.d.red, red, cudaMemcpyDeviceToHost, b.stream));
-    const bool apart = bytes >= (512 << 10);
-    if (apart) {
+    } else if (apart) {
         for (int k = 0; k < m; k++) {
             if (!b.ev_copy[k]) CU(cudaEventCreateWithFlags(&b.ev_copy[k], cudaEventDisableTiming));
-            CU(cudaMemcpyAsync(arrays + k * bytes, b.dense + k * n, bytes, cudaMemcpyDeviceToHost, b.stream));
+            CU(cudaMemcpyAsync(buf.b.p + k * bytes, b.dense + k * n, bytes, cudaMemcpyDeviceToHost, b.stream));
             CU(cudaEventRecord(b.ev_copy[k], b.stream));
         }
     } else {
-        CU(cudaMemcpyAsync(arrays, b.dense, m * bytes, cudaMemcpyDeviceToHost, b.stream));
+        CU(cudaMemcpyAsync(buf.b.p, b.dense, m * bytes, cudaMemcpyDeviceToHost, b.stream));
         CU(cudaStreamSynchronize(b.stream));
     }
-    for (int k = 0; k < m; k++) {
+    for (int k = 0; buf.b.p && k < m; k++) {
         if (apart) CU(cudaEventSynchronize(b.ev_copy[k]));
-        host_copy((char *)host[k], arrays + k * bytes, bytes, m * bytes > 2 * kCoresMin);
+        host_copy((char *)host[k], buf.b.p + k * bytes, bytes, m * bytes > 2 * kCoresMin);
     }
-    if (red) std::memcpy(b.red.data(), buf.b.p, red);
+    buf.settled = true;
+    if (red && sums != b.red.data()) std::memcpy(b.red.data(), sums, red);
     return 0;
 }
 
@@ -1314,9 +1392,8 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
     const int n = b.d.nsolves;
     int rc = 0;
     if (!c.done) {
-        b.flag = pinned_get(sizeof(int));
-        if (!b.flag.p) return fail(UEGCCD_ERR_ALLOC, "no page-locked host memory");
-        c.done = reinterpret_cast<int *>(b.flag.p);
+        if (!b.words && !(b.words = words_get())) return fail(UEGCCD_ERR_ALLOC, "no page-locked host memory");
+        c.done = reinterpret_cast<int *>(b.words);
         for (auto &e : b.ev_iter) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     if (!c.state) {
@@ -2384,14 +2461,15 @@ int uegccd_batch_get_all_amplitudes(UegccdBatch *b, double *t_abab)
     // a page-locked destination takes the copy directly; else through page-locked memory, copied
     // out on all host cores (a pageable copy is staged by the driver on one thread)
     const bool direct = is_pinned(t_abab);
-    PinnedScope buf(direct ? 0 : bytes);
-    if (direct || !buf.b.p) {
+    PinnedScope buf(direct ? 0 : bytes, b->stream);
+    if (!buf.b.p) {
         CU(cudaMemcpyAsync(t_abab, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
         CU(cudaStreamSynchronize(b->stream));
         return UEGCCD_OK;
     }
     CU(cudaMemcpyAsync(buf.b.p, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
     CU(cudaStreamSynchronize(b->stream));
+    buf.settled = true;
     host_copy((char *)t_abab, buf.b.p, bytes, bytes >= kCoresMin);
     return UEGCCD_OK;
 }
@@ -2427,13 +2505,7 @@ int uegccd_batch_structure_factor(UegccdBatch *b, int32_t s, const UegccdSfGrid 
 
 int uegccd_trim_cache(void)
 {
-    std::vector<PinnedBuf> unlock;
-    {
-        std::lock_guard<std::mutex> lock(g_pinned_mu);
-        unlock.swap(g_pinned);
-        g_pinned_bytes = 0;
-    }
-    for (auto &b : unlock) cudaFreeHost(b.p);
+    pinned_trim();
     std::vector<DevChunk> drop;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
