@@ -44,3 +44,71 @@ def test_live_contexts_hold_no_download_buffer():
     assert _locked() - base <= arrays + SLACK, ((_locked() - base) / MB, arrays / MB)
     _capi.trim_cache()
     assert _locked() - base <= SLACK, (_locked() - base) / MB
+
+
+def _host_allocs(call):
+    """How often a call locks host memory anew."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    torch.cuda.init()
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        call()
+    counts = {e.key: e.count for e in p.key_averages()}
+    assert "cudaMemcpyAsync" in counts   # the profile saw the call
+    return counts.get("cudaHostAlloc", 0)
+
+
+@pytest.mark.parametrize("count,electrons,basis", [(2, 14, 60), (30, 54, 485), (22, 114, 1140)])
+def test_batch_downloads_into_ordinary_memory(count, electrons, basis):
+    """Into a new array: 0.04 MB, 80 MB (three pieces) and 590 MB (more than is kept locked).  A
+    second download locks nothing, and both have the values of the solves one by one."""
+    from uegccd_b200 import Batch, _capi
+
+    b = Batch(_systems(count, electrons, basis))
+    b.mp2()
+    _capi.trim_cache()
+    base = _locked()
+    first = b.all_amplitudes()
+    kept = _locked() - base
+    assert kept <= 96 * MB + SLACK, kept / MB
+    got = []
+    assert _host_allocs(lambda: got.append(b.all_amplitudes())) == 0
+    for s in range(b.n):
+        want = b.amplitudes(s)
+        np.testing.assert_array_equal(first[s], want)
+        np.testing.assert_array_equal(got[0][s], want)
+    b.close()
+
+
+def test_many_threads_download_at_once():
+    """Eight threads with three arrays of 28 MB each ask for more than may be locked (8 x 84 MB):
+    those that find none left take the driver's copies, with the same values."""
+    import threading
+
+    from uegccd_b200 import Context, _capi
+
+    system = _systems(1, 114, 1140)[0]
+    contexts = [Context(*system) for _ in range(8)]
+    want = contexts[0].mp2()
+    _capi.trim_cache()
+    base, errors, most = _locked(), [], [0]
+
+    def work(c):
+        try:
+            for _ in range(2):
+                got = c.mp2()
+                most[0] = max(most[0], _locked() - base)
+                assert got[0] == want[0]
+                for x, y in zip(got[1:], want[1:]):
+                    assert np.array_equal(x, y)
+        except Exception as e:   # an assertion of a thread has to reach the test
+            errors.append(repr(e))
+
+    th = [threading.Thread(target=work, args=(c,)) for c in contexts]
+    for x in th:
+        x.start()
+    for x in th:
+        x.join()
+    assert not errors, errors
+    assert most[0] <= 512 * MB + SLACK, most[0] / MB

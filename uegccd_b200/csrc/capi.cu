@@ -1164,9 +1164,54 @@ int pack_from_host(UegccdBatch &b, int s, const double *host_dense)
     return 0;
 }
 
+// One run of device bytes and where it goes.
+struct Piece {
+    char *dst;
+    const char *src;
+    size_t bytes;
+};
+constexpr size_t kPiece = 32ull << 20;
+void add_pieces(std::vector<Piece> &out, char *dst, const char *src, size_t bytes)
+{
+    for (size_t a = 0; a < bytes; a += kPiece) out.push_back(Piece{dst + a, src + a, std::min(kPiece, bytes - a)});
+}
+
+// Pieces into pageable host memory through up to three page-locked slots, the host's copy of one
+// beside the device's of the next, and the stream's work done at the end: what a call locks does not grow with what it downloads.
+// Without page-locked memory the driver copies them.
+int download(UegccdBatch &b, const std::vector<Piece> &v, bool cores)
+{
+    const int n = (int)v.size(), slots = std::min(n, 3);
+    size_t size = 0;
+    for (const auto &p : v) size = std::max(size, (p.bytes + 63) & ~(size_t)63);
+    PinnedScope buf(slots * size, b.stream);
+    if (!buf.b.p) {
+        for (const auto &p : v) CU(cudaMemcpyAsync(p.dst, p.src, p.bytes, cudaMemcpyDeviceToHost, b.stream));
+        CU(cudaStreamSynchronize(b.stream));
+        return 0;
+    }
+    for (int k = 0; k < slots; k++)
+        if (!b.ev_copy[k]) CU(cudaEventCreateWithFlags(&b.ev_copy[k], cudaEventDisableTiming));
+    auto issue = [&](int k) {
+        CU(cudaMemcpyAsync(buf.b.p + (k % slots) * size, v[k].src, v[k].bytes, cudaMemcpyDeviceToHost, b.stream));
+        CU(cudaEventRecord(b.ev_copy[k % slots], b.stream));
+        return 0;
+    };
+    int rc = 0;
+    for (int k = 0; k < slots; k++)
+        if ((rc = issue(k))) return rc;
+    for (int k = 0; k < n; k++) {
+        CU(cudaEventSynchronize(b.ev_copy[k % slots]));
+        host_copy(v[k].dst, buf.b.p + (k % slots) * size, v[k].bytes, cores);
+        if (k + slots < n && (rc = issue(k + slots))) return rc;
+    }
+    buf.settled = true;
+    return 0;
+}
+
 // T2abab / T2abba / T2aaaa of solve s in the reference layout (each may be null) into host
-// arrays; with_red: the batch's reduced sums too, in the same wait.  The arrays leave the device in
-// one run into page-locked memory and go on from there, one copied while the next is on its way: a
+// arrays; with_red: the batch's reduced sums too, in the same wait.  The arrays leave the device
+// through page-locked memory, one copied on while the next is on its way (small ones in one run): a
 // pageable copy waits for the one before it.  MP2 with its three arrays: N=38 (0.7 MB each) 0.48 ->
 // 0.24 ms, N=54 (3.3 MB) 1.28 -> 0.82, N=114 (28 MB) 16 -> 6.5; one array, the residual, of 17 MB
 // 3.9 -> 3.4 ms, but of 28 MB 5.7 -> 7.4: a single one above kAloneMax is left to the driver.
@@ -1193,31 +1238,24 @@ int unpack_to_host(UegccdBatch &b, int s, const double *t_dev, double *ab, doubl
         CU(cudaMemcpyAsync(sums, b.d.red, red, cudaMemcpyDeviceToHost, b.stream));
         b.d2h_bytes += (int64_t)red;
     }
-    constexpr size_t kAloneMax = 24ull << 20;
+    constexpr size_t kAloneMax = 24ull << 20, kApartMin = 512ull << 10;
     bool direct = true;   // page-locked destinations take the copies themselves
     for (int k = 0; k < m; k++) direct = direct && is_pinned(host[k]);
     direct = direct || (m == 1 && bytes > kAloneMax);
-    PinnedScope buf(direct ? 0 : m * bytes, b.stream);
-    const bool apart = bytes >= (512 << 10);
-    if (!buf.b.p) {
-        for (int k = 0; k < m; k++)
+    if (!direct && bytes >= kApartMin) {
+        std::vector<Piece> v;
+        for (int k = 0; k < m; k++) add_pieces(v, (char *)host[k], (const char *)(b.dense + k * n), bytes);
+        const int rc = download(b, v, m * bytes > 2 * kCoresMin);
+        if (rc) return rc;
+    } else {
+        PinnedScope buf(direct ? 0 : m * bytes, b.stream);
+        if (buf.b.p) CU(cudaMemcpyAsync(buf.b.p, b.dense, m * bytes, cudaMemcpyDeviceToHost, b.stream));
+        for (int k = 0; !buf.b.p && k < m; k++)
             CU(cudaMemcpyAsync(host[k], b.dense + k * n, bytes, cudaMemcpyDeviceToHost, b.stream));
         CU(cudaStreamSynchronize(b.stream));
-    } else if (apart) {
-        for (int k = 0; k < m; k++) {
-            if (!b.ev_copy[k]) CU(cudaEventCreateWithFlags(&b.ev_copy[k], cudaEventDisableTiming));
-            CU(cudaMemcpyAsync(buf.b.p + k * bytes, b.dense + k * n, bytes, cudaMemcpyDeviceToHost, b.stream));
-            CU(cudaEventRecord(b.ev_copy[k], b.stream));
-        }
-    } else {
-        CU(cudaMemcpyAsync(buf.b.p, b.dense, m * bytes, cudaMemcpyDeviceToHost, b.stream));
-        CU(cudaStreamSynchronize(b.stream));
+        buf.settled = true;
+        for (int k = 0; buf.b.p && k < m; k++) std::memcpy(host[k], buf.b.p + k * bytes, bytes);
     }
-    for (int k = 0; buf.b.p && k < m; k++) {
-        if (apart) CU(cudaEventSynchronize(b.ev_copy[k]));
-        host_copy((char *)host[k], buf.b.p + k * bytes, bytes, m * bytes > 2 * kCoresMin);
-    }
-    buf.settled = true;
     if (red && sums != b.red.data()) std::memcpy(b.red.data(), sums, red);
     return 0;
 }
@@ -2458,19 +2496,15 @@ int uegccd_batch_get_all_amplitudes(UegccdBatch *b, double *t_abab)
     CU(cudaGetLastError());
     const size_t bytes = b->dense_all_n * sizeof(double);
     b->d2h_bytes += (int64_t)bytes;
-    // a page-locked destination takes the copy directly; else through page-locked memory, copied
-    // out on all host cores (a pageable copy is staged by the driver on one thread)
-    const bool direct = is_pinned(t_abab);
-    PinnedScope buf(direct ? 0 : bytes, b->stream);
-    if (!buf.b.p) {
-        CU(cudaMemcpyAsync(t_abab, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
-        CU(cudaStreamSynchronize(b->stream));
-        return UEGCCD_OK;
+    // a page-locked destination takes the copy directly; else through page-locked memory, large ones
+    // copied on on all host cores (a pageable copy is staged by the driver on one thread)
+    if (!is_pinned(t_abab)) {
+        std::vector<Piece> v;
+        add_pieces(v, (char *)t_abab, (const char *)b->dense_all, bytes);
+        return download(*b, v, bytes >= kCoresMin);
     }
-    CU(cudaMemcpyAsync(buf.b.p, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
+    CU(cudaMemcpyAsync(t_abab, b->dense_all, bytes, cudaMemcpyDeviceToHost, b->stream));
     CU(cudaStreamSynchronize(b->stream));
-    buf.settled = true;
-    host_copy((char *)t_abab, buf.b.p, bytes, bytes >= kCoresMin);
     return UEGCCD_OK;
 }
 
