@@ -112,3 +112,25 @@ def test_many_threads_download_at_once():
         x.join()
     assert not errors, errors
     assert most[0] <= 512 * MB + SLACK, most[0] / MB
+
+
+def test_small_batch_downloads_are_one_copy():
+    """Below 8 MB the driver's own staging is the faster way: a download of 2.0 MB into ordinary memory
+    is one copy to pageable memory, one of 10.7 MB comes through page-locked memory."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    from uegccd_b200 import Batch
+
+    torch.cuda.init()
+    for count, electrons, basis, key in ((3, 38, 247, "Pageable"), (4, 54, 485, "Pinned")):
+        b = Batch(_systems(count, electrons, basis))
+        b.mp2()
+        first = b.all_amplitudes()
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+            again = b.all_amplitudes()
+        copies = [e.key for e in p.key_averages() if "Memcpy DtoH" in e.key]
+        assert copies == [f"Memcpy DtoH (Device -> {key})"], copies
+        for x, y in zip(first, again):
+            np.testing.assert_array_equal(x, y)
+        b.close()
