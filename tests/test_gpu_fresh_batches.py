@@ -1,0 +1,90 @@
+"""What a program that makes a batch for every step pays for beside the batch itself: streams,
+events, page-locked and device memory come from the batches before."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+DIIS = dict(scheme=1, ndiis=6, denom_factor=1.0)
+
+
+def _systems(count, electrons, basis, seed=3):
+    from uegccd_b200 import heg
+
+    h = heg.Heg(heg.default_input(nelectron=electrons, maxkpoint=50, rsmin=1.0, rsmax=1.0,
+                                  fcut=(basis / (electrons // 2)) ** (2.0 / 3.0)))
+    return h.twist_systems(np.random.default_rng(seed).random((count, 3)) - 0.5)[0]
+
+
+def _step(systems, drpa):
+    from uegccd_b200 import Batch
+
+    b = Batch(systems)
+    _, e2, res = b.solve(drpa=drpa, **({} if drpa else DIIS))
+    out = list(e2), [r["ecorr"] for r in res], [t.copy() for t in b.all_amplitudes()]
+    b.close()
+    return out
+
+
+@pytest.mark.parametrize("drpa", [False, True], ids=["ccd", "drpa"])
+@pytest.mark.parametrize("count,electrons,basis", [(3, 14, 42), (10, 38, 228)])
+def test_a_batch_takes_over_what_the_last_one_used(count, electrons, basis, drpa):
+    """A second batch makes its own stream and nothing more, dRPA (which has no side streams) from the
+    first one on; and its values are the first one's."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    from uegccd_b200 import _capi
+
+    torch.cuda.init()
+    systems = _systems(count, electrons, basis)
+    _capi.trim_cache()
+    counts, outs = [], []
+    for _ in range(2):
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+            outs.append(_step(systems, drpa))
+        counts.append({e.key: e.count for e in p.key_averages()})
+    assert counts[1]["cudaGraphLaunch"] > 0   # the profile saw the solve
+    for c in counts[0 if drpa else 1:]:
+        assert c["cudaStreamCreateWithFlags"] == 1 and c["cudaStreamDestroy"] == 1, c
+    assert "cudaHostAlloc" not in counts[1] and "cudaFreeHost" not in counts[1], counts[1]
+    assert "cudaMalloc" not in counts[1] and "cudaFree" not in counts[1], counts[1]
+    (a2, a, ta), (b2, b, tb) = outs
+    assert a2 == b2 and a == b and all(np.array_equal(x, y) for x, y in zip(ta, tb))
+
+
+def test_side_streams_of_many_threads_and_live_batches():
+    """Six threads make, solve and release batches of two sizes while other batches stay alive, and
+    the idle sets are given up in between: the values are those of one batch alone."""
+    from uegccd_b200 import Batch, _capi
+
+    sets = [_systems(3, 14, 60), _systems(2, 54, 485)]
+    want = [_step(s, False) for s in sets]
+    live = [Batch(s) for s in sets]
+    for b in live:
+        b.solve(**DIIS)
+    errors = []
+
+    def work(k):
+        try:
+            for rep in range(3):
+                q = (k + rep) % 2
+                got = _step(sets[q], False)
+                assert got[0] == want[q][0] and got[1] == want[q][1]
+                assert all(np.array_equal(x, y) for x, y in zip(got[2], want[q][2]))
+                if k == 0:
+                    _capi.trim_cache()
+        except Exception as e:   # an assertion of a thread has to reach the test
+            errors.append(repr(e))
+
+    th = [threading.Thread(target=work, args=(k,)) for k in range(6)]
+    for x in th:
+        x.start()
+    for x in th:
+        x.join()
+    assert not errors, errors
+    for b, w in zip(live, want):
+        assert [r["ecorr"] for r in b.solve(**DIIS)[2]] == w[1]
+        b.close()

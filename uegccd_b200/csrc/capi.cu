@@ -305,6 +305,112 @@ void pinned_trim()
     for (char *p : drop) cudaFreeHost(p);
 }
 
+// Side streams and untimed events of destroyed batches, kept for the next batch of their device (at
+// most kIdleForks sets and kIdleEvents events a process, until uegccd_trim_cache).  Making and destroying a set
+// with each batch took 0.3-0.5 ms, as long as the rest of a small batch's making: 3 twists of N=14 made,
+// solved and released, 1.42 -> 1.80 ms.
+constexpr size_t kIdleForks = 32, kIdleEvents = 256;
+template <class T>
+struct Idle {
+    int dev;
+    T x;
+};
+std::mutex g_idle_mu;
+std::vector<Idle<Fork>> g_forks;
+std::vector<Idle<cudaEvent_t>> g_events;
+
+template <class T>
+bool idle_get(std::vector<Idle<T>> &v, int dev, T &x)
+{
+    std::lock_guard<std::mutex> lock(g_idle_mu);
+    for (size_t k = v.size(); k-- > 0;)
+        if (v[k].dev == dev) {
+            x = v[k].x;
+            v.erase(v.begin() + k);
+            return true;
+        }
+    return false;
+}
+template <class T>
+bool idle_put(std::vector<Idle<T>> &v, size_t most, int dev, const T &x)
+{
+    std::lock_guard<std::mutex> lock(g_idle_mu);
+    if (v.size() >= most) return false;
+    v.push_back(Idle<T>{dev, x});
+    return true;
+}
+
+void fork_destroy(Fork &f)
+{
+    for (cudaEvent_t e : {f.start, f.staged})
+        if (e) cudaEventDestroy(e);
+    for (auto &e : f.done)
+        if (e) cudaEventDestroy(e);
+    for (auto &x : f.s)
+        if (x) cudaStreamDestroy(x);
+    f = Fork{};
+}
+
+// The side streams of a batch on device dev (current): a whole set, or none.
+bool fork_get(Fork &f, int dev)
+{
+    if (idle_get(g_forks, dev, f)) return true;
+    bool ok = cudaEventCreateWithFlags(&f.start, cudaEventDisableTiming) == cudaSuccess &&
+              cudaEventCreateWithFlags(&f.staged, cudaEventDisableTiming) == cudaSuccess;
+    for (int k = 0; k < kSideStreams; k++)
+        ok = ok && cudaStreamCreateWithFlags(&f.s[k], cudaStreamNonBlocking) == cudaSuccess &&
+             cudaEventCreateWithFlags(&f.done[k], cudaEventDisableTiming) == cudaSuccess;
+    if (ok) return true;
+    cudaGetLastError();
+    fork_destroy(f);
+    return false;
+}
+
+// Back for another batch; a set with work left on a stream, or one that a failed capture still
+// holds, is destroyed.
+void fork_put(Fork &f, int dev)
+{
+    if (!f.s[0]) return;
+    bool ok = true;
+    for (auto &x : f.s) {
+        cudaStreamCaptureStatus c = cudaStreamCaptureStatusNone;
+        ok = ok && cudaStreamIsCapturing(x, &c) == cudaSuccess && c == cudaStreamCaptureStatusNone &&
+             cudaStreamQuery(x) == cudaSuccess;
+    }
+    if (!ok) cudaGetLastError();
+    if (!ok || !idle_put(g_forks, kIdleForks, dev, f)) fork_destroy(f);
+}
+
+cudaError_t event_get(cudaEvent_t &e, int dev)
+{
+    return idle_get(g_events, dev, e) ? cudaSuccess : cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
+}
+
+void event_put(cudaEvent_t e, int dev)
+{
+    if (e && !idle_put(g_events, kIdleEvents, dev, e)) cudaEventDestroy(e);
+}
+
+// The idle sets and events back to their devices.
+void idle_trim()
+{
+    std::vector<Idle<Fork>> f;
+    std::vector<Idle<cudaEvent_t>> e;
+    {
+        std::lock_guard<std::mutex> lock(g_idle_mu);
+        f.swap(g_forks);
+        e.swap(g_events);
+    }
+    for (auto &k : f) {
+        DeviceScope scope(k.dev);
+        fork_destroy(k.x);
+    }
+    for (auto &k : e) {
+        DeviceScope scope(k.dev);
+        cudaEventDestroy(k.x);
+    }
+}
+
 bool is_pinned(const void *p)
 {
     cudaPointerAttributes pa;
@@ -526,16 +632,9 @@ struct UegccdBatch {
         if (ev_solve1) cudaEventDestroy(ev_solve1);
         pinned_put(pin);
         words_put(words);
-        for (auto &e : ev_iter)
-            if (e) cudaEventDestroy(e);
-        for (auto &e : ev_copy)
-            if (e) cudaEventDestroy(e);
-        for (cudaEvent_t e : {fork.start, fork.staged})
-            if (e) cudaEventDestroy(e);
-        for (auto &e : fork.done)
-            if (e) cudaEventDestroy(e);
-        for (auto &x : fork.s)
-            if (x) cudaStreamDestroy(x);
+        for (auto &e : ev_iter) event_put(e, dev);
+        for (auto &e : ev_copy) event_put(e, dev);
+        fork_put(fork, dev);
         if (stream) cudaStreamDestroy(stream);
     }
 
@@ -1191,7 +1290,7 @@ int download(UegccdBatch &b, const std::vector<Piece> &v, bool cores)
         return 0;
     }
     for (int k = 0; k < slots; k++)
-        if (!b.ev_copy[k]) CU(cudaEventCreateWithFlags(&b.ev_copy[k], cudaEventDisableTiming));
+        if (!b.ev_copy[k]) CU(event_get(b.ev_copy[k], b.dev));
     auto issue = [&](int k) {
         CU(cudaMemcpyAsync(buf.b.p + (k % slots) * size, v[k].src, v[k].bytes, cudaMemcpyDeviceToHost, b.stream));
         CU(cudaEventRecord(b.ev_copy[k % slots], b.stream));
@@ -1430,9 +1529,10 @@ int ctl_alloc(UegccdBatch &b, int ndiis, int max_rec)
     const int n = b.d.nsolves;
     int rc = 0;
     if (!c.done) {
+        for (auto &e : b.ev_iter)
+            if (!e) CU(event_get(e, b.dev));
         if (!b.words && !(b.words = words_get())) return fail(UEGCCD_ERR_ALLOC, "no page-locked host memory");
         c.done = reinterpret_cast<int *>(b.words);
-        for (auto &e : b.ev_iter) CU(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
     }
     if (!c.state) {
         const UegccdBatch::Mark m = b.mark();
@@ -1487,16 +1587,9 @@ const Fork *fork_of(UegccdBatch &b)
 {
     if (!b.fork_made) {
         b.fork_made = true;
-        Fork &f = b.fork;
-        f.terms = b.d.namp <= kForkAmps || b.d.nsolves <= kForkSolves;
-        bool ok = cudaEventCreateWithFlags(&f.start, cudaEventDisableTiming) == cudaSuccess &&
-                  cudaEventCreateWithFlags(&f.staged, cudaEventDisableTiming) == cudaSuccess;
-        for (int k = 0; k < kSideStreams; k++)
-            ok = ok && cudaStreamCreateWithFlags(&f.s[k], cudaStreamNonBlocking) == cudaSuccess &&
-                 cudaEventCreateWithFlags(&f.done[k], cudaEventDisableTiming) == cudaSuccess;
-        if (!ok) cudaGetLastError();   // one stream then serves all
+        if (fork_get(b.fork, b.dev)) b.fork.terms = b.d.namp <= kForkAmps || b.d.nsolves <= kForkSolves;
     }
-    return b.fork.done[kSideStreams - 1] ? &b.fork : nullptr;
+    return b.fork.s[0] ? &b.fork : nullptr;   // else one stream serves all
 }
 
 // Captures one iteration as a CUDA graph.
@@ -1507,7 +1600,7 @@ int capture_iteration(UegccdBatch &b, const TermFlags &f, double tol, int max_it
     if (G.valid && G.key == key) return 0;
     G.valid = false;
     if (G.exec) { cudaGraphExecDestroy(G.exec); G.exec = nullptr; }
-    const Fork *fork = fork_of(b);
+    const Fork *fork = f.drpa ? nullptr : fork_of(b);   // dRPA's terms follow one another
     cudaGraph_t g = nullptr;
     CU(cudaStreamBeginCapture(b.stream, cudaStreamCaptureModeThreadLocal));
     int nl = launch_iteration(b.d, b.ctl, f, tol, max_iter, ndiis, b.stream, nullptr, fork);
@@ -2541,6 +2634,7 @@ int uegccd_batch_structure_factor(UegccdBatch *b, int32_t s, const UegccdSfGrid 
 int uegccd_trim_cache(void)
 {
     pinned_trim();
+    idle_trim();
     std::vector<DevChunk> drop;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
