@@ -255,7 +255,8 @@ struct PinnedScope {
 // Page-locked words an object keeps for its life (the flag of an iteration, small reads): kWords
 // bytes each, cut from slabs of their own.
 constexpr size_t kWords = 4096, kSlab = 64ull << 10;
-constexpr size_t kFlagBytes = 64;   // of a batch's words, for CtlBuffers::done
+constexpr size_t kFlagBytes = 64;   // of a batch's words: CtlBuffers::done, then the two-channel results
+constexpr size_t kReadAt = kFlagBytes + kTcWords * sizeof(double);   // then small reads
 std::vector<char *> g_slabs, g_words;   // slabs, and their free pieces (under g_pinned_mu)
 
 char *words_get()
@@ -462,6 +463,43 @@ void drop_cached(int dev)
     for (auto &c : drop) cudaFree(c.p);
 }
 
+// Device memory that makes a call faster and that it can do without, of one holder: kept between its
+// calls, and given up then to an allocation that finds no room (under g_pool_mu).
+struct SpareChunk {
+    DevChunk c{nullptr, 0, -1};
+    bool busy = false;
+    size_t refused = 0;          // bytes there was no room for, at g_released
+    uint64_t refused_at = 0;
+};
+uint64_t g_released = 0;              // how often memory was given back or the limit moved
+std::vector<SpareChunk *> g_spares;   // those with a chunk
+
+// Returns the idle spare chunks of device dev (-1: of all) to the driver, as drop_cached.
+bool drop_spares(int dev)
+{
+    std::vector<DevChunk> drop;
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        for (size_t k = 0; k < g_spares.size();) {
+            SpareChunk &s = *g_spares[k];
+            if (s.busy || (dev >= 0 && s.c.dev != dev)) {
+                k++;
+                continue;
+            }
+            drop.push_back(s.c);
+            g_dev_bytes[s.c.dev % kMaxDevices] -= (int64_t)s.c.size;
+            s.c = DevChunk{nullptr, 0, -1};
+            g_released++;
+            g_spares.erase(g_spares.begin() + k);
+        }
+    }
+    for (auto &c : drop) {
+        DeviceScope scope(c.dev);
+        cudaFree(c.p);
+    }
+    return !drop.empty();
+}
+
 // True when `need` more bytes on dev stay within the limit (under g_pool_mu).
 bool within_limit(int dev, size_t need)
 {
@@ -470,8 +508,9 @@ bool within_limit(int dev, size_t need)
 
 // A chunk of at least `need` bytes on device dev (current): from the cache, else cudaMalloc.
 // Past the memory limit, or when cudaMalloc fails, the device's cache goes back to the driver
-// and the request is tried once more; then cudaErrorMemoryAllocation.
-cudaError_t chunk_get(size_t need, int dev, DevChunk &out)
+// and the request is tried once more; then, unless it is for a spare chunk itself, with the idle spare
+// chunks back too; then cudaErrorMemoryAllocation.
+cudaError_t chunk_get(size_t need, int dev, DevChunk &out, bool spare = false)
 {
     bool fits = true;
     {
@@ -490,15 +529,19 @@ cudaError_t chunk_get(size_t need, int dev, DevChunk &out)
         fits = within_limit(dev, need);
     }
     if (!fits) {
+        auto room = [&]() {
+            std::lock_guard<std::mutex> lock(g_pool_mu);
+            return within_limit(dev, need);
+        };
         drop_cached(dev);
-        std::lock_guard<std::mutex> lock(g_pool_mu);
-        if (!within_limit(dev, need)) return cudaErrorMemoryAllocation;
+        if (!room() && (spare || !drop_spares(dev) || !room())) return cudaErrorMemoryAllocation;
     }
     void *p = nullptr;
     cudaError_t e = cudaMalloc(&p, need);
-    if (e != cudaSuccess) {
+    for (int k = 0; k < 2 && e != cudaSuccess; k++) {
         cudaGetLastError();
-        drop_cached(dev);
+        if (k == 0) drop_cached(dev);
+        else if (spare || !drop_spares(dev)) break;
         e = cudaMalloc(&p, need);
     }
     if (e == cudaSuccess) {
@@ -515,6 +558,7 @@ void chunk_free(const DevChunk &c)
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
         g_dev_bytes[c.dev % kMaxDevices] -= (int64_t)c.size;
+        g_released++;
     }
     cudaFree(c.p);
 }
@@ -524,6 +568,7 @@ void chunk_put(const DevChunk &c)
 {
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
+        g_released++;
         if (g_pool_bytes + c.size <= kPoolCap) {
             g_pool.push_back(c);
             g_pool_bytes += c.size;
@@ -532,6 +577,58 @@ void chunk_put(const DevChunk &c)
         g_dev_bytes[c.dev % kMaxDevices] -= (int64_t)c.size;
     }
     cudaFree(c.p);
+}
+
+// The chunk of s for one call, at least `need` bytes on device dev (current): the one it has kept, else
+// another (fresh = true), else none.
+char *spare_hold(SpareChunk &s, size_t need, int dev, bool &fresh)
+{
+    DevChunk old{nullptr, 0, -1};
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        if (s.c.p && s.c.size >= need) {
+            s.busy = true;
+            fresh = false;
+            return s.c.p;
+        }
+        if (s.refused > 0 && need >= s.refused && s.refused_at == g_released) return nullptr;
+        if (s.c.p) {
+            old = s.c;
+            s.c = DevChunk{nullptr, 0, -1};
+            g_spares.erase(std::find(g_spares.begin(), g_spares.end(), &s));
+        }
+    }
+    if (old.p) chunk_put(old);
+    DevChunk c;
+    const bool found = chunk_get(need, dev, c, true) == cudaSuccess;
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    s.refused = found ? 0 : need;   // not asked for again before memory was given back somewhere
+    s.refused_at = g_released;
+    if (!found) return nullptr;
+    s.c = c;
+    s.busy = true;
+    g_spares.push_back(&s);
+    fresh = true;
+    return c.p;
+}
+
+void spare_rest(SpareChunk &s)
+{
+    std::lock_guard<std::mutex> lock(g_pool_mu);
+    s.busy = false;
+}
+
+void spare_free(SpareChunk &s)
+{
+    DevChunk c{nullptr, 0, -1};
+    {
+        std::lock_guard<std::mutex> lock(g_pool_mu);
+        if (!s.c.p) return;
+        c = s.c;
+        s.c = DevChunk{nullptr, 0, -1};
+        g_spares.erase(std::find(g_spares.begin(), g_spares.end(), &s));
+    }
+    chunk_put(c);
 }
 }  // namespace
 
@@ -547,7 +644,7 @@ struct UegccdBatch {
     std::vector<DevChunk> big;       // chunks of one large array each
     cudaStream_t stream = nullptr;
     cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev_solve0 = nullptr, ev_solve1 = nullptr;
-    char *words = nullptr;           // page-locked words (on first use): CtlBuffers::done, then small reads
+    char *words = nullptr;           // page-locked words (on first use; kFlagBytes, kReadAt)
     PinnedBuf pin;                   // where small reads land that the words do not hold
     cudaEvent_t ev_iter[2] = {nullptr, nullptr};            // the two latest iterations
     cudaEvent_t ev_copy[3] = {nullptr, nullptr, nullptr};   // arrays of a download (on first use)
@@ -613,6 +710,8 @@ struct UegccdBatch {
     // amplitudes hold T2abab of such a solve (the spin relation does not give T2abba)
     std::vector<std::unique_ptr<uegccd::TwoChannel>> tcs;
     std::vector<std::vector<double>> tc_en, tc_dt;
+    SpareChunk tc_work;              // the workspace their matrix-product form shares
+    const void *tc_work_user = nullptr;   // the state that used it last
     bool two_channel_amps = false;
     double *sf_grid = nullptr;
     int *sf_err = nullptr;
@@ -624,6 +723,7 @@ struct UegccdBatch {
         if (kt_events)
             for (auto &e : kt.ev) cudaEventDestroy(e);
         if (stream) cudaStreamSynchronize(stream);
+        spare_free(tc_work);
         for (auto &c : chunks) chunk_put(c);
         for (auto &c : big) chunk_put(c);
         if (ev0) cudaEventDestroy(ev0);
@@ -1220,9 +1320,9 @@ int set_active_all(UegccdBatch &b, uint8_t v)
 // kernels before it; the caller's own memory when there is none.
 void *small_read(UegccdBatch &b, void *own, size_t bytes)
 {
-    if (bytes <= kWords - kFlagBytes) {
+    if (bytes <= kWords - kReadAt) {
         if (!b.words) b.words = words_get();
-        return b.words ? b.words + kFlagBytes : own;
+        return b.words ? b.words + kReadAt : own;
     }
     if (b.pin.bytes < bytes) {
         pinned_put(b.pin);
@@ -2044,6 +2144,16 @@ int make_two_channel(UegccdBatch &b, int s, std::unique_ptr<uegccd::TwoChannel> 
     };
     al.begin = [ar]() { ar->m = ar->b->mark(); };
     al.rollback = [ar]() { ar->b->rollback(ar->m); };
+    al.hold = [ar](const void *who, size_t bytes, bool *kept) -> void * {
+        bool fresh = false;
+        char *p = spare_hold(ar->b->tc_work, bytes, ar->b->dev, fresh);
+        *kept = p && !fresh && ar->b->tc_work_user == who;
+        ar->b->tc_work_user = p ? who : nullptr;
+        return p;
+    };
+    al.rest = [ar]() { spare_rest(ar->b->tc_work); };
+    if (!b.words && !(b.words = words_get())) return fail(UEGCCD_ERR_ALLOC, "no page-locked host memory");
+    al.words = reinterpret_cast<double *>(b.words + kFlagBytes);
     auto tc = std::make_unique<uegccd::TwoChannel>();
     const int rc = tc->init(b.sys[s], b.plans[s], b.stream, al);
     if (rc) return rc;
@@ -2635,6 +2745,7 @@ int uegccd_trim_cache(void)
 {
     pinned_trim();
     idle_trim();
+    drop_spares(-1);
     std::vector<DevChunk> drop;
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
@@ -2648,6 +2759,7 @@ int uegccd_trim_cache(void)
     {
         std::lock_guard<std::mutex> lock(g_pool_mu);
         for (auto &c : drop) g_dev_bytes[c.dev % kMaxDevices] -= (int64_t)c.size;
+        g_released++;
     }
     return UEGCCD_OK;
 }
@@ -2657,6 +2769,7 @@ int uegccd_set_memory_limit(int64_t bytes)
     if (bytes < 0) return fail(UEGCCD_ERR_ARG, "memory limit must be >= 0");
     std::lock_guard<std::mutex> lock(g_pool_mu);
     g_mem_limit = bytes;
+    g_released++;
     return UEGCCD_OK;
 }
 

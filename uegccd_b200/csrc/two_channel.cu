@@ -712,7 +712,6 @@ TwoChannel::TwoChannel() = default;
 
 TwoChannel::~TwoChannel()
 {
-    if (out_) cudaFreeHost(out_);
     if (evo_) cudaEventDestroy(evo_);
     if (ev0_) cudaEventDestroy(ev0_);
     if (ev1_) cudaEventDestroy(ev1_);
@@ -770,8 +769,7 @@ int TwoChannel::init(const SystemHost &sys, const SolvePlan &plan, cudaStream_t 
         (rc = alloc((void **)&vt_, (size_t)8 * nq_ * sizeof(double))) ||
         (rc = alloc((void **)&eig_, M_ * sizeof(double))) || (rc = alloc((void **)&cube_d, cube.size() * sizeof(int))) ||
         (rc = alloc((void **)&jvv_, V_ * sizeof(double))) || (rc = alloc((void **)&joo_, O_ * sizeof(double))) ||
-        (rc = alloc((void **)&part_, (size_t)2 * std::max(nblk_, 1) * kMaxDiis * sizeof(double))) ||
-        (rc = host_words())) {
+        (rc = alloc((void **)&part_, (size_t)2 * std::max(nblk_, 1) * kMaxDiis * sizeof(double)))) {
         al_.rollback();
         return rc;
     }
@@ -798,6 +796,8 @@ int TwoChannel::init(const SystemHost &sys, const SolvePlan &plan, cudaStream_t 
     k2_find<<<blocks_of(nf), kThreads, 0, st_>>>(D, cube_d, R, F_);
     TCU(cudaGetLastError());
     TCU(cudaStreamSynchronize(st_));
+    out_ = al_.words;
+    if (!evo_) TCU(cudaEventCreateWithFlags(&evo_, cudaEventDisableTiming));
     if (!ev0_) TCU(cudaEventCreate(&ev0_));
     if (!ev1_) TCU(cudaEventCreate(&ev1_));
     UegccdRangeTerms none{};
@@ -854,88 +854,108 @@ int TwoChannel::set_integrals(int routine, const UegccdRangeTerms &fl, int core_
     return 0;
 }
 
-// Whether the residual can take the form of two_channel_mm.cu; its arrays on the first call, as
-// long as memory holds them (the loops serve the system otherwise).
-bool TwoChannel::mm_ready()
+// The matrix-product form of this system: its sizes and lists.
+void TwoChannel::mm_make()
 {
-    if (mm_state_ != 0) return mm_state_ > 0;
-    mm_state_ = -1;
-    auto m = std::make_unique<TcMm>();
-    TcMm &D = *m;
+    mm_ = std::make_unique<TcMm>();
+    TcMm &D = *mm_;
     const int O2 = O_ * O_;
     D.O = O_, D.V = V_, D.n = (int)n_, D.nq = nq_;
     D.F = F_, D.nv = nv_, D.vt = vt_;
+    D.gr[0] = r_[0], D.gr[1] = r_[1], D.gx[0] = x_[0], D.gx[1] = x_[1];
     D.ring_smem = 0;
     for (const auto &P : pairs_) D.ring_smem = std::max(D.ring_smem, tc_mm_ring_smem(P.y, P.w));
-    if (D.ring_smem > kTcMmSmemMax || tc_mm_stage_smem(O_) > kTcMmSmemMax) return false;
+    mm_fits_ = D.ring_smem <= kTcMmSmemMax && tc_mm_stage_smem(O_) <= kTcMmSmemMax;
+    if (!mm_fits_) return;
     auto up = [](int64_t x, int64_t k) { return (x + k - 1) / k * k; };
-    const int64_t ldw = up(2 * (int64_t)(V_ + O_), 64), ldt = up(2 * (int64_t)O2, 64);
-    D.ldw = (int)ldw, D.ldt = (int)ldt, D.kdim = (int)up(V_, 16);
-    std::vector<int> kl0(O2 + 1, 0), kl, kl_ij;
+    D.ldw = (int)up(2 * (int64_t)(V_ + O_), 64), D.ldt = (int)up(2 * (int64_t)O2, 64), D.kdim = (int)up(V_, 16);
+    kl0_.assign(O2 + 1, 0);
     for (int ij = 0; ij < O2; ij++) {
         const auto &a = occ_[ij % O_], &b = occ_[ij / O_];
         for (int k = 0; k < O_; k++)
             for (int l = 0; l < O_; l++)
                 if (a[0] + b[0] == occ_[k][0] + occ_[l][0] && a[1] + b[1] == occ_[k][1] + occ_[l][1] &&
                     a[2] + b[2] == occ_[k][2] + occ_[l][2]) {
-                    kl.push_back(k | l << 16);
-                    kl_ij.push_back(ij);
+                    kl_.push_back(k | l << 16);
+                    kl_ij_.push_back(ij);
                 }
-        kl0[ij + 1] = (int)kl.size();
+        kl0_[ij + 1] = (int)kl_.size();
     }
-    D.nkl = (int)kl.size();
+    D.nkl = (int)kl_.size();
     D.npairs = (int)pairs_.size();
-    int *kl0_d = nullptr, *kl_d = nullptr, *klij_d = nullptr, *ph_d = nullptr;
-    int4 *pairs_d = nullptr;
-    al_.begin();
-    if (alloc((void **)&D.w, D.kdim * ldw * sizeof(double)) || alloc((void **)&D.t, D.kdim * ldt * sizeof(double)) ||
-        alloc((void **)&D.c, ldw * ldt * sizeof(double)) || alloc((void **)&D.jpart, (size_t)V_ * O_ * sizeof(double)) ||
-        alloc((void **)&D.done, sizeof(int)) || alloc((void **)&kl0_d, kl0.size() * sizeof(int)) ||
-        alloc((void **)&kl_d, kl.size() * sizeof(int)) || alloc((void **)&klij_d, kl.size() * sizeof(int)) ||
-        alloc((void **)&D.h2, kl.size() * sizeof(double)) || alloc((void **)&D.h3, kl.size() * sizeof(double)) ||
-        alloc((void **)&pairs_d, pairs_.size() * sizeof(int4)) || alloc((void **)&ph_d, ph_.size() * sizeof(int))) {
-        al_.rollback();
-        return false;
-    }
-    D.kl0 = kl0_d, D.kl = kl_d, D.kl_ij = klij_d, D.pairs = pairs_d, D.ph = ph_d;
-    D.gr[0] = r_[0], D.gr[1] = r_[1], D.gx[0] = x_[0], D.gx[1] = x_[1];
-    cudaError_t e = tc_mm_limits(D);
-    auto copy = [&](void *dst, const void *src, size_t bytes) {
-        if (e == cudaSuccess && bytes > 0) e = cudaMemcpyAsync(dst, src, bytes, cudaMemcpyHostToDevice, st_);
-    };
-    copy(kl0_d, kl0.data(), kl0.size() * sizeof(int));
-    copy(kl_d, kl.data(), kl.size() * sizeof(int));
-    copy(klij_d, kl_ij.data(), kl_ij.size() * sizeof(int));
-    copy(pairs_d, pairs_.data(), pairs_.size() * sizeof(int4));
-    copy(ph_d, ph_.data(), ph_.size() * sizeof(int));
-    if (e == cudaSuccess) e = cudaMemsetAsync(D.w, 0, D.kdim * ldw * sizeof(double), st_);   // the padding stays 0
-    if (e == cudaSuccess) e = cudaMemsetAsync(D.t, 0, D.kdim * ldt * sizeof(double), st_);
-    if (e == cudaSuccess) e = cudaMemsetAsync(D.done, 0, sizeof(int), st_);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st_);
-    if (e != cudaSuccess) {
-        al_.rollback();
-        return false;
-    }
-    mm_ = std::move(m);
-    mm_state_ = 1;
-    return true;
 }
+
+// The workspace of the matrix-product form for one call that can take it, if there is one to be
+// had: the loops serve the call otherwise.  Another system of the owner may have used it in between, so
+// what this one keeps there (the lists, the zero padding of W and T, W) is made again then.
+struct TwoChannel::Workspace {
+    TwoChannel &t;
+    Workspace(TwoChannel &tc, bool drpa) : t(tc)
+    {
+        t.mm_on_ = false;
+        if (drpa || !t.plain_ || !t.mm_fits_) return;
+        if (!t.mm_) t.mm_make();
+        if (!t.mm_fits_) return;
+        TcMm &D = *t.mm_;
+        size_t bytes = 0;
+        auto place = [&bytes](size_t k) {
+            const size_t at = bytes;
+            bytes += (k + 255) & ~(size_t)255;
+            return at;
+        };
+        const size_t nw = (size_t)D.kdim * D.ldw * sizeof(double), nt = (size_t)D.kdim * D.ldt * sizeof(double);
+        const size_t w = place(nw), tt = place(nt), c = place((size_t)D.ldw * D.ldt * sizeof(double));
+        const size_t jpart = place((size_t)t.V_ * t.O_ * sizeof(double)), done = place(sizeof(int));
+        const size_t h2 = place(t.kl_.size() * sizeof(double)), h3 = place(t.kl_.size() * sizeof(double));
+        const size_t kl0 = place(t.kl0_.size() * sizeof(int)), kl = place(t.kl_.size() * sizeof(int));
+        const size_t klij = place(t.kl_ij_.size() * sizeof(int)), pairs = place(t.pairs_.size() * sizeof(int4));
+        const size_t ph = place(t.ph_.size() * sizeof(int));
+        bool kept = false;
+        char *base = static_cast<char *>(t.al_.hold(&t, bytes, &kept));
+        if (!base) return;
+        t.mm_on_ = true;
+        if (kept && D.w == reinterpret_cast<double *>(base + w)) return;
+        D.w = reinterpret_cast<double *>(base + w), D.t = reinterpret_cast<double *>(base + tt);
+        D.c = reinterpret_cast<double *>(base + c), D.jpart = reinterpret_cast<double *>(base + jpart);
+        D.done = reinterpret_cast<int *>(base + done);
+        D.h2 = reinterpret_cast<double *>(base + h2), D.h3 = reinterpret_cast<double *>(base + h3);
+        D.kl0 = reinterpret_cast<int *>(base + kl0), D.kl = reinterpret_cast<int *>(base + kl);
+        D.kl_ij = reinterpret_cast<int *>(base + klij), D.pairs = reinterpret_cast<int4 *>(base + pairs);
+        D.ph = reinterpret_cast<int *>(base + ph);
+        cudaError_t e = tc_mm_limits(D);
+        auto copy = [&](size_t at, const void *src, size_t n) {
+            if (e == cudaSuccess && n > 0) e = cudaMemcpyAsync(base + at, src, n, cudaMemcpyHostToDevice, t.st_);
+        };
+        copy(kl0, t.kl0_.data(), t.kl0_.size() * sizeof(int));
+        copy(kl, t.kl_.data(), t.kl_.size() * sizeof(int));
+        copy(klij, t.kl_ij_.data(), t.kl_ij_.size() * sizeof(int));
+        copy(pairs, t.pairs_.data(), t.pairs_.size() * sizeof(int4));
+        copy(ph, t.ph_.data(), t.ph_.size() * sizeof(int));
+        if (e == cudaSuccess) e = cudaMemsetAsync(D.w, 0, nw, t.st_);
+        if (e == cudaSuccess) e = cudaMemsetAsync(D.t, 0, nt, t.st_);
+        if (e == cudaSuccess) e = cudaMemsetAsync(D.done, 0, sizeof(int), t.st_);
+        t.weights_ = false;
+        if (e != cudaSuccess) {
+            D.w = nullptr;   // nothing is kept of it
+            t.mm_on_ = false;
+            cudaStreamSynchronize(t.st_);
+            t.al_.rest();
+        }
+    }
+    ~Workspace()
+    {
+        if (!t.mm_on_) return;
+        cudaStreamSynchronize(t.st_);   // a call that failed may have left work behind
+        t.mm_on_ = false;
+        t.al_.rest();
+    }
+    Workspace(const Workspace &) = delete;
+    Workspace &operator=(const Workspace &) = delete;
+};
 
 int TwoChannel::upload_t(const double *h, double *d)
 {
     TCU(cudaMemcpyAsync(d, h, n_ * sizeof(double), cudaMemcpyHostToDevice, st_));
-    return 0;
-}
-
-// Where the reductions' results land: page-locked host memory, written by the kernels.
-int TwoChannel::host_words()
-{
-    if (!out_ && cudaHostAlloc((void **)&out_, 2 * kMaxDiis * sizeof(double), cudaHostAllocPortable) != cudaSuccess) {
-        cudaGetLastError();
-        out_ = nullptr;
-        return set_last_error(UEGCCD_ERR_ALLOC, "no page-locked host memory");
-    }
-    if (!evo_) TCU(cudaEventCreateWithFlags(&evo_, cudaEventDisableTiming));
     return 0;
 }
 
@@ -957,7 +977,7 @@ int TwoChannel::read_out(int k, double *h)
 // One residual G of the terms in mask from t_ into g_.
 int TwoChannel::residual(bool drpa, int mask)
 {
-    if (!drpa && plain_ && mm_ready()) {
+    if (mm_on_) {
         mm_->sets = f_.lad_lin_d == f_.lad_lin_x && f_.lad_quad_d == f_.lad_quad_x ? 1 : 2;
         if (!weights_) tc_mm_weights(*mm_, f_, st_);
         weights_ = true;
@@ -1001,6 +1021,7 @@ int TwoChannel::residual(bool drpa, int mask)
 int TwoChannel::ccd_g2(const double *t_abab, const double *t_abba, int mask, double *g_abab, double *g_abba)
 {
     int rc;
+    Workspace ws(*this, false);
     if ((rc = upload_t(t_abab, t_[0])) || (rc = upload_t(t_abba, t_[1])) || (rc = residual(false, mask))) return rc;
     TCU(cudaMemcpyAsync(g_abab, g_[0], n_ * sizeof(double), cudaMemcpyDeviceToHost, st_));
     TCU(cudaMemcpyAsync(g_abba, g_[1], n_ * sizeof(double), cudaMemcpyDeviceToHost, st_));
@@ -1067,6 +1088,7 @@ int TwoChannel::solve(const UegccdOptions &opt, bool drpa, const std::vector<dou
         while ((rc = diis_alloc(nd)) == UEGCCD_ERR_ALLOC && nd > 2) nd--;
         if (rc) return rc;
     }
+    Workspace ws(*this, drpa);   // after the history, which comes before it
     View2 D{O_, M_, V_, nq_, core_n_, (int)n_, F_, nv_, vt_, eig_, f_};
     const int mask = drpa ? (1 | (opt.do_mosaic ? 2 : 0) | (opt.do_ring ? 8 : 0))
                           : (1 | (opt.do_mosaic ? 2 : 0) | (opt.do_ladder ? 4 : 0) | (opt.do_ring ? 8 : 0) |

@@ -25,9 +25,17 @@ int tc_pick_routine(const UegccdRangeTerms &flags, int safe_eri, int core_n, dou
 // Device memory for the two-channel state, carved from the owning context's allocations.
 // get returns 0 or an error status; begin/rollback bracket a group of allocations so that a
 // failed group leaves nothing behind (the DIIS history steps its depth down on failure).
+// hold lends `who` at least `bytes` for one call, until rest: one workspace, which the systems of
+// an owner share and which goes to whoever finds no memory between calls (nullptr: none to be had);
+// *kept: it still holds what `who` left in it.  words: kTcWords doubles of page-locked host memory, the
+// owner's too.
+constexpr int kTcWords = 32;
 struct TcAlloc {
     std::function<int(void **, size_t)> get;
     std::function<void()> begin, rollback;
+    std::function<void *(const void *who, size_t bytes, bool *kept)> hold;
+    std::function<void()> rest;
+    double *words = nullptr;
 };
 
 // The integral flag of each integral of the terms, after the Max(...) of CCD.f90:620-937.
@@ -87,12 +95,13 @@ private:
     double *ht_[2] = {nullptr, nullptr}, *hr_[2] = {nullptr, nullptr};
     cudaEvent_t ev0_ = nullptr, ev1_ = nullptr, evo_ = nullptr;
     int launches_ = 0;
-    // the residual as matrix products (two_channel_mm.cu): device arrays on the first CCD residual
-    // that can take that form; mm_state_ 0 not tried, 1 ready, -1 not for this system
-    std::unique_ptr<TcMm> mm_;
-    int mm_state_ = 0;
+    // the residual as matrix products (two_channel_mm.cu), in a lent workspace
+    std::unique_ptr<TcMm> mm_;  // made on the first call that can take that form
+    bool mm_fits_ = true;       // its shared memory suffices
+    bool mm_on_ = false;        // this call has the workspace
+    std::vector<int> kl0_, kl_, kl_ij_;   // TcMm's lists
     bool plain_ = false;        // no integral excluded, no core orbital
-    bool weights_ = false;      // mm_'s W holds the current integrals
+    bool weights_ = false;      // the workspace's W holds the current integrals
     std::vector<std::array<int, 3>> occ_;
     std::vector<int4> pairs_;   // {Q, -Q} pairs of particle-hole groups: first row and rows of each
     std::vector<int> ph_;       // rows i | x << 16
@@ -100,11 +109,11 @@ private:
     int alloc(void **p, size_t bytes);
     int upload_t(const double *h, double *d);
     int residual(bool drpa, int mask);
-    int host_words();
     int note_out();
     int read_out(int k, double *h);
     int diis_alloc(int ndiis);
-    bool mm_ready();
+    void mm_make();
+    struct Workspace;
 };
 
 }  // namespace uegccd
