@@ -1561,31 +1561,37 @@ int drpa_alloc(UegccdBatch &b)
     DevBatch &d = b.d;
     if (d.drs2) return 0;
     const int n = d.nsolves;
-    std::vector<int2> list;
+    std::vector<int4> list;
     std::vector<DrpaSolveDev> ds(n);
     int64_t rij = 0, cp = 0, ph = 0;
+    int ranges = 0, jp = 0;
     for (int s = 0; s < n; s++) {
         const SolvePlan &P = b.plans[s];
-        ds[s] = DrpaSolveDev{rij, cp};
+        const int nc = (P.V + kDrpaCols - 1) / kDrpaCols;
+        ds[s] = DrpaSolveDev{rij, cp, ranges, nc, jp, 0};
+        ranges += nc;
+        jp += nc > 1 ? P.O * nc : 0;
         rij += (int64_t)P.O * P.O;
         cp += (int64_t)P.blocks.size() * P.V;
         ph += (int64_t)P.O * P.V;
-        for (int i = 0; i < P.O; i++) list.push_back(make_int2(s, i));
+        for (int c = 0; c < nc; c++)
+            for (int i = 0; i < P.O; i++) list.push_back(make_int4(s, i, c, 0));
     }
     const UegccdBatch::Mark m = b.mark();
     DevBatch x = d;
     int rc = 0;
     if ((rc = b.upload(x.drlist, list)) || (rc = b.upload(x.drsolves, ds)) || (rc = b.alloc(x.drows, (size_t)rij)) ||
-        (rc = b.alloc(x.colpos, (size_t)cp)) || (rc = b.alloc(x.drdone, n)) || (rc = b.alloc(x.dru, (size_t)ph)) ||
-        (rc = b.alloc(x.drs2, (size_t)ph))) {
+        (rc = b.alloc(x.colpos, (size_t)cp)) || (rc = b.alloc(x.drdone, ranges + n)) ||
+        (rc = b.alloc(x.drj, (size_t)jp)) || (rc = b.alloc(x.dru, (size_t)ph)) || (rc = b.alloc(x.drs2, (size_t)ph))) {
         cudaStreamSynchronize(b.stream);   // the uploads above read host vectors of this call
         b.rollback(m);
         return rc;
     }
     x.ndrlist = (int)list.size();
+    x.ndrranges = ranges;
     CU(cudaMemsetAsync(x.drows, 0xff, (size_t)rij * sizeof(int4), b.stream));
     CU(cudaMemsetAsync(x.colpos, 0xff, (size_t)cp * sizeof(int16_t), b.stream));
-    CU(cudaMemsetAsync(x.drdone, 0, n * sizeof(int), b.stream));
+    CU(cudaMemsetAsync(x.drdone, 0, (ranges + n) * sizeof(int), b.stream));
     launch_drpa_tables(x, b.stream);
     CU(cudaGetLastError());
     CU(cudaStreamSynchronize(b.stream));

@@ -45,14 +45,15 @@ struct DevBatch {
     double *eigen = nullptr, *vtab = nullptr;
     double *t = nullptr, *t_new = nullptr, *g = nullptr;
     double *jvv = nullptr, *joo = nullptr;
-    // dRPA (on the first dRPA solve): k_drpa_sums' CTA list {solve, i}, row and column lookups,
-    // and its U, S2 per (i, x) at phr0 + i*V + x - O; per solve the count of finished CTAs
-    int2 *drlist = nullptr;
-    int ndrlist = 0;
+    // dRPA (on the first dRPA solve): k_drpa_sums' CTA list {solve, i, column range}, row and column
+    // lookups, its U, S2 per (i, x) at phr0 + i*V + x - O, and Joo's terms per range; the count of
+    // finished CTAs per range, then of finished ranges per solve
+    int4 *drlist = nullptr;
+    int ndrlist = 0, ndrranges = 0;
     DrpaSolveDev *drsolves = nullptr;
     int4 *drows = nullptr;
     int16_t *colpos = nullptr;
-    double *dru = nullptr, *drs2 = nullptr;
+    double *dru = nullptr, *drs2 = nullptr, *drj = nullptr;
     int *drdone = nullptr;
     double *part_e = nullptr, *part_dt = nullptr, *part_r = nullptr;
     double *red = nullptr;           // 3 per solve: sum e, max dt, max |r|
@@ -197,6 +198,8 @@ struct TermFlags {
 void launch_mp2(const DevBatch &d, cudaStream_t st);
 void launch_reduce(const DevBatch &d, cudaStream_t st);
 void launch_energy(const DevBatch &d, int kind, double csosex, cudaStream_t st);
+// virtuals a CTA of k_drpa_sums takes at most
+constexpr int kDrpaCols = 1024;
 // d.t <- T2aaaa of d.t (t(ij,a) - t(ij,b))
 void launch_to_aaaa(const DevBatch &d, cudaStream_t st);
 // drows and colpos (pre-set to -1) of the dRPA sums from the blocks

@@ -325,9 +325,10 @@ __global__ void __launch_bounds__(256) k_mosaic_sum(const int2 *__restrict__ tar
 //   Joo(k) = sum_c U(k,c),   Jvv(c) = sum_k U(k,c).
 // k_update then reads three values per amplitude where it walked 3 NOcc of them.
 //
-// One CTA per (solve, i), a thread per virtual x: each k adds one value of row (i,k) and one
-// of its mirror (k,i), at the column of x in that row's block (colpos), in ascending k.  The
-// last CTA of a solve to finish adds the columns of U up for Jvv.
+// One CTA per (solve, i) and range of at most kDrpaCols virtuals, a thread per virtual x: each k adds
+// one value of row (i,k) and one of its mirror (k,i), at the column of x in that row's block (colpos),
+// in ascending k.  The last CTA of a range to finish adds the columns of U up for Jvv, the last
+// range's the terms of Joo.  (One CTA for all of a wide basis: N=14 with 9,000 plane waves 135 us.)
 // Bound by memory latency: every amplitude read twice, near-coalesced (18 bytes with the column
 // index).  30 twists of N=54, 485 plane waves, per iteration: 0.052 ms here and 0.072 ms in
 // k_update, against 0.489 ms for the (i, x, l) intermediate, 0.048 ms of mosaic kernels and
@@ -354,20 +355,22 @@ __global__ void k_drpa_tables(const BlockDev *__restrict__ blocks, const SolveDe
 }
 
 __global__ void __launch_bounds__(kDrpaThreads)
-    k_drpa_sums(const int2 *__restrict__ list, const SolveDev *__restrict__ solves,
+    k_drpa_sums(const int4 *__restrict__ list, const SolveDev *__restrict__ solves,
                 const DrpaSolveDev *__restrict__ ds, const int4 *__restrict__ drows,
                 const int16_t *__restrict__ colpos, const int4 *__restrict__ nv4, const double *__restrict__ vtab,
-                const double *__restrict__ t, double *u, double *__restrict__ s2, double *__restrict__ jvv,
-                double *__restrict__ joo, int *__restrict__ done, const uint8_t *__restrict__ active)
+                const double *__restrict__ t, double *u, double *__restrict__ s2, double *jpart,
+                double *__restrict__ jvv, double *__restrict__ joo, int *done, int nranges,
+                const uint8_t *__restrict__ active)
 {
-    const int2 L = list[blockIdx.x];
+    const int4 L = list[blockIdx.x];
     if (!active[L.x]) return;
     const SolveDev s = solves[L.x];
     const DrpaSolveDev D = ds[L.x];
     const int O = s.O, V = s.V, i = L.y;
+    const int x0 = L.z * kDrpaCols, x1 = min(x0 + kDrpaCols, V), range = D.ch0 + L.z;
     __shared__ int4 row[kMaxOcc];
     __shared__ int mrow[kMaxOcc];
-    __shared__ bool last;
+    __shared__ bool last, whole;
     for (int k = threadIdx.x; k < O; k += kDrpaThreads) {
         row[k] = drows[D.rij0 + (int64_t)i * O + k];
         mrow[k] = drows[D.rij0 + (int64_t)k * O + i].x;
@@ -375,7 +378,7 @@ __global__ void __launch_bounds__(kDrpaThreads)
     __syncthreads();
     const int16_t *cp = colpos + D.cp0;
     double usum = 0.0;
-    for (int x = threadIdx.x; x < V; x += kDrpaThreads) {
+    for (int x = x0 + threadIdx.x; x < x1; x += kDrpaThreads) {
         double a1 = 0.0, a2 = 0.0;
 #pragma unroll 4
         for (int k = 0; k < O; k++) {
@@ -393,20 +396,35 @@ __global__ void __launch_bounds__(kDrpaThreads)
         usum += y;
     }
     usum = block_sum<kDrpaThreads>(usum);
-    if (threadIdx.x == 0) joo[s.joo0 + i] = usum;
-    // Jvv by the solve's last CTA: its reads of u follow every other CTA's fence and count
+    if (threadIdx.x == 0) {
+        if (D.nc == 1) joo[s.joo0 + i] = usum;
+        else jpart[D.jp0 + i * D.nc + L.z] = usum;
+    }
+    // Jvv by the range's last CTA: its reads of u follow every other CTA's fence and count
     __threadfence();
     __syncthreads();
-    if (threadIdx.x == 0) last = atomicAdd(&done[L.x], 1) == O - 1;
+    if (threadIdx.x == 0) last = atomicAdd(&done[range], 1) == O - 1;
     __syncthreads();
     if (!last) return;
     __threadfence();
-    for (int x = threadIdx.x; x < V; x += kDrpaThreads) {
+    for (int x = x0 + threadIdx.x; x < x1; x += kDrpaThreads) {
         double a = 0.0;
         for (int k = 0; k < O; k++) a += __ldcg(&u[s.phr0 + (int64_t)k * V + x]);
         jvv[s.jvv0 + x] = a;
     }
-    if (threadIdx.x == 0) done[L.x] = 0;
+    if (threadIdx.x == 0) {
+        done[range] = 0;
+        whole = D.nc > 1 && atomicAdd(&done[nranges + L.x], 1) == D.nc - 1;
+    }
+    __syncthreads();
+    if (!whole) return;
+    __threadfence();
+    for (int k = threadIdx.x; k < O; k += kDrpaThreads) {
+        double a = 0.0;
+        for (int c = 0; c < D.nc; c++) a += __ldcg(&jpart[D.jp0 + k * D.nc + c]);
+        joo[s.joo0 + k] = a;
+    }
+    if (threadIdx.x == 0) done[nranges + L.x] = 0;
 }
 
 // (The rings and crossed rings, CCD.f90:689-940, are in rings.cu.)
@@ -1035,7 +1053,8 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
     if ((f.do_ring || f.do_mosaic) && f.drpa) {
         kt->begin(KID_DRPA_SUMS, st);
         k_drpa_sums<<<d.ndrlist, kDrpaThreads, 0, st>>>(d.drlist, d.solves, d.drsolves, d.drows, d.colpos, d.nv4,
-                                                        d.vtab, d.t, d.dru, d.drs2, d.jvv, d.joo, d.drdone, d.active);
+                                                        d.vtab, d.t, d.dru, d.drs2, d.drj, d.jvv, d.joo, d.drdone,
+                                                        d.ndrranges, d.active);
         kt->end(st);
         n++;
     }

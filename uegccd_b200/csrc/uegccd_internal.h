@@ -110,9 +110,10 @@ struct RingPairDev {
 };
 
 // Where a solve's dRPA lookups start: rows of its pairs (O*O entries), columns of its blocks
-// (nblk*V entries).
+// (nblk*V entries); its nc column ranges, the first of which is ch0, and their sums (O*nc entries).
 struct DrpaSolveDev {
     int64_t rij0, cp0;
+    int ch0, nc, jp0, pad;
 };
 
 // Pairs [first, first + count) of one solve and one row class, done by one CTA of k_rings.
