@@ -67,3 +67,21 @@ def test_drpa_over_column_ranges(electrons, virtuals):
     (want,) = x.iterate([p + m], lambda a: (x.drpa_residual(a),), 1e-8, 2.0)
     want = x.out(want)
     assert np.abs(t[0] - want).max() <= 1e-12 * np.abs(want).max()
+
+
+@pytest.mark.parametrize("electrons,basis,name", [(2, 3000, "k_ladder_fma"), (14, 3000, "k_ladder_fma"),
+                                                  (54, 485, "k_ladder_mma"), (54, 1500, "k_ladder_fma")])
+def test_a_short_ladder_is_spread_over_the_sms(electrons, basis, name):
+    """Beside other kernels an SM takes no more of the ladder's CTAs than their share of the GPU: what
+    shared memory each one holds leaves no room for another.  (Packed on the first SMs that come free, an
+    iteration took up to four times as long, at random.)"""
+    from uegccd_b200 import Batch
+
+    b = Batch([_system(electrons, basis)])
+    launches = _kernels(lambda: b.solve(scheme=1, ndiis=6, denom_factor=1.0, max_iter=4, raise_on_error=False), name)
+    assert launches
+    for grid, shared in launches:
+        share = -(-grid // SMS)
+        assert share <= 4
+        assert SM_SHARED // (shared + 1024) == share, (grid, shared)
+    b.close()

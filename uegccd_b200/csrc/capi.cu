@@ -1160,7 +1160,7 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     d.ntargets = (int)targets.size();
     d.max_v = max_v;
     for (int f = 0; f < 2; f++) {
-        d.ladder_smem[f] = ladder_smem_bytes(q2m, n2m, max_rows, f);
+        d.ladder_smem[f] = ladder_smem_bytes(q2m, n2m, max_rows, f, d.nltiles[f]);
         set_ladder_smem_limit(d.ladder_smem[f]);
     }
     // K blocks of more than some 9000 virtuals are outside what the kernels are checked for

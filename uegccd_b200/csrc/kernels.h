@@ -105,8 +105,8 @@ constexpr int kLadderFmaRows = 4, kLadderMmaRows = 16;
 constexpr int kLadderFmaCols = 256;
 constexpr int ladder_pass_cols(int np) { return np <= 8 ? 128 : 64; }
 // dynamic shared memory for |q|^2 tables up to q2max, |n|^2 up to n2max and blocks of at most
-// max_rows rows i <= j; form 0 FMA, 1 DMMA
-size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form);
+// max_rows rows i <= j, launched in so many tiles; form 0 FMA, 1 DMMA
+size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form, int tiles);
 void set_ladder_smem_limit(size_t bytes);
 // G of the rows i <= j: the particle-particle ladder of t (do_pp), the hole-hole one (do_hh); the
 // DMMA form on st_mma.  Returns the launches.

@@ -539,16 +539,33 @@ size_t fma_bytes(int r)
 
 }  // namespace
 
-size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form)
+// A launch of fewer tiles than the GPU holds at a time asks for so much shared memory that no SM takes
+// more of them than its share: with the rings and the mosaics running beside it, the ladder's CTAs are
+// else packed on the SMs that come free first, up to seven on one.  Up to four tiles an SM;
+// with more the packing costs nothing.  Times of one iteration in us, not spread (the range of six
+// graphs of the same batch) and spread: N=2, 6,000 plane waves (12 tiles) 290 to 1,150, 293; N=14, 3,000 (131) 176
+// to 520, 176, and 9,000 (385) 890 to 2,020, 893 to 978; N=30, 2,500 (281) 362 to 502, 246; N=54, 2,500
+// (466, and 256 of the DMMA form) 562 to 591, 394; one N=54 system with 485 plane waves (114 and 52) 73, 71,
+// three 96, 87, eight (908 and 442, five an SM) 156 and, spread over five, 163.
+constexpr int kSms = 148, kSpread = 4;
+constexpr size_t kSmShared = 228 * 1024;   // of an SM; each CTA takes 1 KB of it for itself
+size_t spread_bytes(int tiles)
+{
+    const int per_sm = (tiles + kSms - 1) / kSms;
+    return per_sm >= 1 && per_sm <= kSpread ? kSmShared / (per_sm + 1) : 0;
+}
+
+size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form, int tiles)
 {
     const size_t tab = tab_bytes(tab_form(q2max, n2max), q2max);
     if (form == 0) {
         size_t b = 0;
         for (int r = 1; r <= std::min(max_rows, kLadderFmaRows); r++) b = std::max(b, fma_bytes(r));
-        return tab + b;
+        return std::max(tab + b, spread_bytes(tiles));
     }
     const int nr = max_rows <= 8 ? 8 : 16;
-    return tab + sizeof(int2) * 2 * kKC + sizeof(double) * (2 * 2 * (size_t)nr * kLd + 2 * (size_t)nr * kHLd);
+    return std::max(tab + sizeof(int2) * 2 * kKC + sizeof(double) * (2 * 2 * (size_t)nr * kLd + 2 * (size_t)nr * kHLd),
+                    spread_bytes(tiles));
 }
 
 void set_ladder_smem_limit(size_t bytes)
