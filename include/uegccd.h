@@ -314,9 +314,9 @@ int uegccd_trim_cache(void);
 int uegccd_batch_history(UegccdBatch *b, int32_t s, double *energies, double *dts, int32_t max_rec,
                          int32_t *n_recorded);
 
-/* CTA sizes of the ring kernel's pair classes: up to 256 threads each, the same for every batch
- * (eight, four or two small pairs, or one large one, a CTA).  Writes at most max values; returns
- * how many. */
+/* CTA sizes of the ring kernel, by the group pairs a CTA works on at a time (eight, four, two, one):
+ * the largest of each kind, the same for every batch (a kind has CTAs of 192 threads too).  Writes at
+ * most max values; returns how many. */
 int32_t uegccd_batch_ring_threads(UegccdBatch *b, int32_t *threads, int32_t max);
 /* The launch shapes of a batch (new; the reference has no launches): the four ring CTA sizes
  * above, the CTA size of the ring staging kernel (64, 128 or 256: picked by timing on the batch's

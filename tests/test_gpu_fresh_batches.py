@@ -88,3 +88,39 @@ def test_side_streams_of_many_threads_and_live_batches():
     for b, w in zip(live, want):
         assert [r["ecorr"] for r in b.solve(**DIIS)[2]] == w[1]
         b.close()
+
+
+def test_reported_launch_shapes_are_those_launched():
+    """ring_threads and launch_shapes against the profile of a solve with ring groups of all sizes."""
+    import json
+    import os
+    import re
+    import tempfile
+
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    from uegccd_b200 import Batch
+
+    torch.cuda.init()
+    b = Batch(_systems(1, 114, 1140))
+    b.solve(**DIIS)
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        b.solve(**DIIS)
+    with tempfile.TemporaryDirectory() as d:
+        path = os.path.join(d, "trace.json")
+        p.export_chrome_trace(path)
+        with open(path) as f:
+            events = [e for e in json.load(f)["traceEvents"] if e.get("cat") == "kernel"]
+    sizes = {}   # rows of group 1 in eights -> threads
+    for e in events:
+        m = re.search(r"k_rings<\w+, (\d)>", e["name"])
+        if m:
+            sizes[int(m.group(1))] = e["args"]["block"][0]
+    assert sorted(sizes) == [1, 2, 3, 4, 6, 8]
+    of = {8: [1], 4: [2], 2: [3, 4], 1: [6, 8]}   # pairs a CTA
+    shapes = b.launch_shapes()
+    assert b.ring_threads() == shapes["ring_threads"] == [max(sizes[n] for n in of[k]) for k in (8, 4, 2, 1)]
+    stage = {e["args"]["block"][0] for e in events if "k_ring_stage" in e["name"]}
+    assert stage == {shapes["stage_threads"]}
+    b.close()

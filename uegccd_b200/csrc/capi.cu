@@ -2574,14 +2574,14 @@ int uegccd_batch_advance(UegccdBatch *b, int32_t rounds, int32_t *n_active, int3
     return session_advance(*b, rounds, n_active, n_done, done_ids, done_results);
 }
 
-// Values of the four ring entries of the two calls below: k_rings' CTAs are of one size.
-static constexpr int kRingShapes = 4, kRingCta = 256;
+// The four ring entries of the two calls below, by the pairs a CTA of k_rings works on at a time
+static constexpr int kRingShapes = 4, kRingPairs[kRingShapes] = {8, 4, 2, 1};
 
 int32_t uegccd_batch_ring_threads(UegccdBatch *b, int32_t *threads, int32_t max)
 {
     if (!b || !threads || max <= 0) return fail(UEGCCD_ERR_ARG, "bad argument");
     const int n = std::min<int>(max, kRingShapes);
-    for (int c = 0; c < n; c++) threads[c] = kRingCta;
+    for (int c = 0; c < n; c++) threads[c] = ring_cta_threads(kRingPairs[c]);
     return n;
 }
 
@@ -2589,10 +2589,10 @@ int32_t uegccd_batch_launch_shapes(UegccdBatch *b, int32_t *vals, int32_t max)
 {
     if (!b || !vals || max <= 0) return fail(UEGCCD_ERR_ARG, "bad argument");
     int32_t v[kRingShapes + 3];
-    for (int c = 0; c < kRingShapes; c++) v[c] = kRingCta;
+    for (int c = 0; c < kRingShapes; c++) v[c] = ring_cta_threads(kRingPairs[c]);
     v[kRingShapes] = b->d.stage_threads;
-    v[kRingShapes + 1] = 1;    // ladder tiles: always the longest first
-    v[kRingShapes + 2] = 32;   // virtuals per staged chunk of the DMMA ladder
+    v[kRingShapes + 1] = 1;   // ladder tiles: always the longest first (ladder_tiles)
+    v[kRingShapes + 2] = ladder_chunk();
     const int n = std::min<int>(max, kRingShapes + 3);
     for (int k = 0; k < n; k++) vals[k] = v[k];
     return n;

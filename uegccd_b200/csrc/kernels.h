@@ -108,6 +108,7 @@ constexpr int ladder_pass_cols(int np) { return np <= 8 ? 128 : 64; }
 // max_rows rows i <= j, launched in so many tiles; form 0 FMA, 1 DMMA
 size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form, int tiles);
 void set_ladder_smem_limit(size_t bytes);
+int ladder_chunk();   // virtuals per staged chunk of the DMMA form
 // G of the rows i <= j: the particle-particle ladder of t (do_pp), the hole-hole one (do_hh); the
 // DMMA form on st_mma.  Returns the launches.
 int launch_ladder(const DevBatch &d, const double *t, int do_pp, int do_hh, double *g, cudaStream_t st,
@@ -117,6 +118,7 @@ constexpr int kRingClasses = 6;
 constexpr int kRingFrags[kRingClasses] = {1, 2, 3, 4, 6, 8};
 int ring_class(int n1);             // -1: more than 64 rows (NOcc <= 64 keeps every group below)
 int ring_pairs_per_pass(int c);     // pairs a CTA works on at a time
+int ring_cta_threads(int pairs);    // the largest CTA of the classes that work on so many pairs at a time
 int ring_doubles(int c, int max_n2);
 size_t ring_smem_bytes(const DevBatch &d, int c, int max_n2);
 void set_rings_smem_limit(size_t bytes);

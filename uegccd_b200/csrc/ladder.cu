@@ -568,6 +568,8 @@ size_t ladder_smem_bytes(int q2max, int n2max, int max_rows, int form, int tiles
                     spread_bytes(tiles));
 }
 
+int ladder_chunk() { return kKC; }
+
 void set_ladder_smem_limit(size_t bytes)
 {
     static std::mutex mu;

@@ -329,6 +329,14 @@ int ring_class(int n1)
 
 int ring_pairs_per_pass(int c) { return ring_groups(kRingFrags[c]); }
 
+int ring_cta_threads(int pairs)
+{
+    int t = 0;
+    for (int nf : kRingFrags)
+        if (ring_groups(nf) == pairs) t = std::max(t, ring_threads(nf));
+    return t;
+}
+
 size_t ring_smem_bytes(const DevBatch &d, int c, int max_n2)
 {
     return tab_bytes(d) + sizeof(double) * (size_t)ring_buffers(kRingFrags[c]) * ring_groups(kRingFrags[c]) * pair_doubles(kRingFrags[c], max_n2);

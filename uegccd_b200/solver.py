@@ -233,7 +233,7 @@ class Batch:
         return _sf_call(self._systems[s], lambda g: capi.lib().uegccd_batch_structure_factor(self._h, s, g))
 
     def ring_threads(self) -> list:
-        """CTA size of each ring pair class."""
+        """Largest CTA of the ring kernel for eight, four, two and one pairs a CTA."""
         a = (C.c_int32 * 8)()
         n = capi.lib().uegccd_batch_ring_threads(self._h, a, 8)
         if n < 0:
@@ -241,7 +241,7 @@ class Batch:
         return list(a[:n])
 
     def launch_shapes(self) -> dict:
-        """Ring CTA sizes per class, the ring staging CTA size (picked on the first CCD solve),
+        """Ring CTA sizes (ring_threads), the ring staging CTA size (picked on the first CCD solve),
         the ladder tile order (0 block order, 1 longest first), the ladder's column chunk."""
         a = (C.c_int32 * 8)()
         n = capi.lib().uegccd_batch_launch_shapes(self._h, a, 8)
