@@ -124,3 +124,31 @@ def test_reported_launch_shapes_are_those_launched():
     stage = {e["args"]["block"][0] for e in events if "k_ring_stage" in e["name"]}
     assert stage == {shapes["stage_threads"]}
     b.close()
+
+
+@pytest.mark.parametrize("options", [dict(), DIIS, dict(DIIS, precision=1), dict(drpa=True), dict(do_ring=1, do_xring=0)],
+                         ids=["replay", "diis", "mixed", "drpa", "two channels"])
+@pytest.mark.parametrize("count,electrons,basis", [(2, 54, 485), (3, 14, 60)])
+def test_reported_launches_are_those_made(count, electrons, basis, options):
+    """kernel_launches of a solve against the kernels of its profile: all but the MP2 start's two (or
+    three, with dRPA's T2aaaa), which are not the solve's."""
+    import torch
+    from torch.profiler import ProfilerActivity, profile
+
+    from uegccd_b200 import Batch
+
+    torch.cuda.init()
+    b = Batch(_systems(count, electrons, basis))
+    b.solve(**options)
+    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+        _, _, res = b.solve(**options)
+    kernels = {e.key: e.count for e in p.key_averages() if "uegccd::" in e.key}
+    two = "do_xring" in options
+    made = sum(n for k, n in kernels.items()
+               if not (two and ("::k_" in k or "k_unpack" in k or "k_pack" in k)))
+    if two:   # one count a system; the batch's own kernels around the solves are not counted
+        assert sum(r["kernel_launches"] for r in res) == made, kernels
+    else:
+        start = 3 if options.get("drpa") else 2
+        assert all(r["kernel_launches"] == made - start for r in res), (res[0]["kernel_launches"], made, kernels)
+    b.close()

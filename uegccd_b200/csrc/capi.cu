@@ -1843,10 +1843,7 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
         for (int round = 0; round < most && stop == 0; round++) {
             // the refresh is not queued ahead: it costs as much as an iteration
             if (f.mixed && it > 0 && (stop = stopped(it - 1)) != 0) break;
-            if (f.mixed) {
-                launch_refresh(d, b.stream);
-                b.launches += 2;
-            }
+            if (f.mixed) b.launches += launch_refresh(d, b.stream);
             for (int k = 0; k < kPoll && stop == 0; k++, it++) {
                 if (b.kt.on && k == kPoll - 1) {
                     // the sampled iteration of the round: direct launches between CUDA events

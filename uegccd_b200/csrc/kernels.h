@@ -237,12 +237,12 @@ void launch_ring_rows(const DevBatch &d, int n, const int *row0, cudaStream_t st
 // lbase: its first list entry; smem: (max V + O) ints)
 void launch_mosaic_targets(const DevBatch &d, const int *tbase, const int64_t *lbase, size_t smem, cudaStream_t st);
 // Mixed precision: FP16 tcgen05 ladder of t - t_ref added to g (plus g_ref); writes the
-// scaled FP16 d tiles first (d.w16 must be built)
-void launch_ladder_tc(const DevBatch &d, const double *t_ref, const double *g_ref, int *err, cudaStream_t st);
+// scaled FP16 d tiles first (d.w16 must be built).  Returns the launches.
+int launch_ladder_tc(const DevBatch &d, const double *t_ref, const double *g_ref, int *err, cudaStream_t st);
 // The static FP16 Coulomb slabs of the tensor-core ladder, from the current |q|^2 tables
 void launch_w16_build(const DevBatch &d, cudaStream_t st);
-// Refresh point: t_ref <- t and g_ref <- FP64 particle-particle ladder of t_ref
-void launch_refresh(const DevBatch &d, cudaStream_t st);
+// Refresh point: t_ref <- t and g_ref <- FP64 particle-particle ladder of t_ref.  Returns the launches.
+int launch_refresh(const DevBatch &d, cudaStream_t st);
 // Device-side iteration control
 void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
                  cudaStream_t st);

@@ -765,10 +765,10 @@ __global__ void k_copy(int64_t n, const double *__restrict__ src, double *__rest
     if (p < n) dst[p] = src[p];
 }
 
-void launch_refresh(const DevBatch &d, cudaStream_t st)
+int launch_refresh(const DevBatch &d, cudaStream_t st)
 {
     k_copy<<<(unsigned)((d.namp + 255) / 256), 256, 0, st>>>(d.namp, d.t, d.t_ref);
-    launch_ladder(d, d.t_ref, 1, 0, d.g_ref, st, st);
+    return 1 + launch_ladder(d, d.t_ref, 1, 0, d.g_ref, st, st);
 }
 
 void launch_tail(const DevBatch &d, const CtlBuffers &c, double tol, int max_iter, int ndiis, int init,
@@ -1034,9 +1034,8 @@ int launch_residual(const DevBatch &d, const TermFlags &f, int mode, double *g_o
         kt->end(st);
         if (f.do_pp && f.mixed) {
             kt->begin(KID_LADDER_TC, st);
-            launch_ladder_tc(d, d.t_ref, d.g_ref, d.tc_err, st);
+            n += launch_ladder_tc(d, d.t_ref, d.g_ref, d.tc_err, st);
             kt->end(st);
-            n += (d.ntc16 > 0) + (d.ntc32 > 0) + (d.ntc64 > 0);
         }
     }
     if (f.do_mosaic && !f.drpa) {

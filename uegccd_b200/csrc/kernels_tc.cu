@@ -361,7 +361,7 @@ void launch_w16_build(const DevBatch &d, cudaStream_t st)
                                                static_cast<__half *>(d.w16));
 }
 
-void launch_ladder_tc(const DevBatch &d, const double *t_ref, const double *g_ref, int *err, cudaStream_t st)
+int launch_ladder_tc(const DevBatch &d, const double *t_ref, const double *g_ref, int *err, cudaStream_t st)
 {
     const __half *w = static_cast<const __half *>(d.w16), *dd = static_cast<const __half *>(d.d16);
     if (d.ndtiles > 0)
@@ -376,6 +376,7 @@ void launch_ladder_tc(const DevBatch &d, const double *t_ref, const double *g_re
     if (d.ntc64)
         k_ladder_tc<64><<<d.ntc64, 128, 0, st>>>(d.tctiles + d.ntc16 + d.ntc32, d.tcx + d.ntc16 + d.ntc32,
                                                   d.blocks, w, dd, d.dscale, g_ref, d.g, d.active, err);
+    return (d.ndtiles > 0) + (d.ntc16 > 0) + (d.ntc32 > 0) + (d.ntc64 > 0);
 }
 
 }  // namespace uegccd

@@ -979,7 +979,10 @@ int TwoChannel::residual(bool drpa, int mask)
 {
     if (mm_on_) {
         mm_->sets = f_.lad_lin_d == f_.lad_lin_x && f_.lad_quad_d == f_.lad_quad_x ? 1 : 2;
-        if (!weights_) tc_mm_weights(*mm_, f_, st_);
+        if (!weights_) {
+            tc_mm_weights(*mm_, f_, st_);
+            launches_++;
+        }
         weights_ = true;
         launches_ += tc_mm_residual(*mm_, f_, mask, t_[0], t_[1], jvv_, joo_, g_[0], g_[1], st_);
         TCU(cudaGetLastError());
