@@ -8,9 +8,12 @@
 
 namespace uegccd {
 
-// Raw device pointers of one batch (owned by the Batch object in capi.cu).
+// The |q|^2 table's form in the ladders and the rings, and of the records both look it up with: 16
+// copies in shared memory and |n|^2 carried in a record's fourth byte.
+inline bool table16(int q2max, int n2max) { return q2max < 256 && n2max < 128; }
 constexpr int kVtabSmemEntries = 1024;   // |q|^2 table entries a kernel stages in shared memory at most
 
+// Raw device pointers of one batch (owned by the Batch object in capi.cu).
 struct DevBatch {
     int nsolves = 0, nblocks = 0, ntiles = 0, nchunks = 0, nrchunks = 0, ntargets = 0;
     int max_v = 0;      // largest v_K

@@ -512,10 +512,7 @@ __global__ void k_ring_rows(int n, const int *__restrict__ row0, int nsolves, co
         else hi = m - 1;
     }
     const SolveDev &s = solves[lo];
-    auto m2 = [&](int p) {
-        const int x = (int8_t)p, y = (int8_t)(p >> 8), z = (int8_t)(p >> 16);
-        return ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16) | (carry ? 1 << 24 : 0);
-    };
+    auto m2 = [&](int p) { return neg2(p) | (carry ? 1 << 24 : 0); };
     const int pi = nvp[s.orb0 + ph_i[r]], px = nvp[s.orb0 + ph_x[r]];
     RingRowDev R;
     const int ni2 = __dp4a(pi, pi, 0);
@@ -529,7 +526,7 @@ __global__ void k_ring_rows(int n, const int *__restrict__ row0, int nsolves, co
 
 void launch_ring_rows(const DevBatch &d, int n, const int *row0, cudaStream_t st)
 {
-    const int carry = d.q2max < 256 && d.n2max < 128;
+    const int carry = table16(d.q2max, d.n2max);
     if (n > 0)
         k_ring_rows<<<(n + 255) / 256, 256, 0, st>>>(n, row0, d.nsolves, d.solves, d.ph_i, d.ph_x, d.nvp, carry, d.rrows);
 }

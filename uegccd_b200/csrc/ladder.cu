@@ -47,6 +47,7 @@
 
 #include "kernels.h"
 #include "uegccd_internal.h"
+#include "warp.cuh"
 
 namespace uegccd {
 
@@ -58,13 +59,6 @@ constexpr int kFC = 256;           // the same, FMA form
 constexpr int kLd = kKC + 4;       // row stride of the DMMA operands: = 4 mod 16 doubles, conflict-free
 constexpr int kHLd = 36;           // row stride of H (at most 32 pairs q <= q'): likewise
 
-__device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 // Table forms: 16 copies or one in shared memory, or global memory.
 enum { kTab16 = 0, kTab1 = 1, kTabGlobal = 2 };
 
@@ -73,15 +67,14 @@ struct Col {
     int m2, base;
 };
 
-// With 16 copies every |n|^2 is at most 127 (launch_ladder's rule): the column side carries it
+// With 16 copies every |n|^2 is at most 127 (table16): the column side carries it
 // in its fourth byte, against a 1 on the row side.
 template <int TAB>
 __device__ __forceinline__ Col make_col(int packed)
 {
-    const int x = (int8_t)packed, y = (int8_t)(packed >> 8), z = (int8_t)(packed >> 16);
-    const int n2 = x * x + y * y + z * z;
+    const int n2 = __dp4a(packed, packed, 0);
     Col c;
-    c.m2 = ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16);   // |n_d| <= 63
+    c.m2 = neg2(packed);
     if (TAB == kTab16) c.m2 |= 1 << 24;
     c.base = TAB == kTab16 ? (n2 << 7) + ((threadIdx.x & 15) << 3) : TAB == kTab1 ? n2 << 3 : n2;
     return c;
@@ -524,7 +517,10 @@ __global__ void __launch_bounds__(kThreads, 5) k_ladder_mma(Args A)
     else ladder_mma<TAB, 2>(A, K, lsm, sm);
 }
 
-int tab_form(int q2max, int n2max) { return q2max < 256 && n2max < 128 ? kTab16 : q2max < 1024 ? kTab1 : kTabGlobal; }
+int tab_form(int q2max, int n2max)
+{
+    return table16(q2max, n2max) ? kTab16 : q2max < kVtabSmemEntries ? kTab1 : kTabGlobal;
+}
 int tab_bytes(int form, int q2max)
 {
     return form == kTab16 ? (q2max + 1) * 128 : form == kTab1 ? ((q2max + 1) * 8 + 15) / 16 * 16 : 0;

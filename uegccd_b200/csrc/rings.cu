@@ -50,6 +50,7 @@
 
 #include "kernels.h"
 #include "uegccd_internal.h"
+#include "warp.cuh"
 
 namespace uegccd {
 
@@ -60,27 +61,11 @@ constexpr int ring_groups(int nf) { return nf == 1 ? 8 : nf == 2 ? 4 : nf <= 4 ?
 constexpr int ring_threads(int nf) { return 32 * nf * ring_groups(nf); }
 constexpr int ring_buffers(int nf) { return nf <= 4 ? 2 : 1; }
 
-__device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-
 // The barrier of one group of warps (0: the whole CTA's)
 __device__ __forceinline__ void group_sync(int id, int threads)
 {
     asm volatile("bar.sync %0, %1;\n" ::"r"(id), "r"(threads) : "memory");
 }
-
-__device__ __forceinline__ void cp_async16(void *dst, const void *src)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 struct Col {
     int m2, base;
@@ -303,7 +288,7 @@ __global__ void __launch_bounds__(ring_threads(NF), NF <= 3 ? 3 : 2) k_rings(Arg
     }
 }
 
-bool tab16(const DevBatch &d) { return d.q2max < 256 && d.n2max < 128; }
+bool tab16(const DevBatch &d) { return table16(d.q2max, d.n2max); }
 int tab_bytes(const DevBatch &d)
 {
     return tab16(d) ? (d.q2max + 1) * 128 : d.q2max < kVtabSmemEntries ? ((d.q2max + 1) * 8 + 15) / 16 * 16 : 0;

@@ -922,7 +922,7 @@ struct TwoChannel::Workspace {
         D.kl0 = reinterpret_cast<int *>(base + kl0), D.kl = reinterpret_cast<int *>(base + kl);
         D.kl_ij = reinterpret_cast<int *>(base + klij), D.pairs = reinterpret_cast<int4 *>(base + pairs);
         D.ph = reinterpret_cast<int *>(base + ph);
-        cudaError_t e = tc_mm_limits(D);
+        cudaError_t e = tc_mm_limits();
         auto copy = [&](size_t at, const void *src, size_t n) {
             if (e == cudaSuccess && n > 0) e = cudaMemcpyAsync(base + at, src, n, cudaMemcpyHostToDevice, t.st_);
         };

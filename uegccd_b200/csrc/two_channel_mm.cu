@@ -18,6 +18,7 @@
 #include <algorithm>
 
 #include "two_channel_mm.h"
+#include "warp.cuh"
 
 namespace uegccd {
 
@@ -39,21 +40,6 @@ __device__ __forceinline__ int q2v(int4 a, int4 b)
     const int x = a.x - b.x, y = a.y - b.y, z = a.z - b.z;
     return x * x + y * y + z * z;
 }
-
-__device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
-{
-    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
-                 : "+d"(d0), "+d"(d1)
-                 : "d"(a), "d"(b));
-}
-__device__ __forceinline__ void cp_async16(double *dst, const double *src)
-{
-    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
-template <int N>
-__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 // W by rows c: direct integrals of the V virtuals and the O occupied orbitals, then (sets = 2)
 // the exchange ones.  The padding stays zero (preset).
@@ -388,14 +374,13 @@ __device__ void rings_pair(const TcMm &D, const TcFlags &f, const int4 P, const 
 }
 
 // Three CTAs an SM (80 registers, some spilled) and the largest pairs first: 43 -> 40 us.
-__global__ void __launch_bounds__(kThreads, 3) k2m_rings(TcMm D, TcFlags f, int rings, int xrings,
+__global__ void __launch_bounds__(kThreads, 3) k2m_rings(TcMm D, TcFlags f, int rings,
                                                       const double *__restrict__ tab, const double *__restrict__ tba)
 {
     extern __shared__ double sm[];
     const int4 P = D.pairs[blockIdx.x];
     if (blockIdx.y == 0 && rings) rings_pair<false>(D, f, P, tab, tba, D.gr[0], D.gr[1], sm);
     else rings_pair<true>(D, f, P, tab, tba, D.gx[0], D.gx[1], sm);
-    (void)xrings;
 }
 
 // Every term of one amplitude x = (i,j,a), b its momentum partner, from the products above.
@@ -463,7 +448,7 @@ size_t tc_mm_ring_smem(int n1, int n2)
 
 size_t tc_mm_stage_smem(int O) { return sizeof(double) * (std::max((size_t)O * O, (size_t)kThreads) + O); }
 
-cudaError_t tc_mm_limits(const TcMm &D)
+cudaError_t tc_mm_limits()
 {
     cudaError_t e = cudaFuncSetAttribute(k2m_gemm, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                          (int)(2 * kStages * kKC * kLd * sizeof(double)));
@@ -472,7 +457,6 @@ cudaError_t tc_mm_limits(const TcMm &D)
         e = cudaFuncSetAttribute(k2m_rings, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcMmSmemMax);
     if (e == cudaSuccess)
         e = cudaFuncSetAttribute(k2m_stage, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTcMmSmemMax);
-    (void)D;
     return e;
 }
 
@@ -494,7 +478,7 @@ int tc_mm_residual(const TcMm &D, const TcFlags &f, int mask, const double *tab,
     }
     const int rings = (mask & 8) != 0, xrings = (mask & 16) != 0;
     if ((rings || xrings) && D.npairs > 0) {
-        k2m_rings<<<dim3(D.npairs, rings + xrings), kThreads, D.ring_smem, st>>>(D, f, rings, xrings, tab, tba);
+        k2m_rings<<<dim3(D.npairs, rings + xrings), kThreads, D.ring_smem, st>>>(D, f, rings, tab, tba);
         n++;
     }
     k2m_assemble<<<(D.n + kThreads - 1) / kThreads, kThreads, 0, st>>>(D, f, mask, tab, tba, jvv, joo, gab, gba);

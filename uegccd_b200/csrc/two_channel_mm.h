@@ -35,7 +35,7 @@ struct TcMm {
 
 size_t tc_mm_ring_smem(int n1, int n2);
 size_t tc_mm_stage_smem(int O);
-cudaError_t tc_mm_limits(const TcMm &D);
+cudaError_t tc_mm_limits();
 void tc_mm_weights(const TcMm &D, const TcFlags &f, cudaStream_t st);
 // G of the terms in mask (two_channel.h); returns the launches.
 int tc_mm_residual(const TcMm &D, const TcFlags &f, int mask, const double *tab, const double *tba, double *jvv,

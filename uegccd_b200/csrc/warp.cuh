@@ -1,4 +1,4 @@
-// Warp reductions and packed-vector arithmetic shared by the kernels.
+// Warp reductions, packed-vector arithmetic and the PTX of the FP64 tensor-core kernels, shared by them.
 #pragma once
 
 #include <cstdint>
@@ -49,5 +49,22 @@ __device__ __forceinline__ int neg2(int p)
     const int x = (int8_t)p, y = (int8_t)(p >> 8), z = (int8_t)(p >> 16);
     return ((-2 * x) & 0xff) | (((-2 * y) & 0xff) << 8) | (((-2 * z) & 0xff) << 16);
 }
+
+// One FP64 product of fragments, 8 x 4 by 4 x 8: d += a b (mma.sync; tcgen05 has no f64 kind)
+__device__ __forceinline__ void dmma_884(double &d0, double &d1, double a, double b)
+{
+    asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
+                 : "+d"(d0), "+d"(d1)
+                 : "d"(a), "d"(b));
+}
+
+__device__ __forceinline__ void cp_async16(void *dst, const void *src)
+{
+    const unsigned d = (unsigned)__cvta_generic_to_shared(dst);
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(d), "l"(src) : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::: "memory"); }
+template <int N>
+__device__ __forceinline__ void cp_async_wait() { asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory"); }
 
 }  // namespace uegccd
