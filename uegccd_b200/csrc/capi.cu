@@ -1273,7 +1273,6 @@ int build_batch(const UegccdSystem *systems, int n, std::unique_ptr<UegccdBatch>
     if ((rc = b->alloc(d.ph_b, phr0))) return rc;
     if ((rc = b->alloc(d.rpos, amp0))) return rc;
     if ((rc = b->alloc(d.t, amp0))) return rc;
-    if ((rc = b->alloc(d.t_new, amp0))) return rc;
     if ((rc = b->alloc(d.g, amp0))) return rc;
     if ((rc = b->alloc(d.jvv, jvv0))) return rc;
     if ((rc = b->alloc(d.joo, joo0))) return rc;
@@ -2405,8 +2404,9 @@ int uegccd_ccd_g2_ex(UegccdCtx *c, const double *t_abab, int32_t mask, int32_t p
         CU(cudaMemsetAsync(d.tc_err, 0, sizeof(int), b.stream));
         f.mixed = 1;
     }
-    // g_out reuses t_new (mode 1 does not write the update)
-    launch_residual(d, f, 1, d.t_new, b.stream);
+    // G takes the ladder's place: k_update reads an amplitude's ladder value where it writes its G, and
+    // none of a mirror
+    launch_residual(d, f, 1, d.g, b.stream);
     CU(cudaGetLastError());
     if (precision == UEGCCD_MIXED) {
         int err = 0;
@@ -2414,7 +2414,7 @@ int uegccd_ccd_g2_ex(UegccdCtx *c, const double *t_abab, int32_t mask, int32_t p
         CU(cudaStreamSynchronize(b.stream));
         if (err) return fail(UEGCCD_ERR_CUDA, "tensor-core ladder: an mbarrier wait expired");
     }
-    return unpack_to_host(b, 0, d.t_new, g_abab, nullptr, nullptr);
+    return unpack_to_host(b, 0, d.g, g_abab, nullptr, nullptr);
 }
 
 int32_t uegccd_sf_length(const UegccdSystem *sys)
@@ -2637,7 +2637,7 @@ int uegccd_footprint(const UegccdSystem *sys, int32_t ndiis, int32_t mixed, int6
     int64_t b = 0;
     int64_t sum_ov = 0;
     for (const auto &B : P.blocks) sum_ov += B.o + B.v;
-    b += A * (8 * 3 + sizeof(AmpInfo) + 4 + 8);      // t, t_new, g; amps; partner, ring positions
+    b += A * (8 * 2 + sizeof(AmpInfo) + 4 + 8);      // t, g; amps; partner, ring positions
     b += sum_ov * (8 + 4) + (V + O + 1) * (4 + 8);   // mosaic partials and target lists
     b += O * O * V * 4;                              // pos
     b += O * V * 8 * 2 + O * O * 16 + nblk * V * 2;  // dRPA sums and lookups (allocated for dRPA only)

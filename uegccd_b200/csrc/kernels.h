@@ -46,7 +46,7 @@ struct DevBatch {
     int4 *nv4 = nullptr;
     int *nvp = nullptr;              // the same vectors packed a component per byte (warp.cuh)
     double *eigen = nullptr, *vtab = nullptr;
-    double *t = nullptr, *t_new = nullptr, *g = nullptr;
+    double *t = nullptr, *g = nullptr;
     double *jvv = nullptr, *joo = nullptr;
     // dRPA (on the first dRPA solve): k_drpa_sums' CTA list {solve, i, column range}, row and column
     // lookups, its U, S2 per (i, x) at phr0 + i*V + x - O, and Joo's terms per range; the count of

@@ -209,7 +209,7 @@ struct UpdateArgs {
     const double *jvv, *joo;
     const double *dru, *drs2;     // dRPA: U and S2 of k_drpa_sums
     double *part_e, *part_dt, *part_r;
-    double *g_out;                // optional: full G per amplitude (term checks)
+    double *g_out;                // optional: full G per amplitude (term checks); may be g_ladder
     const double *rx;             // ring and crossed-ring G, particle-hole layout
     const int2 *rpos;             // where each amplitude's two values sit in it
     const uint8_t *active;
