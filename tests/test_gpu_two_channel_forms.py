@@ -88,3 +88,35 @@ def test_one_context_through_the_forms():
         own.set_eri(FORMS[name][0], safe_eri=True, screening=sd)
         for x, y in zip(ctx.ccd_g2_2ch(tb, tc, 31), own.ccd_g2_2ch(tb, tc, 31)):
             assert np.array_equal(x, y), name
+
+
+@pytest.mark.parametrize("nel,cut", [(2, 3), (14, 5)])
+def test_a_repeated_selection_is_not_made_again(nel, cut):
+    """A second residual with the same integrals uploads the amplitudes and nothing else; a new selection,
+    and the old one after it, are taken up."""
+    o = _setup(nel, cut, ONE)
+    sc = o.scalars()
+    ctx = Context(o.nocc, sc["L"], sc["madelung"], o.eigen(), o.nvec())
+    sd = _screening(2 * o.nocc, sc["L"])
+    _, _, tb, tc, _ = o.mp2()
+    ctx.set_eri(ONE, safe_eri=True, screening=sd)
+    first = ctx.ccd_g2_2ch(tb, tc, 31)
+
+    def copies():
+        import torch
+        from torch.profiler import ProfilerActivity, profile
+
+        torch.cuda.init()
+        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
+            out = ctx.ccd_g2_2ch(tb, tc, 31)
+        return out, {e.key: e.count for e in p.key_averages()}
+
+    again, c = copies()
+    assert c["Memcpy HtoD (Pageable -> Device)"] == 2 and not any("k2m_weights" in k for k in c), c
+    ctx.set_eri(ONE, safe_eri=True, screening=2 * sd)
+    other, c = copies()
+    assert any("k2m_weights" in k for k in c)
+    ctx.set_eri(ONE, safe_eri=True, screening=sd)
+    back = ctx.ccd_g2_2ch(tb, tc, 31)
+    for x, y, z, w in zip(first, again, back, other):
+        assert np.array_equal(x, y) and np.array_equal(x, z) and not np.array_equal(x, w)

@@ -822,13 +822,9 @@ int TwoChannel::set_integrals(int routine, const UegccdRangeTerms &fl, int core_
             for (int q2 = 0; q2 < nq_; q2++)
                 vt[(size_t)(core * 4 + flag) * nq_ + q2] =
                     routine_value(routine, core != 0, flag, L_, madelung_, screening, g, q2);
-    TCU(cudaMemcpyAsync(vt_, vt.data(), vt.size() * sizeof(double), cudaMemcpyHostToDevice, st_));
-    TCU(cudaStreamSynchronize(st_));
-    routine_ = routine;
-    core_n_ = core_n;
     // The Max(...) of each integral's flags (CCD.f90:620-642, 726-750, 782-786, 855-879, 910-914).
     auto m3 = [](int a, int b, int c) { return std::max(a, std::max(b, c)); };
-    TcFlags &f = f_;
+    TcFlags f{};
     f.drv_d = fl.driver_direct;
     f.drv_x = fl.driver_exchange;
     f.mosaic = fl.mosaic;
@@ -845,12 +841,22 @@ int TwoChannel::set_integrals(int routine, const UegccdRangeTerms &fl, int core_
     f.xr_lin_x = m3(fl.xring, fl.exchange_rings, fl.lin_rings);
     f.xr_quad_d = m3(fl.xring, fl.direct_rings, fl.quad_rings);
     f.xr_quad_x = m3(fl.xring, fl.exchange_rings, fl.quad_rings);
+    // A context selects its integrals before every call: mostly the same ones
+    if (vt.size() == vt_host_.size() && std::memcmp(vt.data(), vt_host_.data(), vt.size() * sizeof(double)) == 0 &&
+        std::memcmp(&f, &f_, sizeof f) == 0 && core_n == core_n_)
+        return 0;
+    vt_host_.clear();   // (until the tables are there)
+    TCU(cudaMemcpyAsync(vt_, vt.data(), vt.size() * sizeof(double), cudaMemcpyHostToDevice, st_));
+    TCU(cudaStreamSynchronize(st_));
+    f_ = f;
+    core_n_ = core_n;
     plain_ = core_n == 0;
     for (const int flag : {f.drv_d, f.drv_x, f.mosaic, f.lad_lin_d, f.lad_lin_x, f.lad_quad_d, f.lad_quad_x,
                            f.ring_lin_d, f.ring_lin_x, f.ring_quad_d, f.ring_quad_x, f.xr_lin_d, f.xr_lin_x,
                            f.xr_quad_d, f.xr_quad_x})
         for (int q2 = 0; q2 < nq_ && plain_; q2++) plain_ = vt[(size_t)flag * nq_ + q2] >= -80.0;
     weights_ = false;
+    vt_host_ = std::move(vt);
     return 0;
 }
 

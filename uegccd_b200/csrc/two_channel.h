@@ -72,7 +72,6 @@ private:
     int64_t n_ = 0;
     int nq_ = 0;
     int core_n_ = 0;
-    int routine_ = TC_BASE;
     TcFlags f_{};
     double L_ = 0, madelung_ = 0;
     cudaStream_t st_ = nullptr;
@@ -100,6 +99,7 @@ private:
     bool mm_fits_ = true;       // its shared memory suffices
     bool mm_on_ = false;        // this call has the workspace
     std::vector<int> kl0_, kl_, kl_ij_;   // TcMm's lists
+    std::vector<double> vt_host_;   // vt_'s values
     bool plain_ = false;        // no integral excluded, no core orbital
     bool weights_ = false;      // the workspace's W holds the current integrals
     std::vector<std::array<int, 3>> occ_;
