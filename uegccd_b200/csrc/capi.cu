@@ -3,9 +3,9 @@
 // A context is a batch of one system.  The drivers follow DrvMBPT (MP2.f90:11-157),
 // DrvCCD (CCD.f90:18-183) and DrvdRPA (dRPA.f90:23-174): MP2 guess, then
 // residual -> update -> convergence -> energy per iteration until max|dT| < TolMax
-// or MaxIter, then one final residual for MaxRes.  All amplitudes, index maps
-// and intermediates stay on the device for the whole solve; one small
-// device-to-host read per iteration carries (E, max|dT|, max|R|) of every solve.
+// or MaxIter, then one final residual for MaxRes.  All amplitudes, index maps,
+// intermediates and the iteration's control stay on the device for the whole solve;
+// the host reads a flag in its own memory, and (E, max|dT|, max|R|) of every solve at the end.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -1749,10 +1749,10 @@ int tune_batch(UegccdBatch &b)
 
 // Runs the iteration for all solves of the batch from the amplitudes in d.t (from_mp2: those
 // k_mp2 has just written).
-// Iteration control lives on the device; the host replays a captured iteration
-// graph kPoll times between polls of the number of active solves.  With kernel
-// timing on, the last iteration of each round runs as direct launches between
-// CUDA events: that iteration is the sample the per-kernel times come from.
+// Iteration control lives on the device; the host replays a captured iteration graph, keeps one
+// queued behind the one whose end it waits for, and stops at the flag the last solve to stop
+// sets.  With kernel timing on, the last iteration of each round of kPoll runs as direct
+// launches between CUDA events: that iteration is the sample the per-kernel times come from.
 int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult *res, bool from_mp2 = false)
 {
     constexpr int kPoll = 4;
@@ -1811,9 +1811,8 @@ int run_solves(UegccdBatch &b, const UegccdOptions *opt, int drpa, UegccdResult 
     *(volatile int *)b.ctl.done = 0;
     launch_tail(d, b.ctl, opt->tol, opt->max_iter, ndiis, 1, b.stream);
     b.launches++;
-    // The iterations go in rounds of kPoll.  The host keeps one queued behind the one whose end it
-    // waits for, and looks at the flag of k_tail: the GPU does not wait for the host, and a solve
-    // that has stopped costs one empty iteration.  (A copy of the count and a wait every four
+    // The iterations go in rounds of kPoll (a mixed solve's refreshes).  The GPU does not wait for the
+    // host, and a batch that has stopped costs one empty iteration.  (A copy of the count and a wait every four
     // iterations left the GPU idle for 22 us and up to three iterations empty.)
     const int max_rounds = opt->max_iter / kPoll + 2;
     // mixed precision: tensor-core ladder of t - t_ref, t_ref refreshed (FP64) each round,

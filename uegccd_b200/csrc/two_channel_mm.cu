@@ -2,7 +2,7 @@
 //
 // two_channel.cu forms every term of an amplitude in the reference's loops: per amplitude it
 // walks all virtuals for the particle-particle ladder and NOcc orbitals five times for the
-// hole-hole ladder, the rings and the crossed rings, 0.9 ms a residual at N=54 (485 plane
+// hole-hole ladder, the rings and the crossed rings, 0.84 ms a residual at N=54 (485 plane
 // waves), bound by the latency of its scattered loads.  Where no integral of the tables is
 // excluded (the reference's "Min(V1,V2) < -80 -> Cycle" never fires) and no orbital is core, the
 // two integrals of a term do not depend on each other and the sums are products:
