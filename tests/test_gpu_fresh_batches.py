@@ -5,6 +5,8 @@ import threading
 import numpy as np
 import pytest
 
+from profiled import profiled
+
 pytestmark = pytest.mark.gpu
 
 DIIS = dict(scheme=1, ndiis=6, denom_factor=1.0)
@@ -33,20 +35,16 @@ def _step(systems, drpa):
 def test_a_batch_takes_over_what_the_last_one_used(count, electrons, basis, drpa):
     """A second batch makes its own stream and nothing more, dRPA (which has no side streams) from the
     first one on; and its values are the first one's."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
     from uegccd_b200 import _capi
 
-    torch.cuda.init()
     systems = _systems(count, electrons, basis)
     _capi.trim_cache()
     counts, outs = [], []
     for _ in range(2):
-        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-            outs.append(_step(systems, drpa))
-        counts.append({e.key: e.count for e in p.key_averages()})
-    assert counts[1]["cudaGraphLaunch"] > 0   # the profile saw the solve
+        out, c, _ = profiled(lambda: _step(systems, drpa))
+        outs.append(out)
+        counts.append(c)
+    assert counts[1]["cudaGraphLaunch"] > 0
     for c in counts[0 if drpa else 1:]:
         assert c["cudaStreamCreateWithFlags"] == 1 and c["cudaStreamDestroy"] == 1, c
     assert "cudaHostAlloc" not in counts[1] and "cudaFreeHost" not in counts[1], counts[1]
@@ -92,26 +90,13 @@ def test_side_streams_of_many_threads_and_live_batches():
 
 def test_reported_launch_shapes_are_those_launched():
     """ring_threads and launch_shapes against the profile of a solve with ring groups of all sizes."""
-    import json
-    import os
     import re
-    import tempfile
-
-    import torch
-    from torch.profiler import ProfilerActivity, profile
 
     from uegccd_b200 import Batch
 
-    torch.cuda.init()
     b = Batch(_systems(1, 114, 1140))
     b.solve(**DIIS)
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-        b.solve(**DIIS)
-    with tempfile.TemporaryDirectory() as d:
-        path = os.path.join(d, "trace.json")
-        p.export_chrome_trace(path)
-        with open(path) as f:
-            events = [e for e in json.load(f)["traceEvents"] if e.get("cat") == "kernel"]
+    _, _, events = profiled(lambda: b.solve(**DIIS))
     sizes = {}   # rows of group 1 in eights -> threads
     for e in events:
         m = re.search(r"k_rings<\w+, (\d)>", e["name"])
@@ -132,17 +117,12 @@ def test_reported_launch_shapes_are_those_launched():
 def test_reported_launches_are_those_made(count, electrons, basis, options):
     """kernel_launches of a solve against the kernels of its profile: all but the MP2 start's two (or
     three, with dRPA's T2aaaa), which are not the solve's."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
     from uegccd_b200 import Batch
 
-    torch.cuda.init()
     b = Batch(_systems(count, electrons, basis))
     b.solve(**options)
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-        _, _, res = b.solve(**options)
-    kernels = {e.key: e.count for e in p.key_averages() if "uegccd::" in e.key}
+    (_, _, res), counts, _ = profiled(lambda: b.solve(**options))
+    kernels = {k: n for k, n in counts.items() if "uegccd::" in k}
     two = "do_xring" in options
     made = sum(n for k, n in kernels.items()
                if not (two and ("::k_" in k or "k_unpack" in k or "k_pack" in k)))

@@ -8,6 +8,8 @@ import re
 import numpy as np
 import pytest
 
+from profiled import profiled
+
 pytestmark = pytest.mark.gpu
 
 MB = 1 << 20
@@ -48,14 +50,8 @@ def test_live_contexts_hold_no_download_buffer():
 
 def _host_allocs(call):
     """How often a call locks host memory anew."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
-    torch.cuda.init()
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-        call()
-    counts = {e.key: e.count for e in p.key_averages()}
-    assert "cudaMemcpyAsync" in counts   # the profile saw the call
+    _, counts, _ = profiled(call)
+    assert "cudaMemcpyAsync" in counts
     return counts.get("cudaHostAlloc", 0)
 
 
@@ -117,19 +113,14 @@ def test_many_threads_download_at_once():
 def test_small_batch_downloads_are_one_copy():
     """Below 8 MB the driver's own staging is the faster way: a download of 2.0 MB into ordinary memory
     is one copy to pageable memory, one of 10.7 MB comes through page-locked memory."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
     from uegccd_b200 import Batch
 
-    torch.cuda.init()
     for count, electrons, basis, key in ((3, 38, 247, "Pageable"), (4, 54, 485, "Pinned")):
         b = Batch(_systems(count, electrons, basis))
         b.mp2()
         first = b.all_amplitudes()
-        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-            again = b.all_amplitudes()
-        copies = [e.key for e in p.key_averages() if "Memcpy DtoH" in e.key]
+        again, counts, _ = profiled(b.all_amplitudes)
+        copies = [k for k in counts if "Memcpy DtoH" in k]
         assert copies == [f"Memcpy DtoH (Device -> {key})"], copies
         for x, y in zip(first, again):
             np.testing.assert_array_equal(x, y)

@@ -8,6 +8,7 @@ import numpy as np
 import pytest
 
 from oracle.oracle import Oracle, parse_input_text
+from profiled import profiled
 from test_gpu_two_channel import KEYS, MIXED, _screening
 from uegccd_b200 import Context
 from uegccd_b200 import _capi as capi
@@ -39,16 +40,6 @@ def _setup(nel, cut, flags, factor=1):
     return o
 
 
-def _kernels(call):
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
-    torch.cuda.init()
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-        out = call()
-    return out, " ".join(e.key for e in p.key_averages())
-
-
 @pytest.mark.parametrize("form", FORMS)
 @pytest.mark.parametrize("nel,cut", [(14, 5), (38, 8)])
 def test_terms_and_form(nel, cut, form):
@@ -64,7 +55,8 @@ def test_terms_and_form(nel, cut, form):
     tc = tc + 1e-3 * rng.standard_normal(tc.shape)
     for mask in (4, 8, 16, 31):
         ga, gb = o.ccd_g2(tb, tc, mask)
-        (ha, hb), names = _kernels(lambda: ctx.ccd_g2_2ch(tb, tc, mask))
+        (ha, hb), counts, _ = profiled(lambda: ctx.ccd_g2_2ch(tb, tc, mask))
+        names = " ".join(counts)
         assert ("k2m_assemble" in names) == products and ("k2_assemble" in names) != products, names
         scale = max(np.abs(ga).max(), np.abs(gb).max(), 1e-300)
         assert np.abs(ha - ga).max() <= 1e-12 * scale, (mask, "abab")
@@ -103,13 +95,8 @@ def test_a_repeated_selection_is_not_made_again(nel, cut):
     first = ctx.ccd_g2_2ch(tb, tc, 31)
 
     def copies():
-        import torch
-        from torch.profiler import ProfilerActivity, profile
-
-        torch.cuda.init()
-        with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-            out = ctx.ccd_g2_2ch(tb, tc, 31)
-        return out, {e.key: e.count for e in p.key_averages()}
+        out, counts, _ = profiled(lambda: ctx.ccd_g2_2ch(tb, tc, 31))
+        return out, counts
 
     again, c = copies()
     assert c["Memcpy HtoD (Pageable -> Device)"] == 2 and not any("k2m_weights" in k for k in c), c

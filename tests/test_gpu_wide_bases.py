@@ -1,12 +1,11 @@
 """Systems with few occupied orbitals and thousands of plane waves: one system's work has to reach more
 than a few SMs, and its sums are the reference's at the edges of their ranges."""
-import json
 import math
-import os
-import tempfile
 
 import numpy as np
 import pytest
+
+from profiled import profiled
 
 pytestmark = pytest.mark.gpu
 
@@ -29,19 +28,8 @@ def _system(electrons, basis, seed=5):
 
 def _kernels(call, name):
     """(grid, shared memory) of every launch of a kernel."""
-    import torch
-    from torch.profiler import ProfilerActivity, profile
-
-    torch.cuda.init()
-    with profile(activities=[ProfilerActivity.CPU, ProfilerActivity.CUDA]) as p:
-        call()
-    with tempfile.TemporaryDirectory() as d:
-        path = os.path.join(d, "trace.json")
-        p.export_chrome_trace(path)
-        with open(path) as f:
-            events = json.load(f)["traceEvents"]
-    return [(e["args"]["grid"][0], e["args"]["shared memory"]) for e in events
-            if e.get("cat") == "kernel" and name in e["name"]]
+    _, _, events = profiled(call)
+    return [(e["args"]["grid"][0], e["args"]["shared memory"]) for e in events if name in e["name"]]
 
 
 @pytest.mark.parametrize("electrons,virtuals", [(14, 60), (14, 1024), (14, 1025), (6, 2048), (14, 2049), (4, 5000)])
