@@ -875,16 +875,28 @@ void TwoChannel::mm_make()
     if (!mm_fits_) return;
     auto up = [](int64_t x, int64_t k) { return (x + k - 1) / k * k; };
     D.ldw = (int)up(2 * (int64_t)(V_ + O_), 64), D.ldt = (int)up(2 * (int64_t)O2, 64), D.kdim = (int)up(V_, 16);
+    // the pairs (k,l) by their momentum, each momentum's in ascending k, then l
+    auto momentum = [&](int k, int l) {
+        int64_t key = 0;
+        for (int d = 0; d < 3; d++) key = key << 16 | (uint16_t)(occ_[k][d] + occ_[l][d]);
+        return key;
+    };
+    std::vector<std::pair<int64_t, int>> by(O2);
+    for (int k = 0; k < O_; k++)
+        for (int l = 0; l < O_; l++) by[k * O_ + l] = {momentum(k, l), k * O_ + l};
+    std::sort(by.begin(), by.end());
+    std::vector<std::pair<int, int>> range(O2);   // by pair: its momentum's part of `by`
+    for (int a = 0, e = 0; a < O2; a = e) {
+        while (e < O2 && by[e].first == by[a].first) e++;
+        for (int q = a; q < e; q++) range[by[q].second] = {a, e};
+    }
     kl0_.assign(O2 + 1, 0);
     for (int ij = 0; ij < O2; ij++) {
-        const auto &a = occ_[ij % O_], &b = occ_[ij / O_];
-        for (int k = 0; k < O_; k++)
-            for (int l = 0; l < O_; l++)
-                if (a[0] + b[0] == occ_[k][0] + occ_[l][0] && a[1] + b[1] == occ_[k][1] + occ_[l][1] &&
-                    a[2] + b[2] == occ_[k][2] + occ_[l][2]) {
-                    kl_.push_back(k | l << 16);
-                    kl_ij_.push_back(ij);
-                }
+        const auto r = range[(ij % O_) * O_ + ij / O_];
+        for (int q = r.first; q < r.second; q++) {
+            kl_.push_back(by[q].second / O_ | (by[q].second % O_) << 16);
+            kl_ij_.push_back(ij);
+        }
         kl0_[ij + 1] = (int)kl_.size();
     }
     D.nkl = (int)kl_.size();
