@@ -642,6 +642,9 @@ def main(argv=None):
                        "frac": ach / p64, "avg_ms": avg_s * 1e3, "launches": launches,
                        "peak_source": ("measured in this run: register-only mma.sync m8n8k4 f64 probe"
                                        if g.get("fp64_peak") else "nominal FP64")}
+            if k == "k_ladder":   # a rate of useful work, not a pipe's utilisation
+                kern[k]["note"] = ("flops of the plain form of the ladder; the even and odd halves need about half, "
+                                   "part of them on the FMA pipe")
         else:
             ach = units / avg_s / 1e9
             kern[k] = {"bound": "hbm", "achieved": ach, "peak": HBM_PEAK, "unit": "GB/s", "frac": ach / HBM_PEAK,

@@ -37,8 +37,8 @@
 //               lane makes its own element of the two Coulomb fragments.  8 cycles per 8 rows.
 // Measured per residual, ladders and hole-hole sums together, against DMMA tiles over the full
 // products with a separate hole-hole launch: 100 twists of N=54 (485 plane waves) 0.79 -> 0.38 ms
-// (FMA form 0.20, bound by its shared-memory reads: 0.15 ms of wavefronts; DMMA form 0.17, its
-// pipe 46% busy), four N=114 systems 0.70 -> 0.25 ms, 100 twists of N=14 21 -> 10.5 us.
+// (FMA form 0.20, at the limit of no pipe: shared memory 57%, issue 55%, with 39% of the warps, its
+// largest stalls the barriers and first loads of its short tiles; DMMA form 0.17, its pipe 46% busy), four N=114 systems 0.70 -> 0.25 ms, 100 twists of N=14 21 -> 10.5 us.
 #include <cuda_runtime.h>
 
 #include <algorithm>
